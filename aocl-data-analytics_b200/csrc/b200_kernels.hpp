@@ -127,6 +127,25 @@ cudaError_t launch_knn_merge(const T *part_key, const int *part_idx, int nq, int
 int knn_tile_rows_train(bool fp64);
 int knn_max_k(bool fp64);
 
+// The same search with a bound found first (knn_select.cu): sizes of its
+// passes.  knn_sel_plan is false where they do not apply (too few rows for k).
+constexpr int KNN_SEL_GROUPS = 512; // sample minima per query, at most
+constexpr int KNN_SEL_CAP = 4096;   // listed keys per query, at most
+struct KnnSelPlan {
+    int n_sample, step;          // sample rows: every step-th row
+    int parts, part_rows;        // blocks over the sample, rows of each
+    int groups;                  // minima per query (32 per part)
+    int cap;                     // list entries per query (a power of two)
+};
+bool knn_sel_plan(int n, int nq, int k, bool fp64, KnnSelPlan &pl);
+size_t knn_sel_bytes(const KnnSelPlan &pl, int nq, bool fp64);
+// out_key / out_idx as launch_knn_merge's; *flag is set to 1 when a query's
+// list overflowed or held fewer than k keys (its outputs are then unwritten).
+template <typename T>
+cudaError_t launch_knn_select(const T *Q, int nq, const T *X, int nx, int ld, int d, const T *qn,
+                              const T *xn, const KnnArgs &a, const KnnSelPlan &pl, void *work,
+                              int tf, T *out_key, int *out_idx, int *flag, cudaStream_t s);
+
 // ---------------------------------------------- kNN tensor-core pass ---
 // fp32 euclidean / squared euclidean / cosine: bf16x3 tcgen05 candidate pass with a
 // certified threshold per query, exact re-score of the survivors in the plain

@@ -50,26 +50,6 @@ cudaError_t ensure_smem_limit(const void *func, size_t smem) {
 
 namespace b200 {
 
-// Post-operation of one accumulated pair value (reference post-ops:
-// cosine_distance.cpp:66-88, minkowski_distance.cpp:67-77,
-// euclidean_gemm_distance.cpp:108-135, nearest_neighbors.cpp:662-665).
-template <typename T>
-B200_DEV T post_value(int post, T g, T xn, T yn, T invp) {
-    switch (post) {
-    case POST_SQRT: return sqrt_rn(g);
-    case POST_COSINE: return sub_rn(T(1), div_rn(g, mul_rn(xn, yn)));
-    case POST_GEMM_SQ: return fma_rn(T(-2), g, add_rn(xn, yn));
-    case POST_GEMM_SQRT: return sqrt_rn(fma_rn(T(-2), g, add_rn(xn, yn)));
-    case POST_GEMM_SQ_CLAMP: {
-        T v = fma_rn(T(-2), g, add_rn(xn, yn));
-        return v < T(0) ? T(0) : v;
-    }
-    case POST_POW: return pow_(g, invp);
-    case POST_NEG: return -g;
-    default: return g;
-    }
-}
-
 // ------------------------------------------------------------ pairwise ----
 template <typename T, int ACC>
 __global__ void __launch_bounds__(256)

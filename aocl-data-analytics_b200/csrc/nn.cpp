@@ -4,6 +4,7 @@
 // the top-k selection run on the GPU (dist_simt.cu).
 #include "alg.hpp"
 #include <cstdlib>
+#include <functional>
 #include <map>
 
 namespace b200 {
@@ -536,7 +537,18 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
                           tc_done);
         if (s != da_status_success) return s;
     }
+    // the plain path: bounds first (launch_knn_select) in query batches of at
+    // most 256 MB of lists, each with its own flag after the indices; running
+    // lists (run_lists) where that does not apply or a flag comes back set
+    KnnSelPlan sel{};
+    da_int sel_qb = 0, n_flags = 0;
+    std::function<da_status()> run_lists;
     if (!tc_done) {
+        if (knn_sel_plan((int)n_samples, (int)std::min<da_int>(nq, 65536), (int)k, fp64, sel)) {
+            const size_t per = knn_sel_bytes(sel, 1, fp64);
+            sel_qb = std::min(nq, (da_int)std::max<size_t>(64, ((size_t)1 << 28) / per / 64 * 64));
+            n_flags = (nq + sel_qb - 1) / sel_qb;
+        }
         const T *qn = nullptr, *xn = nullptr;
         if (norm_kind >= 0) {
             if (!dQn.ensure((size_t)nq * sizeof(T)) || !dXn.ensure((size_t)n_samples * sizeof(T)))
@@ -558,43 +570,80 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             return err->error(da_status_not_implemented,
                               "k = " + std::to_string(k) + " exceeds the largest supported number "
                               "of neighbours per query (" + std::to_string(knn_max_k(fp64)) + ").");
-        // chunking of the training rows: enough CTAs to fill 148 SMs several times
-        const int BN = knn_tile_rows_train(fp64);
-        const int q_tiles = (int)((nq + 63) / 64);
-        const int max_chunks = std::max(1, (int)((n_samples + BN - 1) / BN));
-        // enough CTAs to fill the GPU, but at most ~16K partial entries per query
-        // (the merge ranks every entry against every chunk list)
-        int n_chunks = std::max(1, std::min({max_chunks, (148 * 8 + q_tiles - 1) / q_tiles,
-                                             std::max(8, 16384 / (int)k)}));
-        int chunk_rows = (int)((n_samples + n_chunks - 1) / n_chunks);
-        chunk_rows = ((chunk_rows + BN - 1) / BN) * BN;
-        n_chunks = (int)((n_samples + chunk_rows - 1) / chunk_rows);
-        KnnArgs a{acc, post, kc, (double)p, (int)k, chunk_rows, n_chunks};
-        const size_t parts = (size_t)nq * n_chunks * k;
-        if (!dPartK.ensure(parts * sizeof(T)) || !dPartI.ensure(parts * sizeof(int)) ||
-            !dOutK.ensure((size_t)nq * k * sizeof(T)) || !dOutI.ensure((size_t)nq * k * sizeof(int)))
+        if (!dOutK.ensure((size_t)nq * k * sizeof(T)) ||
+            !dOutI.ensure(((size_t)nq * k + n_flags) * sizeof(int)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
-        B200_TRY(cuda->timed("knn_chunks", [&] {
-            return launch_knn_chunks<T>(dQ.as<T>(), ld, (int)nq, dX.as<T>(), ld, (int)n_samples,
-                                        (int)d, qn, xn, a, dPartK.as<T>(), dPartI.as<int>(), nullptr,
-                                        st);
-        }), "kNN distance kernel");
-        B200_TRY(cuda->timed("knn_merge", [&] {
-            return launch_knn_merge<T>(dPartK.as<T>(), dPartI.as<int>(), (int)nq, n_chunks, (int)k,
-                                       tf, dOutK.as<T>(), dOutI.as<int>(), st);
-        }), "kNN merge kernel");
+        if (n_flags > 0) {
+            const KnnArgs a{acc, post, kc, (double)p, (int)k, 0, 0};
+            if (!dPartK.ensure(knn_sel_bytes(sel, (int)sel_qb, fp64)))
+                return err->error(da_status_memory_error, "Device memory allocation failed.");
+            int *flags = dOutI.as<int>() + (size_t)nq * k;
+            for (da_int q0 = 0; q0 < nq; q0 += sel_qb, ++flags) {
+                const da_int nb = std::min(sel_qb, nq - q0);
+                B200_TRY(cuda->timed("knn_select", [&] {
+                    return launch_knn_select<T>(dQ.as<T>() + (size_t)q0 * ld, (int)nb, dX.as<T>(),
+                                                (int)n_samples, ld, (int)d, qn ? qn + q0 : nullptr,
+                                                xn, a, sel, dPartK.p, tf,
+                                                dOutK.as<T>() + (size_t)q0 * k,
+                                                dOutI.as<int>() + (size_t)q0 * k, flags, st);
+                }), "kNN selection kernels");
+            }
+        }
+        run_lists = [&, qn, xn]() -> da_status {
+            // chunking of the training rows: enough CTAs to fill 148 SMs several times
+            const int BN = knn_tile_rows_train(fp64);
+            const int q_tiles = (int)((nq + 63) / 64);
+            const int max_chunks = std::max(1, (int)((n_samples + BN - 1) / BN));
+            // enough CTAs to fill the GPU, but at most ~16K partial entries per query
+            // (the merge ranks every entry against every chunk list)
+            int n_chunks = std::max(1, std::min({max_chunks, (148 * 8 + q_tiles - 1) / q_tiles,
+                                                 std::max(8, 16384 / (int)k)}));
+            int chunk_rows = (int)((n_samples + n_chunks - 1) / n_chunks);
+            chunk_rows = ((chunk_rows + BN - 1) / BN) * BN;
+            n_chunks = (int)((n_samples + chunk_rows - 1) / chunk_rows);
+            KnnArgs a{acc, post, kc, (double)p, (int)k, chunk_rows, n_chunks};
+            const size_t parts = (size_t)nq * n_chunks * k;
+            if (!dPartK.ensure(parts * sizeof(T)) || !dPartI.ensure(parts * sizeof(int)) ||
+                !dOutK.ensure((size_t)nq * k * sizeof(T)) || !dOutI.ensure((size_t)nq * k * sizeof(int)))
+                return err->error(da_status_memory_error, "Device memory allocation failed.");
+            B200_TRY(cuda->timed("knn_chunks", [&] {
+                return launch_knn_chunks<T>(dQ.as<T>(), ld, (int)nq, dX.as<T>(), ld, (int)n_samples,
+                                            (int)d, qn, xn, a, dPartK.as<T>(), dPartI.as<int>(), nullptr,
+                                            st);
+            }), "kNN distance kernel");
+            B200_TRY(cuda->timed("knn_merge", [&] {
+                return launch_knn_merge<T>(dPartK.as<T>(), dPartI.as<int>(), (int)nq, n_chunks, (int)k,
+                                           tf, dOutK.as<T>(), dOutI.as<int>(), st);
+            }), "kNN merge kernel");
+            return da_status_success;
+        };
+        if (n_flags == 0) {
+            s = run_lists();
+            if (s != da_status_success) return s;
+        }
     }
     ind.resize((size_t)nq * k);
-    std::vector<int> tmp((size_t)nq * k);
-    B200_TRY(cudaMemcpyAsync(tmp.data(), dOutI.p, tmp.size() * sizeof(int), cudaMemcpyDeviceToHost, st),
-             "download");
-    if (dist) {
-        dist->resize((size_t)nq * k);
-        B200_TRY(cudaMemcpyAsync(dist->data(), dOutK.p, dist->size() * sizeof(T),
-                                 cudaMemcpyDeviceToHost, st), "download");
+    std::vector<int> tmp((size_t)nq * k + n_flags);
+    for (;;) {
+        B200_TRY(cudaMemcpyAsync(tmp.data(), dOutI.p, ((size_t)nq * k + n_flags) * sizeof(int),
+                                 cudaMemcpyDeviceToHost, st),
+                 "download");
+        if (dist) {
+            dist->resize((size_t)nq * k);
+            B200_TRY(cudaMemcpyAsync(dist->data(), dOutK.p, dist->size() * sizeof(T),
+                                     cudaMemcpyDeviceToHost, st), "download");
+        }
+        B200_TRY(cudaStreamSynchronize(st), "kNN");
+        const bool again = std::any_of(tmp.begin() + (size_t)nq * k, tmp.begin() + (size_t)nq * k + n_flags,
+                                       [](int f) { return f != 0; });
+        if (!again) break;
+        // a query's list overflowed or was short of k keys
+        cuda->stats["knn_select_fallback"] += 1.0;
+        n_flags = 0;
+        s = run_lists();
+        if (s != da_status_success) return s;
     }
-    B200_TRY(cudaStreamSynchronize(st), "kNN");
-    for (size_t i = 0; i < tmp.size(); ++i) ind[i] = (da_int)tmp[i];
+    for (size_t i = 0; i < ind.size(); ++i) ind[i] = (da_int)tmp[i];
     return da_status_success;
 }
 
