@@ -18,7 +18,7 @@
 #include "b200_common.cuh"
 #include <cuda/atomic>
 #include "b200_kernels.hpp"
-#include "simt_engine.cuh"
+#include "tile_sweep.cuh"
 #include <map>
 #include <mutex>
 
@@ -52,75 +52,80 @@ namespace b200 {
 
 // ------------------------------------------------------------ pairwise ----
 template <typename T, int ACC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 pairwise_kernel(const T *X, int m, const T *Y, int n, int ld, int d, const T *xn, const T *yn,
                 int post, int kc, T p, T invp, int x_is_y, int out_rowmajor, T *D, T thr,
-                int *hits, int nch) {
-    using C = SimtCfg<T>;
-    constexpr int TM = C::TM, TN = C::TN, BK = C::BK, BM = 16 * TM, BN = 16 * TN;
-    __shared__ __align__(16) Stage<T, BM, BN, BK> st[2];
+                int *hits, int nch, int tiles) {
+    constexpr int TM = SweepAcc<T, ACC>::TM, TN = SweepAcc<T, ACC>::TN, BN = SweepStage<T>::BN;
+    constexpr int W = SweepCols<T>::W;
+    __shared__ SweepStage<T> st[2];
     const int tid = threadIdx.x;
-    const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
-    Acc<T, TM, TN> acc;
-    compute_tile<T, ACC, TM, TN, BM, BN, BK>(st, X, ld, m, i0, Y, ld, n, j0, d, kc, p, acc, tid);
+    const int i0 = blockIdx.y * SW_BM;
+    const int y_begin = blockIdx.x * tiles * BN, y_end = min(n, y_begin + tiles * BN);
     const int tm = tid / 16, tn = tid % 16;
     // row-major D with n a multiple of 4: a thread's four consecutive columns
     // go out as 16-byte stores (D from cudaMalloc, rows of n elements)
     const bool vec_out = out_rowmajor && (n & 3) == 0 &&
                          (reinterpret_cast<uintptr_t>(D) & 15) == 0;
+    const bool zero_diag = x_is_y && (post == POST_COSINE || post == POST_GEMM_SQ ||
+                                      post == POST_GEMM_SQRT);
     int hit[TM];
+    T xv[TM];
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        hit[i] = 0;
         const int gi = i0 + tm * 4 + i;
-        if (gi >= m) continue;
-        const T xv = xn ? xn[gi] : T(0);
-#pragma unroll
-        for (int g = 0; g < TN / 4; ++g) {
-            const int gj0 = j0 + g * 64 + tn * 4;
-            T v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int gj = gj0 + u;
-                const T yv = (yn && gj < n) ? yn[gj] : T(0);
-                v[u] = post_value<T>(post, acc.g1[i][g * 4 + u], xv, yv, invp);
-                if (x_is_y && gi == gj && (post == POST_COSINE || post == POST_GEMM_SQ ||
-                                           post == POST_GEMM_SQRT))
-                    v[u] = T(0);
-                if (gj < n) hit[i] += v[u] <= thr ? 1 : 0;
-            }
-            if (vec_out && gj0 + 3 < n) {
-                using V = typename Vec16Of<T>::V;
-                constexpr int W = 16 / (int)sizeof(T);
-#pragma unroll
-                for (int u = 0; u < 4; u += W)
-                    *reinterpret_cast<V *>(D + (size_t)gi * n + gj0 + u) =
-                        *reinterpret_cast<const V *>(&v[u]);
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int gj = gj0 + u;
-                    if (gj >= n) continue;
-                    if (out_rowmajor)
-                        D[(size_t)gi * n + gj] = v[u];
-                    else
-                        D[(size_t)gj * m + gi] = v[u];
-                }
-            }
-        }
+        hit[i] = 0;
+        xv[i] = (xn && gi < m) ? xn[gi] : T(0);
     }
+    SweepAcc<T, ACC> acc;
+    sweep_tiles<T, ACC>(
+        st, X, m, i0, Y, (size_t)ld, y_begin, y_end, ld, d, kc, p, acc, tid, [&](int j0) {
+            sweep_post<T, ACC>(acc, post, xv, yn, (size_t)1, j0, n, tn, invp, [&](int i, T (&v)[TN]) {
+                const int gi = i0 + tm * 4 + i;
+                if (gi >= m) return;
+#pragma unroll
+                for (int g = 0; g < TN / W; ++g) {
+                    const int gj0 = j0 + SweepCols<T>::of(g * W, tn);
+                    T *w = &v[g * W];
+                    if (zero_diag) {
+#pragma unroll
+                        for (int u = 0; u < W; ++u)
+                            if (gi == gj0 + u) w[u] = T(0);
+                    }
+                    if (hits) {
+#pragma unroll
+                        for (int u = 0; u < W; ++u) hit[i] += (gj0 + u < n && w[u] <= thr) ? 1 : 0;
+                    }
+                    if (vec_out && gj0 + W <= n) {
+                        typename Vec16Of<T>::V o;
+                        T *op = reinterpret_cast<T *>(&o);
+#pragma unroll
+                        for (int u = 0; u < W; ++u) op[u] = w[u];
+                        *reinterpret_cast<typename Vec16Of<T>::V *>(D + (size_t)gi * n + gj0) = o;
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < W; ++u) {
+                            const int gj = gj0 + u;
+                            if (gj >= n) continue;
+                            if (out_rowmajor) D[(size_t)gi * n + gj] = w[u];
+                            else D[(size_t)gj * m + gi] = w[u];
+                        }
+                    }
+                }
+            });
+        });
     if (!hits) return;
-    // the tile's hits per row: the 16 lanes of a row group (one half-warp)
-    // sum theirs, lane tn = 0 adds them to the row's chunk (a tile lies in
-    // one chunk: RADIUS_CHUNK is a multiple of BN)
-    static_assert(RADIUS_CHUNK % BN == 0, "tiles within one radius chunk");
+    // the block's hits per row: the 16 lanes of a row group (one half-warp)
+    // sum theirs, lane tn = 0 adds them to the row's chunk (a block's tiles,
+    // a power of two up to 8, lie in one chunk)
+    static_assert(RADIUS_CHUNK % (8 * BN) == 0, "blocks within one radius chunk");
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         int c = hit[i];
 #pragma unroll
         for (int off = 8; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
         const int gi = i0 + tm * 4 + i;
-        if (tn == 0 && gi < m && c > 0) atomicAdd(&hits[(size_t)gi * nch + j0 / RADIUS_CHUNK], c);
+        if (tn == 0 && gi < m && c > 0) atomicAdd(&hits[(size_t)gi * nch + y_begin / RADIUS_CHUNK], c);
     }
 }
 
@@ -128,10 +133,14 @@ template <typename T>
 cudaError_t launch_pairwise(const T *X, int ldx, int m, const T *Y, int ldy, int n, int d,
                             const T *xn, const T *yn, const PairwiseArgs &a, T *D,
                             cudaStream_t s) {
-    using C = SimtCfg<T>;
-    constexpr int BM = 16 * C::TM, BN = 16 * C::TN;
+    constexpr int BM = SW_BM, BN = SweepStage<T>::BN;
     if (ldx != ldy) return cudaErrorInvalidValue;
-    dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
+    // tiles per block: up to 8 in a row (one pipeline, the first loads exposed
+    // once) while at least four blocks are left for each of the 296 slots
+    const long long n_tiles = (n + BN - 1) / BN, m_tiles = (m + BM - 1) / BM;
+    int tiles = 1;
+    while (tiles < 8 && n_tiles * m_tiles >= 2 * tiles * 4 * 296) tiles *= 2;
+    dim3 grid((unsigned)((n_tiles + tiles - 1) / tiles), (unsigned)m_tiles);
     const T p = T(a.p);
     const T invp = T(1.0 / (double)p);
     if (a.hits && !a.out_rowmajor) return cudaErrorInvalidValue;
@@ -141,24 +150,22 @@ cudaError_t launch_pairwise(const T *X, int ldx, int m, const T *Y, int ldy, int
     case ACC_SQEUC:
         pairwise_kernel<T, ACC_SQEUC><<<grid, 256, 0, s>>>(X, m, Y, n, ldx, d, xn, yn, a.post,
                                                            a.kc, p, invp, a.x_is_y,
-                                                           a.out_rowmajor, D, thr, a.hits, nch);
+                                                           a.out_rowmajor, D, thr, a.hits, nch, tiles);
         break;
     case ACC_DOT:
         pairwise_kernel<T, ACC_DOT><<<grid, 256, 0, s>>>(X, m, Y, n, ldx, d, xn, yn, a.post, a.kc,
                                                          p, invp, a.x_is_y, a.out_rowmajor, D,
-                                                         thr, a.hits, nch);
+                                                         thr, a.hits, nch, tiles);
         break;
     case ACC_MANHATTAN:
         pairwise_kernel<T, ACC_MANHATTAN><<<grid, 256, 0, s>>>(X, m, Y, n, ldx, d, xn, yn,
                                                                a.post, a.kc, p, invp, a.x_is_y,
-                                                               a.out_rowmajor, D, thr, a.hits,
-                                                               nch);
+                                                               a.out_rowmajor, D, thr, a.hits, nch, tiles);
         break;
     default:
         pairwise_kernel<T, ACC_MINKOWSKI><<<grid, 256, 0, s>>>(X, m, Y, n, ldx, d, xn, yn,
                                                                a.post, a.kc, p, invp, a.x_is_y,
-                                                               a.out_rowmajor, D, thr, a.hits,
-                                                               nch);
+                                                               a.out_rowmajor, D, thr, a.hits, nch, tiles);
         break;
     }
     return cudaGetLastError();
