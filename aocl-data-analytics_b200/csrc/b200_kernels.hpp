@@ -371,7 +371,7 @@ cudaError_t launch_kpp_clamp(T *w, int n, int first, double *bs, int *flag, cuda
 // their number); force_exact redoes all of them.
 template <typename T>
 cudaError_t launch_kpp_draw(const T *w, int n, const double *bs, const double *U, int nt,
-                            int force_exact, int *cand, int *unc, int *exact_count,
+                            int force_exact, int *cand, int *exact_count,
                             cudaStream_t s);
 // Distances of every row to the t candidate rows (D[c*n + i], as
 // launch_kpp_dist) and cost[c] = the serial sum in T, index order from 0, of
@@ -383,6 +383,11 @@ cudaError_t launch_kpp_dist_cost(const T *X, int ldx, int n, int d, const T *xno
                                  void *work, cudaStream_t s, const T *xinv = nullptr,
                                  int cosine = 0);
 size_t kpp_cost_work_bytes(int n, int t);
+// elements between the candidates' rows of D
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+size_t kpp_dist_stride(int n, size_t elem);
 // Choose among the nt candidates by cost (chosen[c]), w_i = max(0, min(w_i,
 // D_best,i)), w_best = 0, block sums of the new w.
 template <typename T>

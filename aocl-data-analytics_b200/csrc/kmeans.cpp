@@ -211,15 +211,14 @@ template <typename T> da_status KMeans<T>::kmeans_plusplus(T *dC) {
     const da_int n = n_samples, k = n_clusters, d = n_features;
     const da_int n_trials = 2 + (da_int)std::log(k);
     const int nb = kpp_num_blocks((int)n);
-    if (!dW.ensure((size_t)n * sizeof(T)) || !dKD.ensure((size_t)n * n_trials * sizeof(T)) ||
+    if (!dW.ensure((size_t)n * sizeof(T)) || !dKD.ensure(kpp_dist_stride((int)n, sizeof(T)) * n_trials * sizeof(T)) ||
         !dCand.ensure((size_t)(2 * n_trials + k + 2) * sizeof(int)) ||
         !dKppU.ensure((size_t)std::max<da_int>(1, (k - 1) * n_trials) * sizeof(double)) ||
         !dKppBs.ensure((size_t)(nb + n_trials) * sizeof(double)) ||
         !dPartials.ensure(kpp_cost_work_bytes((int)n, (int)n_trials)))
         return err->error(da_status_memory_error, "Device memory allocation failed.");
     int *dCandv = dCand.as<int>();
-    int *dUnc = dCandv + n_trials;
-    int *dChosen = dUnc + n_trials;
+    int *dChosen = dCandv + n_trials;
     int *dFlag = dChosen + k;       // [0] a positive weight, [1] redone draws
     double *dBs = dKppBs.as<double>();
     double *dCost = dBs + nb;
@@ -257,7 +256,7 @@ template <typename T> da_status KMeans<T>::kmeans_plusplus(T *dC) {
         const int force_exact = (fe && fe[0] == '1') ? 1 : 0;
         for (da_int c = 1; c < k; ++c) {
             B200_TRY(launch_kpp_draw<T>(dW.as<T>(), (int)n, dBs, dU + (size_t)(c - 1) * n_trials,
-                                        (int)n_trials, force_exact, dCandv, dUnc, dFlag + 1, st),
+                                        (int)n_trials, force_exact, dCandv, dFlag + 1, st),
                      "k-means++ draws");
             B200_TRY(launch_kpp_dist_cost<T>(dX.as<T>(), ld, n, d, dXn.as<T>(), dCandv, n_trials,
                                              dW.as<T>(), dKD.as<T>(), dCost, dPartials.p, st,

@@ -16,12 +16,12 @@
 //     sequential sums, the divisions and the parallel sums).  The index is
 //     certified when u - P'_{i-1} / S' and P'_i / S' - u both exceed the
 //     bound; then the sequential search returns the same index.
-//   * kpp_exact_kernel: the draws that are not certified (about one per
+//   * exact_draw: the draws that are not certified (about one per
 //     k-means++ run on a million rows) are redone with the sequential sums
 //     themselves, in the reference's order of operations.
 // The candidates' distances are the kpp_dist kernel; their costs are the
 // reference's serial sums in the working precision, reproduced exactly by
-// kpp_serial_cost_kernel (at a million fp32 rows the rounding of those sums
+// kpp_walk_kernel (at a million fp32 rows the rounding of those sums
 // decides between candidates whose costs are that close, so an fp64 sum
 // would choose differently); kpp_select_update_kernel picks the candidate
 // with the smallest finite cost (repeats skipped, first strictly smaller wins), writes it to
@@ -29,13 +29,14 @@
 // weight and writes the block sums of the new w.  No host round trip per
 // centre.
 #include "b200_common.cuh"
+#include <algorithm>
 
 namespace b200 {
 
 static constexpr int KPP_THREADS = 256;
 static constexpr int KPP_PER_THREAD = 8;
 static constexpr int KPP_BLOCK = KPP_THREADS * KPP_PER_THREAD;
-static constexpr int KPP_EXACT_TILE = 4096;
+static constexpr int KPP_TRIALS = 64; // candidates per centre, at most (2 + ln k)
 
 __device__ __forceinline__ bool finite_(float v) { return isfinite(v); }
 __device__ __forceinline__ bool finite_(double v) { return isfinite(v); }
@@ -95,13 +96,279 @@ kpp_clamp_kernel(T *w, int n, int first, double *bs, int *flag) {
     if (__syncthreads_or(pos) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 
+// ------------------------------------------------ serial cost sums ------
+// The reference's candidate cost (kmeans.cpp:1624-1636) is the serial sum,
+// in the working precision T and index order from 0, of m_i = max(0,
+// min(w_i, d_i)).  It is reproduced exactly, not approximated.  While the
+// running sum s stays inside one binade [2^E, 2^(E+1)) every addition rounds
+// to the grid g = 2^(E - MANT) (s itself lies on it), so fl(s + m_i) =
+// s + RN_g(m_i) and a run of additions is one integer sum of the
+// independently rounded terms q_i = RN_g(m_i) (a tie, m_i / g exactly half-way,
+// rounds by the running sum's last bit) -- until the sum leaves the binade.
+// Three passes per candidate set:
+//   * kpp_dist_csum_kernel: the candidates' distances and, per 256-row
+//     chunk, the fp64 sum of its terms;
+//   * kpp_chunk_q_kernel: the fp64 prefix of the chunk sums predicts the
+//     binade E_j of the serial sum at each chunk; the chunk's run on that
+//     binade's grid as a parity function (Pf: ties need the sum's last bit);
+//   * kpp_walk_kernel, one block per candidate: adds runs of chunks whole
+//     where the running sum is in their binade and stays there, and the others
+//     term by term.  The prediction only chooses what is added whole; every
+//     such step is checked, so the result is the reference's T value whatever
+//     the fp64 prefix says.
+template <typename T> struct FpTraits;
+template <> struct FpTraits<float> {
+    static constexpr int MANT = 23, EMIN = -126;
+    static __device__ __forceinline__ int exponent(float s) {
+        return (int)((__float_as_uint(s) >> 23) & 0xFF) - 127;
+    }
+};
+template <> struct FpTraits<double> {
+    static constexpr int MANT = 52, EMIN = -1022;
+    static __device__ __forceinline__ int exponent(double s) {
+        return (int)((__double_as_longlong(s) >> 52) & 0x7FF) - 1023;
+    }
+};
+
+__host__ __device__ size_t kpp_dist_stride(int n, size_t elem);
+static constexpr int CK = 256;           // terms per chunk
+static constexpr int WALK_THREADS = 512;
+static constexpr int WALK_PER = 4; // chunk records per thread per pass
+static constexpr int NO_BINADE = -100000; // chunk record: sum it exactly
+static constexpr unsigned long long SC_SAT = 1ull << 62;
+
+__device__ __forceinline__ unsigned long long sat_add(unsigned long long a, unsigned long long b) {
+    const unsigned long long r = a + b; // a, b <= 2^62: no wrap
+    return r > SC_SAT ? SC_SAT : r;
+}
+
+// the reference's works5 element: std::max(0, std::min(w, d))
+template <typename T> __device__ __forceinline__ T kpp_term(T wv, T dv) {
+    const T mn = (dv < wv) ? dv : wv;
+    return (T(0) < mn) ? mn : T(0);
+}
+
+// PER consecutive values from row i0 (a multiple of PER; 0 past the end), with
+// 16-byte loads where they all exist (v starts on 16 bytes).
+template <typename T, int PER>
+__device__ __forceinline__ void kpp_load(const T *v, int n, int i0, T (&o)[PER]) {
+    constexpr int W = 16 / (int)sizeof(T);
+    struct __align__(16) V { T e[W]; };
+    if (i0 + PER <= n) {
+#pragma unroll
+        for (int c = 0; c < PER / W; ++c) {
+            const V a = reinterpret_cast<const V *>(v + i0)[c];
+#pragma unroll
+            for (int u = 0; u < W; ++u) o[c * W + u] = a.e[u];
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < PER; ++u) o[u] = i0 + u < n ? v[i0 + u] : T(0);
+    }
+}
+
+// The grid of the binade of s > 0: raw exponent (subnormals: EMIN - 1),
+// sh = -log2(g), the binade's end in grid units, s in grid units.
+template <typename T> struct Binade {
+    int ex, sh;
+    unsigned long long limit, s_int;
+    __device__ __forceinline__ void set(T s) {
+        using F = FpTraits<T>;
+        ex = F::exponent(s);
+        const bool sub = ex < F::EMIN;
+        sh = F::MANT - (sub ? F::EMIN : ex);
+        limit = sub ? (1ull << F::MANT) : (2ull << F::MANT);
+        s_int = (unsigned long long)ldexp((double)s, sh);
+    }
+    // t = 2 m / g is exact (power-of-two scaling in double, in two factors so
+    // that neither overflows).  q for a term staying inside the binade by
+    // itself: RN_g(m) for a
+    // non-tie; for a tie (m / g = k + 1/2) k, with *tie set (its rounding
+    // depends on the running sum's parity); SC_SAT for a term that leaves
+    // the binade by itself
+    __device__ __forceinline__ unsigned long long qt(T m, bool &tie) const {
+        const int e2 = sh + 1, ea = min(e2, 1000), eb = e2 - ea;
+        const double sa = __longlong_as_double((long long)(ea + 1023) << 52);
+        const double sb = __longlong_as_double((long long)(eb + 1023) << 52);
+        const double tt = ((double)m * sa) * sb;
+        tie = false;
+        if (!(tt < 2.0 * (double)limit)) return SC_SAT;
+        const unsigned long long ti = __double2ull_rz(tt);
+        if ((ti & 1ull) && tt == __ull2double_rn(ti)) {
+            tie = true;
+            return ti >> 1;
+        }
+        return (ti + 1ull) >> 1;
+    }
+    __device__ __forceinline__ T value(unsigned long long units) const {
+        return (T)ldexp((double)units, -sh);
+    }
+};
+
+// A run of additions on one grid as a function of the running sum's parity
+// (its last bit in grid units) at the run's start: q0 / q1 the run's total
+// for start parity 0 / 1, o bit p the parity at its end for start parity p.
+// A non-tie term q: (q, q, parity flips with q's last bit).  A tie term
+// m / g = k + 1/2 rounds to the even neighbour: k + ((R + k) & 1) for a
+// running sum R, after which the sum is even.  Runs compose associatively,
+// so a scan over them gives the running sum before every term.
+struct Pf {
+    unsigned long long q0, q1;
+    int o;
+};
+__device__ __forceinline__ Pf pf_id() { return Pf{0ull, 0ull, 2}; }
+__device__ __forceinline__ Pf pf_term(unsigned long long q, bool tie) {
+    if (!tie) {
+        const int b = (int)(q & 1ull);
+        return Pf{q, q, b | ((1 ^ b) << 1)};
+    }
+    return Pf{q + (q & 1ull), q + ((q + 1ull) & 1ull), 0};
+}
+__device__ __forceinline__ unsigned long long pf_q(const Pf &f, int p) { return p ? f.q1 : f.q0; }
+__device__ __forceinline__ int pf_o(const Pf &f, int p) { return (f.o >> p) & 1; }
+// a, then b
+__device__ __forceinline__ Pf pf_cat(const Pf &a, const Pf &b) {
+    const int a0 = a.o & 1, a1 = (a.o >> 1) & 1;
+    return Pf{sat_add(a.q0, pf_q(b, a0)), sat_add(a.q1, pf_q(b, a1)),
+              pf_o(b, a0) | (pf_o(b, a1) << 1)};
+}
+__device__ __forceinline__ Pf pf_shfl_up(const Pf &v, int off) {
+    return Pf{__shfl_up_sync(0xffffffffu, v.q0, off), __shfl_up_sync(0xffffffffu, v.q1, off),
+              __shfl_up_sync(0xffffffffu, v.o, off)};
+}
+
+// Scan of one run per thread over a block of NT threads in thread order:
+// the composition of the runs before this thread's (`excl`) and of all
+// (`total`).  shm: 2 * (NT / 32) + 1 entries.
+template <int NT>
+__device__ void block_scan_pf(const Pf &v, Pf *shm, Pf &excl, Pf &total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NW = NT / 32;
+    Pf x = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const Pf y = pf_shfl_up(x, off);
+        if (lane >= off) x = pf_cat(y, x);
+    }
+    Pf xe = pf_shfl_up(x, 1);
+    if (lane == 0) xe = pf_id();
+    __syncthreads();
+    if (lane == 31) shm[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        Pf y = lane < NW ? shm[lane] : pf_id();
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const Pf z = pf_shfl_up(y, off);
+            if (lane >= off) y = pf_cat(z, y);
+        }
+        Pf ye = pf_shfl_up(y, 1);
+        if (lane == 0) ye = pf_id();
+        if (lane < NW) shm[NW + lane] = ye;
+        if (lane == NW - 1) shm[2 * NW] = y;
+    }
+    __syncthreads();
+    total = shm[2 * NW];
+    excl = pf_cat(shm[NW + warp], xe);
+}
+
+// The sequential sum in double, from s, of a block's tile of terms in thread
+// order (8 consecutive per thread; v: this thread's, cnt in all): by one scan
+// of the terms' runs on the grid of s where the sum stays in its binade, else
+// by thread 0 term by term.  Every thread returns the new sum.
+__device__ double exact_tile(double s, const double (&v)[KPP_PER_THREAD], int cnt, Pf *shm,
+                             double *tile, double *out) {
+    if (s != 0.0 && isfinite(s)) { // the same for every thread
+        Binade<double> b;
+        b.set(s);
+        Pf loc = pf_id();
+        bool sat = false;
+#pragma unroll
+        for (int u = 0; u < KPP_PER_THREAD; ++u) {
+            bool tie;
+            const unsigned long long q = b.qt(v[u], tie);
+            sat = sat || q == SC_SAT;
+            loc = pf_cat(loc, pf_term(q, tie));
+        }
+        Pf ex, tot;
+        block_scan_pf<KPP_THREADS>(loc, shm, ex, tot);
+        const unsigned long long R = sat_add(b.s_int, pf_q(tot, (int)(b.s_int & 1ull)));
+        if (!__syncthreads_or(sat) && R < b.limit) return b.value(R);
+    }
+#pragma unroll
+    for (int u = 0; u < KPP_PER_THREAD; ++u) tile[threadIdx.x * KPP_PER_THREAD + u] = v[u];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 0; j < cnt; ++j) s = __dadd_rn(s, tile[j]);
+        *out = s;
+    }
+    __syncthreads();
+    s = *out;
+    __syncthreads();
+    return s;
+}
+
+// A draw with the reference's sequential arithmetic: S = sum w (double, index
+// order, from 0), p_i = w_i / S, cp_i = cp_{i-1} + p_i, cp_{n-1} = 1, the first
+// i with !(cp_i < u) (std::lower_bound).  Block-wide, 2,048 terms at a time;
+// the terms that decide the draw are added one by one.  About one draw in a
+// k-means++ run on a million rows comes here: 2 ms there, 12 ms when one
+// thread added all terms.
+template <typename T> __device__ __noinline__ void exact_draw(const T *w, int n, double u, int *out) {
+    __shared__ double tile[KPP_BLOCK];
+    __shared__ Pf shm[2 * (KPP_THREADS / 32) + 1];
+    __shared__ double s_out;
+    __shared__ int s_res;
+    double v[KPP_PER_THREAD], S = 0.0;
+    auto load = [&](int t0) {
+        T x[KPP_PER_THREAD];
+        kpp_load<T, KPP_PER_THREAD>(w, n, t0 + (int)threadIdx.x * KPP_PER_THREAD, x);
+#pragma unroll
+        for (int j = 0; j < KPP_PER_THREAD; ++j) v[j] = (double)x[j];
+    };
+    for (int t0 = 0; t0 < n; t0 += KPP_BLOCK) {
+        load(t0);
+        S = exact_tile(S, v, min(KPP_BLOCK, n - t0), shm, tile, &s_out);
+    }
+    if (threadIdx.x == 0) s_res = n - 1;
+    double cp = 0.0;
+    for (int t0 = 0; t0 < n; t0 += KPP_BLOCK) {
+        load(t0);
+#pragma unroll
+        for (int j = 0; j < KPP_PER_THREAD; ++j) v[j] = __ddiv_rn(v[j], S);
+        const double before = cp;
+        cp = exact_tile(cp, v, min(KPP_BLOCK, n - t0), shm, tile, &s_out);
+        // the tile in which cp reaches u (or the last index, cp = 1), or any
+        // when cp is NaN: with all weights zero (S = 0) the test !(cp < u)
+        // holds at once
+        if (cp < u && t0 + KPP_BLOCK < n) continue;
+#pragma unroll
+        for (int j = 0; j < KPP_PER_THREAD; ++j) tile[threadIdx.x * KPP_PER_THREAD + j] = v[j];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double c = before;
+            for (int j = 0; j < KPP_BLOCK && t0 + j < n; ++j) {
+                c = __dadd_rn(c, tile[j]);
+                if (t0 + j == n - 1) c = 1.0;
+                if (!(c < u)) {
+                    s_res = t0 + j;
+                    break;
+                }
+            }
+        }
+        break;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *out = s_res;
+}
+
 // One block per draw t: the index that std::discrete_distribution gives for
-// u = U[t] over the weights w, certified against the bound (unc[t] = 0), or
-// an approximate index with unc[t] = 1 for the exact kernel to redo.
+// u = U[t] over the weights w, certified against the bound; a draw that is not
+// certified is redone by exact_draw and counted.
 template <typename T>
 __global__ void __launch_bounds__(KPP_THREADS)
 kpp_draw_kernel(const T *w, int n, const double *bs, int nb, const double *U, double bound,
-                int force_exact, int *cand, int *unc) {
+                int force_exact, int *cand, int *exact_count) {
     __shared__ double sh[KPP_THREADS / 32 + 1];
     __shared__ double s_prev;
     __shared__ int s_block, s_idx;
@@ -178,6 +445,7 @@ kpp_draw_kernel(const T *w, int n, const double *bs, int nb, const double *U, do
         s_pim1 = pim1;
     }
     __syncthreads();
+    __shared__ int s_certified;
     if (threadIdx.x == 0) {
         int idx = s_idx;
         bool certified = found_block && idx != 0x7fffffff && S > 0.0 && isfinite(S);
@@ -188,266 +456,16 @@ kpp_draw_kernel(const T *w, int n, const double *bs, int nb, const double *U, do
             certified = hi > bound && lo > bound;
         }
         cand[t] = idx;
-        unc[t] = (certified && !force_exact) ? 0 : 1;
-    }
-}
-
-// The uncertified draws with the reference's sequential arithmetic: S =
-// sum w (double, index order, from 0), p_i = w_i / S, cp_i = cp_{i-1} + p_i,
-// cp_{n-1} = 1, the first i with !(cp_i < u) (std::lower_bound).  One block; thread 0 carries the
-// sequential sums over tiles that all threads stage in shared memory.
-// count[0] accumulates the number of redone draws.
-template <typename T>
-__global__ void __launch_bounds__(KPP_THREADS)
-kpp_exact_kernel(const T *w, int n, const double *U, int nt, int *cand, const int *unc,
-                 int *count) {
-    __shared__ double tile[KPP_EXACT_TILE];
-    __shared__ double s_sum;
-    __shared__ int s_any;
-    if (threadIdx.x == 0) {
-        int a = 0;
-        for (int t = 0; t < nt; ++t) a += unc[t] ? 1 : 0;
-        s_any = a;
-        if (a) atomicAdd(count, a);
+        s_certified = certified && !force_exact;
+        if (!s_certified) atomicAdd(exact_count, 1);
     }
     __syncthreads();
-    if (!s_any) return;
-    // S, sequentially
-    double S = 0.0;
-    for (int t0 = 0; t0 < n; t0 += KPP_EXACT_TILE) {
-        const int m = min(KPP_EXACT_TILE, n - t0);
-        for (int j = threadIdx.x; j < m; j += KPP_THREADS) tile[j] = (double)w[t0 + j];
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (int j = 0; j < m; ++j) S = __dadd_rn(S, tile[j]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) s_sum = S;
-    __syncthreads();
-    S = s_sum;
-    for (int t = 0; t < nt; ++t) {
-        if (!unc[t]) continue;
-        const double u = U[t];
-        __shared__ int s_done, s_res;
-        if (threadIdx.x == 0) {
-            s_done = 0;
-            s_res = n - 1;
-        }
-        __syncthreads();
-        double cp = 0.0;
-        for (int t0 = 0; t0 < n; t0 += KPP_EXACT_TILE) {
-            const int m = min(KPP_EXACT_TILE, n - t0);
-            for (int j = threadIdx.x; j < m; j += KPP_THREADS)
-                tile[j] = __ddiv_rn((double)w[t0 + j], S);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                for (int j = 0; j < m; ++j) {
-                    cp = __dadd_rn(cp, tile[j]);
-                    if (t0 + j == n - 1) cp = 1.0;
-                    // std::lower_bound's test !(cp < u): with all weights
-                    // zero (S = 0) every cp is NaN and the first index wins
-                    if (!(cp < u)) {
-                        s_res = t0 + j;
-                        s_done = 1;
-                        break;
-                    }
-                }
-            }
-            __syncthreads();
-            if (s_done) break;
-        }
-        if (threadIdx.x == 0) cand[t] = s_res;
-        __syncthreads();
-    }
+    if (!s_certified) exact_draw<T>(w, n, u, &cand[t]);
 }
 
-// ------------------------------------------------ serial cost sums ------
-// The reference's candidate cost (kmeans.cpp:1624-1636) is the serial sum,
-// in the working precision T and index order from 0, of m_i = max(0,
-// min(w_i, d_i)).  It is reproduced exactly, not approximated.  While the
-// running sum s stays inside one binade [2^E, 2^(E+1)) every addition rounds
-// to the grid g = 2^(E - MANT) (s itself lies on it), so fl(s + m_i) =
-// s + RN_g(m_i) and a run of additions is one integer sum of the
-// independently rounded terms q_i = RN_g(m_i) -- unless a term is a tie
-// (m_i / g exactly half-way: ties-to-even then depends on the running sum's
-// last bit) or the sum leaves the binade; such a term is added serially in T.
-// Three passes per candidate set:
-//   * kpp_dist_csum_kernel: the candidates' distances and, per 256-row
-//     chunk, the fp64 sum of its terms;
-//   * kpp_chunk_q_kernel: the fp64 prefix of the chunk sums predicts the
-//     binade E_j of the serial sum at each chunk; the chunk's integer total
-//     Q_j on that binade's grid (flagged when a term ties);
-//   * kpp_walk_kernel, one block per candidate: walks the chunk records; a
-//     chunk is added as s += Q_j g when the running sum is in binade E_j, the
-//     chunk has no tie and the sum stays in the binade -- else the chunk is
-//     summed exactly term by term (integer runs, serial steps at the first
-//     tie or binade crossing).  The prediction only chooses the fast path;
-//     every fast step is checked, so the result is the reference's T value
-//     whatever the fp64 prefix says.
-template <typename T> struct FpTraits;
-template <> struct FpTraits<float> {
-    static constexpr int MANT = 23, EMIN = -126;
-    static __device__ __forceinline__ int exponent(float s) {
-        return (int)((__float_as_uint(s) >> 23) & 0xFF) - 127;
-    }
-};
-template <> struct FpTraits<double> {
-    static constexpr int MANT = 52, EMIN = -1022;
-    static __device__ __forceinline__ int exponent(double s) {
-        return (int)((__double_as_longlong(s) >> 52) & 0x7FF) - 1023;
-    }
-};
-
-static constexpr int CK = 256;           // terms per chunk
-static constexpr int WALK_THREADS = 256;
-static constexpr int WALK_PER = 4; // chunk records per thread per pass
-static constexpr int NO_BINADE = -100000; // chunk record: sum it exactly
-static constexpr unsigned long long SC_SAT = 1ull << 62;
-
-__device__ __forceinline__ unsigned long long sat_add(unsigned long long a, unsigned long long b) {
-    const unsigned long long r = a + b; // a, b <= 2^62: no wrap
-    return r > SC_SAT ? SC_SAT : r;
-}
-
-// the reference's works5 element: std::max(0, std::min(w, d))
-template <typename T> __device__ __forceinline__ T kpp_term(T wv, T dv) {
-    const T mn = (dv < wv) ? dv : wv;
-    return (T(0) < mn) ? mn : T(0);
-}
-
-// The grid of the binade of s > 0: raw exponent (subnormals: EMIN - 1),
-// sh = -log2(g), the binade's end in grid units, s in grid units.
-template <typename T> struct Binade {
-    int ex, sh;
-    unsigned long long limit, s_int;
-    __device__ __forceinline__ void set(T s) {
-        using F = FpTraits<T>;
-        ex = F::exponent(s);
-        const bool sub = ex < F::EMIN;
-        sh = F::MANT - (sub ? F::EMIN : ex);
-        limit = sub ? (1ull << F::MANT) : (2ull << F::MANT);
-        s_int = (unsigned long long)ldexp((double)s, sh);
-    }
-    // q = RN_g(m) for a non-tie; SC_SAT for a tie or a term that leaves the
-    // binade by itself.  t = 2 m / g is exact (power-of-two scaling in
-    // double, in two factors so that neither overflows); RN(t / 2) of a
-    // non-tie = (floor(t) + 1) / 2; a tie is t an odd integer.
-    __device__ __forceinline__ unsigned long long q(T m) const {
-        const int e2 = sh + 1, ea = min(e2, 1000), eb = e2 - ea;
-        const double sa = __longlong_as_double((long long)(ea + 1023) << 52);
-        const double sb = __longlong_as_double((long long)(eb + 1023) << 52);
-        const double tt = ((double)m * sa) * sb;
-        if (!(tt < 2.0 * (double)limit)) return SC_SAT;
-        const unsigned long long ti = __double2ull_rz(tt);
-        if ((ti & 1ull) && tt == __ull2double_rn(ti)) return SC_SAT;
-        return (ti + 1ull) >> 1;
-    }
-    // q for a term staying inside the binade by itself: RN_g(m) for a
-    // non-tie; for a tie (m / g = k + 1/2) k, with *tie set (its rounding
-    // depends on the running sum's parity); SC_SAT for a term that leaves
-    // the binade by itself
-    __device__ __forceinline__ unsigned long long qt(T m, bool &tie) const {
-        const int e2 = sh + 1, ea = min(e2, 1000), eb = e2 - ea;
-        const double sa = __longlong_as_double((long long)(ea + 1023) << 52);
-        const double sb = __longlong_as_double((long long)(eb + 1023) << 52);
-        const double tt = ((double)m * sa) * sb;
-        tie = false;
-        if (!(tt < 2.0 * (double)limit)) return SC_SAT;
-        const unsigned long long ti = __double2ull_rz(tt);
-        if ((ti & 1ull) && tt == __ull2double_rn(ti)) {
-            tie = true;
-            return ti >> 1;
-        }
-        return (ti + 1ull) >> 1;
-    }
-    // m stays inside the binade by itself (so SC_SAT from q() means a tie)
-    __device__ __forceinline__ bool q_in_range(T m) const {
-        const int e2 = sh + 1, ea = min(e2, 1000), eb = e2 - ea;
-        const double sa = __longlong_as_double((long long)(ea + 1023) << 52);
-        const double sb = __longlong_as_double((long long)(eb + 1023) << 52);
-        return ((double)m * sa) * sb < 2.0 * (double)limit;
-    }
-    __device__ __forceinline__ T value(unsigned long long units) const {
-        return (T)ldexp((double)units, -sh);
-    }
-};
-
-// A run of additions on one grid as a function of the running sum's parity
-// (its last bit in grid units) at the run's start: q0 / q1 the run's total
-// for start parity 0 / 1, o bit p the parity at its end for start parity p.
-// A non-tie term q: (q, q, parity flips with q's last bit).  A tie term
-// m / g = k + 1/2 rounds to the even neighbour: k + ((R + k) & 1) for a
-// running sum R, after which the sum is even.  Runs compose associatively,
-// so a scan over them gives the running sum before every term.
-struct Pf {
-    unsigned long long q0, q1;
-    int o;
-};
-__device__ __forceinline__ Pf pf_id() { return Pf{0ull, 0ull, 2}; }
-__device__ __forceinline__ Pf pf_term(unsigned long long q, bool tie) {
-    if (!tie) {
-        const int b = (int)(q & 1ull);
-        return Pf{q, q, b | ((1 ^ b) << 1)};
-    }
-    return Pf{q + (q & 1ull), q + ((q + 1ull) & 1ull), 0};
-}
-__device__ __forceinline__ unsigned long long pf_q(const Pf &f, int p) { return p ? f.q1 : f.q0; }
-__device__ __forceinline__ int pf_o(const Pf &f, int p) { return (f.o >> p) & 1; }
-// a, then b
-__device__ __forceinline__ Pf pf_cat(const Pf &a, const Pf &b) {
-    const int a0 = a.o & 1, a1 = (a.o >> 1) & 1;
-    return Pf{sat_add(a.q0, pf_q(b, a0)), sat_add(a.q1, pf_q(b, a1)),
-              pf_o(b, a0) | (pf_o(b, a1) << 1)};
-}
-__device__ __forceinline__ Pf pf_shfl_up(const Pf &v, int off) {
-    return Pf{__shfl_up_sync(0xffffffffu, v.q0, off), __shfl_up_sync(0xffffffffu, v.q1, off),
-              __shfl_up_sync(0xffffffffu, v.o, off)};
-}
-
-// Scan of one run per thread over a block of NT threads in thread order:
-// the composition of the runs before this thread's (`excl`) and of all
-// (`total`).  shm: 2 * (NT / 32) + 1 entries.
-template <int NT>
-__device__ void block_scan_pf(const Pf &v, Pf *shm, Pf &excl, Pf &total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int NW = NT / 32;
-    Pf x = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const Pf y = pf_shfl_up(x, off);
-        if (lane >= off) x = pf_cat(y, x);
-    }
-    Pf xe = pf_shfl_up(x, 1);
-    if (lane == 0) xe = pf_id();
-    __syncthreads();
-    if (lane == 31) shm[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        Pf y = lane < NW ? shm[lane] : pf_id();
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const Pf z = pf_shfl_up(y, off);
-            if (lane >= off) y = pf_cat(z, y);
-        }
-        Pf ye = pf_shfl_up(y, 1);
-        if (lane == 0) ye = pf_id();
-        if (lane < NW) shm[NW + lane] = ye;
-        if (lane == NW - 1) shm[2 * NW] = y;
-    }
-    __syncthreads();
-    total = shm[2 * NW];
-    excl = pf_cat(shm[NW + warp], xe);
-}
-
-// Distances of a 256-row chunk to the candidates (one thread per row), with
-// the chunk's fp64 sum of the cost terms per candidate.  A thread holds 64
-// (fp32) or 32 (fp64) features of its row in registers at a time -- 16
-// independent 16-byte loads in flight -- and runs eight candidates' fma
-// chains over them (features in order), the candidates' values broadcast
-// from shared memory (SMEM) or read through L1.
 template <typename T> struct SegTraits;
 template <> struct SegTraits<float> {
-    static constexpr int SEG = 64; // features per register segment
+    static constexpr int SEG = 64; // features per register segment (kpp_dist_long_kernel)
     using V = float4;
     static constexpr int W = 4;
     static __device__ __forceinline__ void split(const float4 &v, float (&o)[4]) {
@@ -463,23 +481,185 @@ template <> struct SegTraits<double> {
     }
 };
 
-template <typename T, bool SMEM>
-__global__ void __launch_bounds__(CK, 2)
-kpp_dist_csum_kernel(const T *X, int ld, int n, int d, const T *xnorm, const int *cand, int t,
-                     const T *w, T *D, double *csum, int nchunks, const T *xinv, int cosine) {
+// Distances of 256-row chunks to the candidates, with each chunk's fp64 sum of
+// the cost terms per candidate.  Bound: HBM, one read of the rows (256 MB at
+// 1M x 64 fp32: 39 us at the measured copy rate).  Three blocks per SM stay for
+// the whole pass and take every gridDim-th chunk; the rows come in as 128-byte
+// slabs (asynchronous 16-byte copies, the 16-byte parts of a row exchanged by
+// the row's low bits so that eight lanes reading eight rows hit all banks), one
+// slab ahead of the arithmetic, across chunks too.  A thread carries two rows'
+// fma chains (features in order) for G candidates, whose values come from
+// shared memory once for both.  At 1M x 64 and seven candidates: 58 us;
+// one thread per row with its own strided 16-byte loads took 138 us (a warp's
+// load touches 32 lines).
+static constexpr int KD_THREADS = 128;
+static constexpr int KD_SLAB = 128; // bytes of a row per slab
+static constexpr int KD_BLOCKS = 3; // per SM
+
+__device__ __forceinline__ void kd_copy16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src));
+}
+__device__ __forceinline__ void kd_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N> __device__ __forceinline__ void kd_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N));
+}
+
+// bytes of shared memory: two slabs of a chunk's rows, the candidates' rows
+template <typename T> static size_t kd_smem(int t, int ld) {
+    return 2 * (size_t)CK * KD_SLAB + (size_t)t * ld * sizeof(T);
+}
+
+template <typename T, int G>
+__global__ void __launch_bounds__(KD_THREADS, KD_BLOCKS)
+kpp_dist_csum_kernel(const T *X, int ld, int n, const T *xnorm, const int *cand, int c0, int t,
+                     const T *w, T *D, size_t nd, double *csum, int nchunks, const T *xinv,
+                     int cosine) {
     using S = SegTraits<T>;
-    constexpr int NV = S::SEG / S::W;
+    using V = typename S::V;
     extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ double red[CK / 32][8];
-    T *cs = reinterpret_cast<T *>(sm); // [t][dp] when SMEM
-    const int dp = (d + S::W - 1) / S::W * S::W;
-    if (SMEM) {
-        for (int e = threadIdx.x; e < t * dp; e += CK) {
-            const int c = e / dp, f = e % dp;
-            cs[e] = f < d ? X[(size_t)cand[c] * ld + f] : T(0);
+    __shared__ double red[KD_THREADS / 32][G];
+    unsigned char *slab = sm;                                     // [2][CK][KD_SLAB]
+    T *cs = reinterpret_cast<T *>(sm + 2 * (size_t)CK * KD_SLAB); // [t][ld]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row_bytes = ld * (int)sizeof(T); // a multiple of 16, pad columns zero
+    const int nslab = (row_bytes + KD_SLAB - 1) / KD_SLAB;
+    const unsigned char *Xb = reinterpret_cast<const unsigned char *>(X);
+    auto fetch = [&](int chunk, int k, int buf) {
+        const int r0 = chunk * CK;
+#pragma unroll
+        for (int u = 0; u < CK * 8 / KD_THREADS; ++u) {
+            const int e = tid + u * KD_THREADS, r = e >> 3, c = e & 7;
+            const int off = k * KD_SLAB + c * 16;
+            if (r0 + r < n && off < row_bytes)
+                kd_copy16(slab + ((size_t)buf * CK + r) * KD_SLAB + ((c ^ (r & 7)) * 16),
+                          Xb + (size_t)(r0 + r) * row_bytes + off);
+        }
+    };
+    int chunk = blockIdx.x;
+    if (chunk >= nchunks) return;
+    fetch(chunk, 0, 0);
+    kd_commit();
+    for (int e = tid; e < t * ld; e += KD_THREADS)
+        cs[e] = X[(size_t)cand[c0 + e / ld] * ld + e % ld];
+    int cg[G], buf = 0;
+    T cn[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        cg[g] = min(g, t - 1) * ld;
+        cn[g] = xnorm[cand[c0 + min(g, t - 1)]];
+    }
+    for (; chunk < nchunks; chunk += gridDim.x) {
+        const int r0 = chunk * CK;
+        T xn[2], wi[2], s[2][G];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = r0 + tid + h * KD_THREADS;
+            xn[h] = i < n ? xnorm[i] : T(0);
+            wi[h] = i < n ? w[i] : T(0);
+#pragma unroll
+            for (int g = 0; g < G; ++g) s[h][g] = T(0);
+        }
+        for (int k = 0; k < nslab; ++k, buf ^= 1) {
+            // the next slab, of this chunk or of the block's next one, into the
+            // other buffer (whose readers passed the barrier below)
+            if (k + 1 < nslab) fetch(chunk, k + 1, buf ^ 1);
+            else if (chunk + (int)gridDim.x < nchunks) fetch(chunk + gridDim.x, 0, buf ^ 1);
+            kd_commit();
+            kd_wait<1>();
+            __syncthreads();
+            const unsigned char *row = slab + ((size_t)buf * CK + tid) * KD_SLAB;
+            const int nv = min(8, (row_bytes - k * KD_SLAB) / 16);
+            const int f0 = k * (KD_SLAB / (int)sizeof(T));
+#pragma unroll 2
+            for (int v = 0; v < nv; ++v) {
+                const int o = (v ^ (tid & 7)) * 16; // rows tid and tid + 128: the same low bits
+                T x0[S::W], x1[S::W];
+                S::split(*reinterpret_cast<const V *>(row + o), x0);
+                S::split(*reinterpret_cast<const V *>(row + KD_THREADS * KD_SLAB + o), x1);
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    T ce[S::W];
+                    S::split(*reinterpret_cast<const V *>(cs + cg[g] + f0 + v * S::W), ce);
+#pragma unroll
+                    for (int u = 0; u < S::W; ++u) {
+                        s[0][g] = fma_rn(x0[u], ce[u], s[0][g]);
+                        s[1][g] = fma_rn(x1[u], ce[u], s[1][g]);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        double part[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            part[g] = 0.0;
+            if (g < t) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int i = r0 + tid + h * KD_THREADS;
+                    if (i >= n) continue;
+                    const T dv = cosine ? cos_dist_kpp(s[h][g], xinv, i, cand[c0 + g])
+                                        : fma_rn(T(-2), s[h][g], add_rn(xn[h], cn[g]));
+                    D[(size_t)(c0 + g) * nd + i] = dv;
+                    part[g] += (double)kpp_term(wi[h], dv);
+                }
+            }
+        }
+        // sums over the warp: lane bits 4, 3, 2 also split the candidates
+        // while there are several (a quarter of the exchanges of G full sums)
+#pragma unroll
+        for (int off = 16, m = G; off > 0; off >>= 1) {
+            if (m % 2 == 0) {
+                m /= 2;
+                const bool up = lane & off;
+#pragma unroll
+                for (int g = 0; g < G / 2; ++g)
+                    if (g < m) {
+                        const double give = up ? part[g] : part[g + m];
+                        const double keep = up ? part[g + m] : part[g];
+                        part[g] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+                    }
+            } else {
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    if (g < m) part[g] += __shfl_xor_sync(0xffffffffu, part[g], off);
+            }
+        }
+        constexpr int H = G == 8 ? 1 : G == 6 ? 3 : 1; // sums left in a lane
+        constexpr int SPLIT = G / H;                   // lane groups of different ones
+        if ((lane & (32 / SPLIT - 1)) == 0) {
+            // the lane's top bits choose its candidates: bit 4 the upper half
+            int g0 = 0, m = G;
+#pragma unroll
+            for (int off = 16; off >= 32 / SPLIT; off >>= 1) {
+                m /= 2;
+                g0 += (lane & off) ? m : 0;
+            }
+#pragma unroll
+            for (int h = 0; h < H; ++h) red[warp][g0 + h] = part[h];
         }
         __syncthreads();
+        if (tid < G && tid < t) {
+            double a = 0.0;
+#pragma unroll
+            for (int v = 0; v < KD_THREADS / 32; ++v) a += red[v][tid];
+            csum[(size_t)(c0 + tid) * nchunks + chunk] = a;
+        }
+        // red is rewritten after the next chunk's barriers
     }
+}
+
+// The same for rows too long for that (candidates beyond 96 KB of shared
+// memory): one thread per row, the candidates' values through L1.
+template <typename T>
+__global__ void __launch_bounds__(CK, 2)
+kpp_dist_long_kernel(const T *X, int ld, int n, int d, const T *xnorm, const int *cand, int t,
+                     const T *w, T *D, size_t nd, double *csum, int nchunks, const T *xinv, int cosine) {
+    using S = SegTraits<T>;
+    constexpr int NV = S::SEG / S::W;
+    __shared__ double red[CK / 32][8];
     const int i = blockIdx.x * CK + threadIdx.x;
     const bool valid = i < n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -509,12 +689,8 @@ kpp_dist_csum_kernel(const T *X, int ld, int n, int d, const T *xnorm, const int
 #pragma unroll
                     for (int g = 0; g < 8; ++g) {
                         T ce[S::W];
-                        if (SMEM) {
-                            S::split(*reinterpret_cast<const typename S::V *>(cs + (size_t)cg[g] * dp + fb), ce);
-                        } else {
-                            const T *yr = X + (size_t)cand[cg[g]] * ld + fb;
-                            S::split(*reinterpret_cast<const typename S::V *>(yr), ce);
-                        }
+                        const T *yr = X + (size_t)cand[cg[g]] * ld + fb;
+                        S::split(*reinterpret_cast<const typename S::V *>(yr), ce);
 #pragma unroll
                         for (int u = 0; u < S::W; ++u)
                             if (fb + u < d) s[g] = fma_rn(xe[u], ce[u], s[g]);
@@ -530,7 +706,7 @@ kpp_dist_csum_kernel(const T *X, int ld, int n, int d, const T *xnorm, const int
                 const int cc = cand[c0 + g];
                 const T dv = cosine ? cos_dist_kpp(s[g], xinv, i, cc)
                                     : fma_rn(T(-2), s[g], add_rn(xn, xnorm[cc]));
-                D[(size_t)(c0 + g) * n + i] = dv;
+                D[(size_t)(c0 + g) * nd + i] = dv;
                 part[g] = (double)kpp_term(wi, dv);
             }
 #pragma unroll
@@ -549,40 +725,112 @@ kpp_dist_csum_kernel(const T *X, int ld, int n, int d, const T *xnorm, const int
     }
 }
 
-// Exclusive fp64 prefix of the chunk sums of candidate blockIdx.x.
+// Exclusive fp64 prefix of the chunk sums of candidate blockIdx.x: one range
+// of consecutive chunks per thread.
 __global__ void __launch_bounds__(1024) kpp_chunk_prefix_kernel(const double *csum, int nchunks,
                                                                 double *P) {
-    __shared__ double shd[33];
+    __shared__ double shd[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double *cs = csum + (size_t)blockIdx.x * nchunks;
     double *Pt = P + (size_t)blockIdx.x * nchunks;
-    double carry = 0.0;
-    for (int c0 = 0; c0 < nchunks; c0 += 1024) {
-        const int j = c0 + threadIdx.x;
-        const double v = j < nchunks ? cs[j] : 0.0;
-        double x = v;
+    const int per = (nchunks + 1023) / 1024;
+    const int j0 = min(nchunks, (int)threadIdx.x * per), j1 = min(nchunks, j0 + per);
+    double mine = 0.0;
+    for (int j = j0; j < j1; ++j) mine += cs[j];
+    double x = mine;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        __syncthreads();
-        if (lane == 31) shd[warp] = x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0.0;
-            for (int q = 0; q < 32; ++q) {
-                const double tq = shd[q];
-                shd[q] = a;
-                a += tq;
-            }
-            shd[32] = a;
-        }
-        __syncthreads();
-        if (j < nchunks) Pt[j] = carry + shd[warp] + (x - v);
-        carry += shd[32];
+    for (int off = 1; off < 32; off <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+    }
+    if (lane == 31) shd[warp] = x;
+    __syncthreads();
+    double before = lane < warp ? shd[lane] : 0.0;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) before += __shfl_xor_sync(0xffffffffu, before, off);
+    double run = before + (x - mine);
+    for (int j = j0; j < j1; ++j) {
+        Pt[j] = run;
+        run += cs[j];
     }
 }
+
+// The terms of one warp's chunk on one binade's grid, eight consecutive terms a
+// lane, in the integer width that the type's grid needs: 32 bits for fp32 (a
+// binade holds 2^23 grid steps; totals saturate far above that), 64 for fp64.
+// run(): a lane's terms as one parity function; warp_scan(): the runs of the
+// lanes before.  SAT marks a run that leaves the binade.
+template <typename T> struct Grid;
+template <> struct Grid<float> {
+    using U = unsigned;
+    static constexpr U SAT = 1u << 30;
+    U limit, s_int, base; // base: the binade's exponent bits (0: subnormal)
+    float sa, sb;         // terms to half grid steps, in two exact factors
+    __device__ __forceinline__ void set(float s) {
+        const unsigned bits = __float_as_uint(s);
+        base = bits & 0x7f800000u;
+        limit = base ? 1u << 24 : 1u << 23;
+        s_int = (bits & 0x7fffffu) | (base ? 0x800000u : 0u);
+        const int e2 = 24 - (max((int)(base >> 23), 1) - 127), ea = min(e2, 100);
+        sa = __uint_as_float((unsigned)(ea + 127) << 23);
+        sb = __uint_as_float((unsigned)(e2 - ea + 127) << 23);
+    }
+    // the sum of `steps` grid steps, s_int <= steps < limit
+    __device__ __forceinline__ float value(U steps) const {
+        return __uint_as_float(base | (steps & 0x7fffffu));
+    }
+    // RN to the grid of a term that does not tie; k of a tie k + 1/2 (tie set)
+    __device__ __forceinline__ U term(float m, bool &tie) const {
+        const float t = (m * sa) * sb; // exact, or below half a step
+        tie = false;
+        if (!(t < 2.0f * __uint2float_rn(limit))) return SAT;
+        const U ti = __float2uint_rz(t);
+        tie = (ti & 1u) && t == __uint2float_rn(ti);
+        return tie ? ti >> 1 : (ti + 1u) >> 1;
+    }
+    static __device__ __forceinline__ U add(U a, U b) { return min(a + b, SAT); }
+    static __device__ __forceinline__ unsigned long long wide(U v) { return v >= SAT ? SC_SAT : v; }
+};
+template <> struct Grid<double> {
+    using U = unsigned long long;
+    static constexpr U SAT = SC_SAT;
+    U limit, s_int;
+    Binade<double> b;
+    __device__ __forceinline__ void set(double s) {
+        b.set(s);
+        limit = b.limit;
+        s_int = b.s_int;
+    }
+    __device__ __forceinline__ double value(U steps) const { return b.value(steps); }
+    __device__ __forceinline__ U term(double m, bool &tie) const { return b.qt(m, tie); }
+    static __device__ __forceinline__ U add(U a, U b) { return sat_add(a, b); }
+    static __device__ __forceinline__ unsigned long long wide(U v) { return v; }
+};
+// a parity function in the grid's integer width (see Pf)
+template <typename T> struct Run {
+    using G = Grid<T>;
+    using U = typename G::U;
+    U q0, q1;
+    int o;
+    static __device__ __forceinline__ Run id() { return Run{0, 0, 2}; }
+    __device__ __forceinline__ U q(int p) const { return p ? q1 : q0; }
+    __device__ __forceinline__ int par(int p) const { return (o >> p) & 1; }
+    // then one term
+    __device__ __forceinline__ void add_term(U k, bool tie) {
+        const int a0 = o & 1, a1 = (o >> 1) & 1, b = (int)(k & 1);
+        q0 = G::add(q0, tie ? k + (U)(a0 ^ b) : k);
+        q1 = G::add(q1, tie ? k + (U)(a1 ^ b) : k);
+        o = tie ? 0 : (a0 ^ b) | ((a1 ^ b) << 1);
+    }
+    static __device__ __forceinline__ Run cat(const Run &a, const Run &b) {
+        const int a0 = a.par(0), a1 = a.par(1);
+        return Run{G::add(a.q0, b.q(a0)), G::add(a.q1, b.q(a1)), b.par(a0) | (b.par(a1) << 1)};
+    }
+    __device__ __forceinline__ Run up(int off) const {
+        return Run{__shfl_up_sync(0xffffffffu, q0, off), __shfl_up_sync(0xffffffffu, q1, off),
+                   __shfl_up_sync(0xffffffffu, o, off)};
+    }
+};
 
 // Chunk records of candidate blockIdx.y, one warp per chunk: the binade the
 // fp64 prefix predicts for the serial sum at the chunk (raw exponent of
@@ -590,13 +838,17 @@ __global__ void __launch_bounds__(1024) kpp_chunk_prefix_kernel(const double *cs
 // that binade's grid as a parity function (saturating totals).
 template <typename T>
 __global__ void __launch_bounds__(256)
-kpp_chunk_q_kernel(const T *w, const T *D, int n, int nchunks, const double *P,
+kpp_chunk_q_kernel(const T *w, const T *D, size_t nd, int n, int nchunks, const double *P,
                    unsigned long long *Q0, unsigned long long *Q1, int *Or, int *Er) {
-    const int t = blockIdx.y;
+    constexpr int PER = CK / 32;
     const int j = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (j >= nchunks) return;
-    const size_t r = (size_t)t * nchunks + j;
+    const size_t r = (size_t)blockIdx.y * nchunks + j;
+    const int i0 = j * CK + lane * PER;
+    T wv[PER], dv[PER];
+    kpp_load<T, PER>(w, n, i0, wv);
+    kpp_load<T, PER>(D + (size_t)blockIdx.y * nd, n, i0, dv);
     const double Pj = P[r];
     const T Ts = (T)Pj;
     if (!(Pj > 0.0) || !isfinite(Ts) || Ts == T(0)) {
@@ -607,49 +859,216 @@ kpp_chunk_q_kernel(const T *w, const T *D, int n, int nchunks, const double *P,
         }
         return;
     }
-    Binade<T> b;
-    b.set(Ts);
-    const T *Dt = D + (size_t)t * n;
+    Grid<T> g;
+    g.set(Ts);
     // each lane composes 8 consecutive terms, then the lanes' runs in lane
     // order (a tree over neighbouring blocks of lanes)
-    Pf acc = pf_id();
+    Run<T> acc = Run<T>::id();
 #pragma unroll
-    for (int u = 0; u < CK / 32; ++u) {
-        const int i = j * CK + lane * (CK / 32) + u;
-        if (i < n) {
-            bool tie;
-            const unsigned long long q = b.qt(kpp_term(w[i], Dt[i]), tie);
-            acc = pf_cat(acc, pf_term(q, tie));
-        }
+    for (int u = 0; u < PER; ++u) {
+        bool tie;
+        // a term past the end is 0: no change
+        const typename Grid<T>::U k = g.term(kpp_term(wv[u], dv[u]), tie);
+        acc.add_term(k, tie);
     }
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-        const Pf y = Pf{__shfl_down_sync(0xffffffffu, acc.q0, off),
-                        __shfl_down_sync(0xffffffffu, acc.q1, off),
-                        __shfl_down_sync(0xffffffffu, acc.o, off)};
-        if ((lane & (2 * off - 1)) == 0) acc = pf_cat(acc, y);
+        const Run<T> y = Run<T>{__shfl_down_sync(0xffffffffu, acc.q0, off),
+                                __shfl_down_sync(0xffffffffu, acc.q1, off),
+                                __shfl_down_sync(0xffffffffu, acc.o, off)};
+        if ((lane & (2 * off - 1)) == 0) acc = Run<T>::cat(acc, y);
     }
     if (lane == 0) {
-        Q0[r] = acc.q0;
-        Q1[r] = acc.q1;
+        Q0[r] = Grid<T>::wide(acc.q0);
+        Q1[r] = Grid<T>::wide(acc.q1);
         Or[r] = acc.o;
-        Er[r] = b.ex;
+        Er[r] = FpTraits<T>::exponent(Ts);
     }
 }
 
-// The serial sum of candidate blockIdx.x over the chunk records (see above).
+// The serial sum of candidate blockIdx.x over the chunk records (see above),
+// in two parts.  Bound: latency, one block per candidate; the steps below are
+// what it waits for.
+//
+// Fast part.  A chunk whose successor has the same predicted binade is inner:
+// the sum is expected to stay in that binade through it.  The others -- about
+// one per doubling of the sum -- are borders.  One segmented scan over all
+// records gives the composition of the inner chunks before every border; the
+// borders' terms are brought to shared memory together.  One thread then steps
+// from border to border: the inner chunks in one addition (taken only when the
+// running sum is in their binade and stays there), the border chunk's 256
+// terms by 256 dependent additions (0.7 us: less than one block-wide scan to
+// find where the sum leaves its binade).  At 1M rows and seven candidates:
+// 30 us per centre; a block-wide scan per border and per serial step
+// took 93 us.
+//
+// Chunks before the first positive term are left out (their fp64 sums are 0).
+//
+// General part: from the chunk where the fast part stopped (a check that
+// failed, more borders than are kept), block-wide scans from one chunk that
+// cannot be added whole to the next, that chunk's terms serially.
+static constexpr int WALK_BORDERS = 32; // borders kept
+
+struct SegRun { // runs since the last border
+    Pf f;
+    int cut; // a border lies in this range
+};
+__device__ __forceinline__ SegRun seg_cat(const SegRun &a, const SegRun &b) {
+    return SegRun{b.cut ? b.f : pf_cat(a.f, b.f), a.cut | b.cut};
+}
+
+// s + m[0] + m[1] + ... + m[CK - 1], left to right in T (m in shared memory,
+// 16-byte aligned; zero terms change nothing).
+template <typename T> __device__ T serial_sum(T s, const T *m) {
+    constexpr int W = 16 / (int)sizeof(T);
+    struct __align__(16) V { T e[W]; };
+    const V *v = reinterpret_cast<const V *>(m);
+#pragma unroll 8
+    for (int c = 0; c < CK / W; ++c) {
+        const V x = v[c];
+#pragma unroll
+        for (int u = 0; u < W; ++u) s = add_rn(s, x.e[u]);
+    }
+    return s;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(WALK_THREADS)
-kpp_walk_kernel(const T *w, const T *D, int n, int nchunks, const unsigned long long *Q0,
-                const unsigned long long *Q1, const int *Or, const int *Er, double *cost) {
+kpp_walk_kernel(const T *w, const T *D, size_t nd, int n, int nchunks,
+                const unsigned long long *Q0, const unsigned long long *Q1, const int *Or,
+                const int *Er, const double *csum, double *cost) {
     __shared__ Pf shm[2 * (WALK_THREADS / 32) + 1];
     __shared__ int s_f;
     __shared__ T s_val;
+    __shared__ int s_border[WALK_BORDERS], s_ex[WALK_BORDERS];
+    __shared__ Pf s_run[WALK_BORDERS];
+    __shared__ int s_cnt[WALK_THREADS / 32];
+    __shared__ SegRun s_seg[WALK_THREADS / 32];
+    extern __shared__ __align__(16) unsigned char walk_sm[];
+    T *bt = reinterpret_cast<T *>(walk_sm); // [WALK_BORDERS][CK]: the borders' terms
     const int t = blockIdx.x;
-    const T *Dt = D + (size_t)t * n;
+    const T *Dt = D + (size_t)t * nd;
     const size_t ro = (size_t)t * nchunks;
-    T s = T(0);
-    int j = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int first = nchunks; // the first chunk with a positive term
+    for (int c = threadIdx.x; c < nchunks; c += WALK_THREADS)
+        if (!(csum[ro + c] == 0.0)) {
+            first = c;
+            break;
+        }
+    first = __reduce_min_sync(0xffffffffu, first);
+    if (lane == 0) s_cnt[warp] = first;
+    __syncthreads();
+    first = __reduce_min_sync(0xffffffffu, s_cnt[lane & (WALK_THREADS / 32 - 1)]);
+    if (first == nchunks) {
+        if (threadIdx.x == 0) cost[t] = 0.0;
+        return;
+    }
+    __syncthreads();
+    // ---- fast part: borders, in order, and the inner runs before them
+    int nb = 0;
+    {
+        // a thread's range of records, WALK_PER at a time: at(c, border, run)
+        const int per = (nchunks - first + WALK_THREADS - 1) / WALK_THREADS;
+        const int c0 = min(nchunks, first + (int)threadIdx.x * per), c1 = min(nchunks, c0 + per);
+        auto each = [&](auto &&at) {
+            for (int c = c0; c < c1; c += WALK_PER) {
+                Pf f[WALK_PER];
+                int ex[WALK_PER + 1];
+#pragma unroll
+                for (int u = 0; u < WALK_PER; ++u) {
+                    const int r = min(c + u, nchunks - 1);
+                    f[u] = Pf{Q0[ro + r], Q1[ro + r], Or[ro + r]};
+                    ex[u] = Er[ro + r];
+                }
+                ex[WALK_PER] = Er[ro + min(c + WALK_PER, nchunks - 1)];
+#pragma unroll
+                for (int u = 0; u < WALK_PER; ++u)
+                    if (c + u < c1)
+                        at(c + u, c + u + 1 == nchunks || ex[u] == NO_BINADE || ex[u + 1] != ex[u],
+                           f[u], ex[u]);
+            }
+        };
+        SegRun loc{pf_id(), 0};
+        int mine = 0;
+        each([&](int, bool border, const Pf &f, int) {
+            loc = border ? SegRun{pf_id(), 1} : SegRun{pf_cat(loc.f, f), loc.cut};
+            mine += border ? 1 : 0;
+        });
+        SegRun inc = loc;
+        int cinc = mine;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const SegRun y{pf_shfl_up(inc.f, off), __shfl_up_sync(0xffffffffu, inc.cut, off)};
+            const int cy = __shfl_up_sync(0xffffffffu, cinc, off);
+            if (lane >= off) {
+                inc = seg_cat(y, inc);
+                cinc += cy;
+            }
+        }
+        if (lane == 31) {
+            s_seg[warp] = inc;
+            s_cnt[warp] = cinc;
+        }
+        SegRun ex{pf_shfl_up(inc.f, 1), __shfl_up_sync(0xffffffffu, inc.cut, 1)};
+        if (lane == 0) ex = SegRun{pf_id(), 0};
+        __syncthreads();
+        SegRun before{pf_id(), 0};
+        int rank = cinc - mine;
+#pragma unroll
+        for (int v = 0; v < WALK_THREADS / 32; ++v) {
+            if (v < warp) {
+                before = seg_cat(before, s_seg[v]);
+                rank += s_cnt[v];
+            }
+            nb += s_cnt[v];
+        }
+        Pf run = seg_cat(before, ex).f;
+        each([&](int c, bool border, const Pf &f, int e) {
+            if (border) {
+                if (rank < WALK_BORDERS) {
+                    s_border[rank] = c;
+                    s_ex[rank] = e; // the inner chunks before c are in its binade
+                    s_run[rank] = run;
+                }
+                ++rank;
+                run = pf_id();
+            } else {
+                run = pf_cat(run, f);
+            }
+        });
+        nb = min(nb, WALK_BORDERS);
+        __syncthreads();
+        for (int e = threadIdx.x; e < nb * CK; e += WALK_THREADS) {
+            const int i = s_border[e / CK] * CK + e % CK;
+            bt[e] = i < n ? kpp_term(w[i], Dt[i]) : T(0);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        T sum = T(0);
+        int next = first; // the first chunk not yet added
+        for (int b = 0; b < nb && isfinite(sum); ++b) {
+            const int c = s_border[b];
+            if (c > next) { // inner chunks next .. c - 1, one binade
+                if (sum == T(0)) break;
+                Binade<T> bn;
+                bn.set(sum);
+                const unsigned long long R = sat_add(bn.s_int, pf_q(s_run[b], (int)(bn.s_int & 1ull)));
+                if (bn.ex != s_ex[b] || R >= bn.limit) break;
+                sum = bn.value(R);
+            }
+            sum = serial_sum<T>(sum, bt + (size_t)b * CK);
+            next = c + 1;
+        }
+        s_val = sum;
+        s_f = next;
+    }
+    __syncthreads();
+    // ---- general part
+    T s = s_val;
+    int j = s_f;
+    __syncthreads();
     while (j < nchunks && isfinite(s)) {
         Binade<T> b;
         b.ex = NO_BINADE - 1;
@@ -696,66 +1115,18 @@ kpp_walk_kernel(const T *w, const T *D, int n, int nchunks, const unsigned long 
             j += WALK_THREADS * WALK_PER;
             continue;
         }
-        // the records before f on the grid
+        // the records before f on the grid, then chunk j + f term by term
         if (mine == f) s_val = (f == 0) ? s : b.value(R_at);
+        const int c = j + f;
+        for (int e = threadIdx.x; e < CK; e += WALK_THREADS) {
+            const int i = c * CK + e;
+            bt[e] = i < n ? kpp_term(w[i], Dt[i]) : T(0);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_val = serial_sum<T>(s_val, bt);
         __syncthreads();
         s = s_val;
         __syncthreads();
-        // chunk j + f, term by term: ties by their parity rule, a serial
-        // step only where the sum leaves the binade (or a term does by itself)
-        const int c = j + f;
-        int pos = c * CK;
-        const int end = min(n, pos + CK);
-        const int i = pos + (int)threadIdx.x;
-        const T mi = ((int)threadIdx.x < CK && i < end) ? kpp_term(w[i], Dt[i]) : T(0);
-        while (pos < end && isfinite(s)) {
-            const bool in = (int)threadIdx.x < CK && i >= pos && i < end;
-            const T m = in ? mi : T(0);
-            if (s == T(0)) {
-                // 0 + m = m exactly: the first nonzero term starts the sum
-                if (threadIdx.x == 0) s_f = 0x7fffffff;
-                __syncthreads();
-                if (in && m != T(0)) atomicMin(&s_f, i);
-                __syncthreads();
-                const int p = s_f;
-                if (p == 0x7fffffff) {
-                    pos = end;
-                    break;
-                }
-                if (i == p) s_val = m;
-                __syncthreads();
-                s = s_val;
-                pos = p + 1;
-                __syncthreads();
-                continue;
-            }
-            Binade<T> bb;
-            bb.set(s);
-            const int pp = (int)(bb.s_int & 1ull);
-            bool tie = false;
-            const unsigned long long qv = in ? bb.qt(m, tie) : 0ull;
-            const Pf e = in ? pf_term(qv, tie) : pf_id();
-            Pf ex, tot;
-            block_scan_pf<WALK_THREADS>(e, shm, ex, tot);
-            const unsigned long long Rb = bb.s_int + pf_q(ex, pp);
-            const bool bad = in && (qv == SC_SAT || Rb + pf_q(e, pf_o(ex, pp)) >= bb.limit);
-            if (threadIdx.x == 0) s_f = 0x7fffffff;
-            __syncthreads();
-            if (bad) atomicMin(&s_f, i);
-            __syncthreads();
-            const int p = s_f;
-            if (p == 0x7fffffff) {
-                s = bb.value(bb.s_int + pf_q(tot, pp));
-                pos = end;
-                break;
-            }
-            // the terms before p on the grid, then term p serially in T
-            if (i == p) s_val = add_rn(bb.value(Rb), m);
-            __syncthreads();
-            s = s_val;
-            pos = p + 1;
-            __syncthreads();
-        }
         j = c + 1;
     }
     if (threadIdx.x == 0) cost[t] = (double)s;
@@ -775,24 +1146,39 @@ cudaError_t launch_kpp_dist_cost(const T *X, int ldx, int n, int d, const T *xno
     unsigned long long *Q1 = Q0 + (size_t)t * nch;
     int *Or = reinterpret_cast<int *>(Q1 + (size_t)t * nch);
     int *Er = Or + (size_t)t * nch;
-    // candidates' rows padded to 16 bytes, in shared memory when they fit
-    const int W = 16 / (int)sizeof(T);
-    const size_t want = (size_t)t * ((d + W - 1) / W * W) * sizeof(T);
-    if (want <= 96 * 1024) {
-        cudaError_t e = ensure_smem_limit(
-            reinterpret_cast<const void *>(kpp_dist_csum_kernel<T, true>), want);
-        if (e != cudaSuccess) return e;
-        kpp_dist_csum_kernel<T, true><<<nch, CK, want, s>>>(X, ldx, n, d, xnorm, cand, t, w, D,
-                                                            csum, nch, xinv, cosine);
+    const size_t nd = kpp_dist_stride(n, sizeof(T));
+    const size_t cand_bytes = (size_t)t * ldx * sizeof(T);
+    if (cand_bytes <= 96 * 1024) {
+        const int grid = std::min(nch, 148 * KD_BLOCKS);
+        for (int c0 = 0; c0 < t; c0 += 8) {
+            const int m = std::min(8, t - c0);
+            auto kern = m <= 4   ? kpp_dist_csum_kernel<T, 4>
+                        : m <= 6 ? kpp_dist_csum_kernel<T, 6>
+                                 : kpp_dist_csum_kernel<T, 8>;
+            const size_t smem = kd_smem<T>(m, ldx);
+            cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kern), smem);
+            if (e != cudaSuccess) return e;
+            kern<<<grid, KD_THREADS, smem, s>>>(X, ldx, n, xnorm, cand, c0, m, w, D, nd, csum, nch,
+                                                xinv, cosine);
+        }
     } else {
-        kpp_dist_csum_kernel<T, false><<<nch, CK, 0, s>>>(X, ldx, n, d, xnorm, cand, t, w, D, csum,
-                                                          nch, xinv, cosine);
+        kpp_dist_long_kernel<T><<<nch, CK, 0, s>>>(X, ldx, n, d, xnorm, cand, t, w, D, nd, csum,
+                                                   nch, xinv, cosine);
     }
     kpp_chunk_prefix_kernel<<<t, 1024, 0, s>>>(csum, nch, P);
-    kpp_chunk_q_kernel<T><<<dim3((nch + 7) / 8, t), 256, 0, s>>>(w, D, n, nch, P, Q0, Q1, Or,
+    kpp_chunk_q_kernel<T><<<dim3((nch + 7) / 8, t), 256, 0, s>>>(w, D, nd, n, nch, P, Q0, Q1, Or,
                                                                   Er);
-    kpp_walk_kernel<T><<<t, WALK_THREADS, 0, s>>>(w, D, n, nch, Q0, Q1, Or, Er, cost);
+    const size_t wsm = (size_t)WALK_BORDERS * CK * sizeof(T);
+    cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kpp_walk_kernel<T>), wsm);
+    if (e != cudaSuccess) return e;
+    kpp_walk_kernel<T><<<t, WALK_THREADS, wsm, s>>>(w, D, nd, n, nch, Q0, Q1, Or, Er, csum, cost);
     return cudaGetLastError();
+}
+
+// Elements from one candidate's distances to the next: rows start on 16 bytes.
+__host__ __device__ size_t kpp_dist_stride(int n, size_t elem) {
+    const size_t w = 16 / elem;
+    return ((size_t)n + w - 1) / w * w;
 }
 
 size_t kpp_cost_work_bytes(int n, int t) {
@@ -809,18 +1195,25 @@ kpp_select_update_kernel(T *w, const T *D, int n, const double *cost, const int 
                          int *chosen, int c, double *bs) {
     __shared__ double sh[KPP_THREADS / 32 + 1];
     __shared__ int s_best_t, s_best;
+    __shared__ double s_cost[KPP_TRIALS];
+    __shared__ int s_cand[KPP_TRIALS];
+    if ((int)threadIdx.x < nt) {
+        s_cost[threadIdx.x] = cost[threadIdx.x];
+        s_cand[threadIdx.x] = cand[threadIdx.x];
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         int bt = -1, best = 0;
         double bc = __longlong_as_double(0x7ff0000000000000ULL);
         for (int t = 0; t < nt; ++t) {
             bool rep = false;
-            for (int q = 0; q < t; ++q) rep = rep || cand[q] == cand[t];
+            for (int q = 0; q < t; ++q) rep = rep || s_cand[q] == s_cand[t];
             if (rep) continue;
-            const double ct = cost[t];
+            const double ct = s_cost[t];
             if (isfinite(ct) && ct < bc) {
                 bc = ct;
                 bt = t;
-                best = cand[t];
+                best = s_cand[t];
             }
         }
         s_best_t = bt;
@@ -829,9 +1222,28 @@ kpp_select_update_kernel(T *w, const T *D, int n, const double *cost, const int 
     }
     __syncthreads();
     const int bt = s_best_t, best = s_best;
-    const T *Dc = bt >= 0 ? D + (size_t)bt * n : nullptr;
+    const T *Dc = bt >= 0 ? D + (size_t)bt * kpp_dist_stride(n, sizeof(T)) : nullptr;
     const size_t base = (size_t)blockIdx.x * KPP_BLOCK + (size_t)threadIdx.x * KPP_PER_THREAD;
     double s = 0.0;
+    if (Dc && base + KPP_PER_THREAD <= (size_t)n) { // 16-byte loads and stores
+        constexpr int W = 16 / (int)sizeof(T);
+        struct __align__(16) V { T e[W]; };
+        T m[KPP_PER_THREAD], dv[KPP_PER_THREAD];
+        kpp_load<T, KPP_PER_THREAD>(w, n, (int)base, m);
+        kpp_load<T, KPP_PER_THREAD>(Dc, n, (int)base, dv);
+#pragma unroll
+        for (int j = 0; j < KPP_PER_THREAD; ++j) {
+            m[j] = (int)base + j == best ? T(0) : kpp_term(m[j], dv[j]);
+            s += (double)m[j];
+        }
+#pragma unroll
+        for (int v = 0; v < KPP_PER_THREAD / W; ++v) {
+            V o;
+#pragma unroll
+            for (int u = 0; u < W; ++u) o.e[u] = m[v * W + u];
+            reinterpret_cast<V *>(w + base)[v] = o;
+        }
+    } else
 #pragma unroll
     for (int j = 0; j < KPP_PER_THREAD; ++j) {
         const size_t i = base + j;
@@ -868,12 +1280,11 @@ cudaError_t launch_kpp_clamp(T *w, int n, int first, double *bs, int *flag, cuda
 
 template <typename T>
 cudaError_t launch_kpp_draw(const T *w, int n, const double *bs, const double *U, int nt,
-                            int force_exact, int *cand, int *unc, int *exact_count,
+                            int force_exact, int *cand, int *exact_count,
                             cudaStream_t s) {
     const int nb = kpp_num_blocks(n);
     kpp_draw_kernel<T><<<nt, KPP_THREADS, 0, s>>>(w, n, bs, nb, U, kpp_draw_bound(n), force_exact,
-                                                  cand, unc);
-    kpp_exact_kernel<T><<<1, KPP_THREADS, 0, s>>>(w, n, U, nt, cand, unc, exact_count);
+                                                  cand, exact_count);
     return cudaGetLastError();
 }
 
@@ -881,6 +1292,7 @@ template <typename T>
 cudaError_t launch_kpp_select_update(T *w, const T *D, int n, const double *cost,
                                      const int *cand, int nt, int *chosen, int c, double *bs,
                                      cudaStream_t s) {
+    if (nt > KPP_TRIALS) return cudaErrorInvalidValue;
     kpp_select_update_kernel<T><<<kpp_num_blocks(n), KPP_THREADS, 0, s>>>(w, D, n, cost, cand, nt,
                                                                           chosen, c, bs);
     return cudaGetLastError();
@@ -889,7 +1301,7 @@ cudaError_t launch_kpp_select_update(T *w, const T *D, int n, const double *cost
 #define B200_KPP_INST(T)                                                                       \
     template cudaError_t launch_kpp_clamp<T>(T *, int, int, double *, int *, cudaStream_t);     \
     template cudaError_t launch_kpp_draw<T>(const T *, int, const double *, const double *,     \
-                                            int, int, int *, int *, int *, cudaStream_t);       \
+                                            int, int, int *, int *, cudaStream_t);              \
     template cudaError_t launch_kpp_select_update<T>(T *, const T *, int, const double *,       \
                                                      const int *, int, int *, int, double *,    \
                                                      cudaStream_t);                             \
