@@ -127,7 +127,9 @@ template <typename T> struct NN : public AlgBase {
     da_status validate_queries(da_int nq, da_int d, const T *Xt, da_int ldt);
     // tensor-core path; `done` false when the plain path must run instead
     da_status kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_sqrt, bool cosine,
-                            bool &done);
+                            size_t &n_extra, bool &done);
+    da_status tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt, bool cosine,
+                        const int *extra, bool &redone);
     da_status compute_proba(da_int nq, da_int d, const T *Xt, da_int ldt, std::vector<T> &proba);
     // radius mode of predict / predict_proba (outlier handling as the reference)
     da_status radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T r, bool want_val,

@@ -139,6 +139,10 @@ struct KnnSelPlan {
 };
 bool knn_sel_plan(int n, int nq, int k, bool fp64, KnnSelPlan &pl);
 size_t knn_sel_bytes(const KnnSelPlan &pl, int nq, bool fp64);
+// Per query the k-th smallest of `groups` minima (k <= 256 for fp32), +inf
+// where fewer are finite.
+cudaError_t launch_knn_bound(const float *minima, int groups, int nq, int k, float *bound,
+                             cudaStream_t s);
 // out_key / out_idx as launch_knn_merge's; *flag is set to 1 when a query's
 // list overflowed or held fewer than k keys (its outputs are then unwritten).
 template <typename T>
@@ -153,9 +157,17 @@ cudaError_t launch_knn_select(const T *Q, int nq, const T *X, int nx, int ld, in
 // path's; queries the pass cannot certify are flagged in `fallback`
 // (*n_fallback of them) for the plain path.
 int knn_tc_supported(int nx, int d, int k);
-size_t knn_tc_list_cap();                   // list entries per query
-size_t knn_tc_query_bytes(int nq, int d);   // size of qbuf
-int *knn_tc_counts(void *qbuf, int nq, int d); // per-query list lengths inside qbuf
+// Sizes of its passes: sample rows (every step-th), row tiles of a sample work
+// item, minima per query; row tiles of a list work item; list entries per
+// query (8 bytes each).
+struct KnnTcPlan {
+    int n_sample, step, sample_tiles, groups, tiles, cap;
+};
+KnnTcPlan knn_tc_plan(int nx, int nq, int k);
+size_t knn_tc_query_bytes(int nq, int ldbf, const KnnTcPlan &pl); // size of qbuf
+// state words: [0] queries flagged, [1] error code, [2] lists that overflowed,
+// [4] lists short of k
+constexpr int KNN_TC_STATE = 8;
 // dst[i] = src[idx[i]] (rows of ld floats); out[idx[i]] = (key, ind)[i] (rows of k)
 cudaError_t launch_rows_gather(const float *src, int ld, const int *idx, int m, float *dst,
                                cudaStream_t s);
@@ -172,8 +184,8 @@ struct KnnTcCosine {
 cudaError_t launch_recip(const float *v, int n, float *out, cudaStream_t s);
 cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const float *xnorm2,
                           const float *xmax, int nx, int ld, int ldbf, int d, const float *Q,
-                          int nq, int k, int kc, int take_sqrt, void *qbuf, void *list,
-                          int *fallback, int *n_fallback, int *err, float *out_key,
+                          int nq, int k, int kc, int take_sqrt, const KnnTcPlan &pl, void *qbuf,
+                          void *list, int *fallback, int *cnt, int *state, float *out_key,
                           int *out_idx, cudaStream_t s, const KnnTcCosine *cosine = nullptr);
 
 // ------------------------------------------------------------- k-means ---

@@ -291,12 +291,12 @@ template <typename T> da_status NN<T>::ensure_device_data() {
 }
 
 // Tensor-core candidate pass + exact re-score (knn_tc.cu) into dOutK / dOutI,
-// in query batches that bound the candidate lists' memory.  Any query the
-// pass could not certify sends the whole call to the plain path (done =
-// false).
+// in query batches that bound the candidate lists' memory; n_extra ints of
+// state follow the indices, for tc_finish.
+static constexpr da_int KNN_TC_BATCH = 16384;
 template <typename T>
 da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_sqrt,
-                                bool cosine, bool &done) {
+                                bool cosine, size_t &n_extra, bool &done) {
     done = false;
     if constexpr (std::is_same_v<T, float>) {
         cudaStream_t st = cuda->stream;
@@ -330,108 +330,38 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
                      "tensor-core training copies");
             tc_train_ready = true;
         }
-        const da_int QB = 16384;
-        const da_int qb = std::min(nq, QB);
-        if (!dTkQ.ensure(knn_tc_query_bytes((int)qb, (int)d)) ||
-            !dTkList.ensure((size_t)qb * knn_tc_list_cap() * 8) ||
-            !dTkFlag.ensure((size_t)qb * sizeof(int)) ||
+        // batches of queries; their state words and list lengths follow the
+        // indices and come back with them (tc_finish)
+        const da_int qb = std::min<da_int>(nq, KNN_TC_BATCH);
+        const int batches = (int)((nq + KNN_TC_BATCH - 1) / KNN_TC_BATCH);
+        const KnnTcPlan pl = knn_tc_plan((int)n_samples, (int)qb, (int)k);
+        n_extra = (size_t)batches * KNN_TC_STATE + (size_t)nq;
+        if (!dTkQ.ensure(knn_tc_query_bytes((int)qb, ldbf, pl)) ||
+            !dTkList.ensure((size_t)qb * pl.cap * 8) || !dTkFlag.ensure((size_t)nq * sizeof(int)) ||
             !dOutK.ensure((size_t)nq * k * sizeof(float)) ||
-            !dOutI.ensure((size_t)nq * k * sizeof(int)))
+            !dOutI.ensure(((size_t)nq * k + n_extra) * sizeof(int)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
-        int *n_fb = reinterpret_cast<int *>(dTkScal.as<char>() + 16);
-        int *errf = n_fb + 1;
-        int h_state[5] = {0, 0, 0, 0, 0};
-        for (da_int q0 = 0; q0 < nq; q0 += QB) {
-            const da_int nb = std::min(QB, nq - q0);
+        int *state = dOutI.as<int>() + (size_t)nq * k;
+        int *counts = state + (size_t)batches * KNN_TC_STATE;
+        for (da_int q0 = 0; q0 < nq; q0 += KNN_TC_BATCH, state += KNN_TC_STATE) {
+            const da_int nb = std::min<da_int>(KNN_TC_BATCH, nq - q0);
             const KnnTcCosine cs{dXn.as<float>(), dXinv.as<float>(),
                                  cosine ? dQn.as<float>() + q0 : nullptr};
+            // a last batch that fits one M tile has its own sizes
+            const KnnTcPlan pb = nb == qb ? pl : knn_tc_plan((int)n_samples, (int)nb, (int)k);
+            if (!dTkQ.ensure(knn_tc_query_bytes((int)nb, ldbf, pb)) ||
+                !dTkList.ensure((size_t)nb * pb.cap * 8))
+                return err->error(da_status_memory_error, "Device memory allocation failed.");
             B200_TRY(cuda->timed("knn_tc", [&] {
                 return launch_knn_tc(dX.as<float>(), dXh.p, dXl.p, dXsq.as<float>(),
                                      dTkScal.as<float>(), (int)n_samples, ld, tc_ldbf, (int)d,
                                      dQ.as<float>() + (size_t)q0 * ld, (int)nb, (int)k, kc,
-                                     take_sqrt ? 1 : 0, dTkQ.p, dTkList.p, dTkFlag.as<int>(),
-                                     n_fb, errf, dOutK.as<float>() + (size_t)q0 * k,
+                                     take_sqrt ? 1 : 0, pb, dTkQ.p, dTkList.p,
+                                     dTkFlag.as<int>() + q0, counts + q0, state,
+                                     dOutK.as<float>() + (size_t)q0 * k,
                                      dOutI.as<int>() + (size_t)q0 * k, st,
                                      cosine ? &cs : nullptr);
             }), "kNN tensor-core pass");
-            B200_TRY(cudaMemcpyAsync(h_state, n_fb, 5 * sizeof(int), cudaMemcpyDeviceToHost, st),
-                     "copy");
-            std::vector<int> lens((size_t)nb);
-            B200_TRY(cudaMemcpyAsync(lens.data(), knn_tc_counts(dTkQ.p, (int)nb, (int)d),
-                                     lens.size() * sizeof(int), cudaMemcpyDeviceToHost, st),
-                     "copy");
-            B200_TRY(cudaStreamSynchronize(st), "kNN tensor-core pass");
-            double mx = 0, sum = 0;
-            for (int v : lens) {
-                mx = std::max(mx, (double)v);
-                sum += v;
-            }
-            cuda->stats["knn_tc_max_list"] = std::max(cuda->stats["knn_tc_max_list"], mx);
-            cuda->stats["knn_tc_mean_list"] = sum / std::max<double>(1.0, (double)nb);
-            if (h_state[1] != 0)
-                return err->error(da_status_internal_error,
-                                  "The tensor-core kNN kernel timed out waiting on a pipeline "
-                                  "barrier (code " + std::to_string(h_state[1]) + ").");
-            cuda->stats["knn_tc_fallback_queries"] += (double)h_state[0];
-            cuda->stats["knn_tc_fallback_list_overflow"] += (double)h_state[2];
-            cuda->stats["knn_tc_fallback_many_survivors"] += (double)h_state[3];
-            cuda->stats["knn_tc_fallback_few_survivors"] += (double)h_state[4];
-            if (h_state[0] != 0) {
-                // the queries the pass could not certify: the plain path on
-                // just those rows (gathered, searched, scattered back)
-                std::vector<int> flags((size_t)nb), idx;
-                B200_TRY(cudaMemcpyAsync(flags.data(), dTkFlag.p, flags.size() * sizeof(int),
-                                         cudaMemcpyDeviceToHost, st), "copy");
-                B200_TRY(cudaStreamSynchronize(st), "copy");
-                for (int i = 0; i < (int)nb; ++i)
-                    if (flags[i]) idx.push_back(i);
-                const int m = (int)idx.size();
-                const int BN = knn_tile_rows_train(false);
-                const int q_tiles = (m + 63) / 64;
-                const int max_chunks = std::max(1, (int)((n_samples + BN - 1) / BN));
-                // enough CTAs to fill the GPU, but at most ~16K partial entries per query
-                // (the merge ranks every entry against every chunk list)
-                int n_chunks = std::max(1, std::min({max_chunks, (148 * 8 + q_tiles - 1) / q_tiles,
-                                                     std::max(8, 16384 / (int)k)}));
-                int chunk_rows = (int)((n_samples + n_chunks - 1) / n_chunks);
-                chunk_rows = ((chunk_rows + BN - 1) / BN) * BN;
-                n_chunks = (int)((n_samples + chunk_rows - 1) / chunk_rows);
-                // scratch inside the (now free) candidate-list buffer
-                const size_t parts = (size_t)m * n_chunks * k;
-                const size_t need = (size_t)m * 4 + (size_t)m * ld * 4 + parts * 8 +
-                                    (size_t)m * k * 8 + (size_t)m * 4 + 1280;
-                if (!dTkList.ensure(need))
-                    return err->error(da_status_memory_error, "Device memory allocation failed.");
-                char *p = dTkList.as<char>();
-                int *didx = reinterpret_cast<int *>(p);
-                float *qsub = reinterpret_cast<float *>(p + ((size_t)m * 4 + 255) / 256 * 256);
-                float *pk = qsub + (size_t)m * ld;
-                int *pi = reinterpret_cast<int *>(pk + parts);
-                float *ok = reinterpret_cast<float *>(pi + parts);
-                int *oi = reinterpret_cast<int *>(ok + (size_t)m * k);
-                float *qnsub = reinterpret_cast<float *>(oi + (size_t)m * k);
-                KnnArgs pa{cosine ? ACC_DOT : ACC_SQEUC, cosine ? POST_COSINE : POST_NONE, kc, 2.0,
-                           (int)k, chunk_rows, n_chunks};
-                B200_TRY(cudaMemcpyAsync(didx, idx.data(), (size_t)m * 4, cudaMemcpyHostToDevice,
-                                         st), "copy");
-                B200_TRY(launch_rows_gather(dQ.as<float>() + (size_t)q0 * ld, ld, didx, m, qsub,
-                                            st), "gather");
-                if (cosine)
-                    B200_TRY(launch_rows_gather(dQn.as<float>() + q0, 1, didx, m, qnsub, st),
-                             "gather");
-                B200_TRY(launch_knn_chunks<float>(qsub, ld, m, dX.as<float>(), ld,
-                                                  (int)n_samples, (int)d,
-                                                  cosine ? qnsub : nullptr,
-                                                  cosine ? dXn.as<float>() : nullptr, pa, pk,
-                                                  pi, nullptr, st), "kNN distance kernel");
-                B200_TRY(launch_knn_merge<float>(pk, pi, m, n_chunks, (int)k,
-                                                 take_sqrt && !cosine ? 1 : 0, ok, oi, st),
-                         "kNN merge kernel");
-                B200_TRY(launch_results_scatter(ok, oi, didx, m, (int)k,
-                                                dOutK.as<float>() + (size_t)q0 * k,
-                                                dOutI.as<int>() + (size_t)q0 * k, st), "scatter");
-                B200_TRY(cudaStreamSynchronize(st), "kNN fallback");
-            }
         }
         cuda->stats["tensor_core"] = 1.0;
         done = true;
@@ -442,6 +372,92 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
         (void)kc;
         (void)take_sqrt;
         (void)cosine;
+        (void)n_extra;
+    }
+    return da_status_success;
+}
+
+// The state words and list lengths of a tensor-core search (`extra`, as
+// kneighbors_tc laid them out): statistics, errors, and the flagged queries
+// searched on the plain path into dOutK / dOutI (`redone`).
+template <typename T>
+da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt, bool cosine,
+                           const int *extra, bool &redone) {
+    redone = false;
+    if constexpr (std::is_same_v<T, float>) {
+        cudaStream_t st = cuda->stream;
+        const int batches = (int)((nq + KNN_TC_BATCH - 1) / KNN_TC_BATCH);
+        const int *lens = extra + (size_t)batches * KNN_TC_STATE;
+        double mx = 0, sum = 0;
+        int flagged = 0;
+        for (int b = 0; b < batches; ++b) {
+            const int *h = extra + (size_t)b * KNN_TC_STATE;
+            if (h[1] != 0)
+                return err->error(da_status_internal_error,
+                                  "The tensor-core kNN kernel timed out waiting on a pipeline "
+                                  "barrier (code " + std::to_string(h[1]) + ").");
+            flagged += h[0];
+            cuda->stats["knn_tc_fallback_queries"] += (double)h[0];
+            cuda->stats["knn_tc_fallback_list_overflow"] += (double)h[2];
+            cuda->stats["knn_tc_fallback_few_survivors"] += (double)h[4];
+        }
+        for (da_int i = 0; i < nq; ++i) {
+            mx = std::max(mx, (double)lens[i]);
+            sum += lens[i];
+        }
+        cuda->stats["knn_tc_max_list"] = std::max(cuda->stats["knn_tc_max_list"], mx);
+        cuda->stats["knn_tc_mean_list"] = sum / std::max<double>(1.0, (double)nq);
+        if (flagged == 0) return da_status_success;
+        // the queries the pass could not certify: the plain path on just those
+        // rows (gathered, searched, scattered back)
+        redone = true;
+        std::vector<int> flags((size_t)nq), idx;
+        B200_TRY(cudaMemcpyAsync(flags.data(), dTkFlag.p, flags.size() * sizeof(int),
+                                 cudaMemcpyDeviceToHost, st), "copy");
+        B200_TRY(cudaStreamSynchronize(st), "copy");
+        for (int i = 0; i < (int)nq; ++i)
+            if (flags[i]) idx.push_back(i);
+        const int m = (int)idx.size();
+        const int BN = knn_tile_rows_train(false);
+        const int q_tiles = (m + 63) / 64;
+        const int max_chunks = std::max(1, (int)((n_samples + BN - 1) / BN));
+        // enough CTAs to fill the GPU, but at most ~16K partial entries per query
+        // (the merge ranks every entry against every chunk list)
+        int n_chunks = std::max(1, std::min({max_chunks, (148 * 8 + q_tiles - 1) / q_tiles,
+                                             std::max(8, 16384 / (int)k)}));
+        int chunk_rows = (int)((n_samples + n_chunks - 1) / n_chunks);
+        chunk_rows = ((chunk_rows + BN - 1) / BN) * BN;
+        n_chunks = (int)((n_samples + chunk_rows - 1) / chunk_rows);
+        // scratch inside the (now free) candidate-list buffer
+        const size_t parts = (size_t)m * n_chunks * k;
+        const size_t need = (size_t)m * 4 + (size_t)m * ld * 4 + parts * 8 +
+                            (size_t)m * k * 8 + (size_t)m * 4 + 1280;
+        if (!dTkList.ensure(need))
+            return err->error(da_status_memory_error, "Device memory allocation failed.");
+        char *p = dTkList.as<char>();
+        int *didx = reinterpret_cast<int *>(p);
+        float *qsub = reinterpret_cast<float *>(p + ((size_t)m * 4 + 255) / 256 * 256);
+        float *pk = qsub + (size_t)m * ld;
+        int *pi = reinterpret_cast<int *>(pk + parts);
+        float *ok = reinterpret_cast<float *>(pi + parts);
+        int *oi = reinterpret_cast<int *>(ok + (size_t)m * k);
+        float *qnsub = reinterpret_cast<float *>(oi + (size_t)m * k);
+        KnnArgs pa{cosine ? ACC_DOT : ACC_SQEUC, cosine ? POST_COSINE : POST_NONE, kc, 2.0, (int)k,
+                   chunk_rows, n_chunks};
+        B200_TRY(cudaMemcpyAsync(didx, idx.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st),
+                 "copy");
+        B200_TRY(launch_rows_gather(dQ.as<float>(), ld, didx, m, qsub, st), "gather");
+        if (cosine) B200_TRY(launch_rows_gather(dQn.as<float>(), 1, didx, m, qnsub, st), "gather");
+        B200_TRY(launch_knn_chunks<float>(qsub, ld, m, dX.as<float>(), ld, (int)n_samples, (int)d,
+                                          cosine ? qnsub : nullptr,
+                                          cosine ? dXn.as<float>() : nullptr, pa, pk, pi, nullptr,
+                                          st), "kNN distance kernel");
+        B200_TRY(launch_knn_merge<float>(pk, pi, m, n_chunks, (int)k, take_sqrt && !cosine ? 1 : 0,
+                                         ok, oi, st), "kNN merge kernel");
+        B200_TRY(launch_results_scatter(ok, oi, didx, m, (int)k, dOutK.as<float>(),
+                                        dOutI.as<int>(), st), "scatter");
+    } else {
+        (void)nq, (void)d, (void)k, (void)kc, (void)take_sqrt, (void)cosine, (void)extra;
     }
     return da_status_success;
 }
@@ -528,26 +544,33 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
     cuda->stats["knn_tc_fallback_many_survivors"] = 0.0;
     cuda->stats["knn_tc_fallback_few_survivors"] = 0.0;
     bool tc_done = false;
+    size_t n_extra = 0; // ints after the indices: tc_finish's, or the flags below
     const bool tc_metric = metric == M_EUC || metric == M_SQEUC || metric == M_COS ||
                            (metric == M_MINK && p == T(2));
+    // The tensor-core pass from about 5e8 multiply-adds on (a batch counts at
+    // least 64 queries, one tile of either path): there it takes 100 us where
+    // the plain path takes 155 (65,536 x 32, 256 queries, k = 10; 75 against
+    // 194 at 200,000 x 64, one query; 215 against 294 at 16,384 x 32, 2,048
+    // queries).  Below, its five launches are no shorter and its bf16 copies
+    // and lists are more to set up.
     if (!fp64 && tc_metric && opts.key("precision mode") != 0 &&
-        knn_tc_supported((int)n_samples, (int)d, (int)k) && n_samples >= 65536 &&
-        (double)n_samples * (double)std::max<da_int>(nq, 256) * (double)d >= 4.0e9) {
+        knn_tc_supported((int)n_samples, (int)d, (int)k) && n_samples >= 16384 &&
+        (double)n_samples * (double)std::max<da_int>(nq, 64) * (double)d >= 5.0e8) {
         s = kneighbors_tc(nq, d, k, kc, metric != M_SQEUC && metric != M_COS, metric == M_COS,
-                          tc_done);
+                          n_extra, tc_done);
         if (s != da_status_success) return s;
     }
     // the plain path: bounds first (launch_knn_select) in query batches of at
     // most 256 MB of lists, each with its own flag after the indices; running
     // lists (run_lists) where that does not apply or a flag comes back set
     KnnSelPlan sel{};
-    da_int sel_qb = 0, n_flags = 0;
+    da_int sel_qb = 0;
     std::function<da_status()> run_lists;
     if (!tc_done) {
         if (knn_sel_plan((int)n_samples, (int)std::min<da_int>(nq, 65536), (int)k, fp64, sel)) {
             const size_t per = knn_sel_bytes(sel, 1, fp64);
             sel_qb = std::min(nq, (da_int)std::max<size_t>(64, ((size_t)1 << 28) / per / 64 * 64));
-            n_flags = (nq + sel_qb - 1) / sel_qb;
+            n_extra = (size_t)((nq + sel_qb - 1) / sel_qb);
         }
         const T *qn = nullptr, *xn = nullptr;
         if (norm_kind >= 0) {
@@ -571,9 +594,9 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
                               "k = " + std::to_string(k) + " exceeds the largest supported number "
                               "of neighbours per query (" + std::to_string(knn_max_k(fp64)) + ").");
         if (!dOutK.ensure((size_t)nq * k * sizeof(T)) ||
-            !dOutI.ensure(((size_t)nq * k + n_flags) * sizeof(int)))
+            !dOutI.ensure(((size_t)nq * k + n_extra) * sizeof(int)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
-        if (n_flags > 0) {
+        if (n_extra > 0) {
             const KnnArgs a{acc, post, kc, (double)p, (int)k, 0, 0};
             if (!dPartK.ensure(knn_sel_bytes(sel, (int)sel_qb, fp64)))
                 return err->error(da_status_memory_error, "Device memory allocation failed.");
@@ -617,15 +640,15 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             }), "kNN merge kernel");
             return da_status_success;
         };
-        if (n_flags == 0) {
+        if (n_extra == 0) {
             s = run_lists();
             if (s != da_status_success) return s;
         }
     }
     ind.resize((size_t)nq * k);
-    std::vector<int> tmp((size_t)nq * k + n_flags);
+    std::vector<int> tmp((size_t)nq * k + n_extra);
     for (;;) {
-        B200_TRY(cudaMemcpyAsync(tmp.data(), dOutI.p, ((size_t)nq * k + n_flags) * sizeof(int),
+        B200_TRY(cudaMemcpyAsync(tmp.data(), dOutI.p, ((size_t)nq * k + n_extra) * sizeof(int),
                                  cudaMemcpyDeviceToHost, st),
                  "download");
         if (dist) {
@@ -634,14 +657,22 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
                                      cudaMemcpyDeviceToHost, st), "download");
         }
         B200_TRY(cudaStreamSynchronize(st), "kNN");
-        const bool again = std::any_of(tmp.begin() + (size_t)nq * k, tmp.begin() + (size_t)nq * k + n_flags,
-                                       [](int f) { return f != 0; });
-        if (!again) break;
-        // a query's list overflowed or was short of k keys
-        cuda->stats["knn_select_fallback"] += 1.0;
-        n_flags = 0;
-        s = run_lists();
-        if (s != da_status_success) return s;
+        if (n_extra == 0) break;
+        const int *extra = tmp.data() + (size_t)nq * k;
+        if (tc_done) {
+            bool redone = false;
+            s = tc_finish(nq, d, k, kc, metric != M_SQEUC && metric != M_COS, metric == M_COS,
+                          extra, redone);
+            if (s != da_status_success) return s;
+            if (!redone) break;
+        } else {
+            if (std::all_of(extra, extra + n_extra, [](int f) { return f == 0; })) break;
+            // a query's list overflowed or was short of k keys
+            cuda->stats["knn_select_fallback"] += 1.0;
+            s = run_lists();
+            if (s != da_status_success) return s;
+        }
+        n_extra = 0;
     }
     for (size_t i = 0; i < ind.size(); ++i) ind[i] = (da_int)tmp[i];
     return da_status_success;

@@ -95,6 +95,29 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
             smem_u32(bar))
         : "memory");
 }
+// 32 lanes x 32 columns of fp32 from TMEM, without waiting: v holds the values
+// after tmem_ld_wait (which names v, so that no use moves before it).
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, float (&v)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),
+                   "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]),
+                   "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]),
+                   "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
+                   "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]),
+                   "=f"(v[30]), "=f"(v[31])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait(float (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]),
+                   "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]),
+                   "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]), "+f"(v[17]),
+                   "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]),
+                   "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]),
+                   "+f"(v[30]), "+f"(v[31])::"memory");
+}
 // 32 lanes x 32 columns of fp32 from TMEM (lane = thread of the warp).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
@@ -161,15 +184,16 @@ inline EncodeTiledFn tensor_map_encoder() {
 }
 
 // 2-D bf16 row-major matrix (rows x cols, cols a multiple of 64), box of
-// 64 columns (128 bytes, 128-byte swizzle) x box_rows rows (<= 256).
+// 64 columns (128 bytes, 128-byte swizzle) x box_rows rows (<= 256); `step`
+// matrix rows from one row of the map to the next.
 inline bool make_map_bf16_rows(CUtensorMap *m, const void *ptr, int rows, int cols,
-                               int box_rows) {
+                               int box_rows, int step = 1) {
     EncodeTiledFn enc = tensor_map_encoder();
     // rows of any multiple of 8 elements (16 bytes) from 64 up; a 64-column
     // box past the last column reads zeros
     if (!enc || !ptr || box_rows > 256 || cols % 8 != 0 || cols < 64) return false;
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * 2 * (cuuint64_t)step};
     cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box,
