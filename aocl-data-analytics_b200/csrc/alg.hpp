@@ -72,7 +72,13 @@ template <typename T> struct NN : public AlgBase {
     bool classes_done = false;
     // device
     int ld = 0;
-    DevBuf dX, dXn, dQ, dQn, dPartK, dPartI, dOutK, dOutI, dStage;
+    DevBuf dX, dXn, dQ, dQn, dPartK, dPartI, dStage;
+    // a search's nq x k keys, their nk indices, then state words (kneighbors_compute)
+    DevBuf dOutK;
+    static size_t out_bytes(size_t nk, size_t n_extra) {
+        return nk * sizeof(T) + (nk + n_extra) * sizeof(int);
+    }
+    int *out_idx(size_t nk) const { return reinterpret_cast<int *>(dOutK.as<T>() + nk); }
     int xn_kind = -1; // which norms dXn holds: 0 squared, 1 eps1-norm
     // tensor-core candidate pass (fp32 euclidean, cosine): bf16 hi/lo copies
     // of the training rows, their fp32 |x|^2 and max |x|, 1 / |x| (cosine);
@@ -121,8 +127,14 @@ template <typename T> struct NN : public AlgBase {
     da_status load_state(ByteReader &r) override;
 
     // core: q-major results (n_ind[q*k + r]) on the host
+    // (to: the caller's arrays instead, in the storage order ord)
+    struct KnnOut {
+        da_int *ind;
+        T *dist; // or null
+    };
     da_status kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt, da_order ord,
-                                 da_int k, std::vector<da_int> &ind, std::vector<T> *dist);
+                                 da_int k, std::vector<da_int> &ind, std::vector<T> *dist,
+                                 const KnnOut *to = nullptr);
     da_status ensure_device_data();
     da_status validate_queries(da_int nq, da_int d, const T *Xt, da_int ldt);
     // tensor-core path; `done` false when the plain path must run instead

@@ -12,19 +12,21 @@ namespace b200 {
 template <typename T>
 cudaError_t upload_matrix(da_order order, da_int rows, da_int cols, const T *host, da_int ld,
                           T *dst, int ldo, DevBuf &stage, cudaStream_t s) {
-    cudaError_t e;
+    const size_t z = sizeof(T);
+    T *const from = const_cast<T *>(host); // read only
     if (order == row_major) {
-        e = cudaMemcpy2DAsync(dst, (size_t)ldo * sizeof(T), host, (size_t)ld * sizeof(T),
-                              (size_t)cols * sizeof(T), rows, cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) return e;
-        if (ldo > cols)
-            e = cudaMemset2DAsync(dst + cols, (size_t)ldo * sizeof(T), 0,
-                                  (size_t)(ldo - cols) * sizeof(T), rows, s);
-        return e;
+        const XferSeg seg{from, ld * z, dst, ldo * z, cols * z, (size_t)rows};
+        cudaError_t e = cudaSuccess;
+        if (xfer_up(&seg, 1, s, e)) return e;
+        if (ld != cols || ldo == cols || rows < 16) return copy_up(seg, s);
+        // dense rows padded on the device: one copy of all of them and a kernel
+        // (a driver's copy row by row moves 0.8 GB/s)
+        if (!stage.ensure((size_t)rows * cols * z)) return cudaErrorMemoryAllocation;
+        e = cudaMemcpyAsync(stage.p, host, (size_t)rows * cols * z, cudaMemcpyHostToDevice, s);
+        return e == cudaSuccess ? launch_pad_rows<T>(stage.as<T>(), rows, cols, dst, ldo, s) : e;
     }
-    if (!stage.ensure((size_t)rows * cols * sizeof(T))) return cudaErrorMemoryAllocation;
-    e = cudaMemcpy2DAsync(stage.p, (size_t)rows * sizeof(T), host, (size_t)ld * sizeof(T),
-                          (size_t)rows * sizeof(T), cols, cudaMemcpyHostToDevice, s);
+    if (!stage.ensure((size_t)rows * cols * z)) return cudaErrorMemoryAllocation;
+    const cudaError_t e = copy_up({from, ld * z, stage.p, rows * z, rows * z, (size_t)cols}, s);
     if (e != cudaSuccess) return e;
     return launch_colmajor_to_rowmajor<T>(stage.as<T>(), rows, cols, dst, ldo, s);
 }
@@ -242,14 +244,10 @@ da_status pairwise(da_order order, da_int m, da_int n, da_int k, const T *X, da_
     PairwiseArgs a{acc, post, kc, (double)p, x_is_y, order == row_major};
     if (!ok(launch_pairwise<T>(g_X.as<T>(), ld, m, g_Y.as<T>(), ld, n, k, xn, yn, a, g_D.as<T>(), st)))
         return da_status_internal_error;
-    cudaError_t e;
-    if (order == row_major)
-        e = cudaMemcpy2DAsync(D, (size_t)ldd * sizeof(T), g_D.p, (size_t)n * sizeof(T),
-                              (size_t)n * sizeof(T), m, cudaMemcpyDeviceToHost, st);
-    else
-        e = cudaMemcpy2DAsync(D, (size_t)ldd * sizeof(T), g_D.p, (size_t)m * sizeof(T),
-                              (size_t)m * sizeof(T), n, cudaMemcpyDeviceToHost, st);
-    if (!ok(e) || !ok(cudaStreamSynchronize(st))) return da_status_internal_error;
+    const size_t row = (size_t)(order == row_major ? n : m) * sizeof(T);
+    if (!ok(copy_down({D, (size_t)ldd * sizeof(T), g_D.p, row, row,
+                       (size_t)(order == row_major ? m : n)}, st)))
+        return da_status_internal_error;
     return da_status_success;
 }
 
@@ -651,7 +649,18 @@ da_status da_b200_set_stream(da_handle h, void *stream) {
     h->err.clear();
     da_status s = h->cuda.init(h->err);
     if (s != da_status_success) return s;
-    h->cuda.stream = stream ? static_cast<cudaStream_t>(stream) : h->cuda.own_stream;
+    const cudaStream_t to = stream ? static_cast<cudaStream_t>(stream) : h->cuda.own_stream;
+    if (to != h->cuda.stream && h->cuda.stream == h->cuda.own_stream) {
+        // an upload of set_data may still be in flight on the handle's own
+        // stream, which the new one does not wait for (the new one may be
+        // under capture)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaStreamSynchronize(h->cuda.own_stream);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return cuda_status(h->err, e, "stream");
+    }
+    h->cuda.stream = to;
     return da_status_success;
 }
 da_status da_b200_set_stream_priority(da_handle h, da_int priority) {

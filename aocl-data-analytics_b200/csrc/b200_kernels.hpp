@@ -40,6 +40,9 @@ enum PostKind : int {
 
 // ---------------------------------------------------------------- ingest --
 // Dense column-major (rows x cols, ld = rows) -> padded row-major (rows x ldo).
+// Dense rows of cols elements to rows of ldo (pad zero).
+template <typename T>
+cudaError_t launch_pad_rows(const T *src, int rows, int cols, T *dst, int ldo, cudaStream_t s);
 template <typename T>
 cudaError_t launch_colmajor_to_rowmajor(const T *src, int rows, int cols, T *dst, int ldo,
                                         cudaStream_t s);

@@ -502,6 +502,21 @@ __global__ void colmajor_to_rowmajor_kernel(const T *src, int rows, int cols, T 
         if (r < rows && c < ldo) dst[(size_t)r * ldo + c] = (c < cols) ? tile[threadIdx.x][y] : T(0);
     }
 }
+// Dense rows (cols elements) to rows of ldo, the rest zero.
+template <typename T>
+__global__ void pad_rows_kernel(const T *src, size_t rows, int cols, T *dst, int ldo) {
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= rows * ldo) return;
+    const size_t r = e / ldo;
+    const int c = (int)(e - r * ldo);
+    dst[e] = c < cols ? src[r * cols + c] : T(0);
+}
+template <typename T>
+cudaError_t launch_pad_rows(const T *src, int rows, int cols, T *dst, int ldo, cudaStream_t s) {
+    const size_t n = (size_t)rows * ldo;
+    pad_rows_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, (size_t)rows, cols, dst, ldo);
+    return cudaGetLastError();
+}
 template <typename T>
 __global__ void rowmajor_to_colmajor_kernel(const T *src, int rows, int cols, int ldi, T *dst,
                                             long ldc) {
@@ -547,7 +562,8 @@ cudaError_t launch_rowmajor_to_colmajor(const T *src, int rows, int cols, int ld
     template cudaError_t launch_colmajor_to_rowmajor<T>(const T *, int, int, T *, int,         \
                                                         cudaStream_t);                         \
     template cudaError_t launch_rowmajor_to_colmajor<T>(const T *, int, int, int, T *, long,   \
-                                                        cudaStream_t);
+                                                        cudaStream_t);                         \
+    template cudaError_t launch_pad_rows<T>(const T *, int, int, T *, int, cudaStream_t);
 B200_INST(float)
 B200_INST(double)
 

@@ -2,6 +2,7 @@
 // registry, device buffers and the per-handle CUDA context.
 #pragma once
 #include "device_alloc.hpp"
+#include "host_xfer.hpp"
 #include <cstdlib>
 #include <mutex>
 #include "../../include/aoclda_b200.h"
@@ -519,6 +520,18 @@ inline da_status check_2d(ErrorRecord &err, da_order order, da_int n_rows, da_in
             }
     }
     return da_status_success;
+}
+
+// n device ints into the caller's da_int array (synchronises).
+inline cudaError_t download_ints(const int *dev, size_t n, da_int *out, cudaStream_t s) {
+    if (sizeof(da_int) == sizeof(int))
+        return copy_down({out, n * sizeof(int), const_cast<int *>(dev), n * sizeof(int),
+                          n * sizeof(int), 1}, s);
+    std::vector<int> tmp(n);
+    const cudaError_t e = copy_down({tmp.data(), n * sizeof(int), const_cast<int *>(dev),
+                                     n * sizeof(int), n * sizeof(int), 1}, s);
+    std::copy(tmp.begin(), tmp.end(), out);
+    return e;
 }
 
 // Copy a user matrix (order, ld) into a device row-major matrix with padded

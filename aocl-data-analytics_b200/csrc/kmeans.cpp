@@ -1202,10 +1202,7 @@ da_status KMeans<T>::predict(da_int m, da_int d, const T *Y, da_int ldy, da_int 
     B200_TRY(launch_kmeans_assign<T>(dY.as<T>(), ld, m, n_features, dC0.as<T>(), ld, n_clusters,
                                      dCn.as<T>(), dYL.as<int>(), nullptr, nullptr, nullptr, st),
              "assign");
-    std::vector<int> lab(m);
-    B200_TRY(cudaMemcpyAsync(lab.data(), dYL.p, m * sizeof(int), cudaMemcpyDeviceToHost, st), "copy");
-    B200_TRY(cudaStreamSynchronize(st), "predict");
-    for (da_int i = 0; i < m; ++i) labels[i] = lab[i];
+    B200_TRY(download_ints(dYL.as<int>(), (size_t)m, labels, st), "predict");
     return da_status_success;
 }
 
@@ -1252,14 +1249,11 @@ da_status KMeans<T>::transform(da_int m, da_int d, const T *X, da_int ldx, T *Xt
         B200_TRY(launch_pairwise<T>(dY.as<T>(), ld, m, dC0.as<T>(), ld, n_clusters, n_features,
                                     dYL.as<T>(), dCn.as<T>(), a, dKD.as<T>(), st), "transform");
     }
-    std::vector<T> out(outn);
-    B200_TRY(cudaMemcpyAsync(out.data(), dKD.p, outn * sizeof(T), cudaMemcpyDeviceToHost, st), "copy");
-    B200_TRY(cudaStreamSynchronize(st), "transform");
+    // the device block has the storage order of Xt
     const bool rm = order() == row_major;
-    for (da_int i = 0; i < m; ++i)
-        for (da_int j = 0; j < n_clusters; ++j)
-            Xt[rm ? (size_t)i * ldxt + j : i + (size_t)j * ldxt] =
-                out[rm ? (size_t)i * n_clusters + j : i + (size_t)j * m];
+    const size_t row = (size_t)(rm ? n_clusters : m) * sizeof(T);
+    B200_TRY(copy_down({Xt, (size_t)ldxt * sizeof(T), dKD.p, row, row, (size_t)(rm ? m : n_clusters)},
+                       st), "transform");
     return da_status_success;
 }
 
@@ -1323,15 +1317,10 @@ template <typename T> da_status KMeans<T>::get_result_int(da_result q, da_int *d
                              "The array is too small. Please provide an array of at least size: " +
                                  std::to_string(n_samples) + ".");
         }
-        if (!best_labels_on_host) {
-            std::vector<int> lab(n_samples);
-            B200_TRY(cudaMemcpyAsync(lab.data(), dBestL.p, n_samples * sizeof(int),
-                                     cudaMemcpyDeviceToHost, cuda->stream), "copy");
-            B200_TRY(cudaStreamSynchronize(cuda->stream), "copy");
-            best_labels.assign(lab.begin(), lab.end());
-            best_labels_on_host = true;
-        }
-        for (da_int i = 0; i < n_samples; ++i) out[i] = best_labels[i];
+        if (best_labels_on_host)
+            std::copy(best_labels.begin(), best_labels.begin() + n_samples, out);
+        else
+            B200_TRY(download_ints(dBestL.as<int>(), (size_t)n_samples, out, cuda->stream), "copy");
         return da_status_success;
     }
     return err->warn(da_status_unknown_query, "The requested result could not be found.");

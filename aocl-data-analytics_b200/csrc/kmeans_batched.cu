@@ -14,8 +14,8 @@
 //                the sums equal a full recount whatever the order);
 //   kb_finalize  new centres, the shift reduction and the convergence test,
 //                one block per instance;
-// and the whole fit (all iterations, the final relabelling, the inertia) is
-// one CUDA graph replayed without host round trips.  Converged instances
+// and an iteration is one CUDA graph, launched max_iter times without host
+// round trips.  Converged instances
 // skip their items.  The assignment kernel comes in tile shapes -- the row
 // width it holds in registers (16, 32, 64, 128 or any wider) times the
 // centres it scores at once (2, 4 or 8) -- and the shape for each (width,
@@ -32,6 +32,7 @@
 #include "b200_common.cuh"
 #include "b200_kernels.hpp"
 #include "device_alloc.hpp"
+#include "host_xfer.hpp"
 #include "kmeans_fx.cuh"
 #include "../../include/aoclda_b200_ext.h"
 #include <algorithm>
@@ -560,13 +561,28 @@ __global__ void kb_inertia_sum(const KbInst *inst, int n_inst, const double *par
     out[i] = t;
 }
 
-template <typename V> struct DBuf {
+// Device arrays of the call, carved out of one allocation.
+template <typename V> struct Slice {
+    long long n;
     V *p = nullptr;
-    ~DBuf() {
-        if (p) cudaFree(p);
+    size_t bytes() const { return (std::max<size_t>((size_t)n, 1) * sizeof(V) + 255) / 256 * 256; }
+};
+struct Arena {
+    void *base = nullptr;
+    ~Arena() {
+        if (base) cudaFree(base);
     }
-    cudaError_t alloc(size_t n) {
-        return device_alloc(reinterpret_cast<void **>(&p), std::max<size_t>(n, 1) * sizeof(V));
+    template <typename... S> cudaError_t alloc(S &...s) {
+        const size_t total = (s.bytes() + ...);
+        const cudaError_t e = device_alloc(&base, total);
+        if (e != cudaSuccess) return e;
+        char *at = static_cast<char *>(base);
+        auto place = [&](auto &x) {
+            x.p = reinterpret_cast<decltype(x.p)>(at);
+            at += x.bytes();
+        };
+        (place(s), ...);
+        return cudaSuccess;
     }
 };
 
@@ -710,56 +726,47 @@ extern "C" da_status da_b200_kmeans_batched_s(da_int n_inst, const da_int *n_sam
     }
     const int n_queues = NGRP + 2; // assignment groups, update, spare
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    DBuf<float> X, Cb0, Cb1, cn, sc;
-    DBuf<int> lab, cnt, bad, queues;
-    DBuf<int2> chg;
-    DBuf<unsigned> colmax;
-    DBuf<unsigned long long> acc;
-    DBuf<double> inv, scratch, part, inert;
-    DBuf<KbInst> inst;
-    DBuf<KbItem> aitems, ditems, sitems;
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t r) {
         if (e == cudaSuccess) e = r;
         return e == cudaSuccess;
     };
-    ok(X.alloc(xo));
-    ok(Cb0.alloc(co));
-    ok(Cb1.alloc(co));
-    ok(cn.alloc(no));
-    ok(sc.alloc(so));
-    ok(lab.alloc(lo));
-    ok(chg.alloc(lo));
-    ok(cnt.alloc(no));
-    ok(bad.alloc(1));
-    ok(queues.alloc(n_queues));
-    ok(colmax.alloc(so));
-    ok(acc.alloc(ao));
-    ok(inv.alloc(so));
-    ok(scratch.alloc((size_t)n_inst * 2 * 32));
-    ok(part.alloc(scan_items.size()));
-    ok(inert.alloc(n_inst));
-    ok(inst.alloc(n_inst));
-    ok(aitems.alloc(assign_items.size()));
-    ok(ditems.alloc(delta_items.size()));
-    ok(sitems.alloc(scan_items.size()));
-    if (e != cudaSuccess) {
+    // one allocation for the call (each costs 0.3 ms, and as much to free)
+    Arena arena;
+    Slice<float> X{xo}, Cb0{co}, Cb1{co}, cn{no}, sc{so};
+    Slice<int> lab{lo}, cnt{no}, bad{1}, queues{n_queues};
+    Slice<int2> chg{lo};
+    Slice<unsigned> colmax{so};
+    Slice<unsigned long long> acc{ao};
+    Slice<double> inv{so}, scratch{(long long)n_inst * 2 * 32}, part{(long long)scan_items.size()},
+        inert{n_inst};
+    Slice<KbInst> inst{n_inst};
+    Slice<KbItem> aitems{(long long)assign_items.size()}, ditems{(long long)delta_items.size()},
+        sitems{(long long)scan_items.size()};
+    if (!ok(arena.alloc(X, Cb0, Cb1, cn, sc, lab, cnt, bad, queues, chg, colmax, acc, inv, scratch,
+                        part, inert, inst, aitems, ditems, sitems))) {
         cudaGetLastError();
         return da_status_memory_error;
     }
     cudaEvent_t ev[6] = {};
     for (auto &x : ev) ok(cudaEventCreate(&x));
     ok(cudaEventRecord(ev[0], s));
-    // upload: rows padded to ld by the copy engine, initial centres into Cb0
+    // upload: rows padded to ld, initial centres into Cb0
     {
-        ok(cudaMemsetAsync(X.p, 0, xo * sizeof(float), s));
-        ok(cudaMemsetAsync(Cb0.p, 0, co * sizeof(float), s));
-        for (da_int i = 0; i < n_inst && e == cudaSuccess; ++i) {
+        std::vector<XferSeg> segs;
+        for (da_int i = 0; i < n_inst; ++i) {
             const KbInst &I = hi[i];
-            ok(cudaMemcpy2DAsync(X.p + I.xo, (size_t)I.ld * 4, A[i], (size_t)lda[i] * 4,
-                                 (size_t)I.d * 4, I.n, cudaMemcpyHostToDevice, s));
-            ok(cudaMemcpy2DAsync(Cb0.p + I.co, (size_t)I.ld * 4, C_init[i], (size_t)I.d * 4,
-                                 (size_t)I.d * 4, I.k, cudaMemcpyHostToDevice, s));
+            const size_t w = (size_t)I.d * 4, p = (size_t)I.ld * 4;
+            segs.push_back({const_cast<float *>(A[i]), (size_t)lda[i] * 4, X.p + I.xo, p, w,
+                            (size_t)I.n});
+            segs.push_back({const_cast<float *>(C_init[i]), w, Cb0.p + I.co, p, w, (size_t)I.k});
+        }
+        cudaError_t xe = cudaSuccess;
+        if (xfer_up(segs.data(), (int)segs.size(), s, xe)) {
+            ok(xe);
+        } else {
+            for (const XferSeg &g : segs)
+                if (e == cudaSuccess) ok(copy_up(g, s));
         }
         ok(cudaMemcpyAsync(inst.p, hi.data(), hi.size() * sizeof(KbInst), cudaMemcpyHostToDevice, s));
         ok(cudaMemcpyAsync(aitems.p, assign_items.data(), assign_items.size() * sizeof(KbItem),
@@ -868,9 +875,9 @@ extern "C" da_status da_b200_kmeans_batched_s(da_int n_inst, const da_int *n_sam
     ok(ensure_smem_limit(reinterpret_cast<const void *>(kb_delta), dsmem));
     const int dgrid = std::min<int>((int)delta_items.size(),
                                     resident_blocks(reinterpret_cast<const void *>(kb_delta), 256, dsmem));
-    // The whole fit as one CUDA graph: max_iter iterations (finished
-    // instances skip their work), the final relabelling and the inertia;
-    // replayed once.
+    // One Lloyd iteration as a CUDA graph, launched max_iter times (finished
+    // instances skip their work); then the final relabelling and the inertia.
+    // (All iterations in one graph took 3 ms more to capture and instantiate.)
     // The assignment launches (one per tile shape) are parallel branches of
     // the graph: their persistent blocks share the device.
     cudaStream_t cs = nullptr;
@@ -894,21 +901,13 @@ extern "C" da_status da_b200_kmeans_batched_s(da_int n_inst, const da_int *n_sam
         }
     };
     if (e == cudaSuccess && ok(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal))) {
-        for (da_int it = 0; it < max_iter; ++it) {
-            kb_begin<<<n_inst, 128, 0, cs>>>(inst.p, Cb0.p, Cb1.p, cn.p, queues.p, n_queues);
-            assign_all(0);
-            kb_delta<<<dgrid, 256, dsmem, cs>>>(X.p, inst.p, ditems.p, (int)delta_items.size(),
-                                                queues.p + NGRP, chg.p, sc.p, acc.p, cnt.p,
-                                                max_kd, max_k);
-            kb_finalize<<<n_inst, 256, 0, cs>>>(inst.p, Cb0.p, Cb1.p, acc.p, cnt.p, inv.p,
-                                                (int)max_iter, tol, scratch.p);
-        }
-        kb_final_norms<<<n_inst, 128, 0, cs>>>(inst.p, Cb0.p, Cb1.p, cn.p);
-        cudaMemsetAsync(queues.p, 0, n_queues * sizeof(int), cs);
-        assign_all(1);
-        kb_inertia_part<<<(unsigned)scan_items.size(), 256, 0, cs>>>(X.p, inst.p, sitems.p, Cb0.p,
-                                                                      Cb1.p, lab.p, part.p);
-        kb_inertia_sum<<<(n_inst + 127) / 128, 128, 0, cs>>>(inst.p, n_inst, part.p, inert.p);
+        kb_begin<<<n_inst, 128, 0, cs>>>(inst.p, Cb0.p, Cb1.p, cn.p, queues.p, n_queues);
+        assign_all(0);
+        kb_delta<<<dgrid, 256, dsmem, cs>>>(X.p, inst.p, ditems.p, (int)delta_items.size(),
+                                            queues.p + NGRP, chg.p, sc.p, acc.p, cnt.p, max_kd,
+                                            max_k);
+        kb_finalize<<<n_inst, 256, 0, cs>>>(inst.p, Cb0.p, Cb1.p, acc.p, cnt.p, inv.p,
+                                            (int)max_iter, tol, scratch.p);
         const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
         ok(cudaGetLastError());
         ok(ce);
@@ -918,7 +917,16 @@ extern "C" da_status da_b200_kmeans_batched_s(da_int n_inst, const da_int *n_sam
     ok(cudaEventRecord(ev[4], s));
     ok(cudaStreamWaitEvent(cs, ev[4], 0));
     ok(cudaEventRecord(ev[2], cs));
-    if (e == cudaSuccess) ok(cudaGraphLaunch(exec, cs));
+    for (da_int it = 0; it < max_iter && e == cudaSuccess; ++it) ok(cudaGraphLaunch(exec, cs));
+    if (e == cudaSuccess) {
+        kb_final_norms<<<n_inst, 128, 0, cs>>>(inst.p, Cb0.p, Cb1.p, cn.p);
+        ok(cudaMemsetAsync(queues.p, 0, n_queues * sizeof(int), cs));
+        assign_all(1);
+        kb_inertia_part<<<(unsigned)scan_items.size(), 256, 0, cs>>>(X.p, inst.p, sitems.p, Cb0.p,
+                                                                      Cb1.p, lab.p, part.p);
+        kb_inertia_sum<<<(n_inst + 127) / 128, 128, 0, cs>>>(inst.p, n_inst, part.p, inert.p);
+        ok(cudaGetLastError());
+    }
     ok(cudaEventRecord(ev[3], cs));
     ok(cudaStreamSynchronize(cs));
     // results
@@ -927,15 +935,24 @@ extern "C" da_status da_b200_kmeans_batched_s(da_int n_inst, const da_int *n_sam
     ok(cudaMemcpy(fin.data(), inst.p, fin.size() * sizeof(KbInst), cudaMemcpyDeviceToHost));
     ok(cudaMemcpy(hin.data(), inert.p, hin.size() * sizeof(double), cudaMemcpyDeviceToHost));
     ok(cudaEventRecord(ev[4], cs));
+    std::vector<XferSeg> out;
     for (da_int i = 0; i < n_inst && e == cudaSuccess; ++i) {
         const KbInst &I = fin[i];
-        ok(cudaMemcpy2DAsync(C_out[i], (size_t)I.d * 4, (I.fc ? Cb1.p : Cb0.p) + I.co,
-                             (size_t)I.ld * 4, (size_t)I.d * 4, I.k, cudaMemcpyDeviceToHost, cs));
-        ok(cudaMemcpyAsync(labels_out[i], lab.p + I.lo, (size_t)I.n * sizeof(int),
-                           cudaMemcpyDeviceToHost, cs));
+        const size_t w = (size_t)I.d * 4, nl = (size_t)I.n * sizeof(int);
+        out.push_back({C_out[i], w, (I.fc ? Cb1.p : Cb0.p) + I.co, (size_t)I.ld * 4, w, (size_t)I.k});
+        out.push_back({labels_out[i], nl, lab.p + I.lo, nl, nl, 1});
         n_iter[i] = I.n_iter;
         inertia[i] = hin[i];
         converged[i] = I.conv;
+    }
+    cudaError_t xe = cudaSuccess;
+    if (e == cudaSuccess && xfer_down(out.data(), (int)out.size(), cs, xe)) {
+        ok(xe);
+    } else {
+        for (const XferSeg &g : out)
+            if (e == cudaSuccess)
+                ok(cudaMemcpy2DAsync(g.host, g.host_pitch, g.dev, g.dev_pitch, g.row_bytes, g.rows,
+                                     cudaMemcpyDeviceToHost, cs));
     }
     ok(cudaEventRecord(ev[5], cs));
     ok(cudaStreamSynchronize(cs));

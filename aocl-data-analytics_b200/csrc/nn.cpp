@@ -290,7 +290,7 @@ template <typename T> da_status NN<T>::ensure_device_data() {
     return da_status_success;
 }
 
-// Tensor-core candidate pass + exact re-score (knn_tc.cu) into dOutK / dOutI,
+// Tensor-core candidate pass + exact re-score (knn_tc.cu) into dOutK (indices after the distances),
 // in query batches that bound the candidate lists' memory; n_extra ints of
 // state follow the indices, for tc_finish.
 static constexpr da_int KNN_TC_BATCH = 16384;
@@ -338,10 +338,9 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
         n_extra = (size_t)batches * KNN_TC_STATE + (size_t)nq;
         if (!dTkQ.ensure(knn_tc_query_bytes((int)qb, ldbf, pl)) ||
             !dTkList.ensure((size_t)qb * pl.cap * 8) || !dTkFlag.ensure((size_t)nq * sizeof(int)) ||
-            !dOutK.ensure((size_t)nq * k * sizeof(float)) ||
-            !dOutI.ensure(((size_t)nq * k + n_extra) * sizeof(int)))
+            !dOutK.ensure(out_bytes((size_t)nq * k, n_extra)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
-        int *state = dOutI.as<int>() + (size_t)nq * k;
+        int *state = out_idx((size_t)nq * k) + (size_t)nq * k;
         int *counts = state + (size_t)batches * KNN_TC_STATE;
         for (da_int q0 = 0; q0 < nq; q0 += KNN_TC_BATCH, state += KNN_TC_STATE) {
             const da_int nb = std::min<da_int>(KNN_TC_BATCH, nq - q0);
@@ -359,7 +358,7 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
                                      take_sqrt ? 1 : 0, pb, dTkQ.p, dTkList.p,
                                      dTkFlag.as<int>() + q0, counts + q0, state,
                                      dOutK.as<float>() + (size_t)q0 * k,
-                                     dOutI.as<int>() + (size_t)q0 * k, st,
+                                     out_idx((size_t)nq * k) + (size_t)q0 * k, st,
                                      cosine ? &cs : nullptr);
             }), "kNN tensor-core pass");
         }
@@ -379,7 +378,7 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
 
 // The state words and list lengths of a tensor-core search (`extra`, as
 // kneighbors_tc laid them out): statistics, errors, and the flagged queries
-// searched on the plain path into dOutK / dOutI (`redone`).
+// searched on the plain path into dOutK (`redone`).
 template <typename T>
 da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt, bool cosine,
                            const int *extra, bool &redone) {
@@ -455,7 +454,7 @@ da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt
         B200_TRY(launch_knn_merge<float>(pk, pi, m, n_chunks, (int)k, take_sqrt && !cosine ? 1 : 0,
                                          ok, oi, st), "kNN merge kernel");
         B200_TRY(launch_results_scatter(ok, oi, didx, m, (int)k, dOutK.as<float>(),
-                                        dOutI.as<int>(), st), "scatter");
+                                        out_idx((size_t)nq * k), st), "scatter");
     } else {
         (void)nq, (void)d, (void)k, (void)kc, (void)take_sqrt, (void)cosine, (void)extra;
     }
@@ -509,10 +508,12 @@ da_status NN<T>::validate_queries(da_int nq, da_int d, const T *Xt, da_int ldt) 
                     "ldx_test", 1, 1, opts.key("check data") == 1);
 }
 
-// Run the fused distance + top-k kernels; ind/dist are q-major (q*k + r).
+// Run the fused distance + top-k kernels; ind/dist are q-major (q*k + r), or
+// the results go to the caller's arrays in the storage order `ord` (to).
 template <typename T>
 da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt, da_order ord,
-                                    da_int k, std::vector<da_int> &ind, std::vector<T> *dist) {
+                                    da_int k, std::vector<da_int> &ind, std::vector<T> *dist,
+                                    const KnnOut *to) {
     da_status s = ensure_device_data();
     if (s != da_status_success) return s;
     cudaStream_t st = cuda->stream;
@@ -593,14 +594,13 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             return err->error(da_status_not_implemented,
                               "k = " + std::to_string(k) + " exceeds the largest supported number "
                               "of neighbours per query (" + std::to_string(knn_max_k(fp64)) + ").");
-        if (!dOutK.ensure((size_t)nq * k * sizeof(T)) ||
-            !dOutI.ensure(((size_t)nq * k + n_extra) * sizeof(int)))
+        if (!dOutK.ensure(out_bytes((size_t)nq * k, n_extra)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
         if (n_extra > 0) {
             const KnnArgs a{acc, post, kc, (double)p, (int)k, 0, 0};
             if (!dPartK.ensure(knn_sel_bytes(sel, (int)sel_qb, fp64)))
                 return err->error(da_status_memory_error, "Device memory allocation failed.");
-            int *flags = dOutI.as<int>() + (size_t)nq * k;
+            int *flags = out_idx((size_t)nq * k) + (size_t)nq * k;
             for (da_int q0 = 0; q0 < nq; q0 += sel_qb, ++flags) {
                 const da_int nb = std::min(sel_qb, nq - q0);
                 B200_TRY(cuda->timed("knn_select", [&] {
@@ -608,7 +608,7 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
                                                 (int)n_samples, ld, (int)d, qn ? qn + q0 : nullptr,
                                                 xn, a, sel, dPartK.p, tf,
                                                 dOutK.as<T>() + (size_t)q0 * k,
-                                                dOutI.as<int>() + (size_t)q0 * k, flags, st);
+                                                out_idx((size_t)nq * k) + (size_t)q0 * k, flags, st);
                 }), "kNN selection kernels");
             }
         }
@@ -627,7 +627,7 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             KnnArgs a{acc, post, kc, (double)p, (int)k, chunk_rows, n_chunks};
             const size_t parts = (size_t)nq * n_chunks * k;
             if (!dPartK.ensure(parts * sizeof(T)) || !dPartI.ensure(parts * sizeof(int)) ||
-                !dOutK.ensure((size_t)nq * k * sizeof(T)) || !dOutI.ensure((size_t)nq * k * sizeof(int)))
+                !dOutK.ensure(out_bytes((size_t)nq * k, 0)))
                 return err->error(da_status_memory_error, "Device memory allocation failed.");
             B200_TRY(cuda->timed("knn_chunks", [&] {
                 return launch_knn_chunks<T>(dQ.as<T>(), ld, (int)nq, dX.as<T>(), ld, (int)n_samples,
@@ -636,7 +636,7 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             }), "kNN distance kernel");
             B200_TRY(cuda->timed("knn_merge", [&] {
                 return launch_knn_merge<T>(dPartK.as<T>(), dPartI.as<int>(), (int)nq, n_chunks, (int)k,
-                                           tf, dOutK.as<T>(), dOutI.as<int>(), st);
+                                           tf, dOutK.as<T>(), out_idx((size_t)nq * k), st);
             }), "kNN merge kernel");
             return da_status_success;
         };
@@ -645,28 +645,72 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             if (s != da_status_success) return s;
         }
     }
-    ind.resize((size_t)nq * k);
-    std::vector<int> tmp((size_t)nq * k + n_extra);
+    // the indices follow the distances, the state words the indices.  A few
+    // results come back in one copy; many go to the caller's arrays directly,
+    // column-major ones transposed on the device first (the upload's stage is
+    // free by now)
+    const size_t nk = (size_t)nq * k;
+    const bool want = to ? to->dist != nullptr : dist != nullptr;
+    const bool small = out_bytes(nk, n_extra) <= 256 * 1024;
+    const bool cm = to && ord == column_major && nq > 1 && k > 1;
+    std::vector<int> extra, tmp;
+    if (!to) {
+        ind.resize(nk);
+        if (dist) dist->resize(nk);
+    }
+    T *const hd = to ? to->dist : dist ? dist->data() : nullptr;
+    da_int *const hi = to ? to->ind : ind.data();
     for (;;) {
-        B200_TRY(cudaMemcpyAsync(tmp.data(), dOutI.p, ((size_t)nq * k + n_extra) * sizeof(int),
-                                 cudaMemcpyDeviceToHost, st),
-                 "download");
-        if (dist) {
-            dist->resize((size_t)nq * k);
-            B200_TRY(cudaMemcpyAsync(dist->data(), dOutK.p, dist->size() * sizeof(T),
-                                     cudaMemcpyDeviceToHost, st), "download");
+        const T *od = dOutK.as<T>();
+        const int *oi = out_idx(nk);
+        extra.resize(n_extra);
+        if (small) {
+            // in words of four bytes: the distances if wanted, indices, state
+            const size_t dw = want ? nk * sizeof(T) / 4 : 0, words = dw + nk + n_extra;
+            tmp.resize(words);
+            B200_TRY(copy_down({tmp.data(), words * 4, want ? (void *)od : (void *)oi, words * 4,
+                                words * 4, 1}, st), "kNN");
+            const int *ti = tmp.data() + dw;
+            const T *td = reinterpret_cast<const T *>(tmp.data());
+            for (size_t q = 0, e = 0; q < (size_t)nq; ++q)
+                for (size_t r = 0; r < (size_t)k; ++r, ++e) {
+                    const size_t at = cm ? r * nq + q : e;
+                    hi[at] = (da_int)ti[e];
+                    if (want) std::memcpy(&hd[at], &td[e], sizeof(T));
+                }
+            std::copy(ti + nk, ti + nk + n_extra, extra.begin());
+        } else {
+            if (cm) {
+                if (!dStage.ensure(nk * (sizeof(T) + sizeof(int))))
+                    return err->error(da_status_memory_error, "Device memory allocation failed.");
+                T *td = dStage.as<T>();
+                float *ti = reinterpret_cast<float *>(td + nk); // four-byte words
+                B200_TRY(launch_rowmajor_to_colmajor<float>(reinterpret_cast<const float *>(oi),
+                                                            (int)nq, (int)k, (int)k, ti, (long)nq,
+                                                            st), "transpose");
+                if (want)
+                    B200_TRY(launch_rowmajor_to_colmajor<T>(od, (int)nq, (int)k, (int)k, td,
+                                                            (long)nq, st), "transpose");
+                oi = reinterpret_cast<const int *>(ti);
+                od = td;
+            }
+            if (n_extra)
+                B200_TRY(cudaMemcpyAsync(extra.data(), out_idx(nk) + nk, n_extra * sizeof(int),
+                                         cudaMemcpyDeviceToHost, st), "download");
+            if (want)
+                B200_TRY(copy_down({hd, nk * sizeof(T), const_cast<T *>(od), nk * sizeof(T),
+                                    nk * sizeof(T), 1}, st), "download");
+            B200_TRY(download_ints(oi, nk, hi, st), "kNN");
         }
-        B200_TRY(cudaStreamSynchronize(st), "kNN");
         if (n_extra == 0) break;
-        const int *extra = tmp.data() + (size_t)nq * k;
         if (tc_done) {
             bool redone = false;
             s = tc_finish(nq, d, k, kc, metric != M_SQEUC && metric != M_COS, metric == M_COS,
-                          extra, redone);
+                          extra.data(), redone);
             if (s != da_status_success) return s;
             if (!redone) break;
         } else {
-            if (std::all_of(extra, extra + n_extra, [](int f) { return f == 0; })) break;
+            if (std::all_of(extra.begin(), extra.end(), [](int f) { return f == 0; })) break;
             // a query's list overflowed or was short of k keys
             cuda->stats["knn_select_fallback"] += 1.0;
             s = run_lists();
@@ -674,7 +718,6 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
         }
         n_extra = 0;
     }
-    for (size_t i = 0; i < ind.size(); ++i) ind[i] = (da_int)tmp[i];
     return da_status_success;
 }
 
@@ -1004,19 +1047,9 @@ da_status NN<T>::kneighbors(da_int nq, da_int d, const T *Xt, da_int ldt, da_int
     if (return_distance && n_dist == nullptr)
         return err->error(da_status_invalid_pointer, "n_dist is not a valid pointer.");
     std::vector<da_int> ind;
-    std::vector<T> dist;
-    s = kneighbors_compute(nq, d, Xt, ldt, order(), k, ind, return_distance ? &dist : nullptr);
-    if (s != da_status_success) return s;
+    const KnnOut to{n_ind, return_distance ? n_dist : nullptr};
     // outputs: q-major for row-major storage, n_queries x k column-major otherwise
-    const bool cm = order() == column_major;
-    for (da_int q = 0; q < nq; ++q)
-        for (da_int r = 0; r < k; ++r) {
-            const size_t src = (size_t)q * k + r;
-            const size_t dst = cm ? (size_t)r * nq + q : src;
-            n_ind[dst] = ind[src];
-            if (return_distance) n_dist[dst] = dist[src];
-        }
-    return da_status_success;
+    return kneighbors_compute(nq, d, Xt, ldt, order(), k, ind, nullptr, &to);
 }
 
 template <typename T> da_status NN<T>::available_classes() {
@@ -1082,22 +1115,23 @@ da_status NN<T>::compute_proba(da_int nq, da_int d, const T *Xt, da_int ldt,
     const da_int nc = (da_int)classes.size();
     proba.assign((size_t)nq * nc, T(0));
     for (da_int q = 0; q < nq; ++q) {
-        T den = T(0);
-        for (da_int c = 0; c < nc; ++c) {
-            T v = T(0);
-            for (da_int r = 0; r < k; ++r) {
-                const da_int lbl = y_class[ind[(size_t)q * k + r]];
-                if (lbl != classes[c]) continue;
-                if (weights == 0) v += T(1);
-                else {
-                    const T w = dist[(size_t)q * k + r];
-                    v += (w <= std::numeric_limits<T>::epsilon()) ? T(1) : T(1) / w;
-                }
+        T *pq = proba.data() + (size_t)q * nc;
+        // per class, the neighbours' weights in neighbour order
+        for (da_int r = 0; r < k; ++r) {
+            const da_int lbl = y_class[ind[(size_t)q * k + r]];
+            const da_int c = (da_int)(std::lower_bound(classes.begin(), classes.end(), lbl) -
+                                      classes.begin());
+            if (c == nc || classes[c] != lbl) continue;
+            T v = T(1);
+            if (weights != 0) {
+                const T w = dist[(size_t)q * k + r];
+                v = (w <= std::numeric_limits<T>::epsilon()) ? T(1) : T(1) / w;
             }
-            proba[(size_t)q * nc + c] = v;
-            den += v;
+            pq[c] += v;
         }
-        for (da_int c = 0; c < nc; ++c) proba[(size_t)q * nc + c] /= den;
+        T den = T(0);
+        for (da_int c = 0; c < nc; ++c) den += pq[c];
+        for (da_int c = 0; c < nc; ++c) pq[c] /= den;
     }
     return da_status_success;
 }

@@ -79,6 +79,15 @@ class Request:
         return None if self.t_done is None else self.t_done - self.t_submit
 
 
+# A call of a few queries takes 0.1 to 0.2 ms, about as long as a client needs
+# to hand in the next request, so that without a wait each one of a burst is
+# served by a call of its own.  Requests that come less than BURST_GAP seconds
+# apart wait up to LINGER after the last one (2 LINGER in all) for company; a
+# request that comes alone never waits.
+BURST_GAP = 0.5e-3
+LINGER = 0.25e-3
+
+
 class Server:
     """kNN index X (n x d, fp32, euclidean) and k-means models given as
     {name: (training rows, initial centres)}, fitted at start-up.  `workers`
@@ -121,6 +130,9 @@ class Server:
         self.cv = threading.Condition()
         self.pending = {"knn": collections.deque(), "ann": collections.deque(),
                         "predict": collections.deque()}
+        # the last submission of each kind and the time between the last two
+        self.last = dict.fromkeys(self.pending, float("-inf"))
+        self.gap = dict.fromkeys(self.pending, float("inf"))
         self.stopping = False
         self.completed = []
         # every library call: (kind, requests, queries, seconds, largest
@@ -208,6 +220,8 @@ class Server:
             req.parts_left = len(parts)
         with self.cv:
             self.pending[req.kind].extend(parts)
+            self.gap[req.kind] = req.t_submit - self.last[req.kind]
+            self.last[req.kind] = req.t_submit
             self.cv.notify_all()
         return req
 
@@ -231,17 +245,30 @@ class Server:
         blocks until one is pending, None once the server stops.  small_only:
         requests of at most small_queries queries only.  large_first (the
         other workers beside a fast lane): large requests before small ones,
-        unless a small one has waited overflow_ms (the fast lane is behind)."""
+        unless a small one has waited overflow_ms (the fast lane is behind).
+        While requests of the kind arrive less than BURST_GAP apart, a batch
+        with room is held until LINGER after its last arrival."""
         def fits(r):
             return not small_only or r.queries.shape[0] <= self.small_queries
 
         with self.cv:
-            while not any(map(fits, self.pending[kind])) and not self.stopping:
-                self.cv.wait()
-            q = self.pending[kind]
-            if not any(map(fits, q)):
-                return None
-            now = time.perf_counter()
+            held = None  # when the batch being held began to wait
+            while True:
+                q = self.pending[kind]
+                mine = [r.queries.shape[0] for r in q if fits(r)]
+                here, now = sum(mine), time.perf_counter()
+                if not mine:
+                    if self.stopping:
+                        return None
+                    held = None
+                    self.cv.wait()
+                    continue
+                held = held or now
+                left = min(self.last[kind] + LINGER, held + 2 * LINGER) - now
+                if (left <= 0 or self.stopping or self.gap[kind] > BURST_GAP
+                        or 2 * here > cap_queries or 2 * here * per_query_bytes > cap_bytes):
+                    break
+                self.cv.wait(left)
             # aged requests, then small ones, then the rest (oldest first in each)
             def rank(r):
                 wait = now - r.t_submit
