@@ -117,6 +117,7 @@ template <typename T> struct NN : public AlgBase {
     std::vector<T> rnn_val;
     bool rnn_dist = false, rnn_squares = false;
     DevBuf dD, dRc, dRs, dRi, dRv, dRh;
+    double radius_work = 0; // multiply-adds of the searches before the tensor-core copies
     da_status radius_neighbors(da_int nq, da_int d, const T *Xt, da_int ldt, T radius,
                                da_int return_distance, da_int sort_results);
     da_status get_result(da_result q, da_int *dim, double *out) override;
@@ -147,6 +148,12 @@ template <typename T> struct NN : public AlgBase {
     da_status radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T r, bool want_val,
                              std::vector<da_int> &cnt, std::vector<long long> &start,
                              std::vector<da_int> &idx, std::vector<T> &val, bool &squares);
+    // a block of its queries on the tensor cores (fp32; done: false where the
+    // plain path takes it)
+    da_status radius_tc(da_int nq, da_int d, const T *Q, T thr, int kc, bool want_val,
+                        da_int *cnt_out, long long *start_out, std::vector<da_int> &idx_out,
+                        std::vector<T> &val_out, bool &done);
+    cudaError_t tc_train_copies(da_int d);
     da_status compute_proba_rnn(da_int nq, da_int d, const T *Xt, da_int ldt,
                                 std::vector<T> &proba);
     da_status predict_reg_rnn(da_int nq, da_int d, const T *Xt, da_int ldt, T *y);

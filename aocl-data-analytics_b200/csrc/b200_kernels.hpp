@@ -191,6 +191,25 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
                           void *list, int *fallback, int *cnt, int *state, float *out_key,
                           int *out_idx, cudaStream_t s, const KnnTcCosine *cosine = nullptr);
 
+// Radius search, fp32 (squared) euclidean: a mask of the rows whose tensor-core
+// value may be within thr (radius_tc_words(nx) words per query, 32 rows each),
+// their number per query (RADIUS_TC_NO where no bound holds), then offsets and
+// the exact distances.  state: as above ([1] the error code).  hits[q] rows and
+// values follow off[q], in index order.
+constexpr int RADIUS_TC_NO = 1 << 30;
+size_t radius_tc_query_bytes(int nq, int ldbf); // size of qbuf
+int radius_tc_words(int nx);
+cudaError_t launch_radius_tc(const void *Xh, const void *Xl, const float *xnorm2,
+                             const float *xmax, int nx, int ld, int ldbf, int d, const float *Q,
+                             int nq, float thr, void *qbuf, unsigned *mask, int *cnt, int *state,
+                             cudaStream_t s);
+cudaError_t launch_radius_cand_scan(const int *cnt, int nq, long long *off, long long *total,
+                                    cudaStream_t s);
+cudaError_t launch_radius_exact(const float *X, int nx, int ld, int d, const float *Q, int nq,
+                                int kc, float thr, const unsigned *mask, const int *cnt,
+                                const long long *off, int *hits, int *idx, float *val,
+                                cudaStream_t s);
+
 // ------------------------------------------------------------- k-means ---
 struct KmeansWork {
     // per-iteration device scratch owned by the handle

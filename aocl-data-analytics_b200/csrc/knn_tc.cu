@@ -62,7 +62,8 @@ struct KnnTcArgs {
     const float *bound;  // list pass: the k-th smallest sample minimum per query
     const float *margin; // per query: 2 eps_q (nudged up)
     float *minima;       // sample pass: nq x groups
-    int *cnt;            // list pass: values listed per query
+    int *cnt;            // list and mask pass: values below the threshold per query
+    unsigned *mask;      // mask pass: nq x n_xtiles * 8 words, a bit per train row
     int2 *list;          // nq * cap: (value bits, train row)
     int *err;
 };
@@ -116,8 +117,11 @@ template <bool COS> __device__ __forceinline__ void tk_val2(float &a, float &b, 
     b = __uint_as_float((unsigned)(v >> 32));
 }
 
-// One work item: query tile qt against `tiles` consecutive row tiles.  SAMPLE: minima; else lists.
-template <bool COS, bool SAMPLE>
+// What a pass writes: minima, lists, or (radius search) a bit per pair.
+enum { TK_SAMPLE, TK_LIST, TK_MASK };
+
+// One work item: query tile qt against `tiles` consecutive row tiles.
+template <bool COS, int PASS>
 __global__ void __launch_bounds__(TK_THREADS, 1)
 knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ CUtensorMap tmQl,
               const __grid_constant__ CUtensorMap tmXh, const __grid_constant__ CUtensorMap tmXl,
@@ -133,7 +137,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
     unsigned char *Xs = Ql + (size_t)nkb * kQ; // S stages of (Xh, Xl) for one K block
     float *xn_w = reinterpret_cast<float *>(Xs + (size_t)S * 2 * kX); // 8 warps x TK_COLS
     int2 *stash_w = reinterpret_cast<int2 *>(xn_w + 8 * TK_COLS);     // TK_STASH x 256 threads
-    TkShared *sh = reinterpret_cast<TkShared *>(stash_w + (SAMPLE ? 0 : TK_STASH * 256));
+    TkShared *sh = reinterpret_cast<TkShared *>(stash_w + (PASS == TK_LIST ? TK_STASH * 256 : 0));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -258,8 +262,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
         // rows past the end never pass (+inf, or NaN for cosine)
         const float pad = COS ? __int_as_float(0x7fc00000) : inf;
         float theta = -inf, low[4] = {inf, inf, inf, inf};
-        if (!SAMPLE && q < a.nq) theta = nudge_up(a.bound[q] + a.margin[q]);
-        int ns = 0;
+        if (PASS != TK_SAMPLE && q < a.nq) theta = nudge_up(a.bound[q] + a.margin[q]);
+        int ns = 0, found = 0;
         // the stashed values to the query's list
         auto flush = [&]() {
             if (ns > 0) {
@@ -302,6 +306,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
             tmem_ld32_issue(trow, v[0]);
 #pragma unroll 1
             for (int c2 = 0; c2 < TK_COLS / 32; c2 += 2) {
+                unsigned word[2] = {0, 0}; // mask pass
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int c = c2 + h;
@@ -320,7 +325,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
                         a1 = fminf(fminf(a1, w[u + 2]), w[u + 3]);
                     }
                     const float m = fminf(fminf(mp[0], mp[1]), fminf(mp[2], mp[3]));
-                    if (SAMPLE) {
+                    if (PASS == TK_SAMPLE) {
                         if (c2 == 0) low[h] = fminf(low[h], m);
                         else low[h + 2] = fminf(low[h + 2], m);
                         continue;
@@ -330,6 +335,10 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
 #pragma unroll
                     for (int u = 0; u < 32; ++u) part[u & 3] |= (w[u] < theta ? 1u : 0u) << u;
                     unsigned bits = (part[0] | part[1]) | (part[2] | part[3]);
+                    if (PASS == TK_MASK) {
+                        word[h] = bits;
+                        continue;
+                    }
                     const int row = (x0 + t) * TK_ROWS + row_off + c * 32;
                     while (bits) {
                         if (ns == TK_STASH) flush();
@@ -340,11 +349,18 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
                     }
                     __syncwarp();
                 }
+                if (PASS == TK_MASK && q < a.nq) {
+                    found += __popc(word[0]) + __popc(word[1]);
+                    *reinterpret_cast<uint2 *>(a.mask + ((size_t)q * a.n_xtiles + x0 + t) * 8 +
+                                               g * 4 + c2) = make_uint2(word[0], word[1]);
+                }
             }
             tc_fence_before();
             mbar_arrive(&sh->tempty[b]);
         }
-        if (SAMPLE) {
+        if (PASS == TK_MASK) {
+            if (found > 0) atomicAdd(&a.cnt[q], found);
+        } else if (PASS == TK_SAMPLE) {
             if (q < a.nq) {
                 float *o = a.minima + (size_t)q * a.groups + (xc * 2 + g) * 4;
 #pragma unroll
@@ -365,11 +381,13 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
 // -2q split into bf16 hi / lo (rows nq..nq_pad-1 zero) and the margins 2
 // eps_q; the lists' lengths, the fallback flags and the state words cleared.
 // Cosine (qnorm: the plain path's query norms): -2 q / |q| instead, and the
-// margin 2 e1 for every query.
+// margin 2 e1 for every query.  Radius search (bound): thr - |q|^2 per query, the
+// fp32 |q|^2 within eps_q of the exact one; a query whose threshold is not
+// finite gets none (NaN) and RADIUS_TC_NO values.
 __global__ void knn_tc_prep_queries(const float *Q, int ld, int nq, int d, int nq_pad, int ldo,
                                     __nv_bfloat16 *Qh, __nv_bfloat16 *Ql, float e1, float e2,
                                     const float *xmax, float *margin, int *cnt, int *fallback,
-                                    int *state, const float *qnorm) {
+                                    int *state, const float *qnorm, float *bound, float thr) {
     const int qi = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x < KNN_TC_STATE) state[threadIdx.x] = 0;
@@ -392,7 +410,14 @@ __global__ void knn_tc_prep_queries(const float *Q, int ld, int nq, int d, int n
         const float eps = qnorm ? e1 : e1 * xm * qn + e2 * (xm * xm + qn * qn);
         margin[qi] = nudge_up(2.f * eps);
         cnt[qi] = 0;
-        fallback[qi] = 0;
+        if (bound) {
+            const float b = thr - s;
+            const bool finite = isfinite(nudge_up(b + margin[qi]));
+            bound[qi] = finite ? b : __int_as_float(0x7fc00000);
+            if (!finite) cnt[qi] = RADIUS_TC_NO;
+        } else {
+            fallback[qi] = 0;
+        }
     }
 }
 
@@ -575,6 +600,20 @@ __global__ void max_value_kernel(const float *v, int n, float *out) {
 }
 __global__ void sqrt_inplace_kernel(float *v) { *v = sqrtf(*v) * 1.0001f; }
 
+// |v'_tc - v'_plain| <= e1 |x||q| + e2 (|x|^2 + |q|^2)  (u = 2^-24):
+//   bf16 hi/lo split of x and of -2q, dropped lo.lo term: 3.1 2^-16 |x||2q|
+//   fp32 accumulation of K_total = 3 Kp products in the tensor core
+//   (allowing truncation): 2 K_total u |x||2q|
+//   fp32 |x|^2 (Kp-term fma chain) and the final add: (Kp + 2) u |x|^2, u |2xq|
+//   the plain path's direct-difference sum: (d + 4) u (|x| + |q|)^2
+void sqeuc_error(int nkb, int d, double &e1, double &e2) {
+    const double u = std::ldexp(1.0, -24);
+    const double kp = (double)nkb * TK_KB, ktot = 3.0 * kp;
+    e1 = 1.1 * (3.1 * std::ldexp(1.0, -16) * 2.0 + 2.0 * ktot * u * 2.0 + 2.0 * u +
+                (d + 4.0) * u * 2.0);
+    e2 = 1.1 * ((kp + 2.0) * u + (d + 4.0) * u * 2.0 + 2.0 * u);
+}
+
 size_t tk_smem_bytes(int nkb, int stages) {
     return 1024 + (size_t)nkb * 2 * TK_BM * 128 + (size_t)stages * 2 * TK_ROWS * 128 +
            (size_t)8 * TK_COLS * 4 + (size_t)TK_STASH * 256 * 8 + sizeof(TkShared) + 64;
@@ -674,17 +713,10 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
     float *margin = reinterpret_cast<float *>(Ql + (size_t)nq_pad * ldbf);
     float *bound = margin + nq_pad;
     float *minima = bound + nq_pad;
-    // |v'_tc - v'_plain| <= e1 |x||q| + e2 (|x|^2 + |q|^2)  (u = 2^-24):
-    //   bf16 hi/lo split of x and of -2q, dropped lo.lo term: 3.1 2^-16 |x||2q|
-    //   fp32 accumulation of K_total = 3 Kp products in the tensor core
-    //   (allowing truncation): 2 K_total u |x||2q|
-    //   fp32 |x|^2 (Kp-term fma chain) and the final add: (Kp + 2) u |x|^2, u |2xq|
-    //   the plain path's direct-difference sum: (d + 4) u (|x| + |q|)^2
+    double e1, e2;
+    sqeuc_error(nkb, d, e1, e2);
     const double u = std::ldexp(1.0, -24);
     const double kp = (double)nkb * TK_KB, ktot = 3.0 * kp;
-    const double e1 = 1.1 * (3.1 * std::ldexp(1.0, -16) * 2.0 + 2.0 * ktot * u * 2.0 + 2.0 * u +
-                             (d + 4.0) * u * 2.0);
-    const double e2 = 1.1 * ((kp + 2.0) * u + (d + 4.0) * u * 2.0 + 2.0 * u);
     // cosine, r = -2 x.q / (|x| |q|) = 2 (distance - 1), |x|, |q| the plain
     // path's norms: bf16 hi/lo split and fp32 accumulation as above on unit-
     // scale products, the scalings by 1/|q| and 1/|x| (4 u), and twice the
@@ -696,7 +728,7 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
     const int wpb = 8;
     knn_tc_prep_queries<<<(nq_pad + wpb - 1) / wpb, wpb * 32, 0, s>>>(
         Q, ld, nq, d, nq_pad, ldbf, Qh, Ql, (float)(cosm ? ec : e1), (float)e2, xmax, margin, cnt,
-        fallback, state, cosm ? cosine->qnorm : nullptr);
+        fallback, state, cosm ? cosine->qnorm : nullptr, nullptr, 0.f);
     KnnTcArgs a;
     a.nq = nq;
     a.nkb = nkb;
@@ -729,8 +761,9 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
             !make_map_bf16_rows(&mxl, Xl, a.nx, ldbf, TK_ROWS, a.xstep))
             return cudaErrorInvalidValue;
         using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, KnnTcArgs);
-        const Kern kern = sample ? (cosm ? knn_tc_kernel<true, true> : knn_tc_kernel<false, true>)
-                                 : (cosm ? knn_tc_kernel<true, false> : knn_tc_kernel<false, false>);
+        const Kern kern =
+            sample ? (cosm ? knn_tc_kernel<true, TK_SAMPLE> : knn_tc_kernel<false, TK_SAMPLE>)
+                   : (cosm ? knn_tc_kernel<true, TK_LIST> : knn_tc_kernel<false, TK_LIST>);
         cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kern), smem);
         if (e != cudaSuccess) return e;
         // one block per work item: blocks end often, so the kernels of a
@@ -782,6 +815,192 @@ cudaError_t launch_results_scatter(const float *key, const int *ind, const int *
     if (n == 0) return cudaSuccess;
     results_scatter_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(key, ind, idx, m, k,
                                                                         out_key, out_idx);
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------------ radius search ---
+// The mask pass sets a bit for every pair whose v'_tc is below the query's
+// threshold (thr - |q|^2 + 2 eps_q): every row the plain path finds within thr,
+// in index order, whatever their number.  The offsets of a query's set bits
+// follow, and one block per query computes the plain path's distances of its
+// rows, keeping those at most thr.
+
+// off[q] = cnt[0] + .. + cnt[q - 1], *total = all.  One block.
+__global__ void __launch_bounds__(1024)
+radius_cand_scan(const int *cnt, int nq, long long *off, long long *total) {
+    __shared__ long long part[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long before = 0;
+    for (int q0 = 0; q0 < nq; q0 += 1024) {
+        const int q = q0 + threadIdx.x;
+        const long long c = q < nq ? cnt[q] : 0;
+        long long inc = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (lane == 31) part[warp] = inc;
+        __syncthreads();
+        long long add = before, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) add += part[w];
+            all += part[w];
+        }
+        if (q < nq) off[q] = add + inc - c;
+        before += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *total = before;
+}
+
+// A query's candidates: the set bits of its mask row gather in a shared list
+// (the bits are sparse: without it most threads of the distances below would
+// idle), RX_LIST at a time.
+constexpr int RX_THREADS = 256, RX_LIST = 2048;
+__global__ void __launch_bounds__(RX_THREADS)
+radius_exact_kernel(const float *X, const float *Q, int ld, int d, int kc, float thr,
+                    const unsigned *mask, int words, const int *cnt, const long long *off,
+                    int *hits, int *idx, float *val) {
+    extern __shared__ __align__(16) float rx_smem[];
+    __shared__ int rows[RX_LIST], part[RX_THREADS / 32];
+    const int q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (cnt[q] == 0) {
+        if (tid == 0) hits[q] = 0;
+        return;
+    }
+    for (int f = tid; f < d; f += RX_THREADS) rx_smem[f] = Q[(size_t)q * ld + f];
+    // the sum over the block of v before this thread's, and over all
+    auto scan = [&](int v, int &all) {
+        int inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        __syncthreads(); // part is free again
+        if (lane == 31) part[warp] = inc;
+        __syncthreads();
+        int add = 0;
+        all = 0;
+#pragma unroll
+        for (int w = 0; w < RX_THREADS / 32; ++w) {
+            if (w < warp) add += part[w];
+            all += part[w];
+        }
+        return add + inc - v;
+    };
+    int have = 0, kept = 0;
+    auto emit = [&]() { // the listed rows
+        __syncthreads();
+        for (int i0 = 0; i0 < have; i0 += RX_THREADS) {
+            const int i = i0 + tid;
+            float v = 0.f;
+            if (i < have) v = sqeuc_ref(X + (size_t)rows[i] * ld, rx_smem, d, kc);
+            const bool in = i < have && v <= thr;
+            int all;
+            const int at = scan(in ? 1 : 0, all);
+            if (in) {
+                idx[off[q] + kept + at] = rows[i];
+                val[off[q] + kept + at] = v;
+            }
+            kept += all;
+        }
+        have = 0;
+        __syncthreads();
+    };
+    const uint4 *m4 = reinterpret_cast<const uint4 *>(mask + (size_t)q * words);
+    for (int w0 = 0; w0 < words / 4; w0 += RX_THREADS) {
+        uint4 m = make_uint4(0, 0, 0, 0);
+        if (w0 + tid < words / 4) m = m4[w0 + tid];
+        const unsigned wd[4] = {m.x, m.y, m.z, m.w};
+        int all;
+        const int at = scan(__popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w), all);
+        for (int done = 0; done < all;) {
+            const int take = min(RX_LIST - have, all - done);
+            int p = at - done; // of this thread's first bit, from the window's start
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                for (unsigned b = wd[u]; b; b &= b - 1, ++p)
+                    if (p >= 0 && p < take)
+                        rows[have + p] = (w0 + tid) * 128 + u * 32 + __ffs(b) - 1;
+            have += take;
+            done += take;
+            if (have == RX_LIST) emit();
+        }
+    }
+    emit();
+    if (tid == 0) hits[q] = kept;
+}
+
+size_t radius_tc_query_bytes(int nq, int ldbf) {
+    const size_t nq_pad = ((size_t)nq + TK_BM - 1) / TK_BM * TK_BM;
+    return nq_pad * ldbf * 2 * 2 + nq_pad * 8 + 256;
+}
+int radius_tc_words(int nx) { return (nx + TK_ROWS - 1) / TK_ROWS * 8; }
+
+// Device time at 200,000 x 32, 2,000 queries, 140,000 hits: 185 us (the mask 136), where a
+// block of distances written, counted and compacted takes 2.03 ms (1.44 of it
+// the distances).  Bound by the epilogue's instructions (1.5 per pair).
+cudaError_t launch_radius_tc(const void *Xh, const void *Xl, const float *xnorm2,
+                             const float *xmax, int nx, int ld, int ldbf, int d, const float *Q,
+                             int nq, float thr, void *qbuf, unsigned *mask, int *cnt, int *state,
+                             cudaStream_t s) {
+    const int nkb = (ldbf + TK_KB - 1) / TK_KB;
+    const int n_qtiles = (nq + TK_BM - 1) / TK_BM, nq_pad = n_qtiles * TK_BM;
+    __nv_bfloat16 *Qh = static_cast<__nv_bfloat16 *>(qbuf);
+    __nv_bfloat16 *Ql = Qh + (size_t)nq_pad * ldbf;
+    float *margin = reinterpret_cast<float *>(Ql + (size_t)nq_pad * ldbf);
+    float *bound = margin + nq_pad;
+    double e1, e2;
+    sqeuc_error(nkb, d, e1, e2);
+    const int wpb = 8;
+    knn_tc_prep_queries<<<(nq_pad + wpb - 1) / wpb, wpb * 32, 0, s>>>(
+        Q, ld, nq, d, nq_pad, ldbf, Qh, Ql, (float)e1, (float)e2, xmax, margin, cnt, nullptr,
+        state, nullptr, bound, thr);
+    KnnTcArgs a{};
+    a.nx = nx;
+    a.nq = nq;
+    a.nkb = nkb;
+    a.kk_last = (d - (nkb - 1) * TK_KB + 15) / 16;
+    a.n_qtiles = n_qtiles;
+    a.n_xtiles = (nx + TK_ROWS - 1) / TK_ROWS;
+    a.tiles = tk_item_tiles(a.n_xtiles, n_qtiles);
+    a.n_items = n_qtiles * ((a.n_xtiles + a.tiles - 1) / a.tiles);
+    a.xstep = 1;
+    a.xnorm = xnorm2;
+    a.bound = bound;
+    a.margin = margin;
+    a.cnt = cnt;
+    a.mask = mask;
+    a.err = state + 1;
+    a.stages = 8;
+    while (a.stages > 2 && tk_smem_bytes(nkb, a.stages) > TK_SMEM) --a.stages;
+    const size_t smem = tk_smem_bytes(nkb, a.stages);
+    CUtensorMap mqh, mql, mxh, mxl;
+    if (!make_map_bf16_rows(&mqh, Qh, nq_pad, ldbf, TK_BM) ||
+        !make_map_bf16_rows(&mql, Ql, nq_pad, ldbf, TK_BM) ||
+        !make_map_bf16_rows(&mxh, Xh, nx, ldbf, TK_ROWS, 1) ||
+        !make_map_bf16_rows(&mxl, Xl, nx, ldbf, TK_ROWS, 1))
+        return cudaErrorInvalidValue;
+    const auto kern = knn_tc_kernel<false, TK_MASK>;
+    const cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kern), smem);
+    if (e != cudaSuccess) return e;
+    kern<<<a.n_items, TK_THREADS, smem, s>>>(mqh, mql, mxh, mxl, a);
+    return cudaGetLastError();
+}
+cudaError_t launch_radius_cand_scan(const int *cnt, int nq, long long *off, long long *total,
+                                    cudaStream_t s) {
+    radius_cand_scan<<<1, 1024, 0, s>>>(cnt, nq, off, total);
+    return cudaGetLastError();
+}
+cudaError_t launch_radius_exact(const float *X, int nx, int ld, int d, const float *Q, int nq,
+                                int kc, float thr, const unsigned *mask, const int *cnt,
+                                const long long *off, int *hits, int *idx, float *val,
+                                cudaStream_t s) {
+    const size_t smem = (size_t)((d + 3) & ~3) * sizeof(float);
+    radius_exact_kernel<<<nq, RX_THREADS, smem, s>>>(X, Q, ld, d, kc, thr, mask,
+                                                     radius_tc_words(nx), cnt, off, hits, idx, val);
     return cudaGetLastError();
 }
 

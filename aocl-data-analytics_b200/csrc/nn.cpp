@@ -290,6 +290,29 @@ template <typename T> da_status NN<T>::ensure_device_data() {
     return da_status_success;
 }
 
+// The training rows' tensor-core copies: bf16 rows of d rounded up to 8 (at
+// least 64): no padded K block is stored or read (the tensor maps zero-fill past
+// the row).  cudaErrorMemoryAllocation: nothing was built.
+template <typename T> cudaError_t NN<T>::tc_train_copies(da_int d) {
+    if constexpr (std::is_same_v<T, float>) {
+        const int ldbf = d <= 64 ? 64 : (int)((d + 7) / 8 * 8);
+        if (tc_train_ready && tc_ldbf == ldbf) return cudaSuccess;
+        const size_t xb = (size_t)n_samples * ldbf * 2;
+        tc_train_ready = false;
+        tc_ldbf = ldbf;
+        if (!dXh.ensure(xb) || !dXl.ensure(xb) || !dXsq.ensure((size_t)n_samples * 4) ||
+            !dTkScal.ensure(64))
+            return cudaErrorMemoryAllocation;
+        const cudaError_t e = launch_knn_tc_train_prep(
+            dX.as<float>(), ld, (int)n_samples, (int)d, dXh.p, dXl.p, ldbf, dXsq.as<float>(),
+            dTkScal.as<float>(), cuda->stream);
+        tc_train_ready = e == cudaSuccess;
+        return e;
+    } else {
+        return cudaErrorNotSupported;
+    }
+}
+
 // Tensor-core candidate pass + exact re-score (knn_tc.cu) into dOutK (indices after the distances),
 // in query batches that bound the candidate lists' memory; n_extra ints of
 // state follow the indices, for tc_finish.
@@ -315,21 +338,11 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
             B200_TRY(launch_recip(dXn.as<float>(), (int)n_samples, dXinv.as<float>(), st),
                      "norms");
         }
-        // bf16 rows of d rounded up to 8 (at least 64): no padded K block is
-        // stored or read (the tensor maps zero-fill past the row)
-        const int ldbf = d <= 64 ? 64 : (int)((d + 7) / 8 * 8);
-        if (!tc_train_ready || tc_ldbf != ldbf) {
-            tc_ldbf = ldbf;
-            const size_t xb = (size_t)n_samples * tc_ldbf * 2;
-            if (!dXh.ensure(xb) || !dXl.ensure(xb) || !dXsq.ensure((size_t)n_samples * 4) ||
-                !dTkScal.ensure(64))
-                return err->error(da_status_memory_error, "Device memory allocation failed.");
-            B200_TRY(launch_knn_tc_train_prep(dX.as<float>(), ld, (int)n_samples, (int)d, dXh.p,
-                                              dXl.p, tc_ldbf, dXsq.as<float>(),
-                                              dTkScal.as<float>(), st),
-                     "tensor-core training copies");
-            tc_train_ready = true;
-        }
+        const cudaError_t te = tc_train_copies(d);
+        if (te == cudaErrorMemoryAllocation)
+            return err->error(da_status_memory_error, "Device memory allocation failed.");
+        B200_TRY(te, "tensor-core training copies");
+        const int ldbf = tc_ldbf;
         // batches of queries; their state words and list lengths follow the
         // indices and come back with them (tc_finish)
         const da_int qb = std::min<da_int>(nq, KNN_TC_BATCH);
@@ -721,6 +734,100 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
     return da_status_success;
 }
 
+// The queries Q (nq rows on the device) on the tensor cores: the rows that may
+// be within thr, then their exact distances (knn_tc.cu).  Not taken where a
+// buffer is not to be had, where a query has no finite threshold, and from one
+// pair in eight on, where re-scoring them one by one costs what the plain
+// path's block does.
+template <typename T>
+da_status NN<T>::radius_tc(da_int nq, da_int d, const T *Q, T thr, int kc, bool want_val,
+                           da_int *cnt_out, long long *start_out, std::vector<da_int> &idx_out,
+                           std::vector<T> &val_out, bool &done) {
+    done = false;
+    if constexpr (std::is_same_v<T, float>) {
+        cudaStream_t st = cuda->stream;
+        const cudaError_t te = tc_train_copies(d);
+        if (te == cudaErrorMemoryAllocation) return da_status_success;
+        B200_TRY(te, "tensor-core training copies");
+        const int n = (int)n_samples, words = radius_tc_words(n);
+        // state words, their number of candidates; offsets; per query counts
+        // of candidates and hits
+        struct Head {
+            int state[KNN_TC_STATE];
+            long long total;
+        } head;
+        const size_t off_at = 64, hit_at = off_at + (size_t)nq * 8, cnt_at = hit_at + (size_t)nq * 4;
+        if (!dTkQ.ensure(radius_tc_query_bytes((int)nq, tc_ldbf)) ||
+            !dD.ensure((size_t)nq * words * 4) || !dRs.ensure(cnt_at + (size_t)nq * 4))
+            return da_status_success;
+        char *w = dRs.as<char>();
+        int *state = reinterpret_cast<int *>(w), *hits = reinterpret_cast<int *>(w + hit_at),
+            *cnt = reinterpret_cast<int *>(w + cnt_at);
+        long long *off = reinterpret_cast<long long *>(w + off_at);
+        B200_TRY(cuda->timed("radius_distances", [&] {
+            return launch_radius_tc(dXh.p, dXl.p, dXsq.as<float>(), dTkScal.as<float>(), n, ld,
+                                    tc_ldbf, (int)d, Q, (int)nq, thr, dTkQ.p, dD.as<unsigned>(),
+                                    cnt, state, st);
+        }), "radius search's tensor-core pass");
+        B200_TRY(cuda->timed("radius_count", [&] {
+            return launch_radius_cand_scan(cnt, (int)nq, off,
+                                           reinterpret_cast<long long *>(w + sizeof(head.state)), st);
+        }), "count");
+        B200_TRY(cudaMemcpyAsync(&head, w, sizeof(head), cudaMemcpyDeviceToHost, st), "copy");
+        B200_TRY(cudaStreamSynchronize(st), "radius search");
+        if (head.state[1] != 0)
+            return err->error(da_status_internal_error,
+                              "The radius search's tensor-core kernel timed out waiting on a "
+                              "pipeline barrier (code " + std::to_string(head.state[1]) + ").");
+        const size_t tot = (size_t)head.total;
+        if (tot > (size_t)nq * n / 8) return da_status_success;
+        if (!dRi.ensure(std::max<size_t>(tot, 1) * sizeof(int)) ||
+            !dRv.ensure(std::max<size_t>(tot, 1) * sizeof(T)))
+            return da_status_success;
+        B200_TRY(cuda->timed("radius_emit", [&] {
+            return launch_radius_exact(dX.as<float>(), n, ld, (int)d, Q, (int)nq, kc, thr,
+                                       dD.as<unsigned>(), cnt, off, hits, dRi.as<int>(),
+                                       dRv.as<float>(), st);
+        }), "compaction");
+        std::vector<char> meta(cnt_at - off_at);
+        B200_TRY(cudaMemcpyAsync(meta.data(), off, meta.size(), cudaMemcpyDeviceToHost, st), "copy");
+        size_t at = idx_out.size();
+        const size_t from = at;
+        idx_out.resize(at + tot);
+        if (want_val) val_out.resize(at + tot);
+        if (tot > 0) {
+            B200_TRY(download_ints(dRi.as<int>(), tot, idx_out.data() + at, st), "copy");
+            if (want_val)
+                B200_TRY(copy_down({val_out.data() + at, tot * sizeof(T), dRv.p, tot * sizeof(T),
+                                    tot * sizeof(T), 1}, st), "copy");
+        }
+        B200_TRY(cudaStreamSynchronize(st), "radius search");
+        // a query's hits are its first candidates: move them together
+        const long long *ho = reinterpret_cast<const long long *>(meta.data());
+        const int *hh = reinterpret_cast<const int *>(meta.data() + (hit_at - off_at));
+        for (da_int i = 0; i < nq; ++i) {
+            start_out[i] = (long long)at;
+            cnt_out[i] = (da_int)hh[i];
+            const size_t o = from + (size_t)ho[i];
+            if (o != at) {
+                std::copy(idx_out.begin() + o, idx_out.begin() + o + hh[i], idx_out.begin() + at);
+                if (want_val)
+                    std::copy(val_out.begin() + o, val_out.begin() + o + hh[i],
+                              val_out.begin() + at);
+            }
+            at += (size_t)hh[i];
+        }
+        idx_out.resize(at);
+        if (want_val) val_out.resize(at);
+        cuda->stats["tensor_core"] = 1.0;
+        done = true;
+    } else {
+        (void)nq, (void)d, (void)Q, (void)thr, (void)kc, (void)want_val, (void)cnt_out;
+        (void)start_out, (void)idx_out, (void)val_out;
+    }
+    return da_status_success;
+}
+
 // Core of the radius search (radius_neighbors_compute, nearest_neighbors.cpp:
 // 1983-2068): per query its count and start in the flat index / value arrays,
 // rows in index order; values (only when want_val) as computed, squared for
@@ -777,8 +884,38 @@ da_status NN<T>::radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T 
         qn = dQn.as<T>();
         xn = dXn.as<T>();
     }
-    // query blocks whose distance rows fit in 256 MB
+    cuda->stats["tensor_core"] = 0.0;
     const size_t n = (size_t)n_samples;
+    // testing hook: the offsets' waits run out (AOCLDA_B200_TEST_RADIUS_WAIT=1)
+    const char *tw = std::getenv("AOCLDA_B200_TEST_RADIUS_WAIT");
+    const int test_wait = (tw && tw[0] == '1') ? 1 : 0;
+    // the tensor-core path, block by block until one is not taken; in blocks
+    // whose masks fit in 256 MB.  The rule is that of kneighbors (200,000 x 64,
+    // one query: 117 us, the plain path 189; 16,384 x 64, 512 queries: 125
+    // against 180), once the copies of the training rows exist or the handle's
+    // radius searches come to 4e9 multiply-adds: the copies and buffers cost
+    // 0.6 ms to set up, what a search of that size saves (3.1 -> 0.9 ms at
+    // 1.3e10, 200,000 x 32, 2,000 queries).
+    da_int first = 0;
+    const double work = (double)n * (double)std::max<da_int>(nq, 64) * (double)d;
+    if (!fp64 && acc == ACC_SQEUC && std::isfinite((double)thr) && test_wait == 0 &&
+        opts.key("precision mode") != 0 && knn_tc_supported((int)n, (int)d, 1) && n >= 16384 &&
+        work >= 5.0e8 && (tc_train_ready || (radius_work += work) >= 4.0e9)) {
+        da_int Bt = (da_int)std::max<size_t>(
+            1, std::min<size_t>({(size_t)nq, (256u << 20) / ((size_t)radius_tc_words((int)n) * 4),
+                                 (size_t)65535}));
+        if (Bt < nq && Bt > 128) Bt -= Bt % 128;
+        bool done = true;
+        while (done && first < nq) {
+            const da_int b = std::min<da_int>(Bt, nq - first);
+            s = radius_tc(b, d, dQ.as<T>() + (size_t)first * ld, thr, kc, want_val,
+                          cnt_out.data() + first, start_out.data() + first, idx_out, val_out, done);
+            if (s != da_status_success) return s;
+            if (done) first += b;
+        }
+        if (first == nq) return da_status_success;
+    }
+    // query blocks whose distance rows fit in 256 MB
     // (at most 65,535 rows: the count / compaction grids put the rows on y)
     // (and a whole number of the distance kernel's 64-row tiles when there
     // are more queries: a partial last tile row costs a full one)
@@ -791,9 +928,6 @@ da_status NN<T>::radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T 
         !dRs.ensure((size_t)B * nch * sizeof(long long)) ||
         !dRh.ensure((size_t)B * nch * sizeof(int)))
         return err->error(da_status_memory_error, "Device memory allocation failed.");
-    // testing hook: the offsets' waits run out (AOCLDA_B200_TEST_RADIUS_WAIT=1)
-    const char *tw = std::getenv("AOCLDA_B200_TEST_RADIUS_WAIT");
-    const int test_wait = (tw && tw[0] == '1') ? 1 : 0;
     std::vector<long long> start((size_t)B * nch + 2);
     // the distance kernel also counts each (row, chunk) piece's hits
     PairwiseArgs pa{acc, post, kc, (double)p, false, true};
@@ -802,7 +936,7 @@ da_status NN<T>::radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T 
     long long *d_total = reinterpret_cast<long long *>(dRc.as<char>() +
                                                        radius_scan_work_bytes((int)B, (int)n));
     int *d_err = reinterpret_cast<int *>(d_total + 1);
-    for (da_int q0 = 0; q0 < nq; q0 += B) {
+    for (da_int q0 = first; q0 < nq; q0 += B) {
         const int b = (int)std::min<da_int>(B, nq - q0);
         B200_TRY(cudaMemsetAsync(dRh.p, 0, (size_t)b * nch * sizeof(int), st), "memset");
         B200_TRY(cuda->timed("radius_distances", [&] {
