@@ -224,7 +224,8 @@ struct KmeansWork {
     double *scalars;      // [0]=normc^2 [1]=shift^2 [2]=inertia ...
     int *flags;           // [0]=labels changed [1]=n_empty
 };
-int kmeans_assign_block_rows();
+int kmeans_sort_block_rows(int k);
+struct LloydLoopState;
 int kmeans_max_clusters_fused();
 // Lloyd assignment: label_i = argmin_j (|c_j|^2 - 2 x_i.c_j), ties -> lower j.
 // Also writes per-block label histograms (for the counting sort) and raises
@@ -242,12 +243,15 @@ cudaError_t launch_kmeans_sort(const int *labels, int n, int k, const int *block
 // cluster, combined in chunk order; C_new = sum / max(count,1) (an empty
 // cluster becomes the zero vector, kmeans_lloyd.hpp:364-377).  Also computes
 // |C_prev|_F^2 and |C_prev - C_new|_F^2 in fp64 into scalars[0], scalars[1].
+// With ls (the Lloyd loop as a CUDA graph) it also makes the convergence test of
+// iteration ls->it, as launch_kmeans_update_fx_loop does.
 template <typename T>
 cudaError_t launch_kmeans_update(const T *X, int ldx, int n, int d, int k,
                                  const int *sorted_rows, const int *offsets,
                                  const int *seg_chunk_start, int seg_rows, double *chunk_sums,
                                  const int *counts, const T *C_prev, T *C_new, int ldc,
-                                 double *scalars, int *flags, cudaStream_t s);
+                                 double *scalars, int *flags, cudaStream_t s,
+                                 LloydLoopState *ls = nullptr, unsigned long long cond = 0);
 // Fixed-point centroid update for fp32 data (order-independent integer sums,
 // so deterministic without sorting): supported when the shared-memory
 // accumulators (k x d int64) fit.  launch_col_absmax gives the per-feature

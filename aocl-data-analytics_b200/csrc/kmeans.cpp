@@ -143,7 +143,7 @@ template <typename T> da_status KMeans<T>::set_init_centres(const T *C, da_int l
 
 template <typename T> da_status KMeans<T>::alloc_work() {
     const size_t n = n_samples, k = n_clusters;
-    const size_t nblk = (n + kmeans_assign_block_rows() - 1) / kmeans_assign_block_rows();
+    const size_t rows = (size_t)kmeans_sort_block_rows((int)k), nblk = (n + rows - 1) / rows;
     const size_t nchunks = n / SEG_ROWS + k + 1;
     const size_t nfin = (k * n_features + 255) / 256;
     bool ok = dC0.ensure(k * ld * sizeof(T)) && dC1.ensure(k * ld * sizeof(T)) &&
@@ -777,6 +777,43 @@ template <typename T> void KMeans<T>::drop_loop_graph() {
     loop_key.clear();
 }
 
+// A graph of one WHILE node, its body captured from st by launches(cond).
+template <typename F>
+static bool while_graph(cudaStream_t st, cudaGraph_t &graph, cudaGraphExec_t &exec, F launches) {
+    cudaGraph_t g = nullptr;
+    if (cudaGraphCreate(&g, 0) != cudaSuccess) return false;
+    cudaGraphConditionalHandle cond = 0;
+    cudaGraphNodeParams p = {};
+    cudaGraphNode_t node;
+    bool ok = cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+    if (ok) {
+        p.type = cudaGraphNodeTypeConditional;
+        p.conditional.handle = cond;
+        p.conditional.type = cudaGraphCondTypeWhile;
+        p.conditional.size = 1;
+        ok = cudaGraphAddNode(&node, g, nullptr, 0, &p) == cudaSuccess;
+    }
+    cudaGraph_t body = ok ? p.conditional.phGraph_out[0] : nullptr;
+    if (ok)
+        ok = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
+                                           cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    if (ok) {
+        const bool launched = launches((unsigned long long)cond);
+        cudaGraph_t captured = nullptr;
+        const bool ended = cudaStreamEndCapture(st, &captured) == cudaSuccess;
+        ok = launched && ended;
+    }
+    if (ok) ok = cudaGraphInstantiate(&exec, g, 0) == cudaSuccess;
+    if (!ok) {
+        cudaGetLastError();
+        exec = nullptr;
+        cudaGraphDestroy(g);
+        return false;
+    }
+    graph = g;
+    return true;
+}
+
 template <typename T> bool KMeans<T>::build_loop_graph(T *dC, int *dL) {
     if constexpr (!std::is_same_v<T, float>) {
         (void)dC, (void)dL;
@@ -784,31 +821,13 @@ template <typename T> bool KMeans<T>::build_loop_graph(T *dC, int *dL) {
     } else {
         cudaStream_t st = cuda->stream;
         const int n = n_samples, k = n_clusters, d = n_features;
-        cudaGraph_t g = nullptr;
-        if (cudaGraphCreate(&g, 0) != cudaSuccess) return false;
-        cudaGraphConditionalHandle cond = 0;
-        cudaGraphNodeParams p = {};
-        cudaGraphNode_t node;
-        bool ok = cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault) ==
-                  cudaSuccess;
-        if (ok) {
-            p.type = cudaGraphNodeTypeConditional;
-            p.conditional.handle = cond;
-            p.conditional.type = cudaGraphCondTypeWhile;
-            p.conditional.size = 1;
-            ok = cudaGraphAddNode(&node, g, nullptr, 0, &p) == cudaSuccess;
-        }
-        cudaGraph_t body = ok ? p.conditional.phGraph_out[0] : nullptr;
-        if (ok)
-            ok = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
-                                               cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-        if (ok) {
+        const bool ok = while_graph(st, loop_graph, loop_exec, [&](unsigned long long cond) {
             // the assignment lists its changed rows for the incremental update;
             // the centre norms come with the operands (aaug_ready: iteration 0
             // set the constant operand), the counters are re-armed by the
             // finalize of the previous iteration (and before the graph starts)
             chg_capture = true;
-            bool launched = aaug_ready && assign(dC, dL, dL) == da_status_success;
+            const bool launched = aaug_ready && assign(dC, dL, dL) == da_status_success;
             chg_capture = false;
             ChangeList chg;
             chg.count = dChg.as<int>();
@@ -822,29 +841,75 @@ template <typename T> bool KMeans<T>::build_loop_graph(T *dC, int *dL) {
             amb.ncand = amb.rows + n;
             amb.cand = amb.rows + 2 * (size_t)n;
             amb.count = reinterpret_cast<const int *>(dTcScal.as<char>() + 16);
-            launched = launched &&
-                       launch_kmeans_update_fx_loop(
-                           dX.as<float>(), ld, n, d, k, dL, reinterpret_cast<const float *>(scale),
-                           scale + d, dFxAcc.p, dC, dCounts.as<int>(), dScalars.as<double>() + 8,
-                           dScalars.as<double>(), dFlags.as<int>(), dFxTicket.as<unsigned>(),
-                           dLoop.as<LloydLoopState>(), (unsigned long long)cond, chg,
-                           reinterpret_cast<int *>(dTcScal.as<char>() + 16), dCn.as<float>(), amb,
-                           chg.news + chg_cap, st) == cudaSuccess;
-            cudaGraph_t captured = nullptr;
-            const bool ended = cudaStreamEndCapture(st, &captured) == cudaSuccess;
-            ok = launched && ended;
-        }
-        if (ok) ok = cudaGraphInstantiate(&loop_exec, g, 0) == cudaSuccess;
-        if (!ok) {
-            cudaGetLastError();
-            err->clear();
-            loop_exec = nullptr;
-            cudaGraphDestroy(g);
-            return false;
-        }
-        loop_graph = g;
-        return true;
+            return launched &&
+                   launch_kmeans_update_fx_loop(
+                       dX.as<float>(), ld, n, d, k, dL, reinterpret_cast<const float *>(scale),
+                       scale + d, dFxAcc.p, dC, dCounts.as<int>(), dScalars.as<double>() + 8,
+                       dScalars.as<double>(), dFlags.as<int>(), dFxTicket.as<unsigned>(),
+                       dLoop.as<LloydLoopState>(), cond, chg,
+                       reinterpret_cast<int *>(dTcScal.as<char>() + 16), dCn.as<float>(), amb,
+                       chg.news + chg_cap, st) == cudaSuccess;
+        });
+        if (!ok) err->clear();
+        return ok;
     }
+}
+
+// The loop with the update by counting sort: in place too (a row's label and a
+// centre's element are read by the thread that then writes them).
+template <typename T> bool KMeans<T>::build_sort_graph(T *dC, int *dL) {
+    cudaStream_t st = cuda->stream;
+    const int n = n_samples, k = n_clusters, d = n_features;
+    const bool ok = while_graph(st, loop_graph, loop_exec, [&](unsigned long long cond) {
+        return launch_centre_norms<T>(dC, ld, k, d, dCn.as<T>(), st) == cudaSuccess &&
+               assign(dC, dL, dL) == da_status_success &&
+               launch_kmeans_sort(dL, n, k, dBlockCounts.as<int>(), dCounts.as<int>(),
+                                  dOffsets.as<int>(), dSegStart.as<int>(), SEG_ROWS,
+                                  dSorted.as<int>(), dFlags.as<int>(), st) == cudaSuccess &&
+               launch_kmeans_update<T>(update_rows(), ld, n, d, k, dSorted.as<int>(),
+                                       dOffsets.as<int>(), dSegStart.as<int>(), SEG_ROWS,
+                                       dChunkSums.as<double>(), dCounts.as<int>(), dC, dC, ld,
+                                       dScalars.as<double>(), dFlags.as<int>(), st,
+                                       dLoop.as<LloydLoopState>(), cond) == cudaSuccess;
+    });
+    if (!ok) err->clear();
+    return ok;
+}
+
+template <typename T>
+da_status KMeans<T>::lloyd_sort_graph(T *dC, int *dL, da_int &n_iter_out, int &converged, bool &ran) {
+    ran = false;
+    cudaStream_t st = cuda->stream;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return da_status_success; // the caller captures: run the host loop
+    }
+    if (!dLoop.ensure(sizeof(LloydLoopState))) return da_status_success;
+    const std::vector<uintptr_t> key = {
+        1, (uintptr_t)st, (uintptr_t)dC, (uintptr_t)dL, (uintptr_t)update_rows(),
+        (uintptr_t)dX.p, (uintptr_t)dCn.p, (uintptr_t)dFlags.p, (uintptr_t)dScalars.p,
+        (uintptr_t)dCounts.p, (uintptr_t)dLoop.p, (uintptr_t)dBlockCounts.p, (uintptr_t)dOffsets.p,
+        (uintptr_t)dSegStart.p, (uintptr_t)dSorted.p, (uintptr_t)dChunkSums.p,
+        (uintptr_t)n_samples, (uintptr_t)n_clusters, (uintptr_t)n_features, (uintptr_t)ld};
+    if (!loop_exec || key != loop_key) {
+        drop_loop_graph();
+        if (!build_sort_graph(dC, dL)) return da_status_success;
+        loop_key = key;
+    }
+    char *hb = static_cast<char *>(h_small);
+    LloydLoopState *hs = reinterpret_cast<LloydLoopState *>(hb + 128);
+    LloydLoopState *ho = reinterpret_cast<LloydLoopState *>(hb + 160);
+    *hs = LloydLoopState{1, (int)max_iter, 0, 0, (double)tol};
+    B200_TRY(cudaMemcpyAsync(dLoop.p, hs, sizeof(LloydLoopState), cudaMemcpyHostToDevice, st), "copy");
+    B200_TRY(cudaMemsetAsync(dFlags.p, 0, 8 * sizeof(int), st), "memset");
+    B200_TRY(cudaGraphLaunch(loop_exec, st), "Lloyd loop graph");
+    B200_TRY(cudaMemcpyAsync(ho, dLoop.p, sizeof(LloydLoopState), cudaMemcpyDeviceToHost, st), "copy");
+    B200_TRY(cudaStreamSynchronize(st), "Lloyd loop graph");
+    n_iter_out = ho->n_iter;
+    converged = ho->conv;
+    ran = true;
+    return da_status_success;
 }
 
 template <typename T>
@@ -940,14 +1005,15 @@ da_status KMeans<T>::run_lloyd(T *&dCcur, T *&dCprev, int *&dLcur, int *&dLprev,
     converged = 0;
     empty_found = false;
     // iterations 1.. as one graph launch where the loop allows it
-    const bool graph = use_fx && use_tc && empty_mode == EC_IGNORE && !cuda->timing && !sph;
+    const bool graph = use_fx == use_tc && empty_mode == EC_IGNORE && !cuda->timing && !sph;
     da_int it = 0;
     for (it = 0; it < max_iter; ++it) {
         if (graph && it == 1) {
             bool ran = false;
             da_int nit = 0;
             int conv = 0;
-            da_status s = lloyd_graph(dCcur, dLcur, nit, conv, ran);
+            da_status s = use_tc ? lloyd_graph(dCcur, dLcur, nit, conv, ran)
+                                 : lloyd_sort_graph(dCcur, dLcur, nit, conv, ran);
             if (s != da_status_success) return s;
             cuda->stats["graph_loop"] = ran ? 1.0 : 0.0;
             if (ran) {

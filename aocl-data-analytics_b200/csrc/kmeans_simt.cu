@@ -19,9 +19,10 @@
 
 namespace b200 {
 
-static constexpr int SORT_ROWS = 1024; // rows per counting-sort block
-
-int kmeans_assign_block_rows() { return SORT_ROWS; }
+// Rows per counting-sort block (one warp scatters them, 32 at a time: 98 blocks of
+// 1,024 took 12.5 us at 100,000 rows, 391 of 256 take 4.5); many clusters keep
+// the table of per-block counts small.
+int kmeans_sort_block_rows(int k) { return k <= 256 ? 256 : 1024; }
 int kmeans_max_clusters_fused() { return 1 << 20; }
 
 // ------------------------------------------------------------- assign ----
@@ -99,12 +100,92 @@ kmeans_assign_kernel(const T *X, int n, int ld, int d, const T *C, int k, const 
     if (tid == 0 && changed && flags) atomicOr(&flags[0], 1);
 }
 
+// Few clusters: a thread holds one row and AR_K values x.c at a time, the
+// centres pass through shared memory AR_D features at a time (every lane reads
+// the same address).  The tiles above score a whole tile of 64 (fp64) or 128
+// centres whatever k is.  Same chain over the features, same order of the
+// centres.  Bound by the FMAs and the shared-memory reads, a 16-byte read per 2
+// (fp64) or 4 of them: 37 -> 10 us at 100,000 x 20, k = 16 in fp64.
+constexpr int AR_THREADS = 128, AR_D = 32;
+template <typename T, int AR_K>
+__global__ void __launch_bounds__(AR_THREADS)
+kmeans_assign_rows_kernel(const T *X, int n, int ld, int d, const T *C, int k, const T *cnorm,
+                          int *labels, const int *labels_prev, int *flags) {
+    __shared__ __align__(16) T cs[AR_D][AR_K + 16 / sizeof(T)]; // filled along f
+    const int i = blockIdx.x * AR_THREADS + threadIdx.x;
+    const T *x = X + (size_t)min(i, n - 1) * ld;
+    T best = Lim<T>::inf();
+    int bidx = 0x7fffffff;
+    for (int j0 = 0; j0 < k; j0 += AR_K) {
+        T acc[AR_K];
+#pragma unroll
+        for (int j = 0; j < AR_K; ++j) acc[j] = T(0);
+        for (int f0 = 0; f0 < d; f0 += AR_D) {
+            const int nf = min(AR_D, d - f0);
+            __syncthreads();
+            for (int e = threadIdx.x; e < AR_D * AR_K; e += AR_THREADS) {
+                const int f = e % AR_D, j = e / AR_D;
+                if (f < nf) cs[f][j] = j0 + j < k ? C[(size_t)(j0 + j) * ld + f0 + f] : T(0);
+            }
+            __syncthreads();
+            // rows are padded to whole groups of four
+            for (int g = 0; g < nf; g += 4) {
+                const V4<T> xv = ld4_global(x + f0 + g);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (g + u >= nf) break;
+#pragma unroll
+                    for (int j = 0; j < AR_K; j += 4) {
+                        const V4<T> cv = ld4_shared(&cs[g + u][j]);
+#pragma unroll
+                        for (int w = 0; w < 4; ++w)
+                            acc[j + w] = fma_rn(xv.v[u], cv.v[w], acc[j + w]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < AR_K; ++j) {
+            if (j0 + j >= k) break;
+            const T v = fma_rn(T(-2), acc[j], cnorm[j0 + j]);
+            if (key_less(v, j0 + j, best, bidx)) {
+                best = v;
+                bidx = j0 + j;
+            }
+        }
+    }
+    int ch = 0;
+    if (i < n) {
+        const int lbl = bidx == 0x7fffffff ? 0 : bidx; // NaN distances, as above
+        if (labels_prev && labels_prev[i] != lbl) ch = 1;
+        labels[i] = lbl;
+    }
+    ch = __syncthreads_or(ch);
+    if (threadIdx.x == 0 && ch && flags) atomicOr(&flags[0], 1);
+}
+// Where it is the faster one (100,000 x 32, k = 16: 22 us against 53 in fp64, 16
+// against 34 in fp32; k = 32: 37 against 53, 21 against 34; k = 48: equal; 20,000 x
+// 8: k = 16 9 against 12 and 9 against 10, k = 32 13 against 12 and 10.6 against
+// 9.9; a kernel timed by events, 5 us of it the launch).
+bool assign_by_rows(int n, int k) { return k <= 16 || (k <= 32 && n >= 65536); }
+
 template <typename T>
 cudaError_t launch_kmeans_assign(const T *X, int ldx, int n, int d, const T *C, int ldc, int k,
                                  const T *cnorm, int *labels, const int *labels_prev,
                                  int *block_counts, int *flags, cudaStream_t s) {
     (void)block_counts;
     if (ldx != ldc) return cudaErrorInvalidValue;
+    if (assign_by_rows(n, k)) {
+        constexpr int AR_K = sizeof(T) == 8 ? 16 : 32;
+        const int nb = (n + AR_THREADS - 1) / AR_THREADS;
+        if (k <= AR_K / 2)
+            kmeans_assign_rows_kernel<T, AR_K / 2><<<nb, AR_THREADS, 0, s>>>(
+                X, n, ldx, d, C, k, cnorm, labels, labels_prev, flags);
+        else
+            kmeans_assign_rows_kernel<T, AR_K><<<nb, AR_THREADS, 0, s>>>(
+                X, n, ldx, d, C, k, cnorm, labels, labels_prev, flags);
+        return cudaGetLastError();
+    }
     using Cf = SimtCfg<T>;
     constexpr int BM = 16 * Cf::TM;
     kmeans_assign_kernel<T><<<(n + BM - 1) / BM, 256, 0, s>>>(X, n, ldx, d, C, k, cnorm, labels,
@@ -113,37 +194,86 @@ cudaError_t launch_kmeans_assign(const T *X, int ldx, int n, int d, const T *C, 
 }
 
 // ------------------------------------------------------- counting sort ---
-// (1) per SORT_ROWS block histogram of labels.
-__global__ void label_hist_kernel(const int *labels, int n, int k, int *block_counts) {
+// (1) per block of `rows` rows, the histogram of labels.
+__global__ void label_hist_kernel(const int *labels, int n, int k, int rows, int *block_counts) {
     extern __shared__ int h[];
     for (int j = threadIdx.x; j < k; j += blockDim.x) h[j] = 0;
     __syncthreads();
-    const int r0 = blockIdx.x * SORT_ROWS;
-    const int r1 = min(n, r0 + SORT_ROWS);
+    const int r0 = blockIdx.x * rows;
+    const int r1 = min(n, r0 + rows);
     for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) atomicAdd(&h[labels[i]], 1);
     __syncthreads();
     for (int j = threadIdx.x; j < k; j += blockDim.x)
         block_counts[(size_t)blockIdx.x * k + j] = h[j];
 }
-// (2) one warp per cluster: exclusive scan of its block counts (in place).
+// (2) one warp per cluster: exclusive scan of its block counts (in place), eight
+// loads in flight.  The cluster's rows.
+__device__ __forceinline__ int scan_block_counts(int *block_counts, int nblocks, int k, int j) {
+    const int lane = threadIdx.x & 31;
+    int carry = 0;
+    constexpr int U = 8;
+    for (int b0 = 0; b0 < nblocks; b0 += U * 32) {
+        int v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int b = b0 + u * 32 + lane;
+            v[u] = (b < nblocks) ? block_counts[(size_t)b * k + j] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int b = b0 + u * 32 + lane;
+            int x = v[u];
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, off);
+                if (lane >= off) x += y;
+            }
+            if (b < nblocks) block_counts[(size_t)b * k + j] = carry + x - v[u];
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+    }
+    return carry;
+}
 __global__ void block_scan_kernel(int *block_counts, int nblocks, int k, int *counts) {
     const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
     if (j >= k) return;
-    int carry = 0;
-    for (int b0 = 0; b0 < nblocks; b0 += 32) {
-        const int b = b0 + lane;
-        const int v = (b < nblocks) ? block_counts[(size_t)b * k + j] : 0;
-        int x = v;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        if (b < nblocks) block_counts[(size_t)b * k + j] = carry + x - v;
-        carry += __shfl_sync(0xffffffffu, x, 31);
+    const int c = scan_block_counts(block_counts, nblocks, k, j);
+    if ((threadIdx.x & 31) == 0) counts[j] = c;
+}
+// (2) and (3) for at most 32 clusters: one block, a warp per cluster, then the
+// offsets by one of them.
+__global__ void __launch_bounds__(1024)
+small_offsets_kernel(int *block_counts, int nblocks, int k, int *counts, int seg_rows,
+                     int *offsets, int *seg_chunk_start, int *flags) {
+    __shared__ int total[32];
+    const int j = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (j < k) {
+        const int c = scan_block_counts(block_counts, nblocks, k, j);
+        if (lane == 0) total[j] = c;
     }
-    if (lane == 0) counts[j] = carry;
+    __syncthreads();
+    if (j != 0) return;
+    const int c = lane < k ? total[lane] : 0, sc = (c + seg_rows - 1) / seg_rows;
+    int a = c, b = sc;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int ya = __shfl_up_sync(0xffffffffu, a, off), yb = __shfl_up_sync(0xffffffffu, b, off);
+        if (lane >= off) {
+            a += ya;
+            b += yb;
+        }
+    }
+    if (lane < k) {
+        counts[lane] = c;
+        offsets[lane] = a - c;
+        seg_chunk_start[lane] = b - sc;
+    }
+    const unsigned empty = __ballot_sync(0xffffffffu, lane < k && c == 0);
+    if (lane == 31) {
+        offsets[k] = a;
+        seg_chunk_start[k] = b;
+        if (flags) flags[1] = __popc(empty);
+    }
 }
 // (3) single CTA: cluster offsets and per-cluster segment-chunk starts.
 __global__ void cluster_offsets_kernel(const int *counts, int k, int seg_rows, int *offsets,
@@ -191,16 +321,17 @@ __global__ void cluster_offsets_kernel(const int *counts, int k, int seg_rows, i
     __syncthreads();
     if (threadIdx.x == 0 && flags) flags[1] = s_empty;
 }
-// (4) one warp per SORT_ROWS block: stable scatter of row ids.
-__global__ void label_scatter_kernel(const int *labels, int n, int k, const int *block_offsets,
-                                     const int *offsets, int *sorted_rows) {
+// (4) one warp per block of rows: stable scatter of row ids.
+__global__ void label_scatter_kernel(const int *labels, int n, int k, int rows,
+                                     const int *block_offsets, const int *offsets,
+                                     int *sorted_rows) {
     extern __shared__ int ctr[];
     const int b = blockIdx.x;
     const int lane = threadIdx.x;
     for (int j = lane; j < k; j += 32) ctr[j] = offsets[j] + block_offsets[(size_t)b * k + j];
     __syncwarp();
-    const int r0 = b * SORT_ROWS;
-    const int r1 = min(n, r0 + SORT_ROWS);
+    const int r0 = b * rows;
+    const int r1 = min(n, r0 + rows);
     for (int base = r0; base < r1; base += 32) {
         const int i = base + lane;
         const bool valid = i < r1;
@@ -222,13 +353,19 @@ cudaError_t launch_kmeans_sort(const int *labels, int n, int k, const int *block
                                int *counts, int *offsets, int *seg_chunk_start, int seg_rows,
                                int *sorted_rows, int *flags, cudaStream_t s) {
     int *block_counts = const_cast<int *>(block_counts_in);
-    const int nblocks = (n + SORT_ROWS - 1) / SORT_ROWS;
+    const int rows = kmeans_sort_block_rows(k);
+    const int nblocks = (n + rows - 1) / rows;
     const size_t hs = (size_t)k * sizeof(int);
-    label_hist_kernel<<<nblocks, 256, hs, s>>>(labels, n, k, block_counts);
-    block_scan_kernel<<<(k * 32 + 255) / 256, 256, 0, s>>>(block_counts, nblocks, k, counts);
-    cluster_offsets_kernel<<<1, 1024, 0, s>>>(counts, k, seg_rows, offsets, seg_chunk_start,
-                                              flags);
-    label_scatter_kernel<<<nblocks, 32, hs, s>>>(labels, n, k, block_counts, offsets,
+    label_hist_kernel<<<nblocks, 256, hs, s>>>(labels, n, k, rows, block_counts);
+    if (k <= 32) {
+        small_offsets_kernel<<<1, 1024, 0, s>>>(block_counts, nblocks, k, counts, seg_rows, offsets,
+                                                seg_chunk_start, flags);
+    } else {
+        block_scan_kernel<<<(k * 32 + 255) / 256, 256, 0, s>>>(block_counts, nblocks, k, counts);
+        cluster_offsets_kernel<<<1, 1024, 0, s>>>(counts, k, seg_rows, offsets, seg_chunk_start,
+                                                  flags);
+    }
+    label_scatter_kernel<<<nblocks, 32, hs, s>>>(labels, n, k, rows, block_counts, offsets,
                                                  sorted_rows);
     return cudaGetLastError();
 }
@@ -254,15 +391,54 @@ __global__ void seg_sum_kernel(const T *X, int ld, int d, int k, const int *sort
     const int r_begin = offsets[j] + (w - seg_chunk_start[j]) * seg_rows;
     const int r_end = min(offsets[j + 1], r_begin + seg_rows);
     double *out = chunk_sums + (size_t)w * ld;
+    // the sums of one row order, NC features a lane; U rows' loads in flight (a
+    // row at a time waits for its id, then for its features)
+    if (d <= 32) {
+        constexpr int U = 16;
+        const int c = min(lane, d - 1);
+        double a = 0;
+        for (int r0 = r_begin; r0 < r_end; r0 += 32) {
+            const int m = min(32, r_end - r0);
+            const int id = sorted_rows[r0 + min(lane, m - 1)];
+            for (int u0 = 0; u0 < m; u0 += U) {
+                T v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) // past the end: the last row, not added
+                    v[u] = X[(size_t)__shfl_sync(0xffffffffu, id, u0 + u) * ld + c];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (u0 + u < m) a += (double)v[u];
+            }
+        }
+        if (lane < d) out[lane] = a;
+        return;
+    }
     for (int d0 = 0; d0 < d; d0 += 128) {
+        constexpr int U = 4;
         double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
         const int c0 = d0 + lane, c1 = c0 + 32, c2 = c0 + 64, c3 = c0 + 96;
-        for (int r = r_begin; r < r_end; ++r) {
-            const T *x = X + (size_t)sorted_rows[r] * ld;
-            if (c0 < d) a0 += (double)x[c0];
-            if (c1 < d) a1 += (double)x[c1];
-            if (c2 < d) a2 += (double)x[c2];
-            if (c3 < d) a3 += (double)x[c3];
+        for (int r0 = r_begin; r0 < r_end; r0 += 32) {
+            const int m = min(32, r_end - r0);
+            const int id = sorted_rows[r0 + min(lane, m - 1)];
+            for (int u0 = 0; u0 < m; u0 += U) {
+                T v[U][4];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const T *x = X + (size_t)__shfl_sync(0xffffffffu, id, u0 + u) * ld;
+                    v[u][0] = x[min(c0, d - 1)];
+                    v[u][1] = x[min(c1, d - 1)];
+                    v[u][2] = x[min(c2, d - 1)];
+                    v[u][3] = x[min(c3, d - 1)];
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (u0 + u >= m) break;
+                    a0 += (double)v[u][0];
+                    a1 += (double)v[u][1];
+                    a2 += (double)v[u][2];
+                    a3 += (double)v[u][3];
+                }
+            }
         }
         if (c0 < d) out[c0] = a0;
         if (c1 < d) out[c1] = a1;
@@ -282,8 +458,17 @@ __global__ void centre_finalize_kernel(int k, int d, int ld, const int *counts,
     if (e < k * d) {
         const int j = e / d, f = e % d;
         double sum = 0.0;
-        for (int c = seg_chunk_start[j]; c < seg_chunk_start[j + 1]; ++c)
-            sum += chunk_sums[(size_t)c * ld + f];
+        const int c1 = seg_chunk_start[j + 1];
+        constexpr int U = 8; // loads in flight, sums in order (32: slower, by its code)
+        int c = seg_chunk_start[j];
+        for (; c + U <= c1; c += U) {
+            double v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = chunk_sums[(size_t)(c + u) * ld + f];
+#pragma unroll
+            for (int u = 0; u < U; ++u) sum += v[u];
+        }
+        for (; c < c1; ++c) sum += chunk_sums[(size_t)c * ld + f];
         const int cnt = counts[j];
         const T cn = T(sum / (double)(cnt > 0 ? cnt : 1));
         const size_t o = (size_t)j * ld + f;
@@ -321,13 +506,48 @@ __global__ void sum_partials_kernel(const double *partials, int nblocks, int str
     }
 }
 
+// The convergence test of iteration ls->it inside the graph loop (scalars[0..1] =
+// |C_prev|^2 and |C_prev - C_new|^2, flags[0]: a label changed), as the host
+// loop makes it; ends the WHILE node (cond) when it passes or max_iter is
+// reached, and re-arms the flags.  One lane.
+__device__ __forceinline__ void lloyd_test(LloydLoopState *ls, unsigned long long cond, double norm2,
+                                           double shift2, int *flags) {
+    const int it = ls->it;
+    int conv = 0;
+    if (it > 1 && *((volatile int *)flags) == 0) conv = 2;
+    if (conv == 0 && sqrt(shift2) < ls->tol * sqrt(norm2)) conv = 1;
+    const int next = it + 1;
+    const bool stop = conv > 0 || next >= ls->max_iter;
+    ls->conv = conv;
+    ls->n_iter = conv > 0 ? it : next;
+    ls->it = next;
+    if (stop) cudaGraphSetConditional(cond, 0);
+    flags[0] = 0;
+    flags[1] = 0;
+}
+// sum_partials_kernel's two sums, then the test.  Single warp.
+__global__ void lloyd_control_kernel(const double *partials, int nblocks, double *scalars,
+                                     LloydLoopState *ls, unsigned long long cond, int *flags) {
+    const int lane = threadIdx.x;
+    double sv[2];
+    for (int v = 0; v < 2; ++v) {
+        double a = 0.0;
+        for (int b = lane; b < nblocks; b += 32) a += partials[(size_t)b * 2 + v];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xffffffffu, a, off);
+        if (lane == 0) scalars[v] = a;
+        sv[v] = a;
+    }
+    if (lane == 0) lloyd_test(ls, cond, sv[0], sv[1], flags);
+}
+
 template <typename T>
 cudaError_t launch_kmeans_update(const T *X, int ldx, int n, int d, int k,
                                  const int *sorted_rows, const int *offsets,
                                  const int *seg_chunk_start, int seg_rows, double *chunk_sums,
                                  const int *counts, const T *C_prev, T *C_new, int ldc,
-                                 double *scalars, int *flags, cudaStream_t s) {
-    (void)flags;
+                                 double *scalars, int *flags, cudaStream_t s,
+                                 LloydLoopState *ls, unsigned long long cond) {
     (void)n;
     if (ldx != ldc) return cudaErrorInvalidValue;
     // chunk count upper bound: n / seg_rows + k
@@ -340,7 +560,8 @@ cudaError_t launch_kmeans_update(const T *X, int ldx, int n, int d, int k,
     double *partials = scalars + 8;
     centre_finalize_kernel<T><<<nb, 256, 0, s>>>(k, d, ldc, counts, seg_chunk_start, chunk_sums,
                                                  C_prev, C_new, partials);
-    sum_partials_kernel<<<1, 32, 0, s>>>(partials, nb, 2, 2, scalars);
+    if (ls) lloyd_control_kernel<<<1, 32, 0, s>>>(partials, nb, scalars, ls, cond, flags);
+    else sum_partials_kernel<<<1, 32, 0, s>>>(partials, nb, 2, 2, scalars);
     return cudaGetLastError();
 }
 
@@ -530,7 +751,8 @@ cudaError_t launch_kpp_update(T *w, const T *Dc, int n, int chosen, cudaStream_t
     template cudaError_t launch_kmeans_update<T>(const T *, int, int, int, int, const int *,    \
                                                  const int *, const int *, int, double *,       \
                                                  const int *, const T *, T *, int, double *,    \
-                                                 int *, cudaStream_t);                          \
+                                                 int *, cudaStream_t, LloydLoopState *,         \
+                                                 unsigned long long);                           \
     template cudaError_t launch_centre_norms<T>(const T *, int, int, int, T *, cudaStream_t);   \
     template cudaError_t launch_kmeans_inertia<T>(const T *, int, int, int, const T *, int,     \
                                                   const int *, double *, double *,              \
@@ -1174,22 +1396,11 @@ fx_finalize_kernel(int k, int d, int ld, const unsigned long long *gsum, const C
         }
         if (lane == 0) *ticket = 0u;
         if (ls && lane == 0) {
-            const int it = ls->it;
-            int conv = 0;
-            if (it > 1 && *((volatile int *)flags) == 0) conv = 2;
-            if (conv == 0 && sqrt(sv[1]) < ls->tol * sqrt(sv[0])) conv = 1;
-            const int next = it + 1;
-            const bool stop = conv > 0 || next >= ls->max_iter;
-            ls->conv = conv;
-            ls->n_iter = conv > 0 ? it : next;
-            ls->it = next;
-            if (stop) cudaGraphSetConditional(cond, 0);
+            lloyd_test(ls, cond, sv[0], sv[1], flags);
             // the next iteration's counters start at zero: the label-change and
-            // empty-cluster flags (read above), the relabel list count and its
+            // empty-cluster flags (by the test), the relabel list count and its
             // full-scan count (rearm0[0], rearm0[2]; rearm0[1] is the sticky
             // error word), the changed-row count (rearm1[0])
-            flags[0] = 0;
-            flags[1] = 0;
             if (rearm0) {
                 rearm0[0] = 0;
                 rearm0[2] = 0;
