@@ -1004,8 +1004,14 @@ da_status KMeans<T>::run_lloyd(T *&dCcur, T *&dCprev, int *&dLcur, int *&dLprev,
     int *h_flags = reinterpret_cast<int *>(static_cast<char *>(h_small) + 64);
     converged = 0;
     empty_found = false;
-    // iterations 1.. as one graph launch where the loop allows it
-    const bool graph = use_fx == use_tc && empty_mode == EC_IGNORE && !cuda->timing && !sph;
+    // iterations 1.. as one graph launch where the loop allows it; with the update
+    // by sorting only for short iterations: it saves the host's 20 to 50 us each
+    // (100,000 x 20, k = 16: 95 -> 50 us), but the SIMT assignment runs up to 30%
+    // slower in a conditional node's body (1M x 64, k = 64: 17.4 ms for 15
+    // iterations against 22.7; 300,000 x 32, k = 200: 9.1 against 9.8; 200,000 x 32, k = 39: 2.96
+    // against 3.09; 20,000 x 100, k = 100 and 1M x 15, k = 16 are faster as a graph)
+    const bool graph = use_fx == use_tc && empty_mode == EC_IGNORE && !cuda->timing && !sph &&
+                       (use_tc || (double)n_samples * n_clusters * n_features <= 2e8);
     da_int it = 0;
     for (it = 0; it < max_iter; ++it) {
         if (graph && it == 1) {
