@@ -16,6 +16,7 @@
 #endif
 #include <mutex>
 #include <thread>
+#include <unistd.h>
 #include <vector>
 
 namespace b200 {
@@ -90,7 +91,13 @@ void stream_copy(char *to, const char *from, size_t bytes) {
 
 class Ring {
   public:
-    ~Ring() { release(); }
+    ~Ring() {
+        if (!workers_.empty() && pid_ != getpid()) { // a forked child: the threads are the parent's
+            for (auto &t : workers_) t.detach();
+            return;
+        }
+        release();
+    }
     bool run(const XferSeg *segs, int n, bool up, cudaStream_t s, cudaError_t &e) {
         size_t total = 0;
         for (int i = 0; i < n; ++i) total += segs[i].rows * segs[i].row_bytes;
@@ -111,7 +118,7 @@ class Ring {
             seen_ += total;
             if (seen_ < XFER_AFTER || !set_up(dev)) return false;
         }
-        if (dev != device_) return false;
+        if (dev != device_ || pid_ != getpid()) return false;
         Job job;
         job.segs = segs;
         job.first.assign(1, 0);
@@ -147,6 +154,7 @@ class Ring {
     std::chrono::steady_clock::time_point used_;
     // set while use_mu_ is held
     int threads_ = 0, device_ = -1;
+    pid_t pid_ = 0;
     size_t seen_ = 0;
     char *pinned_ = nullptr;
     std::vector<cudaEvent_t> ev_;
@@ -164,6 +172,7 @@ class Ring {
         }
         pinned_ = static_cast<char *>(p);
         device_ = dev;
+        pid_ = getpid();
         threads_ = t;
         ev_.assign(2 * t, nullptr);
         recorded_.assign(2 * t, 0);
