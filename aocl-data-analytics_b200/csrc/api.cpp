@@ -17,7 +17,8 @@ cudaError_t upload_matrix(da_order order, da_int rows, da_int cols, const T *hos
     if (order == row_major) {
         const XferSeg seg{from, ld * z, dst, ldo * z, cols * z, (size_t)rows};
         cudaError_t e = cudaSuccess;
-        if (xfer_up(&seg, 1, s, e)) return e;
+        const bool direct = ld == cols && host_pinned(host);
+        if (!direct && xfer_up(&seg, 1, s, e)) return e;
         if (ld != cols || ldo == cols || rows < 16) return copy_up(seg, s);
         // dense rows padded on the device: one copy of all of them and a kernel
         // (a driver's copy row by row moves 0.8 GB/s)

@@ -102,6 +102,11 @@ class Ring {
         size_t total = 0;
         for (int i = 0; i < n; ++i) total += segs[i].rows * segs[i].row_bytes;
         if (total < XFER_MIN) return false;
+        // what the device reads or writes itself, at the link's rate
+        const XferSeg *big = std::max_element(segs, segs + n, [](const XferSeg &a, const XferSeg &b) {
+            return a.rows * a.row_bytes < b.rows * b.row_bytes;
+        });
+        if (flat(*big) && host_pinned(big->host)) return false;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
             cudaGetLastError();
@@ -352,6 +357,14 @@ Ring &ring() {
 
 } // namespace
 
+bool host_pinned(const void *p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
 bool xfer_up(const XferSeg *segs, int n, cudaStream_t s, cudaError_t &e) {
     return ring().run(segs, n, true, s, e);
 }

@@ -23,11 +23,14 @@ struct XferSeg {
 
 // Copies all segments, ordered after the work on stream s.  Up: returns with the
 // transfers enqueued on s and the host memory read; down: with the host memory
-// written.  False: not taken (too small, the ring in use by another thread, not
+// written.  False: not taken (too small, page-locked dense rows, the ring in use by another thread, not
 // set up yet, another device, s being captured) -- nothing was done and the
 // caller copies by other means; e: the error of a copy that was taken.
 bool xfer_up(const XferSeg *segs, int n, cudaStream_t s, cudaError_t &e);
 bool xfer_down(const XferSeg *segs, int n, cudaStream_t s, cudaError_t &e);
+
+// Host memory that is page-locked (such rows need no ring).
+bool host_pinned(const void *p);
 
 // One segment, either way, with the driver's copy where the ring does not take
 // it (up: like cudaMemcpy2DAsync from pageable memory; down: synchronises).

@@ -128,3 +128,26 @@ def test_stream_set_after_the_data(warm, ab, n, d):
         km.call("da_b200_kmeans_shard_colmax_s", ab.ptr(out))
         km.close()
         np.testing.assert_array_equal(out, np.arange(2, d + 2, dtype=np.float32))
+
+
+@pytest.mark.parametrize("order,d", [(0, 32), (0, 37), (1, 37)])
+def test_page_locked_rows(warm, ab, order, d):
+    """Page-locked training rows and outputs: the same results."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(d)
+    n, m = 60_000, 900
+    shape = (n, d) if order == 0 else (d, n)
+    lock = torch.empty(shape, dtype=torch.float32, pin_memory=True).numpy()
+    lock[:] = rng.standard_normal(shape)
+    X = lock if order == 0 else lock.T
+    Q = np.array(X[:m], order="C" if order == 0 else "F")
+    res = []
+    for rows in (X, np.array(X, order="C" if order == 0 else "F")):
+        nn = ab.KNN("s", order=order, metric="manhattan", algorithm="brute").fit(rows)
+        res.append(nn.kneighbors(Q, 3))
+        nn.close()
+        st, D = ab.pairwise_distances(rows[:m], rows[m:3 * m], "manhattan", prec="s", order=order)
+        assert st == 0
+        res[-1] += (D,)
+    for a, b in zip(*res):
+        np.testing.assert_array_equal(a, b)
