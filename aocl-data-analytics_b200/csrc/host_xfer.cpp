@@ -39,33 +39,41 @@ struct Job {
     std::atomic<int> error{0};
 };
 
-// A piece of a segment: rows r .. r + n - 1, or (n = 0) bytes of row r.
+// A piece of a segment: rows r .. r + n - 1, or (n = 0) bytes of row r, the last
+// `pad` of them past the row (zeros, going up).
 struct Piece {
-    size_t r, n, off, bytes;
+    size_t r, n, off, bytes, pad;
 };
-bool flat(const XferSeg &g) {
-    return g.rows == 1 || (g.host_pitch == g.row_bytes && g.dev_pitch == g.row_bytes);
+// One run of bytes on both sides.  Going up, a single row that is padded on the
+// device is not: its pad is written too.
+bool flat(const XferSeg &g, bool up) {
+    return (g.rows == 1 && !(up && g.dev_pitch > g.row_bytes)) ||
+           (g.host_pitch == g.row_bytes && g.dev_pitch == g.row_bytes);
 }
-size_t pieces(const XferSeg &g) {
-    if (flat(g)) return (g.rows * g.row_bytes + XFER_SLOT - 1) / XFER_SLOT;
+// bytes that one row takes on the device
+size_t row_span(const XferSeg &g, bool up) { return up ? g.dev_pitch : g.row_bytes; }
+size_t pieces(const XferSeg &g, bool up) {
+    if (flat(g, up)) return (g.rows * g.row_bytes + XFER_SLOT - 1) / XFER_SLOT;
     if (g.dev_pitch <= XFER_SLOT) {
         const size_t per = XFER_SLOT / g.dev_pitch;
         return (g.rows + per - 1) / per;
     }
-    return g.rows * ((g.row_bytes + XFER_SLOT - 1) / XFER_SLOT);
+    return g.rows * ((row_span(g, up) + XFER_SLOT - 1) / XFER_SLOT);
 }
-Piece piece(const XferSeg &g, size_t i) {
-    if (flat(g)) {
+Piece piece(const XferSeg &g, size_t i, bool up) {
+    if (flat(g, up)) {
         const size_t off = i * XFER_SLOT;
-        return {0, 0, off, std::min(XFER_SLOT, g.rows * g.row_bytes - off)};
+        return {0, 0, off, std::min(XFER_SLOT, g.rows * g.row_bytes - off), 0};
     }
     if (g.dev_pitch <= XFER_SLOT) {
         const size_t per = XFER_SLOT / g.dev_pitch, r = i * per, n = std::min(per, g.rows - r);
         // the last row's pad may lie past the device buffer on the way down
-        return {r, n, 0, (n - 1) * g.dev_pitch + g.row_bytes};
+        return {r, n, 0, (n - 1) * g.dev_pitch + g.row_bytes, 0};
     }
-    const size_t per = (g.row_bytes + XFER_SLOT - 1) / XFER_SLOT, off = i % per * XFER_SLOT;
-    return {i / per, 0, off, std::min(XFER_SLOT, g.row_bytes - off)};
+    const size_t span = row_span(g, up), per = (span + XFER_SLOT - 1) / XFER_SLOT;
+    const size_t off = i % per * XFER_SLOT, bytes = std::min(XFER_SLOT, span - off);
+    const size_t past = off + bytes > g.row_bytes ? off + bytes - g.row_bytes : 0;
+    return {i / per, 0, off, bytes, std::min(past, bytes)};
 }
 
 // Into a pinned slot past the caches: the device reads lines that a core's
@@ -106,7 +114,7 @@ class Ring {
         const XferSeg *big = std::max_element(segs, segs + n, [](const XferSeg &a, const XferSeg &b) {
             return a.rows * a.row_bytes < b.rows * b.row_bytes;
         });
-        if (flat(*big) && host_pinned(big->host)) return false;
+        if (flat(*big, up) && host_pinned(big->host)) return false;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
             cudaGetLastError();
@@ -127,7 +135,7 @@ class Ring {
         Job job;
         job.segs = segs;
         job.first.assign(1, 0);
-        for (int i = 0; i < n; ++i) job.first.push_back(job.first.back() + pieces(segs[i]));
+        for (int i = 0; i < n; ++i) job.first.push_back(job.first.back() + pieces(segs[i], up));
         job.up = up;
         job.device = dev;
         job.s = s;
@@ -274,7 +282,7 @@ class Ring {
         const size_t k = std::upper_bound(job.first.begin(), job.first.end(), i) -
                          job.first.begin() - 1;
         g = &job.segs[k];
-        p = piece(*g, i - job.first[k]);
+        p = piece(*g, i - job.first[k], job.up);
         return true;
     }
     static char *dev_at(const XferSeg &g, const Piece &p) {
@@ -308,7 +316,8 @@ class Ring {
                 if (!wait(k)) return;
                 size_t bytes = p[0].bytes;
                 if (p[0].n == 0) {
-                    stream_copy(slot[k], host_at(*g[0], p[0]), bytes);
+                    if (bytes > p[0].pad) stream_copy(slot[k], host_at(*g[0], p[0]), bytes - p[0].pad);
+                    std::memset(slot[k] + bytes - p[0].pad, 0, p[0].pad);
                 } else {
                     const size_t pad = g[0]->dev_pitch - g[0]->row_bytes;
                     for (size_t r = 0; r < p[0].n; ++r) {
@@ -375,7 +384,7 @@ bool xfer_down(const XferSeg *segs, int n, cudaStream_t s, cudaError_t &e) {
 cudaError_t copy_up(const XferSeg &g, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
     if (xfer_up(&g, 1, s, e)) return e;
-    if (flat(g))
+    if (flat(g, true))
         return cudaMemcpyAsync(g.dev, g.host, g.rows * g.row_bytes, cudaMemcpyHostToDevice, s);
     e = cudaMemcpy2DAsync(g.dev, g.dev_pitch, g.host, g.host_pitch, g.row_bytes, g.rows,
                           cudaMemcpyHostToDevice, s);
@@ -387,7 +396,7 @@ cudaError_t copy_up(const XferSeg &g, cudaStream_t s) {
 cudaError_t copy_down(const XferSeg &g, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
     if (xfer_down(&g, 1, s, e)) return e;
-    if (flat(g))
+    if (flat(g, false))
         e = cudaMemcpyAsync(g.host, g.dev, g.rows * g.row_bytes, cudaMemcpyDeviceToHost, s);
     else
         e = cudaMemcpy2DAsync(g.host, g.host_pitch, g.dev, g.dev_pitch, g.row_bytes, g.rows,

@@ -1,0 +1,31 @@
+"""The host transfer ring's paths without a GPU: csrc/host_xfer.cpp compiled
+against a stand-in for the CUDA runtime (xfer_stub.cpp), one process a mode."""
+import os
+import subprocess
+
+import pytest
+
+from conftest import PKG, ROOT
+
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def stub(tmp_path_factory):
+    exe = tmp_path_factory.mktemp("xfer") / "xfer_stub"
+    subprocess.run(["g++", "-O1", "-g", "-std=c++17", f"-I{CUDA}/include",
+                    os.path.join(ROOT, "tests", "xfer_stub.cpp"),
+                    os.path.join(PKG, "csrc", "host_xfer.cpp"), "-lpthread", "-o", str(exe)],
+                   check=True)
+    return str(exe)
+
+
+def run(stub, mode, limit=60):
+    r = subprocess.run([stub, mode], capture_output=True, text=True, timeout=limit)
+    assert r.returncode == 0, (mode, r.returncode, r.stderr)
+
+
+def test_rows_and_their_pads(stub):
+    """Rows arrive, the pads of the device's rows are zero (one row and rows longer
+    than a slot among them), nothing else is written."""
+    run(stub, "copies")

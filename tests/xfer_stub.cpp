@@ -1,0 +1,147 @@
+// The host transfer ring (csrc/host_xfer.cpp) against a stand-in for the part of
+// the CUDA runtime that it calls, so that its paths run without a GPU: "device"
+// memory is host memory and a copy is complete when the call returns.
+//
+//   xfer_stub MODE      exit status 0: as it should be
+#include "../aocl-data-analytics_b200/csrc/host_xfer.hpp"
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <mutex>
+#include <sys/mman.h>
+#include <thread>
+#include <vector>
+
+// ----------------------------------------------------------- the stand-in --
+namespace {
+std::mutex g_mu;
+int g_ring_copies = 0; // copies issued by threads other than the caller's
+std::thread::id g_main;
+void note_thread() {
+    if (std::this_thread::get_id() != g_main) {
+        std::lock_guard<std::mutex> lk(g_mu);
+        ++g_ring_copies;
+    }
+}
+} // namespace
+
+extern "C" {
+cudaError_t cudaMallocHost(void **p, size_t n) {
+    *p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void *) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+    *e = reinterpret_cast<cudaEvent_t>(std::malloc(1));
+    return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+    std::free(e);
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind, cudaStream_t) {
+    note_thread();
+    std::memcpy(to, from, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy2DAsync(void *to, size_t tp, const void *from, size_t fp, size_t w, size_t h,
+                              cudaMemcpyKind, cudaStream_t) {
+    for (size_t r = 0; r < h; ++r) std::memcpy((char *)to + r * tp, (const char *)from + r * fp, w);
+    return cudaSuccess;
+}
+cudaError_t cudaMemset2DAsync(void *p, size_t pitch, int v, size_t w, size_t h, cudaStream_t) {
+    for (size_t r = 0; r < h; ++r) std::memset((char *)p + r * pitch, v, w);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus *s) {
+    *s = cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int *d) {
+    *d = 0;
+    return cudaSuccess;
+}
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
+    std::memset(a, 0, sizeof *a);
+    a->type = cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+} // extern "C"
+
+// ---------------------------------------------------------------- checks --
+using namespace b200;
+namespace {
+#define CHECK(c)                                                                              \
+    do {                                                                                      \
+        if (!(c)) {                                                                           \
+            std::fprintf(stderr, "line %d: %s\n", __LINE__, #c);                              \
+            std::exit(1);                                                                     \
+        }                                                                                     \
+    } while (0)
+
+cudaStream_t const S = reinterpret_cast<cudaStream_t>(0x1000);
+
+// bytes copied through the driver's path until the ring takes a copy
+bool warm(cudaStream_t s = S) {
+    std::vector<char> host(8 << 20, 1), dev(8 << 20);
+    for (int i = 0; i < 20; ++i) {
+        const XferSeg g{host.data(), host.size(), dev.data(), host.size(), host.size(), 1};
+        cudaError_t e = cudaSuccess;
+        if (xfer_up(&g, 1, s, e)) return true;
+    }
+    return false;
+}
+
+// rows of w bytes, pitched on either side, up and down again: the rows arrive,
+// the device rows' pads are zero, the host's bytes between rows stay
+void round_trip(size_t rows, size_t w, size_t host_pitch, size_t dev_pitch, int times) {
+    std::vector<unsigned char> from(rows * host_pitch), dev(rows * dev_pitch + 64, 0xFF),
+        to(rows * host_pitch, 0xAA);
+    for (size_t i = 0; i < from.size(); ++i) from[i] = (unsigned char)(i * 31 + i / 251 + 1);
+    for (int t = 0; t < times; ++t) {
+        std::fill(dev.begin(), dev.end(), 0xFF);
+        CHECK(copy_up({from.data(), host_pitch, dev.data(), dev_pitch, w, rows}, S) == cudaSuccess);
+        for (size_t r = 0; r < rows; ++r) {
+            CHECK(std::memcmp(&dev[r * dev_pitch], &from[r * host_pitch], w) == 0);
+            for (size_t c = w; c < dev_pitch; ++c) CHECK(dev[r * dev_pitch + c] == 0);
+        }
+        for (int i = 0; i < 64; ++i) CHECK(dev[rows * dev_pitch + i] == 0xFF);
+        std::fill(to.begin(), to.end(), 0xAA);
+        CHECK(copy_down({to.data(), host_pitch, dev.data(), dev_pitch, w, rows}, S) == cudaSuccess);
+        for (size_t r = 0; r < rows; ++r) {
+            CHECK(std::memcmp(&to[r * host_pitch], &from[r * host_pitch], w) == 0);
+            for (size_t c = w; c < host_pitch; ++c) CHECK(to[r * host_pitch + c] == 0xAA);
+        }
+    }
+}
+
+int copies() {
+    for (int pass = 0; pass < 2; ++pass) { // without the ring, then with it
+        round_trip(1, 12, 12, 16, 1);
+        round_trip(1, 3 << 20, 3 << 20, (3 << 20) + 12, 1); // one padded row of many pieces
+        round_trip(1, (512 * 1024) * 5 - 8, (512 * 1024) * 5 - 8, 512 * 1024 * 5, 1);
+        round_trip(1, 512 * 1024 * 5, 512 * 1024 * 5, 512 * 1024 * 5 + 16, 1); // a piece of pad alone
+        round_trip(5, 600'004, 600'004, 600'016, 1);                         // rows over a slot
+        round_trip(30'000, 148, 148, 160, 1);
+        round_trip(30'000, 148, 152, 160, 1);
+        round_trip(30'001, 96, 96, 96, 1);
+        round_trip(30'001, 96, 100, 96, 1);
+        if (pass == 0) CHECK(warm());
+    }
+    CHECK(g_ring_copies > 0);
+    return 0;
+}
+} // namespace
+
+int main(int argc, char **argv) {
+    g_main = std::this_thread::get_id();
+    const char *m = argc > 1 ? argv[1] : "";
+    if (!std::strcmp(m, "copies")) return copies();
+    return 2;
+}
