@@ -110,6 +110,8 @@ class Ring {
         size_t total = 0;
         for (int i = 0; i < n; ++i) total += segs[i].rows * segs[i].row_bytes;
         if (total < XFER_MIN) return false;
+        // this name means another stream in each of the ring's threads
+        if (s == cudaStreamPerThread) return false;
         // what the device reads or writes itself, at the link's rate
         const XferSeg *big = std::max_element(segs, segs + n, [](const XferSeg &a, const XferSeg &b) {
             return a.rows * a.row_bytes < b.rows * b.row_bytes;

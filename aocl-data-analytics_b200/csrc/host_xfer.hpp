@@ -23,9 +23,10 @@ struct XferSeg {
 
 // Copies all segments, ordered after the work on stream s.  Up: returns with the
 // transfers enqueued on s and the host memory read; down: with the host memory
-// written.  False: not taken (too small, page-locked dense rows, the ring in use by another thread, not
-// set up yet, another device, s being captured) -- nothing was done and the
-// caller copies by other means; e: the error of a copy that was taken.
+// written.  False: not taken (too small, page-locked dense rows, the ring in use
+// by another thread, not set up yet, another device, s being captured or the
+// calling thread's own default stream) -- nothing was done and the caller copies
+// by other means; e: the error of a copy that was taken.
 bool xfer_up(const XferSeg *segs, int n, cudaStream_t s, cudaError_t &e);
 bool xfer_down(const XferSeg *segs, int n, cudaStream_t s, cudaError_t &e);
 

@@ -29,3 +29,8 @@ def test_rows_and_their_pads(stub):
     """Rows arrive, the pads of the device's rows are zero (one row and rows longer
     than a slot among them), nothing else is written."""
     run(stub, "copies")
+
+
+def test_per_thread_stream(stub):
+    """No transfer of a copy on cudaStreamPerThread is issued by another thread."""
+    run(stub, "per_thread")

@@ -17,11 +17,13 @@
 namespace {
 std::mutex g_mu;
 int g_ring_copies = 0; // copies issued by threads other than the caller's
+int g_strays = 0;      // calls of theirs that name their own stream, not the caller's
 std::thread::id g_main;
-void note_thread() {
+void note_thread(cudaStream_t s) {
     if (std::this_thread::get_id() != g_main) {
         std::lock_guard<std::mutex> lk(g_mu);
         ++g_ring_copies;
+        if (s == cudaStreamPerThread) ++g_strays;
     }
 }
 } // namespace
@@ -42,8 +44,8 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind, cudaStream_t) {
-    note_thread();
+cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind, cudaStream_t s) {
+    note_thread(s);
     std::memcpy(to, from, n);
     return cudaSuccess;
 }
@@ -137,11 +139,28 @@ int copies() {
     CHECK(g_ring_copies > 0);
     return 0;
 }
+
+// cudaStreamPerThread names another stream in every thread: all of a copy's
+// pieces have to be the caller's
+int per_thread() {
+    CHECK(warm());
+    const size_t w = 8 << 20;
+    std::vector<char> from(w, 7), dev(w), to(w);
+    CHECK(copy_up({from.data(), w, dev.data(), w, w, 1}, cudaStreamPerThread) == cudaSuccess);
+    CHECK(copy_down({to.data(), w, dev.data(), w, w, 1}, cudaStreamPerThread) == cudaSuccess);
+    CHECK(to == from);
+    CHECK(g_strays == 0);
+    const int before = g_ring_copies;
+    CHECK(copy_up({from.data(), w, dev.data(), w, w, 1}, S) == cudaSuccess);
+    CHECK(g_ring_copies > before); // other streams: as before
+    return 0;
+}
 } // namespace
 
 int main(int argc, char **argv) {
     g_main = std::this_thread::get_id();
     const char *m = argc > 1 ? argv[1] : "";
     if (!std::strcmp(m, "copies")) return copies();
+    if (!std::strcmp(m, "per_thread")) return per_thread();
     return 2;
 }
