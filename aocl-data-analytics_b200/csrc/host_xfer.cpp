@@ -27,7 +27,10 @@ constexpr size_t XFER_SLOT = 512 * 1024;   // bytes per slot, two slots a thread
 constexpr size_t XFER_MIN = 2 << 20;       // smaller copies: the driver is as fast
 constexpr size_t XFER_AFTER = 64u << 20;   // bytes before the ring is set up
 constexpr int XFER_THREADS = 8;            // with the caller's, at most
-constexpr int XFER_IDLE = 20;              // seconds
+#ifndef XFER_IDLE_SECONDS // (a test's build sets fewer)
+#define XFER_IDLE_SECONDS 20
+#endif
+constexpr int XFER_IDLE = XFER_IDLE_SECONDS;
 
 struct Job {
     const XferSeg *segs = nullptr;
@@ -99,12 +102,19 @@ void stream_copy(char *to, const char *from, size_t bytes) {
 
 class Ring {
   public:
-    ~Ring() {
-        if (!workers_.empty() && pid_ != getpid()) { // a forked child: the threads are the parent's
-            for (auto &t : workers_) t.detach();
-            return;
+    // The process ends, or the library is unloaded.  A copy that stays in progress
+    // keeps the ring: its threads end with the process.
+    void end() {
+        if (foreign()) return;
+        std::unique_lock<std::mutex> use(use_mu_, std::try_to_lock);
+        for (int i = 0; i < 100 && !use.owns_lock(); ++i) {
+            std::this_thread::sleep_for(std::chrono::milliseconds(1));
+            (void)use.try_lock();
         }
-        release();
+        if (!use.owns_lock()) return;
+        closed_ = true;
+        join();
+        if (threads_ > 0) free_memory();
     }
     bool run(const XferSeg *segs, int n, bool up, cudaStream_t s, cudaError_t &e) {
         size_t total = 0;
@@ -112,6 +122,7 @@ class Ring {
         if (total < XFER_MIN) return false;
         // this name means another stream in each of the ring's threads
         if (s == cudaStreamPerThread) return false;
+        if (foreign()) return false;
         // what the device reads or writes itself, at the link's rate
         const XferSeg *big = std::max_element(segs, segs + n, [](const XferSeg &a, const XferSeg &b) {
             return a.rows * a.row_bytes < b.rows * b.row_bytes;
@@ -123,7 +134,7 @@ class Ring {
             return false;
         }
         std::unique_lock<std::mutex> use(use_mu_, std::try_to_lock);
-        if (!use.owns_lock()) return false;
+        if (!use.owns_lock() || closed_) return false;
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) {
             cudaGetLastError();
@@ -133,7 +144,7 @@ class Ring {
             seen_ += total;
             if (seen_ < XFER_AFTER || !set_up(dev)) return false;
         }
-        if (dev != device_ || pid_ != getpid()) return false;
+        if (dev != device_) return false;
         Job job;
         job.segs = segs;
         job.first.assign(1, 0);
@@ -158,6 +169,12 @@ class Ring {
     }
 
   private:
+    // a forked child: threads, locks and waiters are the parent's
+    bool foreign() const {
+        const pid_t p = pid_;
+        return p != 0 && p != getpid();
+    }
+
     std::mutex use_mu_; // one copy at a time
     std::mutex mu_;     // the fields below
     std::condition_variable wake_, done_;
@@ -169,7 +186,8 @@ class Ring {
     std::chrono::steady_clock::time_point used_;
     // set while use_mu_ is held
     int threads_ = 0, device_ = -1;
-    pid_t pid_ = 0;
+    bool closed_ = false;
+    std::atomic<pid_t> pid_{0}; // of the process that set the ring up
     size_t seen_ = 0;
     char *pinned_ = nullptr;
     std::vector<cudaEvent_t> ev_;
@@ -232,10 +250,6 @@ class Ring {
         pinned_ = nullptr;
         threads_ = 0;
         seen_ = 0;
-    }
-    void release() {
-        join();
-        if (threads_ > 0) free_memory();
     }
 
     void serve(int id, unsigned long last) {
@@ -361,9 +375,15 @@ class Ring {
     }
 };
 
+// The object stays: in a forked child, destroying a condition variable waits for
+// the parent's waiting threads for ever.
 Ring &ring() {
-    static Ring r;
-    return r;
+    static Ring *const r = new Ring;
+    static const struct End {
+        ~End() { r->end(); }
+    } at_exit;
+    (void)at_exit;
+    return *r;
 }
 
 } // namespace

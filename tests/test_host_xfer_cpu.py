@@ -13,7 +13,7 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 @pytest.fixture(scope="module")
 def stub(tmp_path_factory):
     exe = tmp_path_factory.mktemp("xfer") / "xfer_stub"
-    subprocess.run(["g++", "-O1", "-g", "-std=c++17", f"-I{CUDA}/include",
+    subprocess.run(["g++", "-O1", "-g", "-std=c++17", "-DXFER_IDLE_SECONDS=1", f"-I{CUDA}/include",
                     os.path.join(ROOT, "tests", "xfer_stub.cpp"),
                     os.path.join(PKG, "csrc", "host_xfer.cpp"), "-lpthread", "-o", str(exe)],
                    check=True)
@@ -34,3 +34,9 @@ def test_rows_and_their_pads(stub):
 def test_per_thread_stream(stub):
     """No transfer of a copy on cudaStreamPerThread is issued by another thread."""
     run(stub, "per_thread")
+
+
+@pytest.mark.parametrize("mode", ["fork", "fork_idle"])
+def test_forked_child_exits(stub, mode):
+    """A child forked with the ring set up (or given back) copies and exits."""
+    run(stub, mode)

@@ -9,8 +9,12 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <chrono>
+#include <csignal>
 #include <sys/mman.h>
+#include <sys/wait.h>
 #include <thread>
+#include <unistd.h>
 #include <vector>
 
 // ----------------------------------------------------------- the stand-in --
@@ -155,6 +159,32 @@ int per_thread() {
     CHECK(g_ring_copies > before); // other streams: as before
     return 0;
 }
+
+// Ends by exit() in a child forked while the ring's threads wait, and copies the
+// driver's way there; then the parent's ring goes on.
+int forked(int idle) {
+    CHECK(warm());
+    std::this_thread::sleep_for(std::chrono::milliseconds(idle));
+    const pid_t child = fork();
+    if (child == 0) {
+        const size_t w = 8 << 20;
+        std::vector<char> from(w, 5), dev(w);
+        for (int i = 0; i < 20; ++i) {
+            const XferSeg g{from.data(), w, dev.data(), w, w, 1};
+            cudaError_t e = cudaSuccess;
+            if (xfer_up(&g, 1, S, e)) _exit(3);
+        }
+        std::exit(0);
+    }
+    int status = -1;
+    for (int i = 0; i < 100 && waitpid(child, &status, WNOHANG) == 0; ++i)
+        std::this_thread::sleep_for(std::chrono::milliseconds(50));
+    if (!WIFEXITED(status)) kill(child, SIGKILL);
+    CHECK(WIFEXITED(status) && WEXITSTATUS(status) == 0);
+    round_trip(30'000, 148, 148, 160, 1);
+    CHECK(warm());
+    return 0;
+}
 } // namespace
 
 int main(int argc, char **argv) {
@@ -162,5 +192,7 @@ int main(int argc, char **argv) {
     const char *m = argc > 1 ? argv[1] : "";
     if (!std::strcmp(m, "copies")) return copies();
     if (!std::strcmp(m, "per_thread")) return per_thread();
+    if (!std::strcmp(m, "fork")) return forked(50);
+    if (!std::strcmp(m, "fork_idle")) return forked(2500);
     return 2;
 }
