@@ -1,10 +1,12 @@
 // The pinned ring of host_xfer.hpp.  One per process, for the first device that
-// uses it: 8 MB of pinned memory and its threads, set up once XFER_AFTER bytes
+// uses it, in the runtime's (primary) context of that device: 8 MB of pinned
+// memory and its threads, set up once XFER_AFTER bytes
 // have gone the driver's way (page-locking takes 7 ms: a program that moves
 // little never pays it) and given back after XFER_IDLE seconds without a copy.
 // A copy holds the ring alone; a second thread's copy meanwhile goes the
 // driver's way.
 #include "host_xfer.hpp"
+#include "cuda_context.hpp"
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -114,7 +116,7 @@ class Ring {
         if (!use.owns_lock()) return;
         closed_ = true;
         join();
-        if (threads_ > 0) free_memory();
+        if (threads_ > 0 && current_context_id() == ctx_id_) free_memory();
     }
     bool run(const XferSeg *segs, int n, bool up, cudaStream_t s, cudaError_t &e) {
         size_t total = 0;
@@ -139,6 +141,13 @@ class Ring {
         if (cudaGetDevice(&dev) != cudaSuccess) {
             cudaGetLastError();
             return false;
+        }
+        if (threads_ > 0 && dev == device_ && current_context_id() != ctx_id_) {
+            // another context of the caller's, or the ring's is gone
+            // (cudaDeviceReset), and the slots and events with it
+            if (!in_primary_context(dev)) return false;
+            join();
+            forget_memory();
         }
         if (threads_ == 0) {
             seen_ += total;
@@ -186,6 +195,7 @@ class Ring {
     std::chrono::steady_clock::time_point used_;
     // set while use_mu_ is held
     int threads_ = 0, device_ = -1;
+    unsigned long long ctx_id_ = 0; // the context of the slots and events
     bool closed_ = false;
     std::atomic<pid_t> pid_{0}; // of the process that set the ring up
     size_t seen_ = 0;
@@ -194,6 +204,7 @@ class Ring {
     std::vector<char> recorded_;
 
     bool set_up(int dev) {
+        if (!in_primary_context(dev)) return false; // the one that the threads use
         join(); // threads of a ring that was given back
         const unsigned hw = std::thread::hardware_concurrency();
         const int t = std::max(2, std::min(XFER_THREADS, (int)hw / 2));
@@ -205,6 +216,7 @@ class Ring {
         }
         pinned_ = static_cast<char *>(p);
         device_ = dev;
+        ctx_id_ = current_context_id();
         pid_ = getpid();
         threads_ = t;
         ev_.assign(2 * t, nullptr);
@@ -244,9 +256,12 @@ class Ring {
                 cudaEventSynchronize(x);
                 cudaEventDestroy(x);
             }
-        ev_.clear();
         if (pinned_) cudaFreeHost(pinned_);
         cudaGetLastError();
+        forget_memory();
+    }
+    void forget_memory() {
+        ev_.clear();
         pinned_ = nullptr;
         threads_ = 0;
         seen_ = 0;
@@ -276,8 +291,12 @@ class Ring {
                     stop_ = true;
                     lk.unlock();
                     wake_.notify_all();
-                    cudaSetDevice(device_);
-                    free_memory();
+                    // (a context that is gone is not made again for it)
+                    if (primary_context_active(device_) &&
+                        cudaSetDevice(device_) == cudaSuccess && current_context_id() == ctx_id_)
+                        free_memory();
+                    else
+                        forget_memory();
                     return;
                 }
                 last = ticket_;

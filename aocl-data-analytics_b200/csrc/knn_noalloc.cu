@@ -23,8 +23,8 @@
 // (cudaDeviceReset, or another primary context made current), the next call
 // looks the address up again instead of using the old one.
 #include "b200_kernels.hpp"
+#include "cuda_context.hpp"
 #include "../../include/aoclda_b200_ext.h"
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <mutex>
@@ -41,41 +41,18 @@ struct ScratchSlot {
 };
 ScratchSlot g_scratch[MAX_DEVICES] = {};
 
-typedef CUresult (*CtxGetCurrentFn)(CUcontext *);
-typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long *);
-
-template <typename F> F driver_entry(const char *name) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-        return nullptr;
-    return reinterpret_cast<F>(p);
-}
-
-// Unique id of the calling thread's current context (0 when there is none).
-unsigned long long current_context_id() {
-    static CtxGetCurrentFn get_cur = driver_entry<CtxGetCurrentFn>("cuCtxGetCurrent");
-    static CtxGetIdFn get_id = driver_entry<CtxGetIdFn>("cuCtxGetId");
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (!get_cur || !get_id || get_cur(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS)
-        return 0;
-    return id;
-}
-
 // Device address of the scratch array on the current device, looked up
 // once per device and context.
 cudaError_t scratch_address(int dev, void **out) {
     std::lock_guard<std::mutex> lock(g_setup_mu);
-    const unsigned long long id = current_context_id();
+    const unsigned long long id = b200::current_context_id();
     if (!g_scratch[dev].addr || id == 0 || g_scratch[dev].ctx_id != id) {
         void *p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, knn_noalloc_scratch);
         if (e != cudaSuccess) return e;
         g_scratch[dev].addr = p;
         // the lookup makes the device's primary context current if none was
-        g_scratch[dev].ctx_id = current_context_id();
+        g_scratch[dev].ctx_id = b200::current_context_id();
     }
     *out = g_scratch[dev].addr;
     return cudaSuccess;

@@ -40,3 +40,10 @@ def test_per_thread_stream(stub):
 def test_forked_child_exits(stub, mode):
     """A child forked with the ring set up (or given back) copies and exits."""
     run(stub, mode)
+
+
+@pytest.mark.parametrize("mode", ["contexts", "reset_idle"])
+def test_contexts(stub, mode):
+    """After a reset of the device, and in a context of the program's own, nothing
+    touches slots and events of the ring's former context."""
+    run(stub, mode)

@@ -4,13 +4,17 @@
 //
 //   xfer_stub MODE      exit status 0: as it should be
 #include "../aocl-data-analytics_b200/csrc/host_xfer.hpp"
+#include <cuda.h>
+#include <atomic>
+#include <chrono>
+#include <csignal>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
-#include <chrono>
-#include <csignal>
+#include <string>
 #include <sys/mman.h>
 #include <sys/wait.h>
 #include <thread>
@@ -30,26 +34,124 @@ void note_thread(cudaStream_t s) {
         if (s == cudaStreamPerThread) ++g_strays;
     }
 }
+
+// contexts: the primary one of device 0 (its id changes when it is reset) and one
+// that a program makes by itself; page-locked memory and events belong to the
+// context that they are made in
+std::atomic<unsigned long long> g_primary{1};
+std::atomic<int> g_active{1};
+thread_local int t_ctx = 0; // 0: primary, 1: the program's own
+unsigned long long ctx_id() { return t_ctx ? 77 : g_primary.load(); }
+struct Locked {
+    size_t n;
+    unsigned long long ctx;
+};
+std::map<void *, Locked> g_locked;
+std::map<cudaEvent_t, unsigned long long> g_events;
+int g_bad = 0; // uses of memory or events of another context, or of none
+std::atomic<int> g_freed{0};
+void use_event(cudaEvent_t e) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!g_events.count(e) || g_events[e] != ctx_id()) ++g_bad;
+}
+void use_memory(const void *p) { // a slot that is gone faults by itself
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_locked.upper_bound(const_cast<void *>(p));
+    if (it == g_locked.begin()) return;
+    --it;
+    if ((const char *)p < (const char *)it->first + it->second.n && it->second.ctx != ctx_id())
+        ++g_bad;
+}
+// cudaDeviceReset: page-locked memory is unmapped, events are gone
+void reset(bool again) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    for (auto it = g_locked.begin(); it != g_locked.end();)
+        if (it->second.ctx == g_primary) {
+            mprotect(it->first, it->second.n, PROT_NONE);
+            it = g_locked.erase(it);
+        } else {
+            ++it;
+        }
+    for (auto it = g_events.begin(); it != g_events.end();)
+        it = it->second == g_primary ? g_events.erase(it) : std::next(it);
+    ++g_primary;
+    g_active = again;
+}
+CUresult ctx_get_current(CUcontext *c) {
+    *c = reinterpret_cast<CUcontext>(t_ctx ? 0x200 : 0x100);
+    return CUDA_SUCCESS;
+}
+CUresult ctx_get_id(CUcontext c, unsigned long long *id) {
+    *id = c == reinterpret_cast<CUcontext>(0x200) ? 77 : g_primary.load();
+    return CUDA_SUCCESS;
+}
+CUresult primary_state(CUdevice, unsigned *flags, int *active) {
+    *flags = 0;
+    *active = g_active;
+    return CUDA_SUCCESS;
+}
+CUresult primary_retain(CUcontext *c, CUdevice) {
+    *c = reinterpret_cast<CUcontext>(0x100);
+    return CUDA_SUCCESS;
+}
+CUresult primary_release(CUdevice) { return CUDA_SUCCESS; }
 } // namespace
 
 extern "C" {
-cudaError_t cudaMallocHost(void **p, size_t n) {
-    *p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+cudaError_t cudaGetDriverEntryPoint(const char *name, void **p, unsigned long long,
+                                    cudaDriverEntryPointQueryResult *q) {
+    const std::string n = name;
+    *p = n == "cuCtxGetCurrent"              ? (void *)ctx_get_current
+         : n == "cuCtxGetId"                 ? (void *)ctx_get_id
+         : n == "cuDevicePrimaryCtxGetState" ? (void *)primary_state
+         : n == "cuDevicePrimaryCtxRetain"   ? (void *)primary_retain
+         : n == "cuDevicePrimaryCtxRelease"  ? (void *)primary_release
+                                             : nullptr;
+    *q = *p ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
     return cudaSuccess;
 }
-cudaError_t cudaFreeHost(void *) { return cudaSuccess; }
+cudaError_t cudaMallocHost(void **p, size_t n) {
+    *p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_locked[*p] = {n, ctx_id()};
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void *p) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!g_locked.count(p)) {
+        ++g_bad;
+        return cudaErrorInvalidValue;
+    }
+    munmap(p, g_locked[p].n);
+    g_locked.erase(p);
+    ++g_freed;
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
-    *e = reinterpret_cast<cudaEvent_t>(std::malloc(1));
+    static uintptr_t next = 0x5000;
+    std::lock_guard<std::mutex> lk(g_mu);
+    *e = reinterpret_cast<cudaEvent_t>(next += 16);
+    g_events[*e] = ctx_id();
     return cudaSuccess;
 }
 cudaError_t cudaEventDestroy(cudaEvent_t e) {
-    std::free(e);
+    use_event(e);
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_events.erase(e);
     return cudaSuccess;
 }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    use_event(e);
+    return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+    use_event(e);
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind, cudaStream_t s) {
     note_thread(s);
+    use_memory(to);
+    use_memory(from);
     std::memcpy(to, from, n);
     return cudaSuccess;
 }
@@ -71,7 +173,11 @@ cudaError_t cudaGetDevice(int *d) {
     *d = 0;
     return cudaSuccess;
 }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaSetDevice(int) {
+    t_ctx = 0;
+    g_active = 1;
+    return cudaSuccess;
+}
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
     std::memset(a, 0, sizeof *a);
@@ -185,6 +291,41 @@ int forked(int idle) {
     CHECK(warm());
     return 0;
 }
+
+// A reset of the device takes the slots and events; a context of the program's own
+// has none.
+int contexts() {
+    CHECK(warm());
+    reset(true);
+    round_trip(30'000, 148, 148, 160, 2);
+    CHECK(g_bad == 0);
+    CHECK(warm()); // a ring in the new context
+    t_ctx = 1;
+    const int before = g_ring_copies;
+    round_trip(30'000, 148, 148, 160, 1);
+    CHECK(g_ring_copies == before);
+    CHECK(!warm()); // none is set up there either
+    t_ctx = 0;
+    round_trip(30'000, 148, 148, 160, 1);
+    CHECK(g_ring_copies > before); // the primary's is still there
+    CHECK(g_bad == 0);
+    return 0;
+}
+// The same with the ring's context gone when it is given back: nothing is made
+// again for it, and the program ends.
+int reset_idle() {
+    CHECK(warm());
+    reset(false);
+    std::this_thread::sleep_for(std::chrono::milliseconds(2500));
+    CHECK(g_bad == 0 && g_freed == 0 && g_active == 0);
+    g_active = 1;
+    CHECK(warm());
+    std::this_thread::sleep_for(std::chrono::milliseconds(2500));
+    CHECK(g_freed == 1);
+    CHECK(warm());
+    reset(true);
+    return 0;
+}
 } // namespace
 
 int main(int argc, char **argv) {
@@ -194,5 +335,7 @@ int main(int argc, char **argv) {
     if (!std::strcmp(m, "per_thread")) return per_thread();
     if (!std::strcmp(m, "fork")) return forked(50);
     if (!std::strcmp(m, "fork_idle")) return forked(2500);
+    if (!std::strcmp(m, "contexts")) return contexts();
+    if (!std::strcmp(m, "reset_idle")) return reset_idle();
     return 2;
 }
