@@ -102,6 +102,14 @@ void stream_copy(char *to, const char *from, size_t bytes) {
     std::memcpy(to, from, bytes);
 }
 
+// What the ring page-locks and frees belongs to no capture: such calls must not
+// end one that another thread of the program has in progress.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 class Ring {
   public:
     // The process ends, or the library is unloaded.  A copy that stays in progress
@@ -114,6 +122,7 @@ class Ring {
             (void)use.try_lock();
         }
         if (!use.owns_lock()) return;
+        const RelaxedCapture relaxed;
         closed_ = true;
         join();
         if (threads_ > 0 && current_context_id() == ctx_id_) free_memory();
@@ -137,6 +146,7 @@ class Ring {
         }
         std::unique_lock<std::mutex> use(use_mu_, std::try_to_lock);
         if (!use.owns_lock() || closed_) return false;
+        const RelaxedCapture relaxed;
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) {
             cudaGetLastError();
@@ -268,6 +278,7 @@ class Ring {
     }
 
     void serve(int id, unsigned long last) {
+        const RelaxedCapture relaxed;
         for (;;) {
             Job *job = nullptr;
             {

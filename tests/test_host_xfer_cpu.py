@@ -47,3 +47,8 @@ def test_contexts(stub, mode):
     """After a reset of the device, and in a context of the program's own, nothing
     touches slots and events of the ring's former context."""
     run(stub, mode)
+
+
+def test_capture_of_another_thread(stub):
+    """Setting the ring up and giving it back leave another thread's capture alone."""
+    run(stub, "capture")

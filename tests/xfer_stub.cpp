@@ -48,6 +48,14 @@ struct Locked {
 };
 std::map<void *, Locked> g_locked;
 std::map<cudaEvent_t, unsigned long long> g_events;
+// a thread of the program's captures a graph in the global mode, which calls that
+// page-lock or free memory in any thread end unless that thread's mode is relaxed
+std::atomic<bool> g_capture{false};
+std::atomic<int> g_spoilt{0};
+thread_local cudaStreamCaptureMode t_mode = cudaStreamCaptureModeGlobal;
+void unsafe_call() {
+    if (g_capture && t_mode != cudaStreamCaptureModeRelaxed) ++g_spoilt;
+}
 int g_bad = 0; // uses of memory or events of another context, or of none
 std::atomic<int> g_freed{0};
 void use_event(cudaEvent_t e) {
@@ -110,13 +118,19 @@ cudaError_t cudaGetDriverEntryPoint(const char *name, void **p, unsigned long lo
     *q = *p ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
     return cudaSuccess;
 }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m) {
+    std::swap(*m, t_mode);
+    return cudaSuccess;
+}
 cudaError_t cudaMallocHost(void **p, size_t n) {
+    unsafe_call();
     *p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
     std::lock_guard<std::mutex> lk(g_mu);
     g_locked[*p] = {n, ctx_id()};
     return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void *p) {
+    unsafe_call();
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_locked.count(p)) {
         ++g_bad;
@@ -326,6 +340,18 @@ int reset_idle() {
     reset(true);
     return 0;
 }
+
+// The ring is set up, given back and set up again while another thread captures.
+int capture() {
+    g_capture = true;
+    CHECK(warm());
+    CHECK(t_mode == cudaStreamCaptureModeGlobal); // the caller's mode is its own again
+    std::this_thread::sleep_for(std::chrono::milliseconds(2500));
+    CHECK(g_freed == 1);
+    CHECK(warm());
+    CHECK(g_spoilt == 0);
+    return 0;
+}
 } // namespace
 
 int main(int argc, char **argv) {
@@ -337,5 +363,6 @@ int main(int argc, char **argv) {
     if (!std::strcmp(m, "fork_idle")) return forked(2500);
     if (!std::strcmp(m, "contexts")) return contexts();
     if (!std::strcmp(m, "reset_idle")) return reset_idle();
+    if (!std::strcmp(m, "capture")) return capture();
     return 2;
 }
