@@ -650,19 +650,9 @@ da_status da_b200_set_stream(da_handle h, void *stream) {
     h->err.clear();
     da_status s = h->cuda.init(h->err);
     if (s != da_status_success) return s;
-    const cudaStream_t to = stream ? static_cast<cudaStream_t>(stream) : h->cuda.own_stream;
-    if (to != h->cuda.stream && h->cuda.stream == h->cuda.own_stream) {
-        // an upload of set_data may still be in flight on the handle's own
-        // stream, which the new one does not wait for (the new one may be
-        // under capture)
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        const cudaError_t e = cudaStreamSynchronize(h->cuda.own_stream);
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        if (e != cudaSuccess) return cuda_status(h->err, e, "stream");
-    }
-    h->cuda.stream = to;
-    return da_status_success;
+    const cudaError_t e =
+        h->cuda.bind(stream ? static_cast<cudaStream_t>(stream) : h->cuda.own_stream);
+    return e == cudaSuccess ? da_status_success : cuda_status(h->err, e, "stream");
 }
 da_status da_b200_set_stream_priority(da_handle h, da_int priority) {
     if (!h) return da_status_handle_not_initialized;

@@ -389,6 +389,8 @@ struct CudaCtx {
     int device = -1;
     cudaStream_t stream = nullptr;     // stream all work is enqueued on
     cudaStream_t own_stream = nullptr; // the handle's own stream
+    cudaEvent_t left_ev = nullptr;     // the end of work that a call left in flight
+    bool left = false;                 // it has been recorded
     bool ready = false;
     bool timing = false;
     // Kernel timing: one event pair per timed launch, recorded without
@@ -425,11 +427,50 @@ struct CudaCtx {
         ready = true;
         return da_status_success;
     }
+    // A call may return with work on `stream` still in flight (set_data's upload):
+    // mark its end, for the next stream that the handle is bound to.
+    cudaError_t leave_in_flight() {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return cudaSuccess; // part of the caller's capture
+        }
+        cudaError_t e = cudaSuccess;
+        if (!left_ev) e = cudaEventCreateWithFlags(&left_ev, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventRecord(left_ev, stream);
+        left = left || e == cudaSuccess;
+        return e;
+    }
+    // Bind the handle to another stream, whose work follows what was left in flight.
+    // The former stream is not touched unless it is the handle's own: the caller
+    // may have destroyed it.
+    cudaError_t bind(cudaStream_t to) {
+        if (to == stream) return cudaSuccess;
+        cudaError_t e = stream == own_stream ? leave_in_flight() : cudaSuccess;
+        if (e == cudaSuccess && left) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            if (to != cudaStreamPerThread && cudaStreamIsCapturing(to, &cs) == cudaSuccess &&
+                cs == cudaStreamCaptureStatusNone) {
+                e = cudaStreamWaitEvent(to, left_ev, 0);
+            } else {
+                // a capture cannot wait for what is not part of it, and the per-thread
+                // stream of this thread need not be that of the next call
+                cudaGetLastError();
+                cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+                cudaThreadExchangeStreamCaptureMode(&mode);
+                e = cudaEventSynchronize(left_ev);
+                cudaThreadExchangeStreamCaptureMode(&mode);
+            }
+        }
+        if (e == cudaSuccess) stream = to;
+        return e;
+    }
     ~CudaCtx() {
         for (auto &t : tpool) {
             if (t.ev0) cudaEventDestroy(t.ev0);
             if (t.ev1) cudaEventDestroy(t.ev1);
         }
+        if (left_ev) cudaEventDestroy(left_ev);
         if (own_stream) cudaStreamDestroy(own_stream);
     }
     // Fold the recorded launches into ktime (waits for the last of them).

@@ -112,6 +112,7 @@ template <typename T> da_status KMeans<T>::ensure_device_data() {
              "upload of A");
     B200_TRY(launch_row_sqnorms<T>(dX.as<T>(), ld, n_samples, n_features, dXn.as<T>(), cuda->stream),
              "row norms");
+    B200_TRY(cuda->leave_in_flight(), "upload of A");
     dXbf_stale = true;
     fx_stale = true;
     sph_ready = 0;

@@ -284,6 +284,7 @@ template <typename T> da_status NN<T>::ensure_device_data() {
     B200_TRY(upload_matrix<T>(data_order, n_samples, n_features, X_host, ldx_host, dX.as<T>(),
                               ld, dStage, cuda->stream),
              "upload of X_train");
+    B200_TRY(cuda->leave_in_flight(), "upload of X_train");
     X_on_device = true;
     xn_kind = -1;
     tc_train_ready = false;
