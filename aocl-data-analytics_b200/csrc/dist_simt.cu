@@ -389,7 +389,9 @@ cudaError_t launch_knn_chunks(const T *Q, int ldq, int nq, const T *X, int ldx, 
 // ------------------------------------------------------------ kNN merge ---
 // One warp per query: every element's final rank is its position in its own
 // chunk list plus the number of smaller elements in every other list
-// (binary search); elements with rank < k are written.
+// (binary search); elements with rank < k are written.  The lists' padding
+// ranks after all rows: a query with fewer than k keys that are numbers ends in
+// index -1 at distance +inf.
 template <typename T>
 __global__ void knn_merge_kernel(const T *pk, const int *pi, int nq, int nc, int k, int tf,
                                  int out_colmajor, T *ok, int *oi) {
@@ -415,13 +417,13 @@ __global__ void knn_merge_kernel(const T *pk, const int *pi, int nq, int nc, int
             }
             rank += lo;
         }
-        if (rank < k && idx != 0x7fffffff) {
+        if (rank < k) {
             T v = key;
             if (tf == 1) v = sqrt_rn(v);
             else if (tf == 2) v = -v;
             const size_t o = out_colmajor ? ((size_t)rank * nq + warp) : ((size_t)warp * k + rank);
             ok[o] = v;
-            oi[o] = idx;
+            oi[o] = idx == 0x7fffffff ? -1 : idx;
         }
     }
 }

@@ -245,7 +245,7 @@ template <typename T> da_status IVF<T>::add(da_int n, da_int d, const T *X, da_i
     s = coarse->kneighbors_compute(n, d, X, ldx, ord, 1, near, nullptr);
     if (s != da_status_success) return s;
     for (da_int i = 0; i < n; ++i) {
-        const da_int c = near[i];
+        const da_int c = std::max<da_int>(near[i], 0); // -1: the row is not a number
         auto &rows = list_rows[c];
         T norm = T(0);
         for (da_int j = 0; j < d; ++j) {

@@ -75,6 +75,7 @@ ivf_scan_kernel(const T *__restrict__ Q, const T *__restrict__ qn, int ld, int n
         __syncthreads();
         for (int p = 0; p < n_probe; ++p) {
             const int list = probe[(size_t)q * n_probe + p];
+            if (list < 0) continue; // a query that is not a number has no nearest centroid
             const long long beg = loff[list], end = loff[list + 1];
             for (long long b0 = beg; b0 < end; b0 += IVF_BATCH) {
                 const int nb = (int)((end - b0) < IVF_BATCH ? (end - b0) : IVF_BATCH);

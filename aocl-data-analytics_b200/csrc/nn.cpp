@@ -1253,7 +1253,9 @@ da_status NN<T>::compute_proba(da_int nq, da_int d, const T *Xt, da_int ldt,
         T *pq = proba.data() + (size_t)q * nc;
         // per class, the neighbours' weights in neighbour order
         for (da_int r = 0; r < k; ++r) {
-            const da_int lbl = y_class[ind[(size_t)q * k + r]];
+            const da_int at = ind[(size_t)q * k + r];
+            if (at < 0) continue; // fewer than k rows at a distance that is a number
+            const da_int lbl = y_class[at];
             const da_int c = (da_int)(std::lower_bound(classes.begin(), classes.end(), lbl) -
                                       classes.begin());
             if (c == nc || classes[c] != lbl) continue;
@@ -1483,17 +1485,21 @@ da_status NN<T>::predict_reg(da_int nq, da_int d, const T *Xt, da_int ldt, T *y,
     s = kneighbors_compute(nq, d, Xt, ldt, order(), k, ind, weights == 1 ? &dist : nullptr);
     if (s != da_status_success) return s;
     // nearest_neighbors.cpp:1707-1747
+    // (a query with fewer than k rows at a distance that is a number has no value)
+    const auto target = [&](size_t e) {
+        return ind[e] < 0 ? std::numeric_limits<T>::quiet_NaN() : y_reg[ind[e]];
+    };
     for (da_int q = 0; q < nq; ++q) {
         if (weights == 0) {
             T sum = T(0);
-            for (da_int r = 0; r < k; ++r) sum += y_reg[ind[(size_t)q * k + r]];
+            for (da_int r = 0; r < k; ++r) sum += target((size_t)q * k + r);
             y[q] = sum / T(k);
         } else {
             T num = T(0), den = T(0);
             for (da_int r = 0; r < k; ++r) {
                 const T dv = dist[(size_t)q * k + r];
                 const T w = (dv <= std::numeric_limits<T>::epsilon()) ? T(1) : T(1) / dv;
-                num += y_reg[ind[(size_t)q * k + r]] * w;
+                num += target((size_t)q * k + r) * w;
                 den += w;
             }
             y[q] = num / den;
