@@ -139,10 +139,28 @@ template <typename T> struct NN : public AlgBase {
     da_status ensure_device_data();
     da_status validate_queries(da_int nq, da_int d, const T *Xt, da_int ldt);
     // tensor-core path; `done` false when the plain path must run instead
-    da_status kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_sqrt, bool cosine,
-                            size_t &n_extra, bool &done);
-    da_status tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt, bool cosine,
-                        const int *extra, bool &redone);
+    // (a search's accumulation, post-operation, output transform, block length
+    // and norms)
+    struct KnnWay {
+        int acc, post, tf, kc;
+        const T *qn, *xn;
+    };
+    da_status kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, size_t &n_extra,
+                            bool &done);
+    da_status tc_finish(da_int nq, da_int d, da_int k, const KnnWay &w, const int *extra,
+                        bool &redone);
+    struct Gathered { // some of the queries, and their results
+        T *Q, *qn, *key;
+        int *ind, *number, *redo, *flag;
+    };
+    da_status flagged_queries(const int *words, size_t nq, std::vector<int> &idx);
+    da_status gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g);
+    da_status scatter_results(da_int nq, da_int k, size_t m, const Gathered &g);
+    size_t sel_batch(const KnnSelPlan &pl) const;
+    da_status knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
+                              const std::vector<int> &idx, std::vector<int> &over);
+    da_status knn_lists(da_int nq, da_int d, da_int k, const KnnWay &w,
+                        const std::vector<int> *only);
     da_status compute_proba(da_int nq, da_int d, const T *Xt, da_int ldt, std::vector<T> &proba);
     // radius mode of predict / predict_proba (outlier handling as the reference)
     da_status radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T r, bool want_val,

@@ -146,12 +146,13 @@ size_t knn_sel_bytes(const KnnSelPlan &pl, int nq, bool fp64);
 // where fewer are finite.
 cudaError_t launch_knn_bound(const float *minima, int groups, int nq, int k, float *bound,
                              cudaStream_t s);
-// out_key / out_idx as launch_knn_merge's; *flag is set to 1 when a query's
-// list overflowed or held fewer than k keys (its outputs are then unwritten).
+// out_key / out_idx as launch_knn_merge's; *flag and the query's redo word are
+// set to 1 when its list overflowed (its outputs are then unwritten), else 0.
 template <typename T>
 cudaError_t launch_knn_select(const T *Q, int nq, const T *X, int nx, int ld, int d, const T *qn,
                               const T *xn, const KnnArgs &a, const KnnSelPlan &pl, void *work,
-                              int tf, T *out_key, int *out_idx, int *flag, cudaStream_t s);
+                              int tf, T *out_key, int *out_idx, int *flag, int *redo,
+                              cudaStream_t s);
 
 // ---------------------------------------------- kNN tensor-core pass ---
 // fp32 euclidean / squared euclidean / cosine: bf16x3 tcgen05 candidate pass with a
@@ -171,11 +172,11 @@ size_t knn_tc_query_bytes(int nq, int ldbf, const KnnTcPlan &pl); // size of qbu
 // state words: [0] queries flagged, [1] error code, [2] lists that overflowed,
 // [4] lists short of k
 constexpr int KNN_TC_STATE = 8;
-// dst[i] = src[idx[i]] (rows of ld floats); out[idx[i]] = (key, ind)[i] (rows of k)
-cudaError_t launch_rows_gather(const float *src, int ld, const int *idx, int m, float *dst,
+// dst[i] = src[idx[i]], and dst[idx[i]] = src[i]: rows of row_bytes (a multiple of 4)
+cudaError_t launch_rows_gather(const void *src, size_t row_bytes, const int *idx, int m, void *dst,
                                cudaStream_t s);
-cudaError_t launch_results_scatter(const float *key, const int *ind, const int *idx, int m, int k,
-                                   float *out_key, int *out_idx, cudaStream_t s);
+cudaError_t launch_rows_scatter(const void *src, size_t row_bytes, const int *idx, int m, void *dst,
+                                cudaStream_t s);
 cudaError_t launch_knn_tc_train_prep(const float *X, int ld, int nx, int d, void *Xh, void *Xl,
                                      int ldbf, float *xnorm2, float *xmax, cudaStream_t s);
 // Cosine distance instead (the plain path's value 1 - x.q / (|x| |q|)): the

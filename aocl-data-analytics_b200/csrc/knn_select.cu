@@ -14,8 +14,9 @@
 //   * knn_append_kernel: the keys of all rows; those at or below the bound are
 //     collected in shared memory and go to the query's list in global memory;
 //   * knn_pick_kernel: sorts the list by (key, index) and writes its first k.
-// A list that overflows, or holds fewer than k entries (NaN keys), raises the
-// flag, and the caller runs the search with running lists (knn_chunk_kernel).
+// A list that overflows raises the flag, and the caller searches its query with
+// running lists (knn_chunk_kernel).  Fewer than k entries are all keys that are
+// numbers: fewer than k finite minima leave the bound at +inf.
 //
 // The passes are bound by FP32 / FP64 issue (tile_sweep.cuh).  Measured on a
 // B200, device time against running lists and their merge: 50,000 x 37 fp32,
@@ -107,11 +108,12 @@ template <> struct OrdBits<double> {
 // at or below the k-th); +inf where fewer than k are finite: everything
 // passes.  Found bit by bit from the top: the largest value with fewer than k
 // below it (counting every value's rank took 256 us for 4,096 queries of 512
-// minima, this 14).  Clears the query's list and the overflow flag (cnt null:
-// neither).
+// minima, this 14).  Clears the query's list, its redo word and the overflow flag
+// (cnt null: none of them).
 template <typename T, int R>
 __global__ void __launch_bounds__(128)
-knn_bound_kernel(const T *minima, int groups, int nq, int k, T *bound, int *cnt, int *flag) {
+knn_bound_kernel(const T *minima, int groups, int nq, int k, T *bound, int *cnt, int *flag,
+                 int *redo) {
     using O = OrdBits<T>;
     using U = typename O::U;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -142,20 +144,21 @@ knn_bound_kernel(const T *minima, int groups, int nq, int k, T *bound, int *cnt,
         bound[q] = O::back(kth);
         if (cnt) {
             cnt[q] = 0;
+            redo[q] = 0;
             if (q == 0) *flag = 0;
         }
     }
 }
 template <typename T>
 void bound_pass(const T *minima, int groups, int nq, int k, T *bound, int *cnt, int *flag,
-                cudaStream_t s) {
+                int *redo, cudaStream_t s) {
     const int nb = (nq + 3) / 4;
     if (k <= 16)
-        knn_bound_kernel<T, 2><<<nb, 128, 0, s>>>(minima, groups, nq, k, bound, cnt, flag);
+        knn_bound_kernel<T, 2><<<nb, 128, 0, s>>>(minima, groups, nq, k, bound, cnt, flag, redo);
     else if (k <= 64)
-        knn_bound_kernel<T, 8><<<nb, 128, 0, s>>>(minima, groups, nq, k, bound, cnt, flag);
+        knn_bound_kernel<T, 8><<<nb, 128, 0, s>>>(minima, groups, nq, k, bound, cnt, flag, redo);
     else
-        knn_bound_kernel<T, 16><<<nb, 128, 0, s>>>(minima, groups, nq, k, bound, cnt, flag);
+        knn_bound_kernel<T, 16><<<nb, 128, 0, s>>>(minima, groups, nq, k, bound, cnt, flag, redo);
 }
 
 // Block (query tile, row chunk): appends every (key, row) with key <= the
@@ -235,18 +238,19 @@ knn_append_kernel(const T *Q, int nq, const T *X, int nx, int ld, int d, const T
 }
 
 // One block per query: the listed entries sorted by (key, index), the first k
-// written (tf 1: square root, 2: negated).
+// written (tf 1: square root, 2: negated; past the last entry index -1, distance
+// +inf).
 template <typename T>
 __global__ void __launch_bounds__(128)
 knn_pick_kernel(const int *cnt, const T *list_key, const int *list_idx, int cap, int k, int tf,
-                T *ok, int *oi, int *flag) {
+                T *ok, int *oi, int *flag, int *redo) {
     extern __shared__ __align__(16) unsigned char pick_sm[];
     T *sk = reinterpret_cast<T *>(pick_sm);           // cap
     int *si = reinterpret_cast<int *>(sk + cap);      // cap
     const int q = blockIdx.x;
     const int m = cnt[q];
-    if (m > cap || m < k) {
-        if (threadIdx.x == 0) *flag = 1;
+    if (m > cap) {
+        if (threadIdx.x == 0) *flag = redo[q] = 1;
         return;
     }
     int np2 = 1;
@@ -273,18 +277,18 @@ knn_pick_kernel(const int *cnt, const T *list_key, const int *list_idx, int cap,
             __syncthreads();
         }
     for (int r = threadIdx.x; r < k; r += 128) {
-        T v = sk[r];
+        T v = r < m ? sk[r] : Lim<T>::inf();
         if (tf == 1) v = sqrt_rn(v);
         else if (tf == 2) v = -v;
         ok[(size_t)q * k + r] = v;
-        oi[(size_t)q * k + r] = si[r];
+        oi[(size_t)q * k + r] = r < m ? si[r] : -1;
     }
 }
 
 template <typename T, int ACC>
 cudaError_t select_t(const T *Q, int nq, const T *X, int nx, int ld, int d, const T *qn,
                      const T *xn, const KnnArgs &a, const KnnSelPlan &pl, void *work, int tf,
-                     T *ok, int *oi, int *flag, cudaStream_t s) {
+                     T *ok, int *oi, int *flag, int *redo, cudaStream_t s) {
     constexpr int BM = SW_BM, BN = SweepStage<T>::BN;
     const T p = T(a.p), invp = T(1.0 / (double)p);
     T *list_key = static_cast<T *>(work);
@@ -296,7 +300,7 @@ cudaError_t select_t(const T *Q, int nq, const T *X, int nx, int ld, int d, cons
     knn_min_kernel<T, ACC><<<dim3(qt, pl.parts), 256, 0, s>>>(
         Q, nq, X, pl.step, pl.n_sample, pl.part_rows, ld, d, qn, xn, a.post, a.kc, p, invp, minima,
         pl.groups);
-    bound_pass(minima, pl.groups, nq, a.k, bound, cnt, flag, s);
+    bound_pass(minima, pl.groups, nq, a.k, bound, cnt, flag, redo, s);
     // chunks of whole row tiles: about four blocks per SM slot (two slots per
     // SM), so that the last wave costs little
     const int tiles = (nx + BN - 1) / BN;
@@ -309,7 +313,8 @@ cudaError_t select_t(const T *Q, int nq, const T *X, int nx, int ld, int d, cons
     const size_t smem = (size_t)pl.cap * (sizeof(T) + 4);
     cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(knn_pick_kernel<T>), smem);
     if (e != cudaSuccess) return e;
-    knn_pick_kernel<T><<<nq, 128, smem, s>>>(cnt, list_key, list_idx, pl.cap, a.k, tf, ok, oi, flag);
+    knn_pick_kernel<T><<<nq, 128, smem, s>>>(cnt, list_key, list_idx, pl.cap, a.k, tf, ok, oi, flag,
+                                             redo);
     return cudaGetLastError();
 }
 
@@ -317,7 +322,7 @@ cudaError_t select_t(const T *Q, int nq, const T *X, int nx, int ld, int d, cons
 
 cudaError_t launch_knn_bound(const float *minima, int groups, int nq, int k, float *bound,
                              cudaStream_t s) {
-    bound_pass<float>(minima, groups, nq, k, bound, nullptr, nullptr, s);
+    bound_pass<float>(minima, groups, nq, k, bound, nullptr, nullptr, nullptr, s);
     return cudaGetLastError();
 }
 
@@ -360,29 +365,30 @@ size_t knn_sel_bytes(const KnnSelPlan &pl, int nq, bool fp64) {
 template <typename T>
 cudaError_t launch_knn_select(const T *Q, int nq, const T *X, int nx, int ld, int d, const T *qn,
                               const T *xn, const KnnArgs &a, const KnnSelPlan &pl, void *work,
-                              int tf, T *out_key, int *out_idx, int *flag, cudaStream_t s) {
+                              int tf, T *out_key, int *out_idx, int *flag, int *redo,
+                              cudaStream_t s) {
     switch (a.acc) {
     case ACC_SQEUC:
         return select_t<T, ACC_SQEUC>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key,
-                                      out_idx, flag, s);
+                                      out_idx, flag, redo, s);
     case ACC_DOT:
         return select_t<T, ACC_DOT>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key, out_idx,
-                                    flag, s);
+                                    flag, redo, s);
     case ACC_MANHATTAN:
         return select_t<T, ACC_MANHATTAN>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key,
-                                          out_idx, flag, s);
+                                          out_idx, flag, redo, s);
     default:
         return select_t<T, ACC_MINKOWSKI>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key,
-                                          out_idx, flag, s);
+                                          out_idx, flag, redo, s);
     }
 }
 template cudaError_t launch_knn_select<float>(const float *, int, const float *, int, int, int,
                                               const float *, const float *, const KnnArgs &,
                                               const KnnSelPlan &, void *, int, float *, int *,
-                                              int *, cudaStream_t);
+                                              int *, int *, cudaStream_t);
 template cudaError_t launch_knn_select<double>(const double *, int, const double *, int, int, int,
                                                const double *, const double *, const KnnArgs &,
                                                const KnnSelPlan &, void *, int, double *, int *,
-                                               int *, cudaStream_t);
+                                               int *, int *, cudaStream_t);
 
 } // namespace b200

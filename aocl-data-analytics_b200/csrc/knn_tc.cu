@@ -787,35 +787,30 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
     return cudaGetLastError();
 }
 
-__global__ void rows_gather_kernel(const float *src, int ld, const int *idx, int m, float *dst) {
+// Rows of w words: from rows idx[i] of src to rows i of dst, or the other way.
+__global__ void rows_move_kernel(const int *src, int w, const int *idx, int m, int *dst, int gather) {
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)m * ld) return;
-    const int i = (int)(e / ld), c = (int)(e % ld);
-    dst[e] = src[(size_t)idx[i] * ld + c];
+    if (e >= (size_t)m * w) return;
+    const int i = (int)(e / w), c = (int)(e % w);
+    const size_t far = (size_t)idx[i] * w + c;
+    if (gather) dst[e] = src[far];
+    else dst[far] = src[e];
 }
-__global__ void results_scatter_kernel(const float *key, const int *ind, const int *idx, int m,
-                                       int k, float *out_key, int *out_idx) {
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)m * k) return;
-    const int i = (int)(e / k), r = (int)(e % k);
-    out_key[(size_t)idx[i] * k + r] = key[e];
-    out_idx[(size_t)idx[i] * k + r] = ind[e];
+static cudaError_t rows_move(const void *src, size_t row_bytes, const int *idx, int m, void *dst,
+                             int gather, cudaStream_t s) {
+    const size_t w = row_bytes / 4, n = (size_t)m * w;
+    if (n == 0) return cudaSuccess;
+    rows_move_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+        static_cast<const int *>(src), (int)w, idx, m, static_cast<int *>(dst), gather);
+    return cudaGetLastError();
 }
-
-cudaError_t launch_rows_gather(const float *src, int ld, const int *idx, int m, float *dst,
+cudaError_t launch_rows_gather(const void *src, size_t row_bytes, const int *idx, int m, void *dst,
                                cudaStream_t s) {
-    const size_t n = (size_t)m * ld;
-    if (n == 0) return cudaSuccess;
-    rows_gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, ld, idx, m, dst);
-    return cudaGetLastError();
+    return rows_move(src, row_bytes, idx, m, dst, 1, s);
 }
-cudaError_t launch_results_scatter(const float *key, const int *ind, const int *idx, int m, int k,
-                                   float *out_key, int *out_idx, cudaStream_t s) {
-    const size_t n = (size_t)m * k;
-    if (n == 0) return cudaSuccess;
-    results_scatter_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(key, ind, idx, m, k,
-                                                                        out_key, out_idx);
-    return cudaGetLastError();
+cudaError_t launch_rows_scatter(const void *src, size_t row_bytes, const int *idx, int m, void *dst,
+                                cudaStream_t s) {
+    return rows_move(src, row_bytes, idx, m, dst, 0, s);
 }
 
 // ------------------------------------------------------ radius search ---

@@ -4,7 +4,6 @@
 // the top-k selection run on the GPU (dist_simt.cu).
 #include "alg.hpp"
 #include <cstdlib>
-#include <functional>
 #include <map>
 
 namespace b200 {
@@ -319,11 +318,12 @@ template <typename T> cudaError_t NN<T>::tc_train_copies(da_int d) {
 // state follow the indices, for tc_finish.
 static constexpr da_int KNN_TC_BATCH = 16384;
 template <typename T>
-da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_sqrt,
-                                bool cosine, size_t &n_extra, bool &done) {
+da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, size_t &n_extra,
+                                bool &done) {
     done = false;
     if constexpr (std::is_same_v<T, float>) {
         cudaStream_t st = cuda->stream;
+        const bool cosine = w.post == POST_COSINE;
         if (cosine) {
             // the plain path's norms of the training rows and queries, and the
             // reciprocals of the former
@@ -368,8 +368,8 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
             B200_TRY(cuda->timed("knn_tc", [&] {
                 return launch_knn_tc(dX.as<float>(), dXh.p, dXl.p, dXsq.as<float>(),
                                      dTkScal.as<float>(), (int)n_samples, ld, tc_ldbf, (int)d,
-                                     dQ.as<float>() + (size_t)q0 * ld, (int)nb, (int)k, kc,
-                                     take_sqrt ? 1 : 0, pb, dTkQ.p, dTkList.p,
+                                     dQ.as<float>() + (size_t)q0 * ld, (int)nb, (int)k, w.kc,
+                                     w.tf, pb, dTkQ.p, dTkList.p,
                                      dTkFlag.as<int>() + q0, counts + q0, state,
                                      dOutK.as<float>() + (size_t)q0 * k,
                                      out_idx((size_t)nq * k) + (size_t)q0 * k, st,
@@ -379,26 +379,19 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, int kc, bool take_
         cuda->stats["tensor_core"] = 1.0;
         done = true;
     } else {
-        (void)nq;
-        (void)d;
-        (void)k;
-        (void)kc;
-        (void)take_sqrt;
-        (void)cosine;
-        (void)n_extra;
+        (void)nq, (void)d, (void)k, (void)w, (void)n_extra;
     }
     return da_status_success;
 }
 
 // The state words and list lengths of a tensor-core search (`extra`, as
 // kneighbors_tc laid them out): statistics, errors, and the flagged queries
-// searched on the plain path into dOutK (`redone`).
+// searched again into dOutK (`redone`).
 template <typename T>
-da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt, bool cosine,
-                           const int *extra, bool &redone) {
+da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, const KnnWay &w, const int *extra,
+                           bool &redone) {
     redone = false;
     if constexpr (std::is_same_v<T, float>) {
-        cudaStream_t st = cuda->stream;
         const int batches = (int)((nq + KNN_TC_BATCH - 1) / KNN_TC_BATCH);
         const int *lens = extra + (size_t)batches * KNN_TC_STATE;
         double mx = 0, sum = 0;
@@ -410,7 +403,6 @@ da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt
                                   "The tensor-core kNN kernel timed out waiting on a pipeline "
                                   "barrier (code " + std::to_string(h[1]) + ").");
             flagged += h[0];
-            cuda->stats["knn_tc_fallback_queries"] += (double)h[0];
             cuda->stats["knn_tc_fallback_list_overflow"] += (double)h[2];
             cuda->stats["knn_tc_fallback_few_survivors"] += (double)h[4];
         }
@@ -422,57 +414,146 @@ da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, int kc, bool take_sqrt
         cuda->stats["knn_tc_mean_list"] = sum / std::max<double>(1.0, (double)nq);
         if (flagged == 0) return da_status_success;
         // the queries the pass could not certify: the plain path on just those
-        // rows (gathered, searched, scattered back)
         redone = true;
-        std::vector<int> flags((size_t)nq), idx;
-        B200_TRY(cudaMemcpyAsync(flags.data(), dTkFlag.p, flags.size() * sizeof(int),
-                                 cudaMemcpyDeviceToHost, st), "copy");
-        B200_TRY(cudaStreamSynchronize(st), "copy");
-        for (int i = 0; i < (int)nq; ++i)
-            if (flags[i]) idx.push_back(i);
-        const int m = (int)idx.size();
-        const int BN = knn_tile_rows_train(false);
-        const int q_tiles = (m + 63) / 64;
-        const int max_chunks = std::max(1, (int)((n_samples + BN - 1) / BN));
-        // enough CTAs to fill the GPU, but at most ~16K partial entries per query
-        // (the merge ranks every entry against every chunk list)
-        int n_chunks = std::max(1, std::min({max_chunks, (148 * 8 + q_tiles - 1) / q_tiles,
-                                             std::max(8, 16384 / (int)k)}));
-        int chunk_rows = (int)((n_samples + n_chunks - 1) / n_chunks);
-        chunk_rows = ((chunk_rows + BN - 1) / BN) * BN;
-        n_chunks = (int)((n_samples + chunk_rows - 1) / chunk_rows);
-        // scratch inside the (now free) candidate-list buffer
-        const size_t parts = (size_t)m * n_chunks * k;
-        const size_t need = (size_t)m * 4 + (size_t)m * ld * 4 + parts * 8 +
-                            (size_t)m * k * 8 + (size_t)m * 4 + 1280;
-        if (!dTkList.ensure(need))
-            return err->error(da_status_memory_error, "Device memory allocation failed.");
-        char *p = dTkList.as<char>();
-        int *didx = reinterpret_cast<int *>(p);
-        float *qsub = reinterpret_cast<float *>(p + ((size_t)m * 4 + 255) / 256 * 256);
-        float *pk = qsub + (size_t)m * ld;
-        int *pi = reinterpret_cast<int *>(pk + parts);
-        float *ok = reinterpret_cast<float *>(pi + parts);
-        int *oi = reinterpret_cast<int *>(ok + (size_t)m * k);
-        float *qnsub = reinterpret_cast<float *>(oi + (size_t)m * k);
-        KnnArgs pa{cosine ? ACC_DOT : ACC_SQEUC, cosine ? POST_COSINE : POST_NONE, kc, 2.0, (int)k,
-                   chunk_rows, n_chunks};
-        B200_TRY(cudaMemcpyAsync(didx, idx.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st),
-                 "copy");
-        B200_TRY(launch_rows_gather(dQ.as<float>(), ld, didx, m, qsub, st), "gather");
-        if (cosine) B200_TRY(launch_rows_gather(dQn.as<float>(), 1, didx, m, qnsub, st), "gather");
-        B200_TRY(launch_knn_chunks<float>(qsub, ld, m, dX.as<float>(), ld, (int)n_samples, (int)d,
-                                          cosine ? qnsub : nullptr,
-                                          cosine ? dXn.as<float>() : nullptr, pa, pk, pi, nullptr,
-                                          st), "kNN distance kernel");
-        B200_TRY(launch_knn_merge<float>(pk, pi, m, n_chunks, (int)k, take_sqrt && !cosine ? 1 : 0,
-                                         ok, oi, st), "kNN merge kernel");
-        B200_TRY(launch_results_scatter(ok, oi, didx, m, (int)k, dOutK.as<float>(),
-                                        out_idx((size_t)nq * k), st), "scatter");
+        std::vector<int> idx, over;
+        da_status s = flagged_queries(dTkFlag.as<int>(), (size_t)nq, idx);
+        if (s != da_status_success) return s;
+        cuda->stats["knn_tc_fallback_queries"] = (double)idx.size();
+        s = knn_select_some(nq, d, k, w, idx, over);
+        return s == da_status_success ? knn_lists(nq, d, k, w, &over) : s;
     } else {
-        (void)nq, (void)d, (void)k, (void)kc, (void)take_sqrt, (void)cosine, (void)extra;
+        (void)nq, (void)d, (void)k, (void)w, (void)extra;
     }
     return da_status_success;
+}
+
+// The numbers of the queries whose word is set (synchronises).
+template <typename T>
+da_status NN<T>::flagged_queries(const int *words, size_t nq, std::vector<int> &idx) {
+    std::vector<int> h(nq);
+    B200_TRY(cudaMemcpyAsync(h.data(), words, nq * sizeof(int), cudaMemcpyDeviceToHost,
+                             cuda->stream), "copy");
+    B200_TRY(cudaStreamSynchronize(cuda->stream), "copy");
+    idx.clear();
+    for (size_t i = 0; i < nq; ++i)
+        if (h[i]) idx.push_back((int)i);
+    return da_status_success;
+}
+
+// Queries idx[0 .. m) brought together, with room for their results, in the
+// upload's stage (free by the time a search has run).
+template <typename T>
+da_status NN<T>::gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g) {
+    cudaStream_t st = cuda->stream;
+    const size_t mk = m * k;
+    if (!dStage.ensure((m * ld + m + mk) * sizeof(T) + (mk + 2 * m + 1) * sizeof(int)))
+        return err->error(da_status_memory_error, "Device memory allocation failed.");
+    g.Q = dStage.as<T>();
+    g.qn = g.Q + m * ld;
+    g.key = g.qn + m;
+    g.ind = reinterpret_cast<int *>(g.key + mk);
+    g.number = g.ind + mk;
+    g.redo = g.number + m;
+    g.flag = g.redo + m;
+    B200_TRY(cudaMemcpyAsync(g.number, idx, m * sizeof(int), cudaMemcpyHostToDevice, st), "copy");
+    B200_TRY(launch_rows_gather(dQ.p, ld * sizeof(T), g.number, (int)m, g.Q, st), "gather");
+    if (w.qn) B200_TRY(launch_rows_gather(w.qn, sizeof(T), g.number, (int)m, g.qn, st), "gather");
+    else g.qn = nullptr;
+    return da_status_success;
+}
+template <typename T>
+da_status NN<T>::scatter_results(da_int nq, da_int k, size_t m, const Gathered &g) {
+    cudaStream_t st = cuda->stream;
+    B200_TRY(launch_rows_scatter(g.key, k * sizeof(T), g.number, (int)m, dOutK.p, st), "scatter");
+    B200_TRY(launch_rows_scatter(g.ind, k * sizeof(int), g.number, (int)m, out_idx((size_t)nq * k),
+                                 st), "scatter");
+    return da_status_success;
+}
+
+// Queries per batch of the selection passes: 256 MB of lists.
+template <typename T> size_t NN<T>::sel_batch(const KnnSelPlan &pl) const {
+    const size_t per = knn_sel_bytes(pl, 1, sizeof(T) == 8);
+    return std::max<size_t>(64, ((size_t)1 << 28) / per / 64 * 64);
+}
+
+// Some queries by the selection passes, into dOutK; the numbers of those whose
+// list overflowed in `over` (all where the passes do not apply).
+template <typename T>
+da_status NN<T>::knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
+                                 const std::vector<int> &idx, std::vector<int> &over) {
+    cudaStream_t st = cuda->stream;
+    const bool fp64 = sizeof(T) == 8;
+    over.clear();
+    KnnSelPlan pl{};
+    if (!knn_sel_plan((int)n_samples, (int)std::min<size_t>(idx.size(), 65536), (int)k, fp64, pl)) {
+        over = idx;
+        return da_status_success;
+    }
+    const KnnArgs a{w.acc, w.post, w.kc, (double)p, (int)k, 0, 0};
+    const size_t qb = std::min(idx.size(), sel_batch(pl));
+    for (size_t i0 = 0; i0 < idx.size(); i0 += qb) {
+        const size_t m = std::min(qb, idx.size() - i0);
+        Gathered g;
+        da_status s = gather_queries(idx.data() + i0, m, k, w, g);
+        if (s != da_status_success) return s;
+        if (!dPartK.ensure(knn_sel_bytes(pl, (int)m, fp64)))
+            return err->error(da_status_memory_error, "Device memory allocation failed.");
+        B200_TRY(cuda->timed("knn_select", [&] {
+            return launch_knn_select<T>(g.Q, (int)m, dX.as<T>(), (int)n_samples, ld, (int)d, g.qn,
+                                        w.xn, a, pl, dPartK.p, w.tf, g.key, g.ind, g.flag, g.redo, st);
+        }), "kNN selection kernels");
+        s = scatter_results(nq, k, m, g);
+        if (s != da_status_success) return s;
+        std::vector<int> f;
+        s = flagged_queries(g.redo, m, f);
+        if (s != da_status_success) return s;
+        for (int i : f) over.push_back(idx[i0 + i]);
+    }
+    return da_status_success;
+}
+
+// Running lists and their merge into dOutK, for all queries or those of `only`.
+template <typename T>
+da_status NN<T>::knn_lists(da_int nq, da_int d, da_int k, const KnnWay &w,
+                           const std::vector<int> *only) {
+    cudaStream_t st = cuda->stream;
+    const bool fp64 = sizeof(T) == 8;
+    const size_t m = only ? only->size() : (size_t)nq;
+    if (m == 0) return da_status_success;
+    cuda->stats["knn_select_fallback"] = (double)m;
+    if (m == (size_t)nq) only = nullptr;
+    // chunking of the training rows: enough CTAs to fill 148 SMs several times
+    const int BN = knn_tile_rows_train(fp64);
+    const int q_tiles = (int)((m + 63) / 64);
+    const int max_chunks = std::max(1, (int)((n_samples + BN - 1) / BN));
+    // enough CTAs to fill the GPU; but one warp merges a query's lists, in a time
+    // that grows with the square of their number (391 lists of 5: 8.3 ms, the rows
+    // of as many chunks: 10 us a tile), so for few queries the sum of both is
+    // least near the cube root below
+    const double merge = (double)k * std::log2(k + 1.0);
+    const int balance = std::max(8, (int)std::cbrt(10.0 * (double)n_samples / merge));
+    int n_chunks = std::max(1, std::min({max_chunks, (148 * 8 + q_tiles - 1) / q_tiles, balance}));
+    int chunk_rows = (int)((n_samples + n_chunks - 1) / n_chunks);
+    chunk_rows = ((chunk_rows + BN - 1) / BN) * BN;
+    n_chunks = (int)((n_samples + chunk_rows - 1) / chunk_rows);
+    const KnnArgs a{w.acc, w.post, w.kc, (double)p, (int)k, chunk_rows, n_chunks};
+    const size_t parts = m * k * n_chunks;
+    if (!dPartK.ensure(parts * sizeof(T)) || !dPartI.ensure(parts * sizeof(int)))
+        return err->error(da_status_memory_error, "Device memory allocation failed.");
+    Gathered g{dQ.as<T>(), const_cast<T *>(w.qn), dOutK.as<T>(), out_idx((size_t)nq * k), nullptr, nullptr, nullptr};
+    if (only) {
+        const da_status s = gather_queries(only->data(), m, k, w, g);
+        if (s != da_status_success) return s;
+    }
+    B200_TRY(cuda->timed("knn_chunks", [&] {
+        return launch_knn_chunks<T>(g.Q, ld, (int)m, dX.as<T>(), ld, (int)n_samples, (int)d, g.qn,
+                                    w.xn, a, dPartK.as<T>(), dPartI.as<int>(), nullptr, st);
+    }), "kNN distance kernel");
+    B200_TRY(cuda->timed("knn_merge", [&] {
+        return launch_knn_merge<T>(dPartK.as<T>(), dPartI.as<int>(), (int)m, n_chunks, (int)k, w.tf,
+                                   g.key, g.ind, st);
+    }), "kNN merge kernel");
+    return only ? scatter_results(nq, k, m, g) : da_status_success;
 }
 
 template <typename T> da_status NN<T>::set_labels(da_int n, const da_int *y) {
@@ -554,10 +635,11 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
         return err->error(da_status_memory_error, "Device memory allocation failed.");
     B200_TRY(upload_matrix<T>(ord, nq, d, Xt, ldt, dQ.as<T>(), ld, dStage, st), "upload of X_test");
     cuda->stats["tensor_core"] = 0.0;
+    cuda->stats["knn_select_fallback"] = 0.0;
     cuda->stats["knn_tc_fallback_queries"] = 0.0;
     cuda->stats["knn_tc_fallback_list_overflow"] = 0.0;
-    cuda->stats["knn_tc_fallback_many_survivors"] = 0.0;
     cuda->stats["knn_tc_fallback_few_survivors"] = 0.0;
+    KnnWay way{acc, post, tf, kc, nullptr, nullptr};
     bool tc_done = false;
     size_t n_extra = 0; // ints after the indices: tc_finish's, or the flags below
     const bool tc_metric = metric == M_EUC || metric == M_SQEUC || metric == M_COS ||
@@ -571,23 +653,24 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
     if (!fp64 && tc_metric && opts.key("precision mode") != 0 &&
         knn_tc_supported((int)n_samples, (int)d, (int)k) && n_samples >= 16384 &&
         (double)n_samples * (double)std::max<da_int>(nq, 64) * (double)d >= 5.0e8) {
-        s = kneighbors_tc(nq, d, k, kc, metric != M_SQEUC && metric != M_COS, metric == M_COS,
-                          n_extra, tc_done);
+        s = kneighbors_tc(nq, d, k, way, n_extra, tc_done);
         if (s != da_status_success) return s;
+        if (tc_done && metric == M_COS) {
+            way.qn = dQn.as<T>();
+            way.xn = dXn.as<T>();
+        }
     }
     // the plain path: bounds first (launch_knn_select) in query batches of at
-    // most 256 MB of lists, each with its own flag after the indices; running
-    // lists (run_lists) where that does not apply or a flag comes back set
+    // most 256 MB of lists, each with its own flag after the indices, then a flag
+    // per query; running lists (knn_lists) where that does not apply and for the
+    // queries whose flag comes back set (the others' results stay)
     KnnSelPlan sel{};
     da_int sel_qb = 0;
-    std::function<da_status()> run_lists;
     if (!tc_done) {
         if (knn_sel_plan((int)n_samples, (int)std::min<da_int>(nq, 65536), (int)k, fp64, sel)) {
-            const size_t per = knn_sel_bytes(sel, 1, fp64);
-            sel_qb = std::min(nq, (da_int)std::max<size_t>(64, ((size_t)1 << 28) / per / 64 * 64));
+            sel_qb = std::min(nq, (da_int)sel_batch(sel));
             n_extra = (size_t)((nq + sel_qb - 1) / sel_qb);
         }
-        const T *qn = nullptr, *xn = nullptr;
         if (norm_kind >= 0) {
             if (!dQn.ensure((size_t)nq * sizeof(T)) || !dXn.ensure((size_t)n_samples * sizeof(T)))
                 return err->error(da_status_memory_error, "Device memory allocation failed.");
@@ -601,61 +684,32 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
                     B200_TRY(launch_row_norms_eps1<T>(dX.as<T>(), ld, n_samples, d, dXn.as<T>(), st), "norms");
             }
             xn_kind = norm_kind;
-            qn = dQn.as<T>();
-            xn = dXn.as<T>();
+            way.qn = dQn.as<T>();
+            way.xn = dXn.as<T>();
         }
         if (k > knn_max_k(fp64))
             return err->error(da_status_not_implemented,
                               "k = " + std::to_string(k) + " exceeds the largest supported number "
                               "of neighbours per query (" + std::to_string(knn_max_k(fp64)) + ").");
-        if (!dOutK.ensure(out_bytes((size_t)nq * k, n_extra)))
+        if (!dOutK.ensure(out_bytes((size_t)nq * k, n_extra > 0 ? n_extra + nq : 0)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
         if (n_extra > 0) {
             const KnnArgs a{acc, post, kc, (double)p, (int)k, 0, 0};
             if (!dPartK.ensure(knn_sel_bytes(sel, (int)sel_qb, fp64)))
                 return err->error(da_status_memory_error, "Device memory allocation failed.");
-            int *flags = out_idx((size_t)nq * k) + (size_t)nq * k;
+            int *flags = out_idx((size_t)nq * k) + (size_t)nq * k, *redo = flags + n_extra;
             for (da_int q0 = 0; q0 < nq; q0 += sel_qb, ++flags) {
                 const da_int nb = std::min(sel_qb, nq - q0);
                 B200_TRY(cuda->timed("knn_select", [&] {
-                    return launch_knn_select<T>(dQ.as<T>() + (size_t)q0 * ld, (int)nb, dX.as<T>(),
-                                                (int)n_samples, ld, (int)d, qn ? qn + q0 : nullptr,
-                                                xn, a, sel, dPartK.p, tf,
-                                                dOutK.as<T>() + (size_t)q0 * k,
-                                                out_idx((size_t)nq * k) + (size_t)q0 * k, flags, st);
+                    return launch_knn_select<T>(
+                        dQ.as<T>() + (size_t)q0 * ld, (int)nb, dX.as<T>(), (int)n_samples, ld, (int)d,
+                        way.qn ? way.qn + q0 : nullptr, way.xn, a, sel, dPartK.p, tf,
+                        dOutK.as<T>() + (size_t)q0 * k, out_idx((size_t)nq * k) + (size_t)q0 * k,
+                        flags, redo + q0, st);
                 }), "kNN selection kernels");
             }
-        }
-        run_lists = [&, qn, xn]() -> da_status {
-            // chunking of the training rows: enough CTAs to fill 148 SMs several times
-            const int BN = knn_tile_rows_train(fp64);
-            const int q_tiles = (int)((nq + 63) / 64);
-            const int max_chunks = std::max(1, (int)((n_samples + BN - 1) / BN));
-            // enough CTAs to fill the GPU, but at most ~16K partial entries per query
-            // (the merge ranks every entry against every chunk list)
-            int n_chunks = std::max(1, std::min({max_chunks, (148 * 8 + q_tiles - 1) / q_tiles,
-                                                 std::max(8, 16384 / (int)k)}));
-            int chunk_rows = (int)((n_samples + n_chunks - 1) / n_chunks);
-            chunk_rows = ((chunk_rows + BN - 1) / BN) * BN;
-            n_chunks = (int)((n_samples + chunk_rows - 1) / chunk_rows);
-            KnnArgs a{acc, post, kc, (double)p, (int)k, chunk_rows, n_chunks};
-            const size_t parts = (size_t)nq * n_chunks * k;
-            if (!dPartK.ensure(parts * sizeof(T)) || !dPartI.ensure(parts * sizeof(int)) ||
-                !dOutK.ensure(out_bytes((size_t)nq * k, 0)))
-                return err->error(da_status_memory_error, "Device memory allocation failed.");
-            B200_TRY(cuda->timed("knn_chunks", [&] {
-                return launch_knn_chunks<T>(dQ.as<T>(), ld, (int)nq, dX.as<T>(), ld, (int)n_samples,
-                                            (int)d, qn, xn, a, dPartK.as<T>(), dPartI.as<int>(), nullptr,
-                                            st);
-            }), "kNN distance kernel");
-            B200_TRY(cuda->timed("knn_merge", [&] {
-                return launch_knn_merge<T>(dPartK.as<T>(), dPartI.as<int>(), (int)nq, n_chunks, (int)k,
-                                           tf, dOutK.as<T>(), out_idx((size_t)nq * k), st);
-            }), "kNN merge kernel");
-            return da_status_success;
-        };
-        if (n_extra == 0) {
-            s = run_lists();
+        } else {
+            s = knn_lists(nq, d, k, way, nullptr);
             if (s != da_status_success) return s;
         }
     }
@@ -719,15 +773,14 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
         if (n_extra == 0) break;
         if (tc_done) {
             bool redone = false;
-            s = tc_finish(nq, d, k, kc, metric != M_SQEUC && metric != M_COS, metric == M_COS,
-                          extra.data(), redone);
+            s = tc_finish(nq, d, k, way, extra.data(), redone);
             if (s != da_status_success) return s;
             if (!redone) break;
         } else {
             if (std::all_of(extra.begin(), extra.end(), [](int f) { return f == 0; })) break;
-            // a query's list overflowed or was short of k keys
-            cuda->stats["knn_select_fallback"] += 1.0;
-            s = run_lists();
+            std::vector<int> over; // the queries whose list overflowed
+            s = flagged_queries(out_idx(nk) + nk + n_extra, (size_t)nq, over);
+            if (s == da_status_success) s = knn_lists(nq, d, k, way, &over);
             if (s != da_status_success) return s;
         }
         n_extra = 0;

@@ -25,19 +25,27 @@ def test_few_queries_without_numbers(gpu, ab, orc, dtype, n, nq, metric, order):
     prec = "d" if dtype == np.float64 else "s"
     nn = ab.KNN(prec, order=order, metric=metric, algorithm="brute").fit(X)
     ind, dist = nn.kneighbors(Q, 7)
-    # (a query that is not a number can have neighbours under the reference's cosine)
-    stat = "knn_tc_fallback_queries" if nn.stat("tensor_core") else "knn_select_fallback"
     assert nn.stat("tensor_core") == (n == 70_000)
-    assert nn.stat(stat) == 3
-    good = np.setdiff1d(np.arange(nq), bad)
-    oi, od = orc.knn(X, Q[good], 7, metric)
-    np.testing.assert_array_equal(ind[good], oi)
-    np.testing.assert_array_equal(dist[good], od)
-    alone = nn.kneighbors(Q[bad], 7)
-    np.testing.assert_array_equal(ind[bad], alone[0])
-    np.testing.assert_array_equal(dist[bad], alone[1])
-    assert nn.stat("knn_select_fallback") in (0, 3)
-    clean = nn.kneighbors(Q[good], 7)
-    np.testing.assert_array_equal(ind[good], clean[0])
-    np.testing.assert_array_equal(dist[good], clean[1])
+    if n == 70_000:
+        assert nn.stat("knn_tc_fallback_queries") == 3
     assert nn.stat("knn_select_fallback") == 0
+    oi, od = orc.knn(X, Q, 7, metric)
+    np.testing.assert_array_equal(ind, oi)
+    np.testing.assert_array_equal(dist, od)
+
+
+@pytest.mark.parametrize("prec", ["s", "d"])
+def test_few_queries_among_equal_rows(gpu, ab, orc, prec):
+    """Queries whose bound ties with more rows than a list holds: running lists for
+    them alone."""
+    rng = np.random.default_rng(8)
+    X, Q = rows(rng, 15_000, 20, "f" if prec == "s" else "d"), None
+    X[rng.choice(len(X), 6000, replace=False)] = X[0]
+    Q = rows(rng, 400, 20, X.dtype)
+    Q[[3, 200, 399]] = X[0]
+    nn = ab.KNN(prec, metric="manhattan", algorithm="brute").fit(X)
+    ind, dist = nn.kneighbors(Q, 5)
+    assert 3 <= nn.stat("knn_select_fallback") < 40
+    oi, od = orc.knn(X, Q, 5, "manhattan")
+    np.testing.assert_array_equal(ind, oi)
+    np.testing.assert_array_equal(dist, od)
