@@ -147,18 +147,27 @@ template <typename T> struct NN : public AlgBase {
     };
     da_status kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, size_t &n_extra,
                             bool &done);
+    da_status tc_check(const int *state);
     da_status tc_finish(da_int nq, da_int d, da_int k, const KnnWay &w, const int *extra,
                         bool &redone);
     struct Gathered { // some of the queries, and their results
         T *Q, *qn, *key;
-        int *ind, *number, *redo, *flag;
+        int *ind, *number, *redo, *state; // state: KNN_TC_STATE words, then one a query
     };
-    da_status flagged_queries(const int *words, size_t nq, std::vector<int> &idx);
+    // (again: queries with a closer bound at their first output key; over: without)
+    struct Redo {
+        std::vector<int> again, over;
+    };
+    da_status flagged_queries(const int *words, size_t nq, const int *number, Redo &r);
     da_status gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g);
     da_status scatter_results(da_int nq, da_int k, size_t m, const Gathered &g);
     size_t sel_batch(const KnnSelPlan &pl) const;
     da_status knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
-                              const std::vector<int> &idx, std::vector<int> &over);
+                              const std::vector<int> &idx, bool given, Redo &r);
+    da_status knn_tc_some(da_int nq, da_int d, da_int k, const KnnWay &w,
+                          const std::vector<int> &idx, Redo &r);
+    da_status knn_redo(da_int nq, da_int d, da_int k, const KnnWay &w, std::vector<int> &fresh,
+                       Redo &r);
     da_status knn_lists(da_int nq, da_int d, da_int k, const KnnWay &w,
                         const std::vector<int> *only);
     da_status compute_proba(da_int nq, da_int d, const T *Xt, da_int ldt, std::vector<T> &proba);

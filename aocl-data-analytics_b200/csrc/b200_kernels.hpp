@@ -135,7 +135,7 @@ int knn_max_k(bool fp64);
 constexpr int KNN_SEL_GROUPS = 512; // sample minima per query, at most
 constexpr int KNN_SEL_CAP = 4096;   // listed keys per query, at most
 struct KnnSelPlan {
-    int n_sample, step;          // sample rows: every step-th row
+    int n_sample, step;          // sample rows: one of every `step`
     int parts, part_rows;        // blocks over the sample, rows of each
     int groups;                  // minima per query (32 per part)
     int cap;                     // list entries per query (a power of two)
@@ -147,21 +147,24 @@ size_t knn_sel_bytes(const KnnSelPlan &pl, int nq, bool fp64);
 cudaError_t launch_knn_bound(const float *minima, int groups, int nq, int k, float *bound,
                              cudaStream_t s);
 // out_key / out_idx as launch_knn_merge's; *flag and the query's redo word are
-// set to 1 when its list overflowed (its outputs are then unwritten), else 0.
+// set when its list overflowed: 2 with a closer bound as the query's first
+// output key, 1 where there is none; else 0.  given: such bounds, a.k apart,
+// in place of the sample's.
 template <typename T>
 cudaError_t launch_knn_select(const T *Q, int nq, const T *X, int nx, int ld, int d, const T *qn,
                               const T *xn, const KnnArgs &a, const KnnSelPlan &pl, void *work,
                               int tf, T *out_key, int *out_idx, int *flag, int *redo,
-                              cudaStream_t s);
+                              const T *given, cudaStream_t s);
 
 // ---------------------------------------------- kNN tensor-core pass ---
 // fp32 euclidean / squared euclidean / cosine: bf16x3 tcgen05 candidate pass with a
 // certified threshold per query, exact re-score of the survivors in the plain
 // kernel's order.  Results (q-major, as launch_knn_merge) equal the plain
-// path's; queries the pass cannot certify are flagged in `fallback`
-// (*n_fallback of them) for the plain path.
+// path's; queries the pass cannot certify are flagged in `fallback` (state[0] of
+// them): 2 with a closer bound as the first output key, for another list pass
+// (given: such bounds, k apart, in place of the sample's), 1 for the plain path.
 int knn_tc_supported(int nx, int d, int k);
-// Sizes of its passes: sample rows (every step-th), row tiles of a sample work
+// Sizes of its passes: sample rows (every step-th, a prime), row tiles of a sample work
 // item, minima per query; row tiles of a list work item; list entries per
 // query (8 bytes each).
 struct KnnTcPlan {
@@ -190,7 +193,8 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
                           const float *xmax, int nx, int ld, int ldbf, int d, const float *Q,
                           int nq, int k, int kc, int take_sqrt, const KnnTcPlan &pl, void *qbuf,
                           void *list, int *fallback, int *cnt, int *state, float *out_key,
-                          int *out_idx, cudaStream_t s, const KnnTcCosine *cosine = nullptr);
+                          int *out_idx, cudaStream_t s, const KnnTcCosine *cosine = nullptr,
+                          const float *given = nullptr);
 
 // Radius search, fp32 (squared) euclidean: a mask of the rows whose tensor-core
 // value may be within thr (radius_tc_words(nx) words per query, 32 rows each),

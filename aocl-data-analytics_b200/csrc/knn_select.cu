@@ -6,7 +6,7 @@
 // threshold, so that all of its first keys go through merges, and the blocks'
 // lists are merged once more.  Here three short passes give every query a
 // bound first:
-//   * knn_min_kernel: the keys of an evenly strided sample of the rows; every
+//   * knn_min_kernel: the keys of a sample, one row of every `step`; every
 //     thread keeps the smallest of each query's keys that it sees, one value
 //     per (query, 32 thread groups, block);
 //   * knn_bound_kernel: the k-th smallest of those minima -- k keys of k
@@ -14,8 +14,10 @@
 //   * knn_append_kernel: the keys of all rows; those at or below the bound are
 //     collected in shared memory and go to the query's list in global memory;
 //   * knn_pick_kernel: sorts the list by (key, index) and writes its first k.
-// A list that overflows raises the flag, and the caller searches its query with
-// running lists (knn_chunk_kernel).  Fewer than k entries are all keys that are
+// A list that overflows raises the flag; the k-th of the keys that it holds is a
+// closer bound, with which the caller runs the last two passes again for its
+// query, and running lists (knn_chunk_kernel) where that does not help (ties).
+// Fewer than k entries are all keys that are
 // numbers: fewer than k finite minima leave the bound at +inf.
 //
 // The passes are bound by FP32 / FP64 issue (tile_sweep.cuh).  Measured on a
@@ -41,7 +43,7 @@ B200_DEV double min_num(double a, double b) { return fmin(a, b); }
 // sets of the part's sample rows (thread column x two sets of its columns).
 template <typename T, int ACC>
 __global__ void __launch_bounds__(256, 2)
-knn_min_kernel(const T *Q, int nq, const T *X, int step, int n_sample, int part_rows, int ld,
+knn_min_kernel(const T *Q, int nq, const T *X, SampleRows rows, int n_sample, int part_rows, int ld,
                int d, const T *qn, const T *xn, int post, int kc, T p, T invp, T *minima,
                int groups) {
     constexpr int TM = SweepAcc<T, ACC>::TM, TN = SweepAcc<T, ACC>::TN;
@@ -58,8 +60,8 @@ knn_min_kernel(const T *Q, int nq, const T *X, int step, int n_sample, int part_
     }
     SweepAcc<T, ACC> acc;
     sweep_tiles<T, ACC>(
-        st, Q, nq, q0, X, (size_t)ld * step, x_begin, x_end, ld, d, kc, p, acc, tid, [&](int x0) {
-            sweep_post<T, ACC>(acc, post, qv, xn, (size_t)step, x0, x_end, tn, invp,
+        st, Q, nq, q0, X, rows, x_begin, x_end, ld, d, kc, p, acc, tid, [&](int x0) {
+            sweep_post<T, ACC>(acc, post, qv, xn, rows, x0, x_end, tn, invp,
                                [&](int i, T (&key)[TN]) {
 #pragma unroll
                                    for (int j = 0; j < TN; ++j) {
@@ -164,7 +166,8 @@ void bound_pass(const T *minima, int groups, int nq, int k, T *bound, int *cnt, 
 // Block (query tile, row chunk): appends every (key, row) with key <= the
 // query's bound to its list.  Hits wait in shared memory, HITS per query; one
 // global reservation per query and block moves them, and what does not fit
-// reserves its own slot.
+// reserves its own slot until the list is full (its query then gets a closer
+// bound from what it holds).
 template <typename T> struct SelHits;
 template <> struct SelHits<float> { static constexpr int N = 24; };
 template <> struct SelHits<double> { static constexpr int N = 16; };
@@ -194,9 +197,9 @@ knn_append_kernel(const T *Q, int nq, const T *X, int nx, int ld, int d, const T
     }
     SweepAcc<T, ACC> acc;
     sweep_tiles<T, ACC>(
-        st, Q, nq, q0, X, (size_t)ld, x_begin, x_end, ld, d, kc, p, acc, tid, [&](int x0) {
+        st, Q, nq, q0, X, AllRows{}, x_begin, x_end, ld, d, kc, p, acc, tid, [&](int x0) {
             sweep_post<T, ACC>(
-                acc, post, qv, xn, (size_t)1, x0, x_end, tn, invp, [&](int i, T (&key)[TN]) {
+                acc, post, qv, xn, AllRows{}, x0, x_end, tn, invp, [&](int i, T (&key)[TN]) {
                     // few keys pass: one test for the row first (the minimum
                     // of the keys that are not NaN)
                     T m = key[0];
@@ -218,6 +221,8 @@ knn_append_kernel(const T *Q, int nq, const T *X, int nx, int ld, int d, const T
                             if (gp < cap) {
                                 list_key[(size_t)(q0 + ql) * cap + gp] = key[j];
                                 list_idx[(size_t)(q0 + ql) * cap + gp] = gx;
+                            } else {
+                                thr[i] = -Lim<T>::inf(); // full: it takes no more
                             }
                         }
                     }
@@ -239,20 +244,18 @@ knn_append_kernel(const T *Q, int nq, const T *X, int nx, int ld, int d, const T
 
 // One block per query: the listed entries sorted by (key, index), the first k
 // written (tf 1: square root, 2: negated; past the last entry index -1, distance
-// +inf).
+// +inf).  A list that overflowed: its k-th key at the query's first output, and
+// whether that is below the bound (redo 2) or not (1).
 template <typename T>
 __global__ void __launch_bounds__(128)
 knn_pick_kernel(const int *cnt, const T *list_key, const int *list_idx, int cap, int k, int tf,
-                T *ok, int *oi, int *flag, int *redo) {
+                const T *bound, T *ok, int *oi, int *flag, int *redo) {
     extern __shared__ __align__(16) unsigned char pick_sm[];
     T *sk = reinterpret_cast<T *>(pick_sm);           // cap
     int *si = reinterpret_cast<int *>(sk + cap);      // cap
     const int q = blockIdx.x;
-    const int m = cnt[q];
-    if (m > cap) {
-        if (threadIdx.x == 0) *flag = redo[q] = 1;
-        return;
-    }
+    const bool over = cnt[q] > cap;
+    const int m = min(cnt[q], cap);
     int np2 = 1;
     while (np2 < m) np2 <<= 1; // <= cap, a power of two
     for (int e = threadIdx.x; e < np2; e += 128) {
@@ -276,6 +279,14 @@ knn_pick_kernel(const int *cnt, const T *list_key, const int *list_idx, int cap,
             }
             __syncthreads();
         }
+    if (over) {
+        if (threadIdx.x == 0) {
+            *flag = 1;
+            redo[q] = sk[k - 1] < bound[q] ? 2 : 1;
+            ok[(size_t)q * k] = sk[k - 1];
+        }
+        return;
+    }
     for (int r = threadIdx.x; r < k; r += 128) {
         T v = r < m ? sk[r] : Lim<T>::inf();
         if (tf == 1) v = sqrt_rn(v);
@@ -288,7 +299,7 @@ knn_pick_kernel(const int *cnt, const T *list_key, const int *list_idx, int cap,
 template <typename T, int ACC>
 cudaError_t select_t(const T *Q, int nq, const T *X, int nx, int ld, int d, const T *qn,
                      const T *xn, const KnnArgs &a, const KnnSelPlan &pl, void *work, int tf,
-                     T *ok, int *oi, int *flag, int *redo, cudaStream_t s) {
+                     T *ok, int *oi, int *flag, int *redo, const T *given, cudaStream_t s) {
     constexpr int BM = SW_BM, BN = SweepStage<T>::BN;
     const T p = T(a.p), invp = T(1.0 / (double)p);
     T *list_key = static_cast<T *>(work);
@@ -297,10 +308,20 @@ cudaError_t select_t(const T *Q, int nq, const T *X, int nx, int ld, int d, cons
     int *list_idx = reinterpret_cast<int *>(bound + nq);
     int *cnt = list_idx + (size_t)nq * pl.cap;
     const int qt = (nq + BM - 1) / BM;
-    knn_min_kernel<T, ACC><<<dim3(qt, pl.parts), 256, 0, s>>>(
-        Q, nq, X, pl.step, pl.n_sample, pl.part_rows, ld, d, qn, xn, a.post, a.kc, p, invp, minima,
-        pl.groups);
-    bound_pass(minima, pl.groups, nq, a.k, bound, cnt, flag, redo, s);
+    cudaError_t e = cudaSuccess;
+    if (given) {
+        e = cudaMemcpy2DAsync(bound, sizeof(T), given, a.k * sizeof(T), sizeof(T), nq,
+                              cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, nq * sizeof(int), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(redo, 0, nq * sizeof(int), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, sizeof(int), s);
+        if (e != cudaSuccess) return e;
+    } else {
+        knn_min_kernel<T, ACC><<<dim3(qt, pl.parts), 256, 0, s>>>(
+            Q, nq, X, SampleRows{pl.step, nx}, pl.n_sample, pl.part_rows, ld, d, qn, xn, a.post,
+            a.kc, p, invp, minima, pl.groups);
+        bound_pass(minima, pl.groups, nq, a.k, bound, cnt, flag, redo, s);
+    }
     // chunks of whole row tiles: about four blocks per SM slot (two slots per
     // SM), so that the last wave costs little
     const int tiles = (nx + BN - 1) / BN;
@@ -311,10 +332,10 @@ cudaError_t select_t(const T *Q, int nq, const T *X, int nx, int ld, int d, cons
         Q, nq, X, nx, ld, d, qn, xn, a.post, a.kc, p, invp, chunk_rows, bound, cnt, list_key,
         list_idx, pl.cap);
     const size_t smem = (size_t)pl.cap * (sizeof(T) + 4);
-    cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(knn_pick_kernel<T>), smem);
+    e = ensure_smem_limit(reinterpret_cast<const void *>(knn_pick_kernel<T>), smem);
     if (e != cudaSuccess) return e;
-    knn_pick_kernel<T><<<nq, 128, smem, s>>>(cnt, list_key, list_idx, pl.cap, a.k, tf, ok, oi, flag,
-                                             redo);
+    knn_pick_kernel<T><<<nq, 128, smem, s>>>(cnt, list_key, list_idx, pl.cap, a.k, tf, bound, ok, oi,
+                                             flag, redo);
     return cudaGetLastError();
 }
 
@@ -366,29 +387,29 @@ template <typename T>
 cudaError_t launch_knn_select(const T *Q, int nq, const T *X, int nx, int ld, int d, const T *qn,
                               const T *xn, const KnnArgs &a, const KnnSelPlan &pl, void *work,
                               int tf, T *out_key, int *out_idx, int *flag, int *redo,
-                              cudaStream_t s) {
+                              const T *given, cudaStream_t s) {
     switch (a.acc) {
     case ACC_SQEUC:
         return select_t<T, ACC_SQEUC>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key,
-                                      out_idx, flag, redo, s);
+                                      out_idx, flag, redo, given, s);
     case ACC_DOT:
         return select_t<T, ACC_DOT>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key, out_idx,
-                                    flag, redo, s);
+                                    flag, redo, given, s);
     case ACC_MANHATTAN:
         return select_t<T, ACC_MANHATTAN>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key,
-                                          out_idx, flag, redo, s);
+                                          out_idx, flag, redo, given, s);
     default:
         return select_t<T, ACC_MINKOWSKI>(Q, nq, X, nx, ld, d, qn, xn, a, pl, work, tf, out_key,
-                                          out_idx, flag, redo, s);
+                                          out_idx, flag, redo, given, s);
     }
 }
 template cudaError_t launch_knn_select<float>(const float *, int, const float *, int, int, int,
                                               const float *, const float *, const KnnArgs &,
                                               const KnnSelPlan &, void *, int, float *, int *,
-                                              int *, int *, cudaStream_t);
+                                              int *, int *, const float *, cudaStream_t);
 template cudaError_t launch_knn_select<double>(const double *, int, const double *, int, int, int,
                                                const double *, const double *, const KnnArgs &,
                                                const KnnSelPlan &, void *, int, double *, int *,
-                                               int *, int *, cudaStream_t);
+                                               int *, int *, const double *, cudaStream_t);
 
 } // namespace b200

@@ -13,7 +13,8 @@
 // Two passes of the same kernel.  The first, over an evenly strided sample of
 // the rows, keeps minima of v'_tc over disjoint sets of rows; the k-th smallest
 // of a query's minima is at least v'_tc(k), so theta_q = that + 2 eps_q admits
-// every candidate.  The second appends every (v'_tc, j) with v'_tc < theta_q to
+// every candidate (so does the k-th of any values listed, which a query whose list
+// overflowed takes for another go).  The second appends every (v'_tc, j) with v'_tc < theta_q to
 // the query's list.  The finalize kernel takes the k-th smallest listed v'_tc
 // (that is v'_tc(k)), re-scores the listed rows within 2 eps_q of it exactly
 // (the plain kernel's formula and order) and keeps the k best by (distance,
@@ -264,12 +265,14 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmQh, const __grid_constant__ 
         float theta = -inf, low[4] = {inf, inf, inf, inf};
         if (PASS != TK_SAMPLE && q < a.nq) theta = nudge_up(a.bound[q] + a.margin[q]);
         int ns = 0, found = 0;
-        // the stashed values to the query's list
+        // the stashed values to the query's list; a full one takes no more (its
+        // query gets a closer bound from what it holds)
         auto flush = [&]() {
             if (ns > 0) {
                 const int at = atomicAdd(&a.cnt[q], ns);
                 for (int i = 0; i < ns; ++i)
                     if (at + i < a.cap) a.list[(size_t)q * a.cap + at + i] = stash[i * 256];
+                if (at + ns > a.cap) theta = -inf;
                 ns = 0;
             }
         };
@@ -513,11 +516,12 @@ __device__ unsigned block_kth(const unsigned *keys, int n, int k, int *hist, int
 // One block per query: v'_tc(k) among the listed values, the exact distances of
 // the rows within 2 eps_q of it, sorted by (distance, index); the first k are
 // written (sqrt for euclidean).  A query whose list overflowed or is short of k
-// is flagged for the plain path, counted at state[0] and by reason at state[2]
-// (overflow) and state[4] (short).
+// is flagged, counted at state[0] and by reason at state[2] (overflow) and
+// state[4] (short).  The k-th of an overflowed list's values, where it is below
+// the query's bound, is its next one: flag 2, the value at its first output.
 __global__ void __launch_bounds__(256)
 knn_tc_finalize(const float *X, const float *Q, int ld, int d, int kc, int k, int cap,
-                const float *margin, const int *cnt, const int2 *list, int take_sqrt,
+                const float *margin, const float *bound, const int *cnt, const int2 *list, int take_sqrt,
                 float *out_key, int *out_idx, int *fallback, int *state, const float *xnp,
                 const float *qnp) {
     __shared__ int scount;
@@ -530,15 +534,14 @@ knn_tc_finalize(const float *X, const float *Q, int ld, int d, int kc, int k, in
     int *sidx = srow + cap;                                  // cap: survivors
     float *skey = reinterpret_cast<float *>(sval);
     const int qi = blockIdx.x;
-    const int n = cnt[qi];
-    if (n > cap || n < k) {
-        if (threadIdx.x == 0) {
-            fallback[qi] = 1;
-            atomicAdd(state, 1);
-            atomicAdd(state + (n > cap ? 2 : 4), 1);
-        }
-        return;
+    const bool over = cnt[qi] > cap;
+    const int n = min(cnt[qi], cap);
+    if (threadIdx.x == 0 && (over || n < k)) {
+        fallback[qi] = 1;
+        atomicAdd(state, 1);
+        atomicAdd(state + (over ? 2 : 4), 1);
     }
+    if (n < k) return;
     if (threadIdx.x == 0) scount = 0;
     for (int f = threadIdx.x; f < d; f += blockDim.x) qs[f] = Q[(size_t)qi * ld + f];
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
@@ -548,6 +551,13 @@ knn_tc_finalize(const float *X, const float *Q, int ld, int d, int kc, int k, in
     }
     __syncthreads();
     const float kth = ord_float(block_kth(sval, n, k, hist, sel));
+    if (over) {
+        if (threadIdx.x == 0 && kth < bound[qi]) {
+            fallback[qi] = 2;
+            out_key[(size_t)qi * k] = kth;
+        }
+        return;
+    }
     const unsigned th = ord_bits(nudge_up(kth + margin[qi]));
     for (int e = threadIdx.x; e < n; e += blockDim.x)
         if (sval[e] < th) sidx[atomicAdd(&scount, 1)] = srow[e];
@@ -637,6 +647,21 @@ int knn_tc_supported(int nx, int d, int k) {
     return tk_smem_bytes(nkb, 2) <= TK_SMEM ? 1 : 0;
 }
 
+// Every step-th row: a prime, so that rows in a cyclic order (a customer in turn, an
+// hour of the day) are met in all their phases unless the period is a multiple of
+// it; 11 instead of the shares that give 7 to 10, days of the week being common.
+static int sample_step(int want, int most) {
+    int s = std::max(1, std::min(want, most));
+    if (s >= 7 && s < 11 && most >= 11) return 11;
+    auto prime = [](int v) {
+        for (int q = 2; q * q <= v; ++q)
+            if (v % q == 0) return false;
+        return true;
+    };
+    while (s > 2 && !prime(s)) --s;
+    return s;
+}
+
 // Sample, lists.  A query is expected to list about 1.2 k times the inverse of
 // the sampled share: an eighth of the rows at most (the sample pass costs its
 // share of the tensor work), a 20th at least, else the share that lists about
@@ -648,7 +673,7 @@ KnnTcPlan knn_tc_plan(int nx, int nq, int k) {
     constexpr int slots = 8, rows = TK_ROWS; // minima of a work item
     const double share = std::min(1.0 / 8.0, std::max(1.0 / 20.0, 1.2 * k / 512.0));
     const int least_rows = (2 * k + slots - 1) / slots * rows;
-    p.step = std::max(1, std::min((int)(1.0 / share), nx / least_rows));
+    p.step = sample_step((int)(1.0 / share), nx / least_rows);
     p.n_sample = (nx + p.step - 1) / p.step;
     const int n_qtiles = (nq + TK_BM - 1) / TK_BM;
     const int tiles = (p.n_sample + rows - 1) / rows;
@@ -701,7 +726,8 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
                           const float *xmax, int nx, int ld, int ldbf, int d, const float *Q,
                           int nq, int k, int kc, int take_sqrt, const KnnTcPlan &pl, void *qbuf,
                           void *list, int *fallback, int *cnt, int *state, float *out_key,
-                          int *out_idx, cudaStream_t s, const KnnTcCosine *cosine) {
+                          int *out_idx, cudaStream_t s, const KnnTcCosine *cosine,
+                          const float *given) {
     // ldbf: the bf16 rows' length (d rounded up to 8, at least 64); the MMA
     // runs nkb K blocks of 64, the last with only the 16-column steps that
     // hold data (the tensor maps zero-fill the columns past ldbf)
@@ -750,7 +776,12 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
     if (!make_map_bf16_rows(&mqh, Qh, nq_pad, ldbf, TK_BM) ||
         !make_map_bf16_rows(&mql, Ql, nq_pad, ldbf, TK_BM))
         return cudaErrorInvalidValue;
-    for (int pass = 0; pass < 2; ++pass) {
+    if (given) {
+        const cudaError_t e = cudaMemcpy2DAsync(bound, sizeof(float), given, k * sizeof(float),
+                                                sizeof(float), nq, cudaMemcpyDeviceToDevice, s);
+        if (e != cudaSuccess) return e;
+    }
+    for (int pass = given ? 1 : 0; pass < 2; ++pass) {
         const bool sample = pass == 0;
         a.xstep = sample ? pl.step : 1;
         a.nx = sample ? pl.n_sample : nx;
@@ -779,7 +810,7 @@ cudaError_t launch_knn_tc(const float *X, const void *Xh, const void *Xl, const 
     const size_t fsm = (size_t)((d + 3) & ~3) * sizeof(float) + (size_t)pl.cap * 12;
     cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(knn_tc_finalize), fsm);
     if (e != cudaSuccess) return e;
-    knn_tc_finalize<<<nq, 256, fsm, s>>>(X, Q, ld, d, kc, k, pl.cap, margin, cnt,
+    knn_tc_finalize<<<nq, 256, fsm, s>>>(X, Q, ld, d, kc, k, pl.cap, margin, bound, cnt,
                                          static_cast<const int2 *>(list), cosm ? 0 : take_sqrt,
                                          out_key, out_idx, fallback, state,
                                          cosm ? cosine->xnorm : nullptr,

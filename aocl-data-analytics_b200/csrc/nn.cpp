@@ -384,6 +384,15 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, s
     return da_status_success;
 }
 
+template <typename T> da_status NN<T>::tc_check(const int *state) {
+    if (state[1] == 0) return da_status_success;
+    return err->error(da_status_internal_error,
+                      "The tensor-core kNN kernel timed out waiting on a pipeline barrier (code " +
+                          std::to_string(state[1]) + ").");
+}
+
+static constexpr int KNN_ROUNDS = 3; // list passes with closer bounds, at most
+
 // The state words and list lengths of a tensor-core search (`extra`, as
 // kneighbors_tc laid them out): statistics, errors, and the flagged queries
 // searched again into dOutK (`redone`).
@@ -398,10 +407,8 @@ da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, const KnnWay &w, const
         int flagged = 0;
         for (int b = 0; b < batches; ++b) {
             const int *h = extra + (size_t)b * KNN_TC_STATE;
-            if (h[1] != 0)
-                return err->error(da_status_internal_error,
-                                  "The tensor-core kNN kernel timed out waiting on a pipeline "
-                                  "barrier (code " + std::to_string(h[1]) + ").");
+            const da_status s = tc_check(h);
+            if (s != da_status_success) return s;
             flagged += h[0];
             cuda->stats["knn_tc_fallback_list_overflow"] += (double)h[2];
             cuda->stats["knn_tc_fallback_few_survivors"] += (double)h[4];
@@ -413,30 +420,40 @@ da_status NN<T>::tc_finish(da_int nq, da_int d, da_int k, const KnnWay &w, const
         cuda->stats["knn_tc_max_list"] = std::max(cuda->stats["knn_tc_max_list"], mx);
         cuda->stats["knn_tc_mean_list"] = sum / std::max<double>(1.0, (double)nq);
         if (flagged == 0) return da_status_success;
-        // the queries the pass could not certify: the plain path on just those
+        // the queries the pass could not certify: again with closer bounds while
+        // that helps, the plain path on the rest
         redone = true;
-        std::vector<int> idx, over;
-        da_status s = flagged_queries(dTkFlag.as<int>(), (size_t)nq, idx);
+        Redo r;
+        da_status s = flagged_queries(dTkFlag.as<int>(), (size_t)nq, nullptr, r);
+        cuda->stats["knn_tc_again_queries"] = (double)r.again.size();
+        for (int round = 0; s == da_status_success && round < KNN_ROUNDS && !r.again.empty();
+             ++round) {
+            std::vector<int> idx;
+            idx.swap(r.again);
+            s = knn_tc_some(nq, d, k, w, idx, r);
+        }
         if (s != da_status_success) return s;
-        cuda->stats["knn_tc_fallback_queries"] = (double)idx.size();
-        s = knn_select_some(nq, d, k, w, idx, over);
-        return s == da_status_success ? knn_lists(nq, d, k, w, &over) : s;
+        std::vector<int> fresh;
+        fresh.swap(r.over);
+        fresh.insert(fresh.end(), r.again.begin(), r.again.end());
+        r.again.clear();
+        cuda->stats["knn_tc_fallback_queries"] = (double)fresh.size();
+        return knn_redo(nq, d, k, w, fresh, r);
     } else {
         (void)nq, (void)d, (void)k, (void)w, (void)extra;
     }
     return da_status_success;
 }
 
-// The numbers of the queries whose word is set (synchronises).
+// The queries whose word is set, by their numbers (null: their places).
 template <typename T>
-da_status NN<T>::flagged_queries(const int *words, size_t nq, std::vector<int> &idx) {
+da_status NN<T>::flagged_queries(const int *words, size_t nq, const int *number, Redo &r) {
     std::vector<int> h(nq);
     B200_TRY(cudaMemcpyAsync(h.data(), words, nq * sizeof(int), cudaMemcpyDeviceToHost,
                              cuda->stream), "copy");
     B200_TRY(cudaStreamSynchronize(cuda->stream), "copy");
-    idx.clear();
     for (size_t i = 0; i < nq; ++i)
-        if (h[i]) idx.push_back((int)i);
+        if (h[i]) (h[i] == 2 ? r.again : r.over).push_back(number ? number[i] : (int)i);
     return da_status_success;
 }
 
@@ -446,7 +463,7 @@ template <typename T>
 da_status NN<T>::gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g) {
     cudaStream_t st = cuda->stream;
     const size_t mk = m * k;
-    if (!dStage.ensure((m * ld + m + mk) * sizeof(T) + (mk + 2 * m + 1) * sizeof(int)))
+    if (!dStage.ensure((m * ld + m + mk) * sizeof(T) + (mk + 3 * m + KNN_TC_STATE) * sizeof(int)))
         return err->error(da_status_memory_error, "Device memory allocation failed.");
     g.Q = dStage.as<T>();
     g.qn = g.Q + m * ld;
@@ -454,7 +471,7 @@ da_status NN<T>::gather_queries(const int *idx, size_t m, da_int k, const KnnWay
     g.ind = reinterpret_cast<int *>(g.key + mk);
     g.number = g.ind + mk;
     g.redo = g.number + m;
-    g.flag = g.redo + m;
+    g.state = g.redo + m;
     B200_TRY(cudaMemcpyAsync(g.number, idx, m * sizeof(int), cudaMemcpyHostToDevice, st), "copy");
     B200_TRY(launch_rows_gather(dQ.p, ld * sizeof(T), g.number, (int)m, g.Q, st), "gather");
     if (w.qn) B200_TRY(launch_rows_gather(w.qn, sizeof(T), g.number, (int)m, g.qn, st), "gather");
@@ -476,17 +493,16 @@ template <typename T> size_t NN<T>::sel_batch(const KnnSelPlan &pl) const {
     return std::max<size_t>(64, ((size_t)1 << 28) / per / 64 * 64);
 }
 
-// Some queries by the selection passes, into dOutK; the numbers of those whose
-// list overflowed in `over` (all where the passes do not apply).
+// Some queries by the selection passes, into dOutK, from their own bounds or
+// (given) from those at their first output keys.
 template <typename T>
 da_status NN<T>::knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
-                                 const std::vector<int> &idx, std::vector<int> &over) {
+                                 const std::vector<int> &idx, bool given, Redo &r) {
     cudaStream_t st = cuda->stream;
     const bool fp64 = sizeof(T) == 8;
-    over.clear();
     KnnSelPlan pl{};
     if (!knn_sel_plan((int)n_samples, (int)std::min<size_t>(idx.size(), 65536), (int)k, fp64, pl)) {
-        over = idx;
+        r.over.insert(r.over.end(), idx.begin(), idx.end());
         return da_status_success;
     }
     const KnnArgs a{w.acc, w.post, w.kc, (double)p, (int)k, 0, 0};
@@ -498,18 +514,73 @@ da_status NN<T>::knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
         if (s != da_status_success) return s;
         if (!dPartK.ensure(knn_sel_bytes(pl, (int)m, fp64)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
+        if (given)
+            B200_TRY(launch_rows_gather(dOutK.p, k * sizeof(T), g.number, (int)m, g.key, st), "gather");
         B200_TRY(cuda->timed("knn_select", [&] {
             return launch_knn_select<T>(g.Q, (int)m, dX.as<T>(), (int)n_samples, ld, (int)d, g.qn,
-                                        w.xn, a, pl, dPartK.p, w.tf, g.key, g.ind, g.flag, g.redo, st);
+                                        w.xn, a, pl, dPartK.p, w.tf, g.key, g.ind, g.state, g.redo,
+                                        given ? g.key : nullptr, st);
         }), "kNN selection kernels");
         s = scatter_results(nq, k, m, g);
+        if (s == da_status_success) s = flagged_queries(g.redo, m, idx.data() + i0, r);
         if (s != da_status_success) return s;
-        std::vector<int> f;
-        s = flagged_queries(g.redo, m, f);
-        if (s != da_status_success) return s;
-        for (int i : f) over.push_back(idx[i0 + i]);
     }
     return da_status_success;
+}
+
+// Some queries by the tensor-core list pass, into dOutK, from the bounds at their
+// first output keys.
+template <typename T>
+da_status NN<T>::knn_tc_some(da_int nq, da_int d, da_int k, const KnnWay &w,
+                             const std::vector<int> &idx, Redo &r) {
+    if constexpr (std::is_same_v<T, float>) {
+        cudaStream_t st = cuda->stream;
+        const bool cosine = w.post == POST_COSINE;
+        for (size_t i0 = 0; i0 < idx.size(); i0 += KNN_TC_BATCH) {
+            const size_t m = std::min<size_t>(KNN_TC_BATCH, idx.size() - i0);
+            const KnnTcPlan pl = knn_tc_plan((int)n_samples, (int)m, (int)k);
+            Gathered g;
+            da_status s = gather_queries(idx.data() + i0, m, k, w, g);
+            if (s != da_status_success) return s;
+            if (!dTkQ.ensure(knn_tc_query_bytes((int)m, tc_ldbf, pl)) ||
+                !dTkList.ensure(m * pl.cap * 8))
+                return err->error(da_status_memory_error, "Device memory allocation failed.");
+            B200_TRY(launch_rows_gather(dOutK.p, k * sizeof(T), g.number, (int)m, g.key, st), "gather");
+            const KnnTcCosine cs{dXn.as<float>(), dXinv.as<float>(), g.qn};
+            B200_TRY(cuda->timed("knn_tc", [&] {
+                return launch_knn_tc(dX.as<float>(), dXh.p, dXl.p, dXsq.as<float>(),
+                                     dTkScal.as<float>(), (int)n_samples, ld, tc_ldbf, (int)d, g.Q,
+                                     (int)m, (int)k, w.kc, w.tf, pl, dTkQ.p, dTkList.p, g.redo,
+                                     g.state + KNN_TC_STATE, g.state, g.key, g.ind, st,
+                                     cosine ? &cs : nullptr, g.key);
+            }), "kNN tensor-core pass");
+            int state[KNN_TC_STATE];
+            B200_TRY(cudaMemcpyAsync(state, g.state, sizeof(state), cudaMemcpyDeviceToHost, st), "copy");
+            s = scatter_results(nq, k, m, g);
+            if (s == da_status_success) s = flagged_queries(g.redo, m, idx.data() + i0, r);
+            if (s == da_status_success) s = tc_check(state);
+            if (s != da_status_success) return s;
+        }
+    } else {
+        (void)nq, (void)d, (void)k, (void)w, (void)idx, (void)r;
+    }
+    return da_status_success;
+}
+
+// What a first pass left: `fresh` by the selection passes, again with closer
+// bounds while that helps, the rest by running lists.
+template <typename T>
+da_status NN<T>::knn_redo(da_int nq, da_int d, da_int k, const KnnWay &w, std::vector<int> &fresh,
+                          Redo &r) {
+    da_status s = da_status_success;
+    if (!fresh.empty()) s = knn_select_some(nq, d, k, w, fresh, false, r);
+    for (int round = 0; s == da_status_success && round < KNN_ROUNDS && !r.again.empty(); ++round) {
+        std::vector<int> idx;
+        idx.swap(r.again);
+        s = knn_select_some(nq, d, k, w, idx, true, r);
+    }
+    r.over.insert(r.over.end(), r.again.begin(), r.again.end());
+    return s == da_status_success ? knn_lists(nq, d, k, w, &r.over) : s;
 }
 
 // Running lists and their merge into dOutK, for all queries or those of `only`.
@@ -540,7 +611,8 @@ da_status NN<T>::knn_lists(da_int nq, da_int d, da_int k, const KnnWay &w,
     const size_t parts = m * k * n_chunks;
     if (!dPartK.ensure(parts * sizeof(T)) || !dPartI.ensure(parts * sizeof(int)))
         return err->error(da_status_memory_error, "Device memory allocation failed.");
-    Gathered g{dQ.as<T>(), const_cast<T *>(w.qn), dOutK.as<T>(), out_idx((size_t)nq * k), nullptr, nullptr, nullptr};
+    Gathered g{dQ.as<T>(), const_cast<T *>(w.qn), dOutK.as<T>(), out_idx((size_t)nq * k), nullptr,
+               nullptr, nullptr};
     if (only) {
         const da_status s = gather_queries(only->data(), m, k, w, g);
         if (s != da_status_success) return s;
@@ -636,6 +708,8 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
     B200_TRY(upload_matrix<T>(ord, nq, d, Xt, ldt, dQ.as<T>(), ld, dStage, st), "upload of X_test");
     cuda->stats["tensor_core"] = 0.0;
     cuda->stats["knn_select_fallback"] = 0.0;
+    cuda->stats["knn_select_again"] = 0.0;
+    cuda->stats["knn_tc_again_queries"] = 0.0;
     cuda->stats["knn_tc_fallback_queries"] = 0.0;
     cuda->stats["knn_tc_fallback_list_overflow"] = 0.0;
     cuda->stats["knn_tc_fallback_few_survivors"] = 0.0;
@@ -662,8 +736,8 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
     }
     // the plain path: bounds first (launch_knn_select) in query batches of at
     // most 256 MB of lists, each with its own flag after the indices, then a flag
-    // per query; running lists (knn_lists) where that does not apply and for the
-    // queries whose flag comes back set (the others' results stay)
+    // per query; running lists (knn_lists) where that does not apply.  Queries whose
+    // flag comes back set are searched again (the others' results stay)
     KnnSelPlan sel{};
     da_int sel_qb = 0;
     if (!tc_done) {
@@ -705,7 +779,7 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
                         dQ.as<T>() + (size_t)q0 * ld, (int)nb, dX.as<T>(), (int)n_samples, ld, (int)d,
                         way.qn ? way.qn + q0 : nullptr, way.xn, a, sel, dPartK.p, tf,
                         dOutK.as<T>() + (size_t)q0 * k, out_idx((size_t)nq * k) + (size_t)q0 * k,
-                        flags, redo + q0, st);
+                        flags, redo + q0, nullptr, st);
                 }), "kNN selection kernels");
             }
         } else {
@@ -778,9 +852,12 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             if (!redone) break;
         } else {
             if (std::all_of(extra.begin(), extra.end(), [](int f) { return f == 0; })) break;
-            std::vector<int> over; // the queries whose list overflowed
-            s = flagged_queries(out_idx(nk) + nk + n_extra, (size_t)nq, over);
-            if (s == da_status_success) s = knn_lists(nq, d, k, way, &over);
+            Redo r; // the queries whose list overflowed
+            std::vector<int> fresh;
+            s = flagged_queries(out_idx(nk) + nk + n_extra, (size_t)nq, nullptr, r);
+            if (s != da_status_success) return s;
+            cuda->stats["knn_select_again"] = (double)r.again.size();
+            s = knn_redo(nq, d, k, way, fresh, r);
             if (s != da_status_success) return s;
         }
         n_extra = 0;

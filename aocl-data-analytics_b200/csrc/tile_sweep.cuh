@@ -212,18 +212,32 @@ B200_DEV void sweep_slab(const SweepStage<T> &st, int k0, int d, int kc, T p, Sw
     }
 }
 
-// Global loads of one slab of ROWS rows (`stride` elements apart, `width`
-// readable; zeros elsewhere) into registers.
+// The matrix row that a sweep's row number stands for: itself, or (SampleRows)
+// one of every `step` consecutive rows, at a place that varies, so that rows in a
+// cyclic order are met in all their phases.
+struct AllRows {
+    B200_DEV size_t operator()(int r) const { return (size_t)r; }
+};
+struct SampleRows {
+    int step, n;
+    B200_DEV size_t operator()(int r) const {
+        return (size_t)min(r * step + (int)__umulhi((unsigned)r * 0x9E3779B1u, (unsigned)step), n - 1);
+    }
+};
+
+// Global loads of one slab of ROWS rows (ld elements apart, all readable; zeros
+// elsewhere) into registers.
 template <typename T, int ROWS> struct SweepRegs {
     static constexpr int NV = ROWS * (SW_BK / 4) / 256;
     V4<T> v[NV];
-    B200_DEV void load(const T *M, size_t stride, int width, int row0, int nrows, int k0, int tid) {
+    template <typename R>
+    B200_DEV void load(const T *M, int ld, R rows, int row0, int nrows, int k0, int tid) {
 #pragma unroll
         for (int u = 0; u < NV; ++u) {
             const int e = tid + u * 256;
             const int gr = row0 + e / (SW_BK / 4), gk = k0 + (e % (SW_BK / 4)) * 4;
-            if (gr < nrows && gk < width) {
-                v[u] = ld4_global(M + (size_t)gr * stride + gk);
+            if (gr < nrows && gk < ld) {
+                v[u] = ld4_global(M + rows(gr) * ld + gk);
             } else {
                 v[u].v[0] = v[u].v[1] = v[u].v[2] = v[u].v[3] = T(0);
             }
@@ -252,10 +266,10 @@ B200_DEV void sweep_put(SweepStage<T> &st, const SweepRegs<T, SW_BM> &ra,
 // b_end) of B, tile by tile: epi(b0) runs with the accumulators of the tile at
 // b0 complete.  One pipeline over all (tile, slab) steps: the next step's
 // global loads are in flight while the current slab is consumed, across tile
-// borders too.  Rows are ld elements (padded to four, pad readable); B's rows
-// lie bstride apart.  No barrier separates the last epi from what follows.
-template <typename T, int ACC, typename F>
-B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T *B, size_t bstride,
+// borders too.  Rows are ld elements (padded to four, pad readable).  No barrier
+// separates the last epi from what follows.
+template <typename T, int ACC, typename R, typename F>
+B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T *B, R brows,
                           int b_begin, int b_end, int ld, int d, int kc, T p,
                           SweepAcc<T, ACC> &acc, int tid, F &&epi) {
     constexpr int BN = SweepStage<T>::BN;
@@ -264,8 +278,8 @@ B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T
     SweepRegs<T, SW_BM> ra;
     SweepRegs<T, BN> rb;
     if (b_begin >= b_end) return;
-    ra.load(A, ld, ld, a0, na, 0, tid);
-    rb.load(B, bstride, ld, b_begin, b_end, 0, tid);
+    ra.load(A, ld, AllRows{}, a0, na, 0, tid);
+    rb.load(B, ld, brows, b_begin, b_end, 0, tid);
     sweep_put(st[0], ra, rb, tid);
     __syncthreads();
     int cur = 0;
@@ -276,8 +290,8 @@ B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T
             const int nb0 = last ? b0 + BN : b0, ns = last ? 0 : s + 1;
             const bool more = nb0 < b_end;
             if (more) {
-                ra.load(A, ld, ld, a0, na, ns * SW_BK, tid);
-                rb.load(B, bstride, ld, nb0, b_end, ns * SW_BK, tid);
+                ra.load(A, ld, AllRows{}, a0, na, ns * SW_BK, tid);
+                rb.load(B, ld, brows, nb0, b_end, ns * SW_BK, tid);
             }
             sweep_slab<T, ACC>(st[cur], s * SW_BK, d, kc, p, acc, tm, tn);
             if (more) sweep_put(st[cur ^ 1], ra, rb, tid);
@@ -290,17 +304,17 @@ B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T
 
 // The post-operation over a whole micro-tile (the cases of post_value that the
 // accumulation can have: fewer copies of the code), rows in turn to out(i, v).
-// xv: A rows' norms, yn: B rows' norms, ystep apart.
-template <typename T, int ACC, typename F>
+// xv: A rows' norms, yn: B rows' norms.
+template <typename T, int ACC, typename R, typename F>
 B200_DEV void sweep_post(const SweepAcc<T, ACC> &acc, int post, const T (&xv)[4], const T *yn,
-                         size_t ystep, int b0, int nb, int tn, T invp, F &&out) {
+                         R brows, int b0, int nb, int tn, T invp, F &&out) {
     constexpr int TN = SweepAcc<T, ACC>::TN;
     T yv[TN];
     if (ACC == ACC_DOT && post != POST_NONE && post != POST_NEG) {
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
             const int gb = b0 + SweepCols<T>::of(j, tn);
-            yv[j] = (yn && gb < nb) ? yn[(size_t)gb * ystep] : T(0);
+            yv[j] = (yn && gb < nb) ? yn[brows(gb)] : T(0);
         }
     }
 #pragma unroll
