@@ -16,7 +16,9 @@
 #if defined(__SSE2__)
 #include <emmintrin.h>
 #endif
+#include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <unistd.h>
 #include <vector>
@@ -448,12 +450,35 @@ cudaError_t copy_up(const XferSeg &g, cudaStream_t s) {
 cudaError_t copy_down(const XferSeg &g, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
     if (xfer_down(&g, 1, s, e)) return e;
-    if (flat(g, false))
+    if (flat(g, false)) {
         e = cudaMemcpyAsync(g.host, g.dev, g.rows * g.row_bytes, cudaMemcpyDeviceToHost, s);
-    else
+        return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+    }
+    // Short rows that are dense on the device come down in runs and are dealt out
+    // here: the driver takes 0.2 us a row (1.5 MB of 256-byte rows: 1.0 ms against
+    // 0.30; of 2,048-byte rows 0.27 each way, of 4,096-byte ones 0.20 against 0.26).
+    const size_t per = std::max<size_t>(1, (4u << 20) / g.row_bytes);
+    const std::unique_ptr<char[]> tmp(
+        g.dev_pitch == g.row_bytes && g.row_bytes < 2048
+            ? new (std::nothrow) char[std::min(per, g.rows) * g.row_bytes]
+            : nullptr);
+    if (tmp) {
+        for (size_t r = 0; r < g.rows; r += per) {
+            const size_t n = std::min(per, g.rows - r);
+            e = cudaMemcpyAsync(tmp.get(), static_cast<char *>(g.dev) + r * g.row_bytes,
+                                n * g.row_bytes, cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) return e;
+            char *to = static_cast<char *>(g.host) + r * g.host_pitch;
+            for (size_t i = 0; i < n; ++i)
+                std::memcpy(to + i * g.host_pitch, tmp.get() + i * g.row_bytes, g.row_bytes);
+        }
+    } else {
         e = cudaMemcpy2DAsync(g.host, g.host_pitch, g.dev, g.dev_pitch, g.row_bytes, g.rows,
                               cudaMemcpyDeviceToHost, s);
-    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
+    return e;
 }
 
 } // namespace b200

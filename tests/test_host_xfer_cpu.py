@@ -52,3 +52,9 @@ def test_contexts(stub, mode):
 def test_capture_of_another_thread(stub):
     """Setting the ring up and giving it back leave another thread's capture alone."""
     run(stub, "capture")
+
+
+def test_results_into_wider_rows(stub):
+    """Dense results go into rows with a pitch of their own without the driver's
+    copy row by row."""
+    run(stub, "pitched_results")

@@ -25,6 +25,7 @@
 namespace {
 std::mutex g_mu;
 int g_ring_copies = 0; // copies issued by threads other than the caller's
+int g_row_copies = 0;  // two-dimensional copies: the driver's row by row
 int g_strays = 0;      // calls of theirs that name their own stream, not the caller's
 std::thread::id g_main;
 void note_thread(cudaStream_t s) {
@@ -171,6 +172,7 @@ cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind
 }
 cudaError_t cudaMemcpy2DAsync(void *to, size_t tp, const void *from, size_t fp, size_t w, size_t h,
                               cudaMemcpyKind, cudaStream_t) {
+    ++g_row_copies;
     for (size_t r = 0; r < h; ++r) std::memcpy((char *)to + r * tp, (const char *)from + r * fp, w);
     return cudaSuccess;
 }
@@ -261,6 +263,26 @@ int copies() {
         if (pass == 0) CHECK(warm());
     }
     CHECK(g_ring_copies > 0);
+    return 0;
+}
+
+// Results that are dense on the device come down in runs, whatever the caller's row
+// pitch, with the ring and without.
+int pitched_results() {
+    for (int pass = 0; pass < 2; ++pass) {
+        for (size_t rows : {1, 17, 2000, 30'001, 120'000})
+            for (size_t pitch : {256, 268}) {
+                std::vector<unsigned char> dev(rows * 256), to(rows * pitch, 0xAA);
+                for (size_t i = 0; i < dev.size(); ++i) dev[i] = (unsigned char)(i * 31 + i / 251);
+                CHECK(copy_down({to.data(), pitch, dev.data(), 256, 256, rows}, S) == cudaSuccess);
+                for (size_t r = 0; r < rows; ++r) {
+                    CHECK(std::memcmp(&to[r * pitch], &dev[r * 256], 256) == 0);
+                    for (size_t c = 256; c < pitch; ++c) CHECK(to[r * pitch + c] == 0xAA);
+                }
+            }
+        if (pass == 0) CHECK(warm());
+    }
+    CHECK(g_row_copies == 0);
     return 0;
 }
 
@@ -364,5 +386,6 @@ int main(int argc, char **argv) {
     if (!std::strcmp(m, "contexts")) return contexts();
     if (!std::strcmp(m, "reset_idle")) return reset_idle();
     if (!std::strcmp(m, "capture")) return capture();
+    if (!std::strcmp(m, "pitched_results")) return pitched_results();
     return 2;
 }
