@@ -159,7 +159,7 @@ template <typename T> struct NN : public AlgBase {
         std::vector<int> again, over;
     };
     da_status flagged_queries(const int *words, size_t nq, const int *number, Redo &r);
-    da_status gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g);
+    cudaError_t gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g);
     da_status scatter_results(da_int nq, da_int k, size_t m, const Gathered &g);
     size_t sel_batch(const KnnSelPlan &pl) const;
     da_status knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
@@ -181,6 +181,7 @@ template <typename T> struct NN : public AlgBase {
                         da_int *cnt_out, long long *start_out, std::vector<da_int> &idx_out,
                         std::vector<T> &val_out, bool &done);
     cudaError_t tc_train_copies(da_int d);
+    void drop_tc();
     da_status compute_proba_rnn(da_int nq, da_int d, const T *Xt, da_int ldt,
                                 std::vector<T> &proba);
     da_status predict_reg_rnn(da_int nq, da_int d, const T *Xt, da_int ldt, T *y);

@@ -21,8 +21,8 @@ cudaError_t upload_matrix(da_order order, da_int rows, da_int cols, const T *hos
         if (!direct && xfer_up(&seg, 1, s, e)) return e;
         if (ld != cols || ldo == cols || rows < 16) return copy_up(seg, s);
         // dense rows padded on the device: one copy of all of them and a kernel
-        // (a driver's copy row by row moves 0.8 GB/s)
-        if (!stage.ensure((size_t)rows * cols * z)) return cudaErrorMemoryAllocation;
+        // (a driver's copy row by row moves 0.8 GB/s, but needs no memory)
+        if (!stage.ensure((size_t)rows * cols * z)) return copy_up(seg, s);
         e = cudaMemcpyAsync(stage.p, host, (size_t)rows * cols * z, cudaMemcpyHostToDevice, s);
         return e == cudaSuccess ? launch_pad_rows<T>(stage.as<T>(), rows, cols, dst, ldo, s) : e;
     }

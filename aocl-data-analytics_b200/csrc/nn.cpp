@@ -313,8 +313,16 @@ template <typename T> cudaError_t NN<T>::tc_train_copies(da_int d) {
     }
 }
 
-// Tensor-core candidate pass + exact re-score (knn_tc.cu) into dOutK (indices after the distances),
-// in query batches that bound the candidate lists' memory; n_extra ints of
+// The tensor-core buffers given back: there is no room for all of them, and the
+// plain path needs none.
+template <typename T> void NN<T>::drop_tc() {
+    tc_train_ready = false;
+    for (DevBuf *b : {&dXh, &dXl, &dXsq, &dXinv, &dTkQ, &dTkList, &dTkFlag}) b->release();
+}
+
+// Tensor-core candidate pass + exact re-score (knn_tc.cu) into dOutK (indices
+// after the distances; `done` false where there is no room for its buffers), in
+// query batches that bound the candidate lists' memory; n_extra ints of
 // state follow the indices, for tc_finish.
 static constexpr da_int KNN_TC_BATCH = 16384;
 template <typename T>
@@ -328,8 +336,10 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, s
             // the plain path's norms of the training rows and queries, and the
             // reciprocals of the former
             if (!dQn.ensure((size_t)nq * sizeof(T)) || !dXn.ensure((size_t)n_samples * sizeof(T)) ||
-                !dXinv.ensure((size_t)n_samples * sizeof(float)))
-                return err->error(da_status_memory_error, "Device memory allocation failed.");
+                !dXinv.ensure((size_t)n_samples * sizeof(float))) {
+                drop_tc();
+                return da_status_success;
+            }
             B200_TRY(launch_row_norms_eps1<float>(dQ.as<float>(), ld, (int)nq, (int)d,
                                                   dQn.as<float>(), st), "norms");
             if (xn_kind != 1)
@@ -340,8 +350,10 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, s
                      "norms");
         }
         const cudaError_t te = tc_train_copies(d);
-        if (te == cudaErrorMemoryAllocation)
-            return err->error(da_status_memory_error, "Device memory allocation failed.");
+        if (te == cudaErrorMemoryAllocation) {
+            drop_tc();
+            return da_status_success;
+        }
         B200_TRY(te, "tensor-core training copies");
         const int ldbf = tc_ldbf;
         // batches of queries; their state words and list lengths follow the
@@ -352,8 +364,10 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, s
         n_extra = (size_t)batches * KNN_TC_STATE + (size_t)nq;
         if (!dTkQ.ensure(knn_tc_query_bytes((int)qb, ldbf, pl)) ||
             !dTkList.ensure((size_t)qb * pl.cap * 8) || !dTkFlag.ensure((size_t)nq * sizeof(int)) ||
-            !dOutK.ensure(out_bytes((size_t)nq * k, n_extra)))
-            return err->error(da_status_memory_error, "Device memory allocation failed.");
+            !dOutK.ensure(out_bytes((size_t)nq * k, n_extra))) {
+            drop_tc();
+            return da_status_success;
+        }
         int *state = out_idx((size_t)nq * k) + (size_t)nq * k;
         int *counts = state + (size_t)batches * KNN_TC_STATE;
         for (da_int q0 = 0; q0 < nq; q0 += KNN_TC_BATCH, state += KNN_TC_STATE) {
@@ -363,8 +377,10 @@ da_status NN<T>::kneighbors_tc(da_int nq, da_int d, da_int k, const KnnWay &w, s
             // a last batch that fits one M tile has its own sizes
             const KnnTcPlan pb = nb == qb ? pl : knn_tc_plan((int)n_samples, (int)nb, (int)k);
             if (!dTkQ.ensure(knn_tc_query_bytes((int)nb, ldbf, pb)) ||
-                !dTkList.ensure((size_t)nb * pb.cap * 8))
-                return err->error(da_status_memory_error, "Device memory allocation failed.");
+                !dTkList.ensure((size_t)nb * pb.cap * 8)) {
+                drop_tc();
+                return da_status_success;
+            }
             B200_TRY(cuda->timed("knn_tc", [&] {
                 return launch_knn_tc(dX.as<float>(), dXh.p, dXl.p, dXsq.as<float>(),
                                      dTkScal.as<float>(), (int)n_samples, ld, tc_ldbf, (int)d,
@@ -460,11 +476,11 @@ da_status NN<T>::flagged_queries(const int *words, size_t nq, const int *number,
 // Queries idx[0 .. m) brought together, with room for their results, in the
 // upload's stage (free by the time a search has run).
 template <typename T>
-da_status NN<T>::gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g) {
+cudaError_t NN<T>::gather_queries(const int *idx, size_t m, da_int k, const KnnWay &w, Gathered &g) {
     cudaStream_t st = cuda->stream;
     const size_t mk = m * k;
     if (!dStage.ensure((m * ld + m + mk) * sizeof(T) + (mk + 3 * m + KNN_TC_STATE) * sizeof(int)))
-        return err->error(da_status_memory_error, "Device memory allocation failed.");
+        return cudaErrorMemoryAllocation;
     g.Q = dStage.as<T>();
     g.qn = g.Q + m * ld;
     g.key = g.qn + m;
@@ -472,11 +488,13 @@ da_status NN<T>::gather_queries(const int *idx, size_t m, da_int k, const KnnWay
     g.number = g.ind + mk;
     g.redo = g.number + m;
     g.state = g.redo + m;
-    B200_TRY(cudaMemcpyAsync(g.number, idx, m * sizeof(int), cudaMemcpyHostToDevice, st), "copy");
-    B200_TRY(launch_rows_gather(dQ.p, ld * sizeof(T), g.number, (int)m, g.Q, st), "gather");
-    if (w.qn) B200_TRY(launch_rows_gather(w.qn, sizeof(T), g.number, (int)m, g.qn, st), "gather");
-    else g.qn = nullptr;
-    return da_status_success;
+    cudaError_t e =
+        cudaMemcpyAsync(g.number, idx, m * sizeof(int), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = launch_rows_gather(dQ.p, ld * sizeof(T), g.number, (int)m, g.Q, st);
+    if (!w.qn) g.qn = nullptr;
+    else if (e == cudaSuccess) e = launch_rows_gather(w.qn, sizeof(T), g.number, (int)m, g.qn, st);
+    return e;
 }
 template <typename T>
 da_status NN<T>::scatter_results(da_int nq, da_int k, size_t m, const Gathered &g) {
@@ -510,10 +528,14 @@ da_status NN<T>::knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
     for (size_t i0 = 0; i0 < idx.size(); i0 += qb) {
         const size_t m = std::min(qb, idx.size() - i0);
         Gathered g;
-        da_status s = gather_queries(idx.data() + i0, m, k, w, g);
-        if (s != da_status_success) return s;
-        if (!dPartK.ensure(knn_sel_bytes(pl, (int)m, fp64)))
-            return err->error(da_status_memory_error, "Device memory allocation failed.");
+        const bool room = dPartK.ensure(knn_sel_bytes(pl, (int)m, fp64));
+        const cudaError_t e = room ? gather_queries(idx.data() + i0, m, k, w, g)
+                                   : cudaErrorMemoryAllocation;
+        if (e == cudaErrorMemoryAllocation) {
+            r.over.insert(r.over.end(), idx.begin() + i0, idx.end());
+            return da_status_success;
+        }
+        B200_TRY(e, "gather");
         if (given)
             B200_TRY(launch_rows_gather(dOutK.p, k * sizeof(T), g.number, (int)m, g.key, st), "gather");
         B200_TRY(cuda->timed("knn_select", [&] {
@@ -521,7 +543,7 @@ da_status NN<T>::knn_select_some(da_int nq, da_int d, da_int k, const KnnWay &w,
                                         w.xn, a, pl, dPartK.p, w.tf, g.key, g.ind, g.state, g.redo,
                                         given ? g.key : nullptr, st);
         }), "kNN selection kernels");
-        s = scatter_results(nq, k, m, g);
+        da_status s = scatter_results(nq, k, m, g);
         if (s == da_status_success) s = flagged_queries(g.redo, m, idx.data() + i0, r);
         if (s != da_status_success) return s;
     }
@@ -540,11 +562,15 @@ da_status NN<T>::knn_tc_some(da_int nq, da_int d, da_int k, const KnnWay &w,
             const size_t m = std::min<size_t>(KNN_TC_BATCH, idx.size() - i0);
             const KnnTcPlan pl = knn_tc_plan((int)n_samples, (int)m, (int)k);
             Gathered g;
-            da_status s = gather_queries(idx.data() + i0, m, k, w, g);
-            if (s != da_status_success) return s;
-            if (!dTkQ.ensure(knn_tc_query_bytes((int)m, tc_ldbf, pl)) ||
-                !dTkList.ensure(m * pl.cap * 8))
-                return err->error(da_status_memory_error, "Device memory allocation failed.");
+            const bool room = dTkQ.ensure(knn_tc_query_bytes((int)m, tc_ldbf, pl)) &&
+                              dTkList.ensure(m * pl.cap * 8);
+            const cudaError_t e = room ? gather_queries(idx.data() + i0, m, k, w, g)
+                                       : cudaErrorMemoryAllocation;
+            if (e == cudaErrorMemoryAllocation) {
+                r.over.insert(r.over.end(), idx.begin() + i0, idx.end());
+                return da_status_success;
+            }
+            B200_TRY(e, "gather");
             B200_TRY(launch_rows_gather(dOutK.p, k * sizeof(T), g.number, (int)m, g.key, st), "gather");
             const KnnTcCosine cs{dXn.as<float>(), dXinv.as<float>(), g.qn};
             B200_TRY(cuda->timed("knn_tc", [&] {
@@ -556,7 +582,7 @@ da_status NN<T>::knn_tc_some(da_int nq, da_int d, da_int k, const KnnWay &w,
             }), "kNN tensor-core pass");
             int state[KNN_TC_STATE];
             B200_TRY(cudaMemcpyAsync(state, g.state, sizeof(state), cudaMemcpyDeviceToHost, st), "copy");
-            s = scatter_results(nq, k, m, g);
+            da_status s = scatter_results(nq, k, m, g);
             if (s == da_status_success) s = flagged_queries(g.redo, m, idx.data() + i0, r);
             if (s == da_status_success) s = tc_check(state);
             if (s != da_status_success) return s;
@@ -583,7 +609,8 @@ da_status NN<T>::knn_redo(da_int nq, da_int d, da_int k, const KnnWay &w, std::v
     return s == da_status_success ? knn_lists(nq, d, k, w, &r.over) : s;
 }
 
-// Running lists and their merge into dOutK, for all queries or those of `only`.
+// Running lists and their merge into dOutK, for all queries or those of `only`
+// (all, where there is no room to bring these together).
 template <typename T>
 da_status NN<T>::knn_lists(da_int nq, da_int d, da_int k, const KnnWay &w,
                            const std::vector<int> *only) {
@@ -592,7 +619,14 @@ da_status NN<T>::knn_lists(da_int nq, da_int d, da_int k, const KnnWay &w,
     const size_t m = only ? only->size() : (size_t)nq;
     if (m == 0) return da_status_success;
     cuda->stats["knn_select_fallback"] = (double)m;
+    Gathered g{dQ.as<T>(), const_cast<T *>(w.qn), dOutK.as<T>(), out_idx((size_t)nq * k), nullptr,
+               nullptr, nullptr};
     if (m == (size_t)nq) only = nullptr;
+    if (only) {
+        const cudaError_t e = gather_queries(only->data(), m, k, w, g);
+        if (e == cudaErrorMemoryAllocation) return knn_lists(nq, d, k, w, nullptr);
+        B200_TRY(e, "gather");
+    }
     // chunking of the training rows: enough CTAs to fill 148 SMs several times
     const int BN = knn_tile_rows_train(fp64);
     const int q_tiles = (int)((m + 63) / 64);
@@ -611,12 +645,6 @@ da_status NN<T>::knn_lists(da_int nq, da_int d, da_int k, const KnnWay &w,
     const size_t parts = m * k * n_chunks;
     if (!dPartK.ensure(parts * sizeof(T)) || !dPartI.ensure(parts * sizeof(int)))
         return err->error(da_status_memory_error, "Device memory allocation failed.");
-    Gathered g{dQ.as<T>(), const_cast<T *>(w.qn), dOutK.as<T>(), out_idx((size_t)nq * k), nullptr,
-               nullptr, nullptr};
-    if (only) {
-        const da_status s = gather_queries(only->data(), m, k, w, g);
-        if (s != da_status_success) return s;
-    }
     B200_TRY(cuda->timed("knn_chunks", [&] {
         return launch_knn_chunks<T>(g.Q, ld, (int)m, dX.as<T>(), ld, (int)n_samples, (int)d, g.qn,
                                     w.xn, a, dPartK.as<T>(), dPartI.as<int>(), nullptr, st);
@@ -729,6 +757,7 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
         (double)n_samples * (double)std::max<da_int>(nq, 64) * (double)d >= 5.0e8) {
         s = kneighbors_tc(nq, d, k, way, n_extra, tc_done);
         if (s != da_status_success) return s;
+        if (!tc_done) n_extra = 0;
         if (tc_done && metric == M_COS) {
             way.qn = dQn.as<T>();
             way.xn = dXn.as<T>();
@@ -765,12 +794,12 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             return err->error(da_status_not_implemented,
                               "k = " + std::to_string(k) + " exceeds the largest supported number "
                               "of neighbours per query (" + std::to_string(knn_max_k(fp64)) + ").");
+        // (no room for its lists: the running lists, which take less)
+        if (n_extra > 0 && !dPartK.ensure(knn_sel_bytes(sel, (int)sel_qb, fp64))) n_extra = 0;
         if (!dOutK.ensure(out_bytes((size_t)nq * k, n_extra > 0 ? n_extra + nq : 0)))
             return err->error(da_status_memory_error, "Device memory allocation failed.");
         if (n_extra > 0) {
             const KnnArgs a{acc, post, kc, (double)p, (int)k, 0, 0};
-            if (!dPartK.ensure(knn_sel_bytes(sel, (int)sel_qb, fp64)))
-                return err->error(da_status_memory_error, "Device memory allocation failed.");
             int *flags = out_idx((size_t)nq * k) + (size_t)nq * k, *redo = flags + n_extra;
             for (da_int q0 = 0; q0 < nq; q0 += sel_qb, ++flags) {
                 const da_int nb = std::min(sel_qb, nq - q0);
@@ -793,8 +822,8 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
     // free by now)
     const size_t nk = (size_t)nq * k;
     const bool want = to ? to->dist != nullptr : dist != nullptr;
-    const bool small = out_bytes(nk, n_extra) <= 256 * 1024;
     const bool cm = to && ord == column_major && nq > 1 && k > 1;
+    bool small = out_bytes(nk, n_extra) <= 256 * 1024;
     std::vector<int> extra, tmp;
     if (!to) {
         ind.resize(nk);
@@ -806,6 +835,7 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
         const T *od = dOutK.as<T>();
         const int *oi = out_idx(nk);
         extra.resize(n_extra);
+        if (!small && cm) small = !dStage.ensure(nk * (sizeof(T) + sizeof(int))); // no room there
         if (small) {
             // in words of four bytes: the distances if wanted, indices, state
             const size_t dw = want ? nk * sizeof(T) / 4 : 0, words = dw + nk + n_extra;
@@ -823,8 +853,6 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
             std::copy(ti + nk, ti + nk + n_extra, extra.begin());
         } else {
             if (cm) {
-                if (!dStage.ensure(nk * (sizeof(T) + sizeof(int))))
-                    return err->error(da_status_memory_error, "Device memory allocation failed.");
                 T *td = dStage.as<T>();
                 float *ti = reinterpret_cast<float *>(td + nk); // four-byte words
                 B200_TRY(launch_rowmajor_to_colmajor<float>(reinterpret_cast<const float *>(oi),
@@ -878,7 +906,10 @@ da_status NN<T>::radius_tc(da_int nq, da_int d, const T *Q, T thr, int kc, bool 
     if constexpr (std::is_same_v<T, float>) {
         cudaStream_t st = cuda->stream;
         const cudaError_t te = tc_train_copies(d);
-        if (te == cudaErrorMemoryAllocation) return da_status_success;
+        if (te == cudaErrorMemoryAllocation) {
+            drop_tc();
+            return da_status_success;
+        }
         B200_TRY(te, "tensor-core training copies");
         const int n = (int)n_samples, words = radius_tc_words(n);
         // state words, their number of candidates; offsets; per query counts
@@ -889,8 +920,10 @@ da_status NN<T>::radius_tc(da_int nq, da_int d, const T *Q, T thr, int kc, bool 
         } head;
         const size_t off_at = 64, hit_at = off_at + (size_t)nq * 8, cnt_at = hit_at + (size_t)nq * 4;
         if (!dTkQ.ensure(radius_tc_query_bytes((int)nq, tc_ldbf)) ||
-            !dD.ensure((size_t)nq * words * 4) || !dRs.ensure(cnt_at + (size_t)nq * 4))
+            !dD.ensure((size_t)nq * words * 4) || !dRs.ensure(cnt_at + (size_t)nq * 4)) {
+            drop_tc();
             return da_status_success;
+        }
         char *w = dRs.as<char>();
         int *state = reinterpret_cast<int *>(w), *hits = reinterpret_cast<int *>(w + hit_at),
             *cnt = reinterpret_cast<int *>(w + cnt_at);
