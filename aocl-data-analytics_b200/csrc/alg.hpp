@@ -118,6 +118,14 @@ template <typename T> struct NN : public AlgBase {
     bool rnn_dist = false, rnn_squares = false;
     DevBuf dD, dRc, dRs, dRi, dRv, dRh;
     double radius_work = 0; // multiply-adds of the searches before the tensor-core copies
+    // the threshold of a search that the tensor-core path refused, how many searches
+    // of no smaller one pass it by, and the length of that wait
+    T radius_refused = std::numeric_limits<T>::infinity();
+    int radius_skip = 0, radius_wait = 0;
+    void radius_accepted() {
+        radius_refused = std::numeric_limits<T>::infinity();
+        radius_skip = radius_wait = 0;
+    }
     da_status radius_neighbors(da_int nq, da_int d, const T *Xt, da_int ldt, T radius,
                                da_int return_distance, da_int sort_results);
     da_status get_result(da_result q, da_int *dim, double *out) override;

@@ -284,6 +284,7 @@ template <typename T> da_status NN<T>::ensure_device_data() {
                               ld, dStage, cuda->stream),
              "upload of X_train");
     B200_TRY(cuda->leave_in_flight(), "upload of X_train");
+    radius_accepted();
     X_on_device = true;
     xn_kind = -1;
     tc_train_ready = false;
@@ -983,7 +984,6 @@ da_status NN<T>::radius_tc(da_int nq, da_int d, const T *Q, T thr, int kc, bool 
         }
         idx_out.resize(at);
         if (want_val) val_out.resize(at);
-        cuda->stats["tensor_core"] = 1.0;
         done = true;
     } else {
         (void)nq, (void)d, (void)Q, (void)thr, (void)kc, (void)want_val, (void)cnt_out;
@@ -1059,12 +1059,15 @@ da_status NN<T>::radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T 
     // against 180), once the copies of the training rows exist or the handle's
     // radius searches come to 4e9 multiply-adds: the copies and buffers cost
     // 0.6 ms to set up, what a search of that size saves (3.1 -> 0.9 ms at
-    // 1.3e10, 200,000 x 32, 2,000 queries).
+    // 1.3e10, 200,000 x 32, 2,000 queries).  A refused search has paid for the
+    // mask (a tenth of the plain path): those of no smaller radius after it skip
+    // this path 1, 2, 4 .. 16 times before it is tried again.
     da_int first = 0;
     const double work = (double)n * (double)std::max<da_int>(nq, 64) * (double)d;
     if (!fp64 && acc == ACC_SQEUC && std::isfinite((double)thr) && test_wait == 0 &&
         opts.key("precision mode") != 0 && knn_tc_supported((int)n, (int)d, 1) && n >= 16384 &&
-        work >= 5.0e8 && (tc_train_ready || (radius_work += work) >= 4.0e9)) {
+        work >= 5.0e8 && (tc_train_ready || (radius_work += work) >= 4.0e9) &&
+        !(thr >= radius_refused && --radius_skip >= 0)) {
         da_int Bt = (da_int)std::max<size_t>(
             1, std::min<size_t>({(size_t)nq, (256u << 20) / ((size_t)radius_tc_words((int)n) * 4),
                                  (size_t)65535}));
@@ -1077,7 +1080,13 @@ da_status NN<T>::radius_compute(da_int nq, da_int d, const T *Xt, da_int ldt, T 
             if (s != da_status_success) return s;
             if (done) first += b;
         }
-        if (first == nq) return da_status_success;
+        if (first == nq) {
+            cuda->stats["tensor_core"] = 1.0;
+            if (thr >= radius_refused) radius_accepted();
+            return da_status_success;
+        }
+        radius_refused = thr;
+        radius_skip = radius_wait = std::min(16, std::max(1, 2 * radius_wait));
     }
     // query blocks whose distance rows fit in 256 MB
     // (at most 65,535 rows: the count / compaction grids put the rows on y)
