@@ -308,3 +308,40 @@ def test_serving_two_fast_lanes_with_a_cap():
         assert mine and all(b[2] <= 6 and b[4] <= 4 for b in mine)
     finally:
         server.close()
+
+
+def test_serving_waiting_clients_are_not_held():
+    """Requests of clients that wait for each answer go to a worker at once, however
+    quickly they follow one another; those handed in without waiting are held for
+    company."""
+    sv = _load("aoclda_serving_cpu_hold", os.path.join(PKG, "serving.py"))
+    sv.BURST_GAP, sv.LINGER = 10.0, 0.2
+    rng = np.random.default_rng(5)
+    X = rng.standard_normal((50, 4)).astype(np.float32)
+    server = sv.Server(FakeAB(), X, models={"m": (X, X[:3].copy())}, workers=2)
+    try:
+        def client(kind, n, waits, out):
+            for _ in range(n):
+                r = server.submit(sv.Request(kind, X[:2], k=3 if kind == "knn" else None,
+                                             model="m" if kind == "predict" else None))
+                out.append(r)
+                if waits:
+                    assert r.wait(30)
+
+        for kind in ("knn", "predict"):
+            for clients in (1, 4):
+                reqs = []
+                ts = [threading.Thread(target=client, args=(kind, 10, True, reqs))
+                      for _ in range(clients)]
+                for t in ts:
+                    t.start()
+                for t in ts:
+                    t.join()
+                held = sorted(r.t_start - r.t_submit for r in reqs)
+                assert held[len(held) // 2] < sv.LINGER / 2, held
+            reqs = []
+            client(kind, 8, False, reqs)
+            assert all(r.wait(30) for r in reqs)
+            assert max(b[1] for b in server.batches if b[0] == kind) > 1
+    finally:
+        server.close()
