@@ -250,7 +250,8 @@ template <typename T> struct KMeans : public AlgBase {
     void *h_small = nullptr; // pinned: flags + scalars
     // the same loop with the update by counting sort (fp64, "plain" precision)
     bool build_sort_graph(T *dC, int *dL);
-    da_status lloyd_sort_graph(T *dC, int *dL, da_int &n_iter, int &converged, bool &ran);
+    da_status lloyd_sort_graph(T *dC, int *dL, da_int it, da_int &n_iter, int &converged, bool &ran);
+    int sort_steps = 0; // iterations that the host ran where the graph could
     // Lloyd iterations 1.. as one CUDA graph (a WHILE node whose body is one
     // iteration in place); rebuilt when a pointer or size it holds changes
     cudaGraph_t loop_graph = nullptr;
