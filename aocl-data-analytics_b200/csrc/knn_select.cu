@@ -372,7 +372,9 @@ bool knn_sel_plan(int n, int nq, int k, bool fp64, KnnSelPlan &pl) {
     if (pl.parts < need) return false;
     pl.groups = pl.parts * 32;
     const double expected = std::min((double)n, 1.5 * k * ((double)n / pl.n_sample) + 16.0);
-    const double room = std::min((double)n, expected * (1.0 + 6.0 / std::sqrt((double)k) + 15.0 / k));
+    const double room =
+        pl.step == 1 ? std::min((double)n, 4.0 * k + 64.0) // the minima are over all rows
+                     : std::min((double)n, expected * (1.0 + 6.0 / std::sqrt((double)k) + 15.0 / k));
     pl.cap = 128;
     while (pl.cap < room && pl.cap < KNN_SEL_CAP) pl.cap <<= 1;
     return pl.cap >= room;

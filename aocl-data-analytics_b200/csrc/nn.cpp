@@ -773,6 +773,11 @@ da_status NN<T>::kneighbors_compute(da_int nq, da_int d, const T *Xt, da_int ldt
     if (!tc_done) {
         if (knn_sel_plan((int)n_samples, (int)std::min<da_int>(nq, 65536), (int)k, fp64, sel)) {
             sel_qb = std::min(nq, (da_int)sel_batch(sel));
+            // a handle's first search: lists within 1 MB, in a few batches, come out
+            // of a block that the driver has, where more cost 0.35 ms to allocate
+            const size_t per = knn_sel_bytes(sel, 1, fp64);
+            const da_int few = (da_int)((1u << 20) / per / 64 * 64);
+            if (!dPartK.p && few > 0 && few < nq && (nq + few - 1) / few <= 4) sel_qb = few;
             n_extra = (size_t)((nq + sel_qb - 1) / sel_qb);
         }
         if (norm_kind >= 0) {
