@@ -518,7 +518,8 @@ __device__ unsigned block_kth(const unsigned *keys, int n, int k, int *hist, int
 // written (sqrt for euclidean).  A query whose list overflowed or is short of k
 // is flagged, counted at state[0] and by reason at state[2] (overflow) and
 // state[4] (short).  The k-th of an overflowed list's values, where it is below
-// the query's bound, is its next one: flag 2, the value at its first output.
+// the query's bound by more than half the margin (which another go keeps), is its
+// next one: flag 2, the value at its first output.
 __global__ void __launch_bounds__(256)
 knn_tc_finalize(const float *X, const float *Q, int ld, int d, int kc, int k, int cap,
                 const float *margin, const float *bound, const int *cnt, const int2 *list, int take_sqrt,
@@ -552,7 +553,7 @@ knn_tc_finalize(const float *X, const float *Q, int ld, int d, int kc, int k, in
     __syncthreads();
     const float kth = ord_float(block_kth(sval, n, k, hist, sel));
     if (over) {
-        if (threadIdx.x == 0 && kth < bound[qi]) {
+        if (threadIdx.x == 0 && kth < bound[qi] - 0.5f * margin[qi]) {
             fallback[qi] = 2;
             out_key[(size_t)qi * k] = kth;
         }
@@ -647,25 +648,37 @@ int knn_tc_supported(int nx, int d, int k) {
     return tk_smem_bytes(nkb, 2) <= TK_SMEM ? 1 : 0;
 }
 
+// List entries per query for a sample of every step-th row (see knn_tc_plan).
+static int list_cap(int nx, int k, int step) {
+    const double expected = 1.5 * 1.2 * k * step + 16.0;
+    const double room = std::min((double)nx, expected * (1.0 + 6.0 / std::sqrt((double)k) + 15.0 / k));
+    int cap = 512;
+    while (cap < room && cap < TK_CAP) cap <<= 1;
+    return cap;
+}
+
 // Every step-th row: a prime, so that rows in a cyclic order (a customer in turn, an
 // hour of the day) are met in all their phases unless the period is a multiple of
-// it; 11 instead of the shares that give 7 to 10, days of the week being common.
-static int sample_step(int want, int most) {
-    int s = std::max(1, std::min(want, most));
-    if (s >= 7 && s < 11 && most >= 11) return 11;
+// it; not 7, days of the week being common, where 11 does.  The next one up (a
+// smaller sample) if the lists stay as long, else the next one down.
+static int sample_step(int nx, int k, int want, int most) {
     auto prime = [](int v) {
         for (int q = 2; q * q <= v; ++q)
             if (v % q == 0) return false;
         return true;
     };
-    while (s > 2 && !prime(s)) --s;
-    return s;
+    const int s = std::max(1, std::min(want, most));
+    if (s == 1) return 1;
+    int up = s >= 7 ? std::max(s, 11) : s, down = s;
+    while (!prime(up)) ++up;
+    while (!prime(down)) --down;
+    return up <= most && list_cap(nx, k, up) == list_cap(nx, k, s) ? up : down;
 }
 
 // Sample, lists.  A query is expected to list about 1.2 k times the inverse of
 // the sampled share: an eighth of the rows at most (the sample pass costs its
-// share of the tensor work), a 20th at least, else the share that lists about
-// 512; more where a short set would give fewer than 2 k minima.  A list holds x
+// share of the tensor work), about a 20th at least, else the share that lists
+// about 512; more where a short set would give fewer than 2 k minima.  A list holds x
 // times that with k (x - 1 - ln x) above 18 (the number varies like a sum of k
 // exponentials), and half as much again for the margin.
 KnnTcPlan knn_tc_plan(int nx, int nq, int k) {
@@ -673,7 +686,7 @@ KnnTcPlan knn_tc_plan(int nx, int nq, int k) {
     constexpr int slots = 8, rows = TK_ROWS; // minima of a work item
     const double share = std::min(1.0 / 8.0, std::max(1.0 / 20.0, 1.2 * k / 512.0));
     const int least_rows = (2 * k + slots - 1) / slots * rows;
-    p.step = sample_step((int)(1.0 / share), nx / least_rows);
+    p.step = sample_step(nx, k, (int)(1.0 / share), nx / least_rows);
     p.n_sample = (nx + p.step - 1) / p.step;
     const int n_qtiles = (nq + TK_BM - 1) / TK_BM;
     const int tiles = (p.n_sample + rows - 1) / rows;
@@ -683,10 +696,7 @@ KnnTcPlan knn_tc_plan(int nx, int nq, int k) {
     const int items = std::max(least, std::min(most, (148 + n_qtiles - 1) / n_qtiles));
     p.sample_tiles = (tiles + items - 1) / items;
     p.groups = (tiles + p.sample_tiles - 1) / p.sample_tiles * slots;
-    const double expected = 1.5 * 1.2 * k * p.step + 16.0;
-    const double room = std::min((double)nx, expected * (1.0 + 6.0 / std::sqrt((double)k) + 15.0 / k));
-    p.cap = 512;
-    while (p.cap < room && p.cap < TK_CAP) p.cap <<= 1;
+    p.cap = list_cap(nx, k, p.step);
     p.tiles = tk_item_tiles((nx + TK_ROWS - 1) / TK_ROWS, n_qtiles);
     return p;
 }
