@@ -923,11 +923,11 @@ def run_radius(ab, nx=1_000_000, nq=10_000, d=32, comps=256, target=100, seed=6,
     Gaussian mixture, 10,000 queries from the mixture, the radius at which the
     median query has 100 neighbours.  Each timed call is one
     da_nn_radius_neighbors_s over all queries with host arrays (queries up;
-    counts, indices and distances down; results in index order).  Roofline of
-    the distance-block pipeline: every block of queries writes its distance
-    rows once (the distance kernel also counts the hits) and the compaction
-    reads them once (8 bytes per (query, row) pair) over the three kernels'
-    CUDA-event time.
+    counts, indices and distances down; results in index order).  Roofline: on
+    the tensor-core path the mask pass's bf16x3 products (3 x 2 flop per pair
+    and feature, features in steps of 16) over its CUDA-event time; on the
+    plain path the distance blocks, written once and read once (8 bytes per
+    pair), over the three kernels' time.
     CPU: the oracle on a sample of queries."""
     rng = np.random.default_rng(seed)
     means = rng.uniform(-3.0, 3.0, (comps, d)).astype(np.float32)
@@ -954,10 +954,21 @@ def run_radius(ab, nx=1_000_000, nq=10_000, d=32, comps=256, target=100, seed=6,
     for name in ("radius_distances", "radius_count", "radius_emit"):
         ms_, n_ = nn.kernel_time(name)
         kern[name] = (ms_, n_)
+    tc = nn.stat("tensor_core") == 1.0
     nn.close()
-    total_ms = sum(v[0] for v in kern.values()) / reps
-    bytes_ = 8.0 * nq * (nx)
-    hbm, _, src = load_peaks()
+    hbm, tflops, src = load_peaks()
+    if tc:
+        ms_ = kern["radius_distances"][0] / reps
+        done = 3 * 2.0 * nx * nq * ((d + 15) // 16 * 16) / (ms_ / 1e3) / 1e12
+        roofline = {"bound": "tensor", "achieved": done, "peak": tflops, "unit": "TFLOP/s",
+                    "frac": done / tflops, "peak_source": src, "traffic": None,
+                    "note": "bf16x3 products of the mask pass (K steps of 16)"}
+    else:
+        ms_ = sum(v[0] for v in kern.values()) / reps
+        done = 8.0 * nq * nx / (ms_ / 1e3) / 1e9
+        roofline = {"bound": "hbm", "achieved": done, "peak": hbm, "unit": "GB/s",
+                    "frac": done / hbm, "peak_source": src, "traffic": None,
+                    "note": "8 bytes per (query, row): distance written once, read once"}
     orc = _load("oracle_mod", os.path.join(ORACLE, "oracle.py"))
     t = time.perf_counter()
     ref = orc.radius(X, Q[:cpu_queries], r)
@@ -970,11 +981,7 @@ def run_radius(ab, nx=1_000_000, nq=10_000, d=32, comps=256, target=100, seed=6,
             "neighbours_mean": float(cnt[nq]) / nq,
             "kernel_ms_per_call": {k: v[0] / reps for k, v in kern.items()},
             "launches_per_call": {k: v[1] // reps for k, v in kern.items()},
-            "roofline": {"bound": "hbm", "achieved": bytes_ / (total_ms / 1e3) / 1e9,
-                         "peak": hbm, "unit": "GB/s",
-                         "frac": bytes_ / (total_ms / 1e3) / 1e9 / hbm, "peak_source": src,
-                         "traffic": None,
-                         "note": "8 bytes per (query, row): distance written once, read once"},
+            "tensor_core": tc, "roofline": roofline,
             "identical_to_oracle_sample": bool(same),
             "cpu_baseline": {"value": cpu_queries / cpu_s, "unit": "queries/s", "cores": 1,
                              "kind": "port", "sample": f"{cpu_queries} queries, oracle"},
@@ -989,10 +996,10 @@ def run_ivf(ab, nx=1_000_000, nq=10_000, d=128, k=10, n_list=1024, n_probe=16, c
     k-means, 10 iterations), n_probe = 16, 10,000 queries from the mixture,
     k = 10.  Each timed search is one da_approx_nn_kneighbors_s over all
     queries with host arrays; recall@k against the exact GPU kNN of the same
-    rows.  Roofline of the list scan: the candidate rows it reads (each
-    query's probed lists: 4 * 128 + 8 bytes a row) over its CUDA-event time
-    -- reads that the 126 MB L2 serves count as well, so the figure can pass
-    the HBM copy bandwidth.  CPU: the oracle's search (numpy) on a sample of
+    rows.  Roofline of the list scan: one read of every probed list (4 * 128 +
+    8 bytes a row), which is all that has to come from HBM, over its CUDA-event
+    time; the candidate rows as each query reads them, most of them from L2, are
+    a figure of their own.  CPU: the oracle's search (numpy) on a sample of
     queries, one thread of Python per query."""
     rng = np.random.default_rng(seed)
     means = rng.uniform(-10.0, 10.0, (comps, d)).astype(np.float32)
@@ -1025,7 +1032,8 @@ def run_ivf(ab, nx=1_000_000, nq=10_000, d=128, k=10, n_list=1024, n_probe=16, c
     dc = (Qd * Qd).sum(1)[:, None] + (C * C).sum(1)[None] - 2.0 * Qd @ C.T
     probes = np.argsort(dc, axis=1, kind="stable")[:, :n_probe]
     cand = int(sizes[probes].sum())
-    bytes_ = cand * (4.0 * d + 8.0)
+    row = 4.0 * d + 8.0
+    bytes_ = float(sizes[np.unique(probes)].sum()) * row
     hbm, _, src = load_peaks()
     h.close()
     exact = ab.KNN("s", order=ab.ROW_MAJOR, metric="sqeuclidean").fit(X)
@@ -1050,11 +1058,12 @@ def run_ivf(ab, nx=1_000_000, nq=10_000, d=128, k=10, n_list=1024, n_probe=16, c
             "unit": "queries/s", "qps": nq / min(ts), "train_s": train_s, "add_s": add_s,
             "recall_at_k_vs_exact": recall, "scan_kernel_ms": scan_ms,
             "candidates_per_query": cand / nq,
+            "candidate_gb_per_s_with_l2": cand * row / (scan_ms / 1e3) / 1e9,
             "roofline": {"bound": "hbm", "achieved": bytes_ / (scan_ms / 1e3) / 1e9,
                          "peak": hbm, "unit": "GB/s",
                          "frac": bytes_ / (scan_ms / 1e3) / 1e9 / hbm,
                          "peak_source": src, "traffic": None,
-                         "note": "candidate-row bytes per launch; L2 hits included"},
+                         "note": "one read of the probed lists"},
             "cpu_baseline": {"value": cpu_queries / cpu_s, "unit": "queries/s", "cores": 1,
                              "kind": "port",
                              "sample": f"{cpu_queries} queries, oracle numpy search "
