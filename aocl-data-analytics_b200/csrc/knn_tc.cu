@@ -724,10 +724,12 @@ cudaError_t launch_knn_tc_train_prep(const float *X, int ld, int nx, int d, void
     return cudaGetLastError();
 }
 
-// Device time on a B200 at 1M x 128, 4,096 queries, k = 100: 2.92 ms (list pass
-// 2.39 -- 2.05 of it the MMAs, 1.87 at the measured cuBLAS rate --, sample pass
-// 0.33, finalize 0.17), 7.32 ms before (see the top); at 1M x 96, one query, k =
-// 10: 112 us (list pass 79, 4.9 TB/s of the bf16 rows), 228 before.
+// Device time on a B200 at 1M x 128, 4,096 queries, k = 100: 2.83 ms (list pass
+// 2.45 under ncu -- 2.05 of it the MMAs, 1.87 at the measured cuBLAS rate --,
+// sample pass 0.25, finalize 0.18; 1,296 listed a query), 7.32 ms before (see the
+// top); with every 8th row sampled instead of every 11th 0.33 and 0.17, 925 listed,
+// the sum the same.  At 1M x 96, one query, k = 10: 109 us (list pass 79, 4.9 TB/s
+// of the bf16 rows), 228 before.
 // Variants that were slower at the first size (list pass): all warps storing
 // hits to global memory as they find them 4.6 ms, a warp handling one query's
 // hits together 2.8, hi and lo rows in separate 32 KB stages 3.1, sixteen

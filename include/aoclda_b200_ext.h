@@ -16,7 +16,8 @@ extern "C" {
 
 /* Bind the handle's work to a caller-owned CUDA stream (a cudaStream_t passed
  * as void*); NULL restores the handle's own non-blocking stream.  Calls still
- * return only after their results are complete. */
+ * return only after their results are complete.  Data set before are waited for
+ * on the device, whichever stream they were uploaded on (it may be gone). */
 da_status da_b200_set_stream(da_handle handle, void *stream);
 
 /* Recreate the handle's own stream with a CUDA stream priority: 0 is the
@@ -56,7 +57,11 @@ da_status da_b200_nn_share_data(da_handle handle, da_handle source);
 
 /* Named statistics of the last call: "relabelled_rows" (k-means rows of the
  * last tensor-core assignment whose label needed the exact fp32 re-score),
- * "tensor_core" (1 when the last k-means compute used the tensor cores). */
+ * "tensor_core" (1 when the last k-means compute, kNN search or all blocks of the
+ * last radius search used the tensor cores); kNN: "knn_tc_again_queries" and
+ * "knn_select_again" (queries whose list overflowed and that got a closer bound),
+ * "knn_tc_fallback_queries" (left to the plain path), "knn_select_fallback" (left
+ * to the running lists). */
 da_status da_b200_get_stat(da_handle handle, const char *name, double *value);
 
 /* k-means: run only the configured initialisation method ("initialization
