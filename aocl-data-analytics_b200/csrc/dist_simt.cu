@@ -80,7 +80,7 @@ pairwise_kernel(const T *X, int m, const T *Y, int n, int ld, int d, const T *xn
     SweepAcc<T, ACC> acc;
     sweep_tiles<T, ACC>(
         st, X, m, i0, Y, AllRows{}, y_begin, y_end, ld, d, kc, p, acc, tid, [&](int j0) {
-            sweep_post<T, ACC>(acc, post, xv, yn, AllRows{}, j0, n, tn, invp, [&](int i, T (&v)[TN]) {
+            sweep_post<T, ACC>(acc, post, xv, m - i0 - tm * 4, yn, AllRows{}, j0, n, tn, invp, [&](int i, T (&v)[TN]) {
                 const int gi = i0 + tm * 4 + i;
                 if (gi >= m) return;
 #pragma unroll

@@ -61,7 +61,7 @@ knn_min_kernel(const T *Q, int nq, const T *X, SampleRows rows, int n_sample, in
     SweepAcc<T, ACC> acc;
     sweep_tiles<T, ACC>(
         st, Q, nq, q0, X, rows, x_begin, x_end, ld, d, kc, p, acc, tid, [&](int x0) {
-            sweep_post<T, ACC>(acc, post, qv, xn, rows, x0, x_end, tn, invp,
+            sweep_post<T, ACC>(acc, post, qv, nq - q0 - tm * 4, xn, rows, x0, x_end, tn, invp,
                                [&](int i, T (&key)[TN]) {
 #pragma unroll
                                    for (int j = 0; j < TN; ++j) {
@@ -199,7 +199,8 @@ knn_append_kernel(const T *Q, int nq, const T *X, int nx, int ld, int d, const T
     sweep_tiles<T, ACC>(
         st, Q, nq, q0, X, AllRows{}, x_begin, x_end, ld, d, kc, p, acc, tid, [&](int x0) {
             sweep_post<T, ACC>(
-                acc, post, qv, xn, AllRows{}, x0, x_end, tn, invp, [&](int i, T (&key)[TN]) {
+                acc, post, qv, nq - q0 - tm * 4, xn, AllRows{}, x0, x_end, tn, invp,
+                [&](int i, T (&key)[TN]) {
                     // few keys pass: one test for the row first (the minimum
                     // of the keys that are not NaN)
                     T m = key[0];

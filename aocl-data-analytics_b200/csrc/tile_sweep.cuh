@@ -266,8 +266,10 @@ B200_DEV void sweep_put(SweepStage<T> &st, const SweepRegs<T, SW_BM> &ra,
 // b_end) of B, tile by tile: epi(b0) runs with the accumulators of the tile at
 // b0 complete.  One pipeline over all (tile, slab) steps: the next step's
 // global loads are in flight while the current slab is consumed, across tile
-// borders too.  Rows are ld elements (padded to four, pad readable).  No barrier
-// separates the last epi from what follows.
+// borders too.  Rows are ld elements (padded to four, pad readable).  A warp whose
+// eight rows of A do not exist only loads: with few rows (300,000 x 64 against 2
+// rows) the others' shared-memory reads and arithmetic are what a tile costs.  No
+// barrier separates the last epi from what follows.
 template <typename T, int ACC, typename R, typename F>
 B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T *B, R brows,
                           int b_begin, int b_end, int ld, int d, int kc, T p,
@@ -277,6 +279,7 @@ B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T
     const int nslab = (d + SW_BK - 1) / SW_BK;
     SweepRegs<T, SW_BM> ra;
     SweepRegs<T, BN> rb;
+    const bool some = a0 + (tid >> 5) * 8 < na; // of the warp's rows of A
     if (b_begin >= b_end) return;
     ra.load(A, ld, AllRows{}, a0, na, 0, tid);
     rb.load(B, ld, brows, b_begin, b_end, 0, tid);
@@ -293,7 +296,7 @@ B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T
                 ra.load(A, ld, AllRows{}, a0, na, ns * SW_BK, tid);
                 rb.load(B, ld, brows, nb0, b_end, ns * SW_BK, tid);
             }
-            sweep_slab<T, ACC>(st[cur], s * SW_BK, d, kc, p, acc, tm, tn);
+            if (some) sweep_slab<T, ACC>(st[cur], s * SW_BK, d, kc, p, acc, tm, tn);
             if (more) sweep_put(st[cur ^ 1], ra, rb, tid);
             if (last) epi(b0);
             __syncthreads();
@@ -304,10 +307,11 @@ B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T
 
 // The post-operation over a whole micro-tile (the cases of post_value that the
 // accumulation can have: fewer copies of the code), rows in turn to out(i, v).
-// xv: A rows' norms, yn: B rows' norms.
+// xv: A rows' norms, yn: B rows' norms.  rows: how many of the thread's four exist;
+// the operation (a division, a power) is left out for the others.
 template <typename T, int ACC, typename R, typename F>
-B200_DEV void sweep_post(const SweepAcc<T, ACC> &acc, int post, const T (&xv)[4], const T *yn,
-                         R brows, int b0, int nb, int tn, T invp, F &&out) {
+B200_DEV void sweep_post(const SweepAcc<T, ACC> &acc, int post, const T (&xv)[4], int rows,
+                         const T *yn, R brows, int b0, int nb, int tn, T invp, F &&out) {
     constexpr int TN = SweepAcc<T, ACC>::TN;
     T yv[TN];
     if (ACC == ACC_DOT && post != POST_NONE && post != POST_NEG) {
@@ -323,6 +327,7 @@ B200_DEV void sweep_post(const SweepAcc<T, ACC> &acc, int post, const T (&xv)[4]
 #pragma unroll
         for (int j = 0; j < TN; ++j) v[j] = acc.value(i, j);
         auto each = [&](int as) {
+            if (i >= rows) return;
 #pragma unroll
             for (int j = 0; j < TN; ++j) v[j] = post_value<T>(as, v[j], xv[i], yv[j], invp);
         };
