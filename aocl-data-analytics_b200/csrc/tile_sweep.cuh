@@ -308,7 +308,7 @@ B200_DEV void sweep_tiles(SweepStage<T> *st, const T *A, int na, int a0, const T
 // The post-operation over a whole micro-tile (the cases of post_value that the
 // accumulation can have: fewer copies of the code), rows in turn to out(i, v).
 // xv: A rows' norms, yn: B rows' norms.  rows: how many of the thread's four exist;
-// the operation (a division, a power) is left out for the others.
+// a division or a power is left out for the others.
 template <typename T, int ACC, typename R, typename F>
 B200_DEV void sweep_post(const SweepAcc<T, ACC> &acc, int post, const T (&xv)[4], int rows,
                          const T *yn, R brows, int b0, int nb, int tn, T invp, F &&out) {
@@ -327,7 +327,7 @@ B200_DEV void sweep_post(const SweepAcc<T, ACC> &acc, int post, const T (&xv)[4]
 #pragma unroll
         for (int j = 0; j < TN; ++j) v[j] = acc.value(i, j);
         auto each = [&](int as) {
-            if (i >= rows) return;
+            if ((as == POST_COSINE || as == POST_POW) && i >= rows) return;
 #pragma unroll
             for (int j = 0; j < TN; ++j) v[j] = post_value<T>(as, v[j], xv[i], yv[j], invp);
         };
